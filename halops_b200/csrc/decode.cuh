@@ -11,8 +11,16 @@
 //   * Operands are swapped: 128 weight rows are the M of tcgen05.mma, the activations its
 //     N (16 / 32 / 64 / 128 columns).  One instruction then consumes 4 KB of weights instead
 //     of the 2 KB of a 128 x 64 tile with the activations as M.
-//   * A stage holds 256 bytes of K per row (two 128-byte-swizzled boxes per operand): half
-//     as many barrier round trips and commits per byte of weight.
+//   * A stage holds 256 bytes of K per row (two 128-byte-swizzled k-tiles per operand, brought by
+//     one three-dimensional box each): half as many barrier round trips and commits per byte of weight.
+//   * What paces a k-step is whichever thread has the most to issue, since every asynchronous
+//     instruction holds its thread for about 100 cycles or more.  Measured from SM-clock stamps with the
+//     weight in L2: with one loader thread (six copies) and one thread for the scales (four
+//     tcgen05.cp and a commit) a 32 KB step took 870 cycles, with two loader threads of two
+//     copies each 830, and with the scales moved by four warps (ld.shared, one tcgen05.st) 490,
+//     near what L2 delivers to one SM.  8 x 7168 x 2048 behind its quantizer: 10.0 -> 9.0 us.
+//   * Before it waits for the preceding kernel of the stream a CTA asks for the start of its weight
+//     to be brought into L2 (see DecParams::prefetch_steps): 9.0 -> 8.4 us.
 //   * Two threads issue the MMAs of alternate k-steps into accumulators of their own, so
 //     they need no hand-over; the epilogue adds the two accumulators.  One thread alone
 //     needs about 1000 cycles per 32 KB step (33 bytes per cycle and CTA), less than an SM's
@@ -29,10 +37,10 @@
 //     stores a [16 rows x 32 columns] box of the output with one TMA store, which also clips
 //     rows past M and columns past N.
 //
-// Warps: 0 loader, 1 and 7 MMA issuers (warp 1 allocates tensor memory), 2-5 epilogue,
-// 6 scale copies (tcgen05.cp, a few k-steps ahead of the MMAs).
+// Warps: 0 weight loader, 1 and 10 MMA issuers (warp 1 allocates tensor memory), 2-5 epilogue,
+// 6-9 scales to tensor memory (a few k-steps ahead of the MMAs), 11 activation loader.
 
-constexpr int kDecThreads = 256;
+constexpr int kDecThreads = 384;
 constexpr int kDecRows = 128;      // weight rows per tile (the M of the MMA)
 constexpr int kDecStepBytes = 256; // bytes of K per stage row
 constexpr int kDecIssuers = 2;     // threads issuing MMAs, each into its own accumulator
@@ -138,6 +146,7 @@ struct DecParams {
     int x_rows;           // rows of the activation box (m rounded up to 8)
     int epi_op;
     int early_weights;    // the weight and its scales are read before the preceding kernel is known to be complete
+    int prefetch_steps;   // k-steps of its weight a CTA asks to have in L2 before it waits for the preceding kernel
     DecPlan plan;
 };
 
@@ -238,14 +247,14 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&bars->full[s]), 1);
+            ptx::mbar_init(ptx::smem_u32(&bars->full[s]), 2);  // the weight's and the activation's loader
             ptx::mbar_init(ptx::smem_u32(&bars->empty[s]), 1);
         }
         for (int s = 0; s < C::kAccStages; ++s) {
             ptx::mbar_init(ptx::smem_u32(&bars->acc_full[s]), kDecIssuers);
             ptx::mbar_init(ptx::smem_u32(&bars->acc_empty[s]), kEpiWarps);
         }
-        for (int s = 0; s < C::kSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), 1);
+        for (int s = 0; s < C::kSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), kSfWarps);
         ptx::mbar_init(ptx::smem_u32(&bars->epi_sync), kEpiWarps);
         if (p.plan.cluster > 1) {
             ptx::mbar_init(ptx::smem_u32(&bars->turn[0]), 1);  // "the first CTA's ring is free"
@@ -265,80 +274,74 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     ptx::tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
 
+    // While the preceding kernel of the stream finishes, HBM would idle: bring the start of this
+    // CTA's weight into L2.  Only a hint, so it needs no promise about who writes the weight: L2 is
+    // where a write that is still to come goes, and the loads after the wait read it from there.
+    // (From an epilogue warp, idle until the first tile is done.)
+    if (threadIdx.x == 64 && p.prefetch_steps > 0) {
+        DecWalk ahead(p.plan, cta);
+        DecSeg as;
+        int left = p.prefetch_steps;
+        while (left > 0 && ahead.next(as)) {
+            const uint8_t* const sf_row = p.sfw + int64_t(as.tile) * p.kq_dim * 512;
+            for (int ks = as.k0; ks < as.k1 && left > 0; ++ks, --left) {
+                ptx::tma_prefetch_3d(&tm_w, 0, as.tile * kDecRows, 2 * ks);
+                ptx::bulk_prefetch(sf_row + int64_t(ks) * 1024, uint32_t(min(2, k_tiles - 2 * ks)) * 512);
+            }
+        }
+    }
+    __syncwarp();
+
     // Nothing below may read what the previous kernel wrote before this returns.  With
-    // early_weights only the loader waits, after it has asked for the weight of its first ring
+    // early_weights only the loaders wait, the weight's one after it has asked for its first ring
     // of stages: the caller vouches that the weight and its scales are not written by the
     // preceding kernel.  The other roles touch global memory only behind barriers that the
-    // loader's later copies (the activation) complete, so they run after its wait as well.
+    // activation's loads complete, so they run after that wait as well.
     if (p.early_weights == 0) ptx::pdl_wait();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ loader
+        // ------------------------------------------------------------ weight loader
+        // One box of 128 rows x 256 bytes and one flat copy of scales per k-step.
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            const auto arm = [&](uint32_t s, int boxes) {
-                ptx::mbar_arrive_expect_tx(ptx::smem_u32(&bars->full[s]),
-                                           uint32_t(boxes) * (kDecRows * kBKBytes + p.x_rows * kBKBytes + 1024));
-            };
-            const auto load_weight = [&](uint32_t s, int boxes, int ks, int tile) {
-                const uint32_t full = ptx::smem_u32(&bars->full[s]);
-                for (int b = 0; b < boxes; ++b) {
-                    ptx::tma_load_2d(w_base + s * C::kWBytes + b * (kDecRows * kBKBytes), &tm_w,
-                                     ks * kDecStepBytes + b * kBKBytes, tile * kDecRows, full);
-                }
-            };
-            const auto load_weight_scales = [&](uint32_t s, int boxes, int ks, int tile) {
-                ptx::bulk_load(sfw_base + s * C::kSfBytes, p.sfw + int64_t(tile) * p.kq_dim * 512 + int64_t(ks) * 1024,
-                               uint32_t(boxes) * 512, ptx::smem_u32(&bars->full[s]));
-            };
-            if (p.early_weights != 0) {
-                // the first ring of stages: every stage is free, its barrier is armed for all
-                // the bytes of the step, and the weight's share is asked for now
-                DecWalk ahead(p.plan, cta);
-                DecSeg as;
-                uint32_t pre = 0;
-                while (pre < uint32_t(C::kStages) && ahead.next(as)) {
-                    for (int ks = as.k0; ks < as.k1 && pre < uint32_t(C::kStages); ++ks, ++pre) {
-                        const int boxes = min(2, k_tiles - 2 * ks);
-                        arm(pre, boxes);
-                        load_weight(pre, boxes, ks, as.tile);
-                        load_weight_scales(pre, boxes, ks, as.tile);
-                    }
-                }
-                // (letting the next kernel of the stream start here already, before this one's wait,
-                // measured slower: 7.5 against 7.0 us per GEMM in a chain of 8 x 7168 x 2048)
-                ptx::pdl_wait();
-            }
+            bool waited = p.early_weights == 0;
             DecWalk walk(p.plan, cta);
             DecSeg sg;
             while (ok && walk.next(sg)) {
+                const uint8_t* const sf_row = p.sfw + int64_t(sg.tile) * p.kq_dim * 512;
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
                     const uint32_t s = it % C::kStages;
-                    const int boxes = min(2, k_tiles - 2 * ks);  // 128-byte k-tiles in this step
-                    const bool asked = p.early_weights != 0 && it < uint32_t(C::kStages);
-                    if (!asked) {
+                    if (it >= uint32_t(C::kStages)) {
+                        if (!waited) {
+                            ptx::pdl_wait();
+                            waited = true;
+                        }
                         ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                       kStatusProducer);
                         if (!ok) break;
-                        arm(s, boxes);
-                        // the weight first: it is what the step waits for
-                        load_weight(s, boxes, ks, sg.tile);
                     }
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
-                    for (int b = 0; b < boxes; ++b) {
-                        ptx::tma_load_2d(x_base + s * C::kXBytes + b * (NACT * kBKBytes), &tm_x,
-                                         ks * kDecStepBytes + b * kBKBytes, 0, full);
-                    }
-                    if (!asked) load_weight_scales(s, boxes, ks, sg.tile);
-                    ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, uint32_t(boxes) * 512, full);
+                    const uint32_t sf_bytes = uint32_t(min(2, k_tiles - 2 * ks)) * 512;
+                    // (an odd last k-tile: the box's second half lies past K and arrives as zeros,
+                    // counted like the rest; no MMA reads it)
+                    ptx::mbar_arrive_expect_tx(full, C::kWBytes + sf_bytes);
+                    ptx::tma_load_3d(w_base + s * C::kWBytes, &tm_w, 0, sg.tile * kDecRows, 2 * ks, full);
+                    ptx::bulk_load(sfw_base + s * C::kSfBytes, sf_row + int64_t(ks) * 1024, sf_bytes, full);
                 }
             }
+            if (!waited) ptx::pdl_wait();
+            // (triggering before this kernel's own wait was measured again with the prefetch above, which
+            // then overlaps the preceding GEMM: 64 x 24576 x 1536 15.3 against 14.2 us, 33 x 23552 x 7808
+            // 45.8 against 43.6, 8 x 7168 x 2048 8.5 against 8.4)
             ptx::pdl_launch_dependents();
         }
-    } else if (warp == 6) {
-        // ------------------------------------------------------------ scale copies: shared -> tensor memory
+    } else if (warp == 11) {
+        // ------------------------------------------------------------ activation loader
+        // A thread of its own: every copy holds the thread that issues it for 100 to 125 cycles,
+        // and six of them per k-step were what paced the whole kernel.
         if (lane == 0) {
+            if (p.early_weights != 0) ptx::pdl_wait();
             uint32_t it = 0;
             bool ok = true;
             DecWalk walk(p.plan, cta);
@@ -346,26 +349,54 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             while (ok && walk.next(sg)) {
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
-                    if (ok && it >= uint32_t(C::kSfSets)) {
-                        // the MMAs of step it - kSfSets read this set: done once they released their stage
-                        const uint32_t prev = it - uint32_t(C::kSfSets);
-                        ok = wait_bar(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
-                                      kStatusProducer);
-                    }
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint32_t set = tmem + C::kSfCol0 + (it % C::kSfSets) * 16;
-                    const int boxes = min(2, k_tiles - 2 * ks);
-                    for (int b = 0; b < boxes; ++b) {
-                        ptx::tc_copy_sf<1>(set + b * 4, ptx::smem_desc(sfw_base + s * C::kSfBytes + b * 512, 0, 128, 0));
-                        ptx::tc_copy_sf<1>(set + 8 + b * 4, ptx::smem_desc(sfx_base + s * C::kSfBytes + b * 512, 0, 128, 0));
-                    }
-                    ptx::tc_commit(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]));
+                    const uint32_t full = ptx::smem_u32(&bars->full[s]);
+                    const uint32_t sf_bytes = uint32_t(min(2, k_tiles - 2 * ks)) * 512;
+                    ptx::mbar_arrive_expect_tx(full, uint32_t(2 * p.x_rows * kBKBytes) + sf_bytes);
+                    ptx::tma_load_3d(x_base + s * C::kXBytes, &tm_x, 0, 0, 2 * ks, full);
+                    ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, sf_bytes, full);
                 }
             }
         }
-    } else if (warp == 1 || warp == 7) {
+    } else if (warp >= 6 && warp < 6 + kSfWarps) {
+        // ------------------------------------------------------------ scales: shared -> tensor memory
+        // Each of the four warps fills its own lane quarter of the step's set: the 512-byte image
+        // of an SfAtom, lane l holding row l in 4 columns, the two atoms of the weight and the two
+        // of the activation in one 16-column store.
+        const uint32_t quarter = (uint32_t(warp) & 3u) * 32u;
+        uint32_t it = 0;
+        bool ok = true;
+        DecWalk walk(p.plan, cta);
+        DecSeg sg;
+        while (ok && walk.next(sg)) {
+            for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
+                const uint32_t s = it % C::kStages;
+                ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
+                if (ok && it >= uint32_t(C::kSfSets)) {
+                    // the MMAs of step it - kSfSets read this set: done once they released their stage
+                    const uint32_t prev = it - uint32_t(C::kSfSets);
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
+                                  kStatusProducer);
+                }
+                if (!ok) break;
+                ptx::tc_fence_after();
+                // (a last step of one k-tile leaves the second atoms stale; no MMA uses them)
+                uint32_t r[16];
+                const uint32_t src_w = sfw_base + s * C::kSfBytes + uint32_t(lane) * 16u;
+                const uint32_t src_x = sfx_base + s * C::kSfBytes + uint32_t(lane) * 16u;
+                ptx::ld_shared_v4(src_w, r[0], r[1], r[2], r[3]);
+                ptx::ld_shared_v4(src_w + 512, r[4], r[5], r[6], r[7]);
+                ptx::ld_shared_v4(src_x, r[8], r[9], r[10], r[11]);
+                ptx::ld_shared_v4(src_x + 512, r[12], r[13], r[14], r[15]);
+                ptx::tc_store_32x32_x16(tmem + (quarter << 16) + C::kSfCol0 + (it % C::kSfSets) * 16, r);
+                ptx::tc_wait_st();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]));
+            }
+        }
+    } else if (warp == 1 || warp == 10) {
         // ------------------------------------------------------------ MMA issuers
         // Issuer `me` takes the k-steps of a piece whose index inside the piece is me modulo
         // kDecIssuers and accumulates them in its own columns; nothing orders the two threads.
@@ -400,7 +431,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     const int boxes = min(2, k_tiles - 2 * ks);
                     for (int b = 0; b < boxes; ++b) {
                         const uint64_t wdesc = ptx::smem_desc(w_base + s * C::kWBytes + b * (kDecRows * kBKBytes), 16, 1024, 2);
-                        const uint64_t xdesc = ptx::smem_desc(x_base + s * C::kXBytes + b * (NACT * kBKBytes), 16, 1024, 2);
+                        const uint64_t xdesc = ptx::smem_desc(x_base + s * C::kXBytes + b * p.x_rows * kBKBytes, 16, 1024, 2);
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             // the weights are the instruction's A (128 rows), the activations its B
@@ -699,6 +730,15 @@ inline DecPlan dec_plan(int n, int64_t k_bytes, int sm_count, bool allow_split, 
         p.fits32 = int64_t(p.tiles) * p.ksteps * p.ctas < (int64_t(1) << 32) ? 1 : 0;
     }
     return p;
+}
+
+// k-steps of its weight that a CTA asks for ahead of its wait: 24 MB over the grid (but always one
+// step), about what HBM brings while an activation's quantizer runs and the wait is released.
+// More evicts and queues in front of the loads (whole runs: 33 x 23552 x 7808 45.0 us, 5 steps
+// 43.6, none 44.7), less leaves HBM idle (8 x 7168 x 2048: 2 or 5 steps 8.45 us, all 8 8.2).
+inline int dec_prefetch_steps(const DecPlan& p, int64_t step_bytes) {
+    const int64_t steps = (int64_t(24) << 20) / (int64_t(p.ctas) * step_bytes);
+    return steps < 1 ? 1 : steps > p.ksteps * int64_t(p.tiles) ? int(p.ksteps * int64_t(p.tiles)) : int(steps);
 }
 
 // Host check of the unit deal, for tests: every unit is worked exactly once, the owner

@@ -1930,6 +1930,22 @@ bool make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, const void* base,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same matrix cut into 128-byte k-tiles: [pitch / 128][rows][128 bytes], so that one copy brings
+// `box_tiles` neighbouring k-tiles of `box_rows` rows, each in the 128-byte-swizzled form of its own
+// (a box may stick out past the last k-tile, which then arrives as zeros).
+bool make_tmap_ktiles(CUtensorMap* map, const void* base, uint64_t rows, uint64_t pitch, uint32_t box_rows,
+                      uint32_t box_tiles) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[3] = {uint64_t(kBKBytes), rows, pitch / kBKBytes};
+    const cuuint64_t strides[2] = {pitch, uint64_t(kBKBytes)};
+    const cuuint32_t box[3] = {uint32_t(kBKBytes), box_rows, box_tiles};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Per-device, once: the opt-in to more than 48 KB of dynamic shared memory for one kernel.
 // A failed attempt is not remembered, so the next call tries (and reports) again.
 struct SmemOptIn {
@@ -2281,10 +2297,8 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     const int x_rows = int((g.m + 7) / 8 * 8);
     CUtensorMap tm_w, tm_x, tm_o;
     const bool maps_ok =
-        make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, g.b, uint64_t(g.k_bytes), uint64_t(g.n),
-                     uint64_t(g.k_bytes), kBKBytes, kDecRows, CU_TENSOR_MAP_SWIZZLE_128B) &&
-        make_tmap_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, g.a, uint64_t(g.k_bytes), uint64_t(g.m),
-                     uint64_t(g.k_bytes), kBKBytes, uint32_t(x_rows), CU_TENSOR_MAP_SWIZZLE_128B) &&
+        make_tmap_ktiles(&tm_w, g.b, uint64_t(g.n), uint64_t(g.k_bytes), kDecRows, 2) &&
+        make_tmap_ktiles(&tm_x, g.a, uint64_t(g.m), uint64_t(g.k_bytes), uint32_t(x_rows), 2) &&
         // the epilogue stores [16 rows x 32 columns] boxes; rows past M and columns past N are clipped
         make_tmap_2d(&tm_o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, g.out, uint64_t(g.n), uint64_t(g.m),
                      uint64_t(g.ldo) * 2, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -2293,6 +2307,8 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     }
     p.sfw = g.sfb;
     p.early_weights = g.pdl && g.early_weights ? 1 : 0;
+    // (without a programmatic launch there is nothing to overlap; with early weights the loads are the prefetch)
+    p.prefetch_steps = g.pdl && !g.early_weights ? dec_prefetch_steps(p.plan, C::kWBytes) : 0;
     p.sfx = g.sfa;
     p.scratch = scratch.partials;
     p.counters = scratch.counters;
@@ -2369,10 +2385,8 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     const int x_rows = int((g.m + 7) / 8 * 8);
     CUtensorMap tm_w, tm_x, tm_o;
     const bool maps_ok =
-        make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, g.b, uint64_t(g.k_bytes), uint64_t(g.n),
-                     uint64_t(g.k_bytes), kBKBytes, kDecRows, CU_TENSOR_MAP_SWIZZLE_128B) &&
-        make_tmap_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, g.a, uint64_t(g.k_bytes), uint64_t(g.m),
-                     uint64_t(g.k_bytes), kBKBytes, uint32_t(x_rows), CU_TENSOR_MAP_SWIZZLE_128B) &&
+        make_tmap_ktiles(&tm_w, g.b, uint64_t(g.n), uint64_t(g.k_bytes), kDecRows, 2) &&
+        make_tmap_ktiles(&tm_x, g.a, uint64_t(g.m), uint64_t(g.k_bytes), uint32_t(x_rows), 2) &&
         make_tmap_2d(&tm_o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, g.out, uint64_t(g.n), uint64_t(g.m),
                      uint64_t(g.ldo) * 2, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (!maps_ok) {
@@ -2380,6 +2394,8 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     }
     p.sfw = g.sfb;
     p.early_weights = g.pdl && g.early_weights ? 1 : 0;
+    // (without a programmatic launch there is nothing to overlap; with early weights the loads are the prefetch)
+    p.prefetch_steps = g.pdl && !g.early_weights ? dec_prefetch_steps(p.plan, C::kWBytes) : 0;
     p.sfx = g.sfa;
     p.scratch = scratch.partials;
     p.counters = scratch.counters;

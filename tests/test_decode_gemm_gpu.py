@@ -241,3 +241,30 @@ def test_chain_with_early_weight_loads(hq, monkeypatch, m, n, k, deal):
         outs[use_pdl] = res
     for i in range(layers):
         assert torch.equal(outs[0][i], outs[1][i]) and torch.equal(outs[0][i], outs[2][i]), f"GEMM {i} of the chain differs"
+
+
+@pytest.mark.parametrize("m,n,k,deal", [(8, 7168, 2048, ""), (64, 24576, 1536, ""), (3, 320, 384, ""), (16, 1024, 8192, "split,nocluster")],
+                         ids=lambda v: str(v))
+def test_weight_written_by_the_preceding_kernel(hq, monkeypatch, m, n, k, deal):
+    """With a programmatic launch (use_pdl=True) the kernel asks for its weight in L2 before it waits for
+    the preceding kernel.  That must stay a hint: a weight that the preceding kernel rewrites is
+    used in its new form, bit for bit what a launch after a synchronise gives."""
+    monkeypatch.setenv("HALOPS_B200_DECODE", deal)
+    xq, sfa = hq.group_wise_quant(_rand(m, k, 5, "student_t").cuda())
+    ws = [_rand(n, k, 30 + i, "weight").cuda() for i in range(2)]
+    expected = []
+    for w in ws:
+        wq, sfb = hq.group_wise_quant(w)
+        torch.cuda.synchronize()
+        expected.append(_run(hq, xq, wq, sfa, sfb))
+    assert not torch.equal(expected[0], expected[1])
+    wq, sfb = hq.group_wise_quant(ws[1])
+    outs = [torch.empty([m, n], dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        hq.group_wise_quant(ws[i & 1], "w8a8-mxfp8", True, True, wq, sfb)
+        hq.dense_gemm(xq, wq, sfa, sfb, out, use_pdl=True)
+    torch.cuda.synchronize()
+    assert hq.device_status() == 0
+    for i, out in enumerate(outs):
+        assert torch.equal(out, expected[i & 1]), f"call {i} used stale weight bytes"
