@@ -38,9 +38,16 @@
 //     rows past M and columns past N.
 //
 // Warps: 0 weight loader, 1 and 10 MMA issuers (warp 1 allocates tensor memory), 2-5 epilogue,
-// 6-9 scales to tensor memory (a few k-steps ahead of the MMAs), 11 activation loader.
+// 6-9 scales to tensor memory (a few k-steps ahead of the MMAs), 11 activation loader,
+// 12 scale builder (plain scales only).
+//
+// The same kernel serves the low-latency entry point (at most 16 rows), whose scales come in the
+// plain row-major [rows, K / 32] layout and which has two fused forms: concat-K (a second input /
+// weight pair accumulated into the same output) and dual output (a second weight multiplied by the same
+// input); see DecPlain.  Replaces the reference's low-latency GEMM
+// (csrc/kernel/gemm/low_latency_mma_gemm.cu:23-76).
 
-constexpr int kDecThreads = 384;
+constexpr int kDecThreads = 384;   // with plain scales one warp more, the scale builder
 constexpr int kDecRows = 128;      // weight rows per tile (the M of the MMA)
 constexpr int kDecStepBytes = 256; // bytes of K per stage row
 constexpr int kDecIssuers = 2;     // threads issuing MMAs, each into its own accumulator
@@ -150,6 +157,26 @@ struct DecParams {
     DecPlan plan;
 };
 
+// Plain scales: where the scale bytes are, and the second weight of the fused forms.  A warp assembles
+// the SfAtoms of a step in the stage with 4-byte cp.async copies, one scale word per row and
+// k-tile, and arrives on the stage's barrier.
+template <bool kPlain>
+struct DecPlain {};
+template <>
+struct DecPlain<true> {
+    CUtensorMap w2;  // concat-K: [n, k2]; dual output: [n2, k1]
+    CUtensorMap x2;  // concat-K: [m, k2]
+    CUtensorMap o2;  // dual output: [m, n2]
+    const uint8_t* sfx;
+    const uint8_t* sfw;
+    const uint8_t* sfx2;
+    const uint8_t* sfw2;
+    int64_t sfx_stride, sfw_stride, sfx2_stride, sfw2_stride;  // bytes between scale rows
+    int n2;       // rows of the second weight (dual output)
+    int tiles1;   // tiles of the first weight; those behind it are the second one's (dual output)
+    int ksteps1;  // k-steps of the first pair; those behind it are the second one's (concat-K)
+};
+
 __device__ __forceinline__ void tc_load_32x16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -189,14 +216,26 @@ __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, 
     return true;
 }
 
-// bf16(y) or bf16(sigmoid(y)) in the reference's formulation (see epilogue_chunk), as 16 bits
+// bf16(y) or bf16(sigmoid(y)), as 16 bits.  dense_gemm's sigmoid is the reference's formulation (see
+// epilogue_chunk), that of the low-latency entry point (plain scales) the sigmoid of the bfloat16 result
+// as a float computation.  (Chosen at compile time: the code is unrolled into every store, and
+// with both forms in it the small-M kernel took 9.0 instead of 8.2 us behind its quantizer,
+// 8 x 7168 x 2048, instructions being fetched anew at every launch.)
+template <bool kPlain>
 __device__ __forceinline__ uint16_t dec_finish(float y, int epi_op) {
-    if (epi_op == HQ_EPILOGUE_SIGMOID) y = fmaf(0.5f, tanh_fast(0.5f * y), 0.5f);
+    if (epi_op == HQ_EPILOGUE_SIGMOID) {
+        if constexpr (kPlain) {
+            y = __fdiv_rn(1.0f, 1.0f + expf(-__bfloat162float(__float2bfloat16_rn(y))));
+        } else {
+            y = fmaf(0.5f, tanh_fast(0.5f * y), 0.5f);
+        }
+    }
     return __bfloat16_as_ushort(__float2bfloat16_rn(y));
 }
 
 // Output rows [row0, row0 + 16) x columns [col0, col0 + 32) from the 16 values every lane
 // holds (lane = column, v[j] = row row0 + j): transposed through `buf`, stored by TMA.
+template <bool kPlain>
 __device__ __forceinline__ void dec_store_box(const CUtensorMap* tm_o, uint32_t buf, int lane, const float (&v)[16],
                                               int epi_op, int col0, int row0) {
     // the TMA store that last read this buffer (two stores ago) must be done with it
@@ -204,7 +243,7 @@ __device__ __forceinline__ void dec_store_box(const CUtensorMap* tm_o, uint32_t 
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        asm volatile("st.shared.b16 [%0], %1;" ::"r"(buf + j * 64 + lane * 2), "h"(dec_finish(v[j], epi_op)) : "memory");
+        asm volatile("st.shared.b16 [%0], %1;" ::"r"(buf + j * 64 + lane * 2), "h"(dec_finish<kPlain>(v[j], epi_op)) : "memory");
     }
     ptx::fence_proxy_async_smem();
     __syncwarp();
@@ -214,10 +253,23 @@ __device__ __forceinline__ void dec_store_box(const CUtensorMap* tm_o, uint32_t 
     }
 }
 
-template <int NACT>
-__global__ void __launch_bounds__(kDecThreads, 1)
+// Plain scales: where the weight of one k-step of a tile comes from.
+struct DecSource {
+    bool second;  // dual output: the second weight
+    bool tail;    // concat-K: the second pair
+    bool other;   // either: the second weight's map and scales
+    int row0;     // first weight row
+    int ks;       // k-step inside that weight
+    __device__ __forceinline__ DecSource(const DecPlain<true>& pl, int tile, int k)
+        : second(tile >= pl.tiles1), tail(k >= pl.ksteps1), other(second || tail),
+          row0((second ? tile - pl.tiles1 : tile) * kDecRows), ks(tail ? k - pl.ksteps1 : k) {}
+};
+
+template <int NACT, bool kPlain = false>
+__global__ void __launch_bounds__(kDecThreads + (kPlain ? 32 : 0), 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
-                   const __grid_constant__ CUtensorMap tm_o, const DecParams p) {
+                   const __grid_constant__ CUtensorMap tm_o, const DecParams p,
+                   const __grid_constant__ DecPlain<kPlain> plain) {
     using C = DecCfg<NACT>;
     // the descriptors come from global memory: ask for them before anything else (each request
     // holds its thread for a few hundred cycles, so the loader's thread asks only for the one it
@@ -247,7 +299,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&bars->full[s]), 2);  // the weight's and the activation's loader
+            // the weight's and the activation's loader, and with plain scales the builder's lanes
+            ptx::mbar_init(ptx::smem_u32(&bars->full[s]), kPlain ? 2 + 32 : 2);
             ptx::mbar_init(ptx::smem_u32(&bars->empty[s]), 1);
         }
         for (int s = 0; s < C::kAccStages; ++s) {
@@ -285,8 +338,13 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         while (left > 0 && ahead.next(as)) {
             const uint8_t* const sf_row = p.sfw + int64_t(as.tile) * p.kq_dim * 512;
             for (int ks = as.k0; ks < as.k1 && left > 0; ++ks, --left) {
-                ptx::tma_prefetch_3d(&tm_w, 0, as.tile * kDecRows, 2 * ks);
-                ptx::bulk_prefetch(sf_row + int64_t(ks) * 1024, uint32_t(min(2, k_tiles - 2 * ks)) * 512);
+                if constexpr (kPlain) {
+                    const DecSource src(plain, as.tile, ks);
+                    ptx::tma_prefetch_3d(src.other ? &plain.w2 : &tm_w, 0, src.row0, 2 * src.ks);
+                } else {
+                    ptx::tma_prefetch_3d(&tm_w, 0, as.tile * kDecRows, 2 * ks);
+                    ptx::bulk_prefetch(sf_row + int64_t(ks) * 1024, uint32_t(min(2, k_tiles - 2 * ks)) * 512);
+                }
             }
         }
     }
@@ -322,12 +380,18 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         if (!ok) break;
                     }
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
-                    const uint32_t sf_bytes = uint32_t(min(2, k_tiles - 2 * ks)) * 512;
+                    const uint32_t sf_bytes = kPlain ? 0u : uint32_t(min(2, k_tiles - 2 * ks)) * 512;
                     // (an odd last k-tile: the box's second half lies past K and arrives as zeros,
                     // counted like the rest; no MMA reads it)
                     ptx::mbar_arrive_expect_tx(full, C::kWBytes + sf_bytes);
-                    ptx::tma_load_3d(w_base + s * C::kWBytes, &tm_w, 0, sg.tile * kDecRows, 2 * ks, full);
-                    ptx::bulk_load(sfw_base + s * C::kSfBytes, sf_row + int64_t(ks) * 1024, sf_bytes, full);
+                    if constexpr (kPlain) {
+                        const DecSource src(plain, sg.tile, ks);
+                        ptx::tma_load_3d(w_base + s * C::kWBytes, src.other ? &plain.w2 : &tm_w, 0, src.row0, 2 * src.ks,
+                                         full);
+                    } else {
+                        ptx::tma_load_3d(w_base + s * C::kWBytes, &tm_w, 0, sg.tile * kDecRows, 2 * ks, full);
+                        ptx::bulk_load(sfw_base + s * C::kSfBytes, sf_row + int64_t(ks) * 1024, sf_bytes, full);
+                    }
                 }
             }
             if (!waited) ptx::pdl_wait();
@@ -352,10 +416,59 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
-                    const uint32_t sf_bytes = uint32_t(min(2, k_tiles - 2 * ks)) * 512;
+                    const uint32_t sf_bytes = kPlain ? 0u : uint32_t(min(2, k_tiles - 2 * ks)) * 512;
                     ptx::mbar_arrive_expect_tx(full, uint32_t(2 * p.x_rows * kBKBytes) + sf_bytes);
-                    ptx::tma_load_3d(x_base + s * C::kXBytes, &tm_x, 0, 0, 2 * ks, full);
-                    ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, sf_bytes, full);
+                    const CUtensorMap* tm = &tm_x;
+                    int kx = ks;
+                    if constexpr (kPlain) {
+                        if (ks >= plain.ksteps1) {
+                            tm = &plain.x2;
+                            kx = ks - plain.ksteps1;
+                        }
+                    }
+                    ptx::tma_load_3d(x_base + s * C::kXBytes, tm, 0, 0, 2 * kx, full);
+                    if constexpr (!kPlain) {
+                        ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, sf_bytes, full);
+                    }
+                }
+            }
+        }
+    } else if (kPlain && warp == 12) {
+        // ------------------------------------------------------------ scale builder (plain scales)
+        // lane r writes the scale words of activation row r and of weight rows r, r + 32, r + 64 and r + 96
+        // where the SfAtom has them: byte (row % 32) * 16 + (row / 32) * 4
+        if constexpr (kPlain) {
+            uint32_t it = 0;
+            bool ok = true;
+            DecWalk walk(p.plan, cta);
+            DecSeg sg;
+            while (ok && walk.next(sg)) {
+                for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
+                    const uint32_t s = it % C::kStages;
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
+                    if (!ok) break;
+                    const DecSource src(plain, sg.tile, ks);
+                    const int64_t koff = int64_t(src.ks) * 8;
+                    const uint8_t* const sw = src.other ? plain.sfw2 : plain.sfw;
+                    const int64_t sw_stride = src.other ? plain.sfw2_stride : plain.sfw_stride;
+                    const int n_rows = src.second ? plain.n2 : p.n;
+                    const uint8_t* const sx = src.tail ? plain.sfx2 : plain.sfx;
+                    const int64_t sx_stride = src.tail ? plain.sfx2_stride : plain.sfx_stride;
+                    const uint32_t dst_w = sfw_base + s * C::kSfBytes + uint32_t(lane) * 16u;
+                    const uint32_t dst_x = sfx_base + s * C::kSfBytes + uint32_t(lane) * 16u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int row = src.row0 + lane + 32 * j;
+                        if (row < n_rows) {
+                            ptx::cp_async_4(dst_w + j * 4, sw + row * sw_stride + koff);
+                            ptx::cp_async_4(dst_w + 512 + j * 4, sw + row * sw_stride + koff + 4);
+                        }
+                    }
+                    if (lane < p.m) {
+                        ptx::cp_async_4(dst_x, sx + lane * sx_stride + koff);
+                        ptx::cp_async_4(dst_x + 512, sx + lane * sx_stride + koff + 4);
+                    }
+                    ptx::cp_async_arrive_noinc(ptx::smem_u32(&bars->full[s]));
                 }
             }
         }
@@ -472,8 +585,16 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             ptx::tc_fence_after();
             const uint32_t acc = tmem + as * kDecIssuers * NACT + (lane_base << 16);
             const bool two = sg.k1 - sg.k0 > 1;  // the second issuer had steps of this piece
-            const int col0 = sg.tile * kDecRows + int(lane_base);  // first output column of this warp
-            if (sg.partial && p.plan.cluster > 1) {
+            int col0 = sg.tile * kDecRows + int(lane_base);  // first output column of this warp
+            const CUtensorMap* tm_out = &tm_o;
+            if constexpr (kPlain) {
+                if (sg.tile >= plain.tiles1) {
+                    col0 -= plain.tiles1 * kDecRows;
+                    tm_out = &plain.o2;
+                }
+            }
+            const bool partial = !kPlain && sg.partial;  // (plain scales are always worked in whole tiles)
+            if (partial && p.plan.cluster > 1) {
                 // ---- the tile's CTAs are one cluster: partial tiles go into the first CTA's shared
                 // memory (its operand ring, idle once its MMAs have completed), which adds them in
                 // rank order, i.e. in K order, and stores the result
@@ -530,7 +651,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                                 v[j] += x;
                             }
                         }
-                        dec_store_box(&tm_o, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, v, p.epi_op, col0, ci * 16);
+                        dec_store_box<kPlain>(tm_out, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, v, p.epi_op, col0, ci * 16);
                         ++stores;
                     }
                     ptx::tc_fence_before();
@@ -539,7 +660,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 }
                 continue;
             }
-            float* const mine = !sg.partial ? nullptr
+            float* const mine = !partial ? nullptr
                                 : p.scratch + int64_t(dec_slot(p.plan, cta, sg.tile)) * (NACT * kDecRows) + row;
 #pragma unroll 1
             for (int ci = 0; ci < m_chunks; ++ci) {
@@ -555,8 +676,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = two ? __uint_as_float(r0[j]) + __uint_as_float(r1[j]) : __uint_as_float(r0[j]);
-                if (!sg.partial) {
-                    dec_store_box(&tm_o, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, v, p.epi_op, col0, ci * 16);
+                if (!partial) {
+                    dec_store_box<kPlain>(tm_out, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, v, p.epi_op, col0, ci * 16);
                     ++stores;
                 } else {
                     // this CTA holds only part of the tile's K: float32 partial tile to the scratch buffer
@@ -564,7 +685,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     for (int j = 0; j < 16; ++j) __stcg(mine + (ci * 16 + j) * kDecRows, v[j]);
                 }
             }
-            if (!sg.partial) continue;
+            if (!partial) continue;
             // every thread's stores are visible device-wide before the CTA counts itself
             __threadfence();
             if (!(ok = epi_rendezvous(bars, sync_phase, lane, abort))) break;
@@ -606,7 +727,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         }
                     }
                 }
-                dec_store_box(&tm_o, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, sum, p.epi_op, col0, ci * 16);
+                dec_store_box<kPlain>(tm_out, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, sum, p.epi_op, col0, ci * 16);
                 ++stores;
             }
         }

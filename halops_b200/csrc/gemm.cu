@@ -972,295 +972,6 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(uint64_t limit_ns)
     __syncthreads();
 }
 
-// ---------------------------------------------------------------------------- M <= 16, plain scales
-//
-// Decode-sized GEMM whose block scales come in the plain row-major [rows, K / 32] layout
-// (what the quantizer writes without the SfAtom swizzle), with the two fused forms of the
-// reference's low-latency GEMM (csrc/kernel/gemm/low_latency_mma_gemm.cu:23-76): concat-K
-// (a second input / weight pair accumulated into the same output) and dual output (a
-// second weight multiplied by the same input).  128 x 64 tiles of the tcgen05 path; the
-// 512-byte scale atoms the MMA wants are assembled in shared memory by a warp of 4-byte
-// cp.async copies, one scale word per row and k-tile, that arrive on the stage's barrier.
-
-struct LlParams {
-    const uint8_t* sfa;   // [m, k1 / 32]
-    const uint8_t* sfb;   // [n, k1 / 32]
-    const uint8_t* sfa2;  // concat-K: [m, k2 / 32]
-    const uint8_t* sfb2;  // concat-K: [n, k2 / 32]; dual output: [n2, k1 / 32]
-    int64_t sfa_stride, sfb_stride, sfa2_stride, sfb2_stride;  // bytes between scale rows
-    __nv_bfloat16* out;   // [m, n]
-    __nv_bfloat16* out2;  // dual output: [m, n2]
-    int64_t ldo, ldo2;
-    int m, n, n2;            // n2 = 0 unless dual output
-    int k_tiles1, k_tiles2;  // k_tiles2 = 0 unless concat-K
-    int a_rows;              // rows of the A box (m rounded up to 8)
-    int sigmoid;             // write sigmoid(bf16(result)) instead
-};
-
-// Warps: 0 loader, 1 MMA issuer 0, 2-5 epilogue, 6 scale builder, 7 scale copies, 8 MMA issuer 1.
-// A stage holds 16 rows of A (the MMA reads 128 rows; what follows in shared memory only
-// reaches accumulator rows that are never stored), so 16 stages fit; the scale copies and
-// every second k-tile's MMAs have threads of their own.  Each of the two changes alone left
-// the k-tile time where it was (one issuing thread needs about 640 cycles per k-tile; 8
-// stages of loads that take about 5000 cycles to arrive allow one k-tile per 625 cycles).
-constexpr int kLlThreads = 288;
-constexpr int kLlStages = 16;
-constexpr int kLlABytes = 16 * kBKBytes;
-constexpr int kLlStageBytes = kLlABytes + 64 * kBKBytes + 512 + 512;
-constexpr int kLlSmemBytes = kLlStages * kLlStageBytes + 1024 + 1024;
-constexpr int kLlSfSets = 4;
-
-__global__ void __launch_bounds__(kLlThreads, 1)
-ll_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-               const __grid_constant__ CUtensorMap tm_a2, const __grid_constant__ CUtensorMap tm_b2,
-               const LlParams p) {
-    constexpr int BN = 64;
-    using C = Cfg<BN, 0>;
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* const smem = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
-    const uint32_t a_base = smem_base;
-    const uint32_t b_base = a_base + kLlStages * kLlABytes;
-    const uint32_t sfa_base = b_base + kLlStages * C::kBBytes;
-    const uint32_t sfb_base = sfa_base + kLlStages * C::kSfaBytes;
-    const uint32_t bar_off = kLlStages * kLlStageBytes;
-    static_assert(kLlStages * 64 * kBKBytes >= (kBM - 16) * kBKBytes, "A over-read stays inside the B stages");
-    static_assert(kLlStages <= int(sizeof(Barriers::full) / sizeof(uint64_t)), "one barrier pair per stage");
-    static_assert(sizeof(Barriers) <= 1024, "barrier block");
-    static_assert(C::kSfaCol + kLlSfSets * C::kSfCols <= C::kTmemCols, "scale sets fit the allocation");
-    Barriers* const bars = reinterpret_cast<Barriers*>(smem + bar_off);
-    volatile uint32_t* const abort = &bars->abort;
-
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int tiles1 = (p.n + BN - 1) / BN;
-    const int num_tiles = tiles1 + (p.n2 + BN - 1) / BN;
-    const int k_tiles = p.k_tiles1 + p.k_tiles2;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kLlStages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&bars->full[s]), 33);  // the loader + 32 scale-builder lanes
-            ptx::mbar_init(ptx::smem_u32(&bars->empty[s]), 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&bars->acc_full[s]), 2);  // one commit per MMA-issuing thread
-            ptx::mbar_init(ptx::smem_u32(&bars->acc_empty[s]), kEpiWarps);
-            ptx::mbar_init(ptx::smem_u32(&bars->turn[s]), 1);
-        }
-        for (int s = 0; s < kLlSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), 1);
-        bars->abort = 0;
-        ptx::fence_mbar_init();
-        ptx::prefetch_tmap(&tm_a);
-        ptx::prefetch_tmap(&tm_b);
-        ptx::prefetch_tmap(&tm_a2);
-        ptx::prefetch_tmap(&tm_b2);
-    }
-    if (warp == 1) {
-        ptx::tmem_alloc<1>(ptx::smem_u32(&bars->tmem_base), C::kTmemCols);
-        ptx::tmem_relinquish<1>();
-    }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem = bars->tmem_base;
-    ptx::pdl_wait();
-
-    if (warp == 0) {
-        // ------------------------------------------------------------ box loader
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const bool second = tile >= tiles1;  // dual output: a tile of weight2
-                const int n0 = (second ? tile - tiles1 : tile) * BN;
-                for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kLlStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / kLlStages) & 1u) ^ 1u, abort,
-                                  kStatusProducer);
-                    if (!ok) break;
-                    const uint32_t full = ptx::smem_u32(&bars->full[s]);
-                    ptx::mbar_arrive_expect_tx(full, p.a_rows * kBKBytes + C::kBBytes);
-                    const bool tail = kt >= p.k_tiles1;  // concat-K: the second input / weight pair
-                    const int x = (tail ? kt - p.k_tiles1 : kt) * kBKBytes;
-                    ptx::tma_load_2d(a_base + s * kLlABytes, tail ? &tm_a2 : &tm_a, x, 0, full);
-                    ptx::tma_load_2d(b_base + s * C::kBBytes, (tail || second) ? &tm_b2 : &tm_b, x, n0, full);
-                }
-            }
-            ptx::pdl_launch_dependents();
-        }
-    } else if (warp == 6) {
-        // ------------------------------------------------------------ scale builder
-        // lane r writes the scale words of A row r and of B rows r and r + 32 where the
-        // SfAtom has them: byte (row % 32) * 16 + (row / 32) * 4 of the stage's atom
-        uint32_t it = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-            const bool second = tile >= tiles1;
-            const int n0 = (second ? tile - tiles1 : tile) * BN;
-            const int n_rows = second ? p.n2 : p.n;
-            for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                const uint32_t s = it % kLlStages;
-                ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / kLlStages) & 1u) ^ 1u, abort, kStatusProducer);
-                if (!ok) break;
-                const bool tail = kt >= p.k_tiles1;
-                const int64_t koff = int64_t(tail ? kt - p.k_tiles1 : kt) * 4;
-                const uint8_t* const sa = tail ? p.sfa2 : p.sfa;
-                const int64_t sa_stride = tail ? p.sfa2_stride : p.sfa_stride;
-                const uint8_t* const sb = (tail || second) ? p.sfb2 : p.sfb;
-                const int64_t sb_stride = (tail || second) ? p.sfb2_stride : p.sfb_stride;
-                if (lane < p.m) ptx::cp_async_4(sfa_base + s * C::kSfaBytes + lane * 16, sa + lane * sa_stride + koff);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int row = n0 + lane + 32 * h;
-                    if (row < n_rows) {
-                        ptx::cp_async_4(sfb_base + s * C::kSfbBytes + lane * 16 + h * 4, sb + row * sb_stride + koff);
-                    }
-                }
-                ptx::cp_async_arrive_noinc(ptx::smem_u32(&bars->full[s]));
-            }
-        }
-    } else if (warp == 7) {
-        // ------------------------------------------------------------ scale copies
-        // shared memory -> tensor memory, into scale set it % kLlSfSets
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                    const uint32_t s = it % kLlStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / kLlStages) & 1u, abort, kStatusProducer);
-                    if (!ok) break;
-                    if (it >= uint32_t(kLlSfSets)) {
-                        // the MMAs of k-tile it - kLlSfSets read this set: done once they released their stage
-                        const uint32_t prev = it - uint32_t(kLlSfSets);
-                        ok = wait_bar(ptx::smem_u32(&bars->empty[prev % kLlStages]), (prev / kLlStages) & 1u, abort,
-                                      kStatusProducer);
-                        if (!ok) break;
-                    }
-                    // the scale words were written by ordinary asynchronous copies; the
-                    // tensor-memory copy reads them through the async proxy
-                    ptx::fence_proxy_async_smem();
-                    ptx::tc_fence_after();
-                    const uint32_t set = tmem + (it % kLlSfSets) * C::kSfCols;
-                    ptx::tc_copy_sf<1>(set + C::kSfaCol, ptx::smem_desc(sfa_base + s * C::kSfaBytes, 0, 128, 0));
-                    ptx::tc_copy_sf<1>(set + C::kSfbCol, ptx::smem_desc(sfb_base + s * C::kSfbBytes, 0, 128, 0));
-                    ptx::tc_commit(ptx::smem_u32(&bars->sf_ready[it % kLlSfSets]));
-                }
-            }
-        }
-    } else if (warp == 1 || warp == 8) {
-        // ------------------------------------------------------------ MMA issuers
-        // alternate k-tiles; after its MMAs a thread hands the turn to the other one (tcgen05
-        // fences around an mbarrier arrive), so the MMAs reach the tensor core in k order
-        if (lane == 0) {
-            const uint32_t me = warp == 1 ? 0u : 1u;
-            uint32_t it = 0;
-            uint32_t t = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++t) {
-                const uint32_t as = t & 1u;
-                const uint32_t acc = tmem + as * C::kAccStride;
-                for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                    if ((it & 1u) != me) continue;
-                    const uint32_t s = it % kLlStages;
-                    if (kt == 0) {
-                        ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), ((t >> 1) & 1u) ^ 1u, abort, kStatusMma);
-                        if (!ok) break;
-                    }
-                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % kLlSfSets]), (it / kLlSfSets) & 1u, abort,
-                                  kStatusMma) &&
-                         wait_bar(ptx::smem_u32(&bars->full[s]), (it / kLlStages) & 1u, abort, kStatusMma);
-                    if (ok && it > 0u) {
-                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
-                    }
-                    if (!ok) break;
-                    ptx::tc_fence_after();
-                    const uint32_t set = tmem + (it % kLlSfSets) * C::kSfCols;
-                    const uint64_t adesc = ptx::smem_desc(a_base + s * kLlABytes, 16, 1024, 2);
-                    const uint64_t bdesc = ptx::smem_desc(b_base + s * C::kBBytes, 16, 1024, 2);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        ptx::tc_mma_block_scaled<1, 0>(acc, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2),
-                                                       instr_desc<BN, 0>(uint32_t(k)), set + C::kSfaCol,
-                                                       set + C::kSfbCol, (kt > 0 || k > 0) ? 1u : 0u);
-                    }
-                    ptx::tc_fence_before();
-                    ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1u]));
-                    ptx::tc_commit(ptx::smem_u32(&bars->empty[s]));
-                    // a commit tracks the executing thread's operations: each of the two threads
-                    // commits the accumulator after its own last k-tile (K is a multiple of 256,
-                    // so every tile has k-tiles of both)
-                    if (kt >= k_tiles - 2) ptx::tc_commit(ptx::smem_u32(&bars->acc_full[as]));
-                }
-            }
-        }
-    } else if (warp < 6) {
-        // ------------------------------------------------------------ epilogue
-        const uint32_t lane_base = (warp & 3) * 32;
-        uint32_t t = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++t) {
-            const bool second = tile >= tiles1;
-            const int n0 = (second ? tile - tiles1 : tile) * BN;
-            const int n_rows = second ? p.n2 : p.n;
-            __nv_bfloat16* const out = second ? p.out2 : p.out;
-            const int64_t ldo = second ? p.ldo2 : p.ldo;
-            const uint32_t as = t & 1u;
-            ok = wait_bar(ptx::smem_u32(&bars->acc_full[as]), (t >> 1) & 1u, abort, kStatusEpilogue);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            if (lane_base == 0) {  // the only 32 accumulator rows that can hold one of the m <= 16 rows
-                const uint32_t acc = tmem + as * C::kAccStride;
-#pragma unroll 1
-                for (int c = 0; c < BN / kEpiChunk; ++c) {
-                    uint32_t r[32];
-                    ptx::tc_load_32x32(acc + c * kEpiChunk, r);
-                    ptx::tc_wait_ld();
-                    if (lane < p.m) {
-                        const int col = n0 + c * kEpiChunk;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                float lo = __uint_as_float(r[8 * j + 2 * i]);
-                                float hi = __uint_as_float(r[8 * j + 2 * i + 1]);
-                                if (p.sigmoid) {
-                                    // sigmoid of the bfloat16 result, as a float computation
-                                    lo = __bfloat162float(__float2bfloat16_rn(lo));
-                                    hi = __bfloat162float(__float2bfloat16_rn(hi));
-                                    lo = __fdiv_rn(1.0f, 1.0f + expf(-lo));
-                                    hi = __fdiv_rn(1.0f, 1.0f + expf(-hi));
-                                }
-                                const __nv_bfloat162 v = __float22bfloat162_rn(make_float2(lo, hi));
-                                w[i] = *reinterpret_cast<const uint32_t*>(&v);
-                            }
-                            // weight rows come in multiples of 8: whole 16-byte pieces
-                            if (col + 8 * j < n_rows) {
-                                *reinterpret_cast<uint4*>(out + int64_t(lane) * ldo + col + 8 * j) =
-                                    make_uint4(w[0], w[1], w[2], w[3]);
-                            }
-                        }
-                    }
-                }
-            }
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars->acc_empty[as]));
-        }
-    }
-
-    if (*abort != 0u) {
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    }
-    ptx::tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        ptx::tc_fence_after();
-        ptx::tmem_dealloc<1>(tmem, C::kTmemCols);
-    }
-}
-
 // ---------------------------------------------------------------------------- 2-CTA tiles
 //
 // Pair kernel: a cluster of two CTAs computes one 256 x BN tile with
@@ -2319,7 +2030,7 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
     HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes),
-                       g.stream, g.pdl, unsigned(p.plan.cluster > 1 ? p.plan.cluster : 1), tm_w, tm_x, tm_o, p));
+                       g.stream, g.pdl, unsigned(p.plan.cluster > 1 ? p.plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
     return HQ_OK;
 }
 
@@ -2406,7 +2117,7 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
     HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT>, dim3(plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
-                       g.pdl, unsigned(plan.cluster > 1 ? plan.cluster : 1), tm_w, tm_x, tm_o, p));
+                       g.pdl, unsigned(plan.cluster > 1 ? plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
     return HQ_OK;
 }
 
@@ -3098,52 +2809,67 @@ extern "C" int hq_low_latency_gemm(const void* a, const void* b, const void* sfa
                     "4-byte aligned");
     }
 
-    using C = hq::Cfg<64, 0>;
-    const int a_rows = int((m + 7) / 8 * 8);
-    CUtensorMap tm_a, tm_b, tm_a2, tm_b2;
-    const void* const a_tail = concat ? a2 : a;
-    const int64_t k_tail = concat ? k2 : k1;
-    const void* const b_other = second_weight ? b2 : b;
-    const int64_t rows_other = dual ? n2 : n;
+    if (n == 0) {  // dual output with an empty first weight
+        b = b2;
+        sfb = sfb2;
+        sfb_stride = sfb2_stride;
+        out = out2;
+        ldo = ldo2;
+        n = n2;
+        n2 = 0;
+    }
+    // The kernel of dense_gemm's small M, always on whole tiles: the result may not depend on sm_count,
+    // which a split of K over several CTAs would.
+    using C = hq::DecCfg<16>;
+    hq::DecParams p{};
+    hq::DecPlain<true> plain{};
+    p.x_rows = int((m + 7) / 8 * 8);
+    CUtensorMap tm_w, tm_x, tm_o;
+    const bool second_out = dual && n2 > 0;
     const bool maps_ok =
-        hq::make_tmap_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, uint64_t(k1), uint64_t(m), uint64_t(k1),
-                         hq::kBKBytes, uint32_t(a_rows), CU_TENSOR_MAP_SWIZZLE_128B) &&
-        hq::make_tmap_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, b, uint64_t(k1), uint64_t(n > 0 ? n : 8), uint64_t(k1),
-                         hq::kBKBytes, 64, CU_TENSOR_MAP_SWIZZLE_128B) &&
-        hq::make_tmap_2d(&tm_a2, CU_TENSOR_MAP_DATA_TYPE_UINT8, a_tail, uint64_t(k_tail), uint64_t(m), uint64_t(k_tail),
-                         hq::kBKBytes, uint32_t(a_rows), CU_TENSOR_MAP_SWIZZLE_128B) &&
-        hq::make_tmap_2d(&tm_b2, CU_TENSOR_MAP_DATA_TYPE_UINT8, b_other, uint64_t(k_tail), uint64_t(rows_other),
-                         uint64_t(k_tail), hq::kBKBytes, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+        hq::make_tmap_ktiles(&tm_w, b, uint64_t(n), uint64_t(k1), hq::kDecRows, 2) &&
+        hq::make_tmap_ktiles(&tm_x, a, uint64_t(m), uint64_t(k1), uint32_t(p.x_rows), 2) &&
+        // (a form without a second weight or input gets the first one's map, which is then never used)
+        (concat ? hq::make_tmap_ktiles(&plain.w2, b2, uint64_t(n), uint64_t(k2), hq::kDecRows, 2)
+         : second_out ? hq::make_tmap_ktiles(&plain.w2, b2, uint64_t(n2), uint64_t(k1), hq::kDecRows, 2)
+                      : (plain.w2 = tm_w, true)) &&
+        (concat ? hq::make_tmap_ktiles(&plain.x2, a2, uint64_t(m), uint64_t(k2), uint32_t(p.x_rows), 2)
+                : (plain.x2 = tm_x, true)) &&
+        hq::make_tmap_2d(&tm_o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, uint64_t(n), uint64_t(m), uint64_t(ldo) * 2, 32, 16,
+                         CU_TENSOR_MAP_SWIZZLE_NONE) &&
+        (second_out ? hq::make_tmap_2d(&plain.o2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out2, uint64_t(n2), uint64_t(m),
+                                       uint64_t(ldo2) * 2, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE)
+                    : (plain.o2 = tm_o, true));
     if (!maps_ok) {
         return fail(err, errlen, HQ_ERR_INVALID,
                     "TMA descriptor encoding failed: input and weight must be 16-byte aligned, contiguous rows");
     }
-    hq::LlParams p;
-    p.sfa = static_cast<const uint8_t*>(sfa);
-    p.sfb = static_cast<const uint8_t*>(sfb);
-    p.sfa2 = static_cast<const uint8_t*>(concat ? sfa2 : sfa);
-    p.sfb2 = static_cast<const uint8_t*>(second_weight ? sfb2 : sfb);
-    p.sfa_stride = sfa_stride;
-    p.sfb_stride = sfb_stride;
-    p.sfa2_stride = concat ? sfa2_stride : sfa_stride;
-    p.sfb2_stride = second_weight ? sfb2_stride : sfb_stride;
-    p.out = static_cast<__nv_bfloat16*>(out);
-    p.out2 = static_cast<__nv_bfloat16*>(out2);
-    p.ldo = ldo;
-    p.ldo2 = ldo2;
+    plain.sfx = static_cast<const uint8_t*>(sfa);
+    plain.sfw = static_cast<const uint8_t*>(sfb);
+    plain.sfx2 = static_cast<const uint8_t*>(concat ? sfa2 : sfa);
+    plain.sfw2 = static_cast<const uint8_t*>(second_weight ? sfb2 : sfb);
+    plain.sfx_stride = sfa_stride;
+    plain.sfw_stride = sfb_stride;
+    plain.sfx2_stride = concat ? sfa2_stride : sfa_stride;
+    plain.sfw2_stride = second_weight ? sfb2_stride : sfb_stride;
+    plain.n2 = int(n2);
+    plain.tiles1 = int((n + hq::kDecRows - 1) / hq::kDecRows);
+    plain.ksteps1 = int(k1 / hq::kDecStepBytes);
     p.m = int(m);
     p.n = int(n);
-    p.n2 = int(n2);
-    p.k_tiles1 = int(k1 / hq::kBKBytes);
-    p.k_tiles2 = int(k2 / hq::kBKBytes);
-    p.a_rows = a_rows;
-    p.sigmoid = use_sigmoid ? 1 : 0;
+    p.k_bytes = k1 + k2;
+    p.epi_op = use_sigmoid ? HQ_EPILOGUE_SIGMOID : HQ_EPILOGUE_IDENTITY;
+    p.plan.tiles = plain.tiles1 + int((n2 + hq::kDecRows - 1) / hq::kDecRows);
+    p.plan.ksteps = int((k1 + k2) / hq::kDecStepBytes);
+    p.plan.ctas = std::min(sm, p.plan.tiles);
+    p.plan.aligned = 1;
+    p.prefetch_steps = use_pdl != 0 ? hq::dec_prefetch_steps(p.plan, C::kWBytes) : 0;
 
     static hq::SmemOptIn opt_in;
-    HQ_CUDA_TRY(opt_in.ensure(hq::ll_gemm_kernel, hq::kLlSmemBytes));
-    const int tiles = int((n + 63) / 64 + (n2 + 63) / 64);
-    HQ_CUDA_TRY(hq::launch(hq::ll_gemm_kernel, dim3(std::min(sm, tiles)), dim3(hq::kLlThreads), size_t(hq::kLlSmemBytes),
-                           static_cast<cudaStream_t>(stream), use_pdl != 0, 1, tm_a, tm_b, tm_a2, tm_b2, p));
+    HQ_CUDA_TRY(opt_in.ensure(hq::gemm_decode_kernel<16, true>, C::kSmemBytes));
+    HQ_CUDA_TRY(hq::launch(hq::gemm_decode_kernel<16, true>, dim3(p.plan.ctas), dim3(hq::kDecThreads + 32),
+                           size_t(C::kSmemBytes), static_cast<cudaStream_t>(stream), use_pdl != 0, 1, tm_w, tm_x, tm_o, p,
+                           plain));
     return HQ_OK;
 }
 

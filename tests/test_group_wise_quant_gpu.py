@@ -277,3 +277,26 @@ def test_full_size_operand_properties(hq):
     assert (amax > 448 * s / 4).all(), "a scale is more than one step too large"
     err = (deq - x.float()).abs()
     assert (err <= x.float().abs() * 2 ** -4 + scale * 2 ** -10).all()
+
+
+@pytest.mark.parametrize("m,k", [(1, 128), (5, 1152), (200, 2048)], ids=lambda v: str(v))
+def test_input_written_by_the_preceding_kernel(hq, m, k):
+    """With a programmatic launch the quantizer asks for its input in L2 before it waits for the preceding
+    kernel.  A GEMM right before it rewrites that input: the codes are those of the new values."""
+    g = torch.Generator().manual_seed(m + k)
+    weights = [hq.group_wise_quant(torch.randn([k, 256], generator=g).to(torch.bfloat16).cuda()) for _ in range(2)]
+    a, sfa = hq.group_wise_quant(torch.randn([m, 256], generator=g).to(torch.bfloat16).cuda())
+    x = torch.empty([m, k], dtype=torch.bfloat16, device="cuda")
+    expected = []
+    for w, sfb in weights:
+        hq.dense_gemm(a, w, sfa, sfb, x)
+        torch.cuda.synchronize()
+        expected.append([t.clone() for t in hq.group_wise_quant(x)])
+    torch.cuda.synchronize()
+    got = []
+    for i in range(8):
+        hq.dense_gemm(a, weights[i & 1][0], sfa, weights[i & 1][1], x)
+        got.append(hq.group_wise_quant(x))
+    torch.cuda.synchronize()
+    for i, (q, sf) in enumerate(got):
+        assert torch.equal(q.view(torch.uint8), expected[i & 1][0].view(torch.uint8)) and torch.equal(sf, expected[i & 1][1])

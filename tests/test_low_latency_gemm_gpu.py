@@ -172,3 +172,40 @@ def test_golden_fixture(hq, golden_dir):
     wq = torch.from_numpy(d["w"]).cuda().view(torch.float8_e4m3fn)
     sfa, sfb = _pad_scale_rows(torch.from_numpy(d["sfa"]).cuda()), _pad_scale_rows(torch.from_numpy(d["sfb"]).cuda())
     _check(_run(hq, xq, wq, sfa, sfb), torch.from_numpy(d["out"]))
+
+
+@pytest.mark.parametrize("m,n,n2,k1,k2", [(16, 8, 0, 256, 0), (3, 136, 0, 512, 0), (9, 19000, 0, 512, 0), (16, 8, 264, 256, 0),
+                                          (7, 392, 0, 512, 256), (16, 24576, 0, 1536, 512)],
+                         ids=lambda v: str(v))
+def test_tile_edges(hq, m, n, n2, k1, k2):
+    """128-row weight tiles and 256-byte k-steps: less than a tile, a remainder of 8 rows, more tiles than SMs,
+    the second weight's first tile, and a tail pair of one k-step.  Tolerance: the sums are
+    float32, so the results are the reference's up to a bfloat16 rounding (2^-8 of the value)."""
+    g = torch.Generator().manual_seed(m + n + k1)
+
+    def operand(rows, k, scale):
+        q, sf = hq.group_wise_quant((torch.randn([rows, k], generator=g) * scale).to(torch.bfloat16).cuda(), use_swizzle=False)
+        return q, _pad_scale_rows(sf)
+
+    def dense(q, sf):  # e4m3 codes and UE8M0 bytes of 32-element groups, in float64
+        return q.double() * torch.exp2(sf.double() - 127).repeat_interleave(32, dim=1)
+
+    x, sx = operand(m, k1, 1.0)
+    w, sw = operand(n, k1, 0.02)
+    out = torch.full([m, n], 7.0, dtype=torch.bfloat16, device="cuda")
+    kw, refs = {}, []
+    ref = dense(x, sx) @ dense(w, sw).T
+    if n2:
+        w2, sw2 = operand(n2, k1, 0.02)
+        out2 = torch.full([m, n2], 7.0, dtype=torch.bfloat16, device="cuda")
+        kw = dict(weight2=w2, sfb2=sw2, output2=out2)
+        refs.append((out2, dense(x, sx) @ dense(w2, sw2).T))
+    if k2:
+        x2, sx2 = operand(m, k2, 1.0)
+        w2, sw2 = operand(n, k2, 0.02)
+        kw = dict(input2=x2, weight2=w2, sfa2=sx2, sfb2=sw2)
+        ref = ref + dense(x2, sx2) @ dense(w2, sw2).T
+    hq.low_latency_mma_gemm(x, w, sx, sw, out, **kw)
+    assert hq.device_status() == 0
+    for got, want in [(out, ref)] + refs:
+        assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5).all()
