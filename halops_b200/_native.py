@@ -88,6 +88,48 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+class _NoFastPath:
+    """Stands in while the shared library has not been built: every call takes the wrappers' own
+    way, whose argument checks need no library and whose first use of it says that it is missing."""
+
+    @staticmethod
+    def _none(*args):
+        return None
+
+    group_wise_quant = rms_norm_quant = dense_gemm = grouped_gemm = _none
+
+
+# The module of csrc/fast_path.cpp, which makes the ordinary call of an entry point natively; None until
+# load_fast_path has run.  Its functions return None for a call they leave to the wrapper.
+fast_path = None
+_FAST_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "halops_b200_fast_path.so")
+
+
+def load_fast_path():
+    """Loads the module once and hands it the entry points of the loaded library."""
+    global fast_path
+    if not os.path.exists(_LIB_PATH):
+        return _NoFastPath
+    handle = lib()
+    with _lock:
+        if fast_path is None:
+            if not os.path.exists(_FAST_PATH):
+                raise RuntimeError(f"halops_b200: native module not found at {_FAST_PATH}; build it with "
+                                   "`python -m halops_b200.build` (needs a C++ compiler, no GPU).")
+            import importlib.util
+
+            import torch  # noqa: F401  (the module's symbols are torch's)
+
+            spec = importlib.util.spec_from_file_location("halops_b200_fast_path", _FAST_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
+                "hq_group_wise_quant", "hq_rms_norm_quant", "hq_dense_gemm", "hq_dense_gemm_situ_quant",
+                "hq_describe_group_tile", "hq_group_masked_gemm", "hq_group_contiguous_gemm")))
+            fast_path = module
+    return fast_path
+
+
 def call(name: str, *args) -> None:
     """Calls an entry point whose last two parameters are (err, errlen) and
     raises RuntimeError with the library's message on a non-zero return."""

@@ -1,5 +1,6 @@
 """Builds the C-ABI shared library ``halops_b200/lib/libhalops_b200.so`` in-tree
-with nvcc for sm_100a.  No GPU is needed to build."""
+with nvcc for sm_100a, and beside it the CPython module that the Python entry
+points call it through.  No GPU is needed to build."""
 
 from __future__ import annotations
 
@@ -7,11 +8,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libhalops_b200.so")
+FAST_PATH = os.path.join(LIB_DIR, "halops_b200_fast_path.so")
 SOURCES = ("quant.cu", "gemm.cu")
 HEADERS = ("common.cuh", "ptx.cuh", "decode.cuh", os.path.join("..", "..", "include", "halops_b200.h"))
 
@@ -23,35 +26,56 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
 
 
+def _stale(target: str, deps) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
+
+
 def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    built = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
-    return any(os.path.getmtime(d) > built for d in deps)
+    return _stale(LIB_PATH, [os.path.join(CSRC, f) for f in SOURCES + HEADERS])
+
+
+def _run(cmd, verbose: bool) -> None:
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + " ".join(cmd) + "\n" + proc.stdout + proc.stderr)
+    if verbose:
+        sys.stderr.write(proc.stdout + proc.stderr)
+
+
+def _build_fast_path(force: bool, verbose: bool) -> None:
+    source = os.path.join(CSRC, "fast_path.cpp")
+    if not force and not _stale(FAST_PATH, [source]):
+        return
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    _run([
+        os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+        "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+        "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"],
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+        "-o", FAST_PATH, source,
+        "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+    ], verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every CUDA source for sm_100a and link the shared library."""
-    if not force and not is_stale():
-        return LIB_PATH
+    """Compile every CUDA source for sm_100a and link the shared library, then the CPython module."""
     os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [
-        _nvcc(),
-        "-gencode", "arch=compute_100a,code=sm_100a",
-        "-O3", "-std=c++17", "-lineinfo",
-        "-Xcompiler", "-fPIC",
-        "-shared",
-        "-o", LIB_PATH,
-    ]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += [os.path.join(CSRC, f) for f in SOURCES]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + proc.stdout + proc.stderr)
-    if verbose:
-        sys.stderr.write(proc.stdout + proc.stderr)
+    if force or is_stale():
+        cmd = [
+            _nvcc(),
+            "-gencode", "arch=compute_100a,code=sm_100a",
+            "-O3", "-std=c++17", "-lineinfo",
+            "-Xcompiler", "-fPIC",
+            "-shared",
+            "-o", LIB_PATH,
+        ]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        _run(cmd + [os.path.join(CSRC, f) for f in SOURCES], verbose)
+    _build_fast_path(force, verbose)
     return LIB_PATH
 
 

@@ -101,8 +101,11 @@ def dense_gemm(
         output_sf: SfAtom scales of the quantised output ([ceil(M/128)*128, N/64] uint8).
         situ_beta / situ_linear_beta: gate and up soft-caps.
     """
-    # (the messages are only built when a check fails: this function runs once per GEMM of a
-    # decode step, where the host's time per call is what the step costs)
+    if (_native.fast_path or _native.load_fast_path()).dense_gemm(
+            input, weight, sfa, sfb, output, bias, alpha, sm_count, mode, use_pdl, epilogue, output_sf, situ_beta,
+            situ_linear_beta):
+        return
+    # not an ordinary call, or one with an error (the messages are only built when a check fails)
     if mode not in _native.MODE_IDS:
         raise RuntimeError(f"Unsupported mode: {mode}. Expected 'w8a8-mxfp8', 'w4a4-mxfp4' or 'w4a4-nvfp4'.")
     if input.dim() != 2:

@@ -111,6 +111,9 @@ def group_masked_gemm(
         alpha: float32 [num_experts]; required for ``w4a4-nvfp4``, rejected for ``w4a4-mxfp4``.
         max_m_per_expert: rows per expert slot, a positive multiple of 64.
     """
+    if (_native.fast_path or _native.load_fast_path()).grouped_gemm(
+            2, input, weight, sfa, sfb, masked_m, output, bias, alpha, max_m_per_expert, sm_count, mode):
+        return
     _check(
         mode in _MODES,
         f"Unsupported mode: {mode}. Expected 'w8a8-mxfp8', 'w4a4-nvfp4', 'w4a4-mxfp4' or 'w4a8-mxfp4'.",
@@ -174,6 +177,9 @@ def group_contiguous_gemm(
         output: [M, N] bfloat16, written in place.
         bias / alpha: per expert, as for ``group_masked_gemm``.
     """
+    if (_native.fast_path or _native.load_fast_path()).grouped_gemm(
+            3, input, weight, sfa, sfb, expert_ids, output, bias, alpha, 0, sm_count, mode):
+        return
     _check(
         mode in _MODES,
         f"Unsupported mode: {mode}. Expected 'w8a8-mxfp8', 'w4a4-nvfp4', 'w4a4-mxfp4' or 'w4a8-mxfp4'.",

@@ -47,7 +47,11 @@ def group_wise_quant(
         ``(output_quant, output_sf)``: [m, k] float8_e4m3fn or [m, k/2] uint8,
         and [ceil(m/128)*128 or m, k / group] uint8.
     """
-    # (the messages are only built when a check fails: this runs once per activation of a decode step)
+    result = (_native.fast_path or _native.load_fast_path()).group_wise_quant(
+        input, mode, use_swizzle, use_pdl, output_quant, output_sf)
+    if result is not None:
+        return result
+    # not an ordinary call, or one with an error (the messages are only built when a check fails)
     if input.dim() != 2:
         raise RuntimeError("input must be a 2D tensor of shape [m, k]")
     if input.dtype not in _DTYPE_IDS:

@@ -44,6 +44,9 @@ def rms_norm_quant(
         ``(q, sf)``: [M, K] float8_e4m3fn and uint8 UE8M0 scales,
         [ceil(M/128)*128, K/32] (SfAtom order) or [M, K/32] (row-major).
     """
+    result = (_native.fast_path or _native.load_fast_path()).rms_norm_quant(input, weight, eps, use_swizzle, use_pdl)
+    if result is not None:
+        return result
     _check(input.dim() == 2 and input.dtype == torch.bfloat16, "input must be a 2D bfloat16 tensor [M, K]")
     m, k = input.shape
     _check(

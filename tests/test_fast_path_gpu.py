@@ -1,0 +1,97 @@
+"""The native front of the entry points (csrc/fast_path.cpp) takes the ordinary call of every mode and
+gives what the wrapper's own way gives; whatever is not ordinary it leaves to the wrapper, unlaunched."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+MODES = ("w8a8-mxfp8", "w4a4-mxfp4", "w4a4-nvfp4")
+
+
+@pytest.fixture(scope="module")
+def hq():
+    import halops_b200
+
+    return halops_b200
+
+
+@pytest.fixture(scope="module")
+def native(hq):
+    from halops_b200 import _native
+
+    _native.load_fast_path()
+    return _native
+
+
+class Sub(torch.Tensor):
+    pass
+
+
+def _bytes(*tensors):
+    return [t.view(torch.uint8) for t in tensors]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (130, 256, 512), (256, 384, 1024)], ids=lambda v: str(v))
+def test_same_results_both_ways(hq, native, monkeypatch, mode, m, n, k):
+    g = torch.Generator().manual_seed(m + n)
+    a = torch.randn([m, k], generator=g).to(torch.bfloat16).cuda()
+    b = torch.randn([n, k], generator=g).to(torch.float16).cuda()
+    alpha = torch.full([1], 0.5, device="cuda") if mode == "w4a4-nvfp4" else None
+    results = []
+    for front in (native.fast_path, native._NoFastPath):
+        monkeypatch.setattr(native, "fast_path", front)
+        aq, sfa = hq.group_wise_quant(a, mode)
+        bq, sfb = hq.group_wise_quant(b, mode)
+        out = torch.empty([m, n], dtype=torch.bfloat16, device="cuda")
+        hq.dense_gemm(aq, bq, sfa, sfb, out, alpha=alpha, mode=mode)
+        rows = _bytes(*hq.rms_norm_quant(a, a[0].contiguous(), 1e-5, False))
+        results.append(_bytes(aq, sfa, bq, sfb) + [out] + rows)
+    for x, y in zip(*results):
+        assert x.shape == y.shape and torch.equal(x, y)
+
+
+def test_what_it_takes_and_what_it_leaves(hq, native):
+    f = native.fast_path
+    x = torch.randn([64, 256], device="cuda").to(torch.bfloat16)
+    q, sf = f.group_wise_quant(x, "w8a8-mxfp8", True, True, None, None)
+    assert f.group_wise_quant(x, "w8a8-mxfp8", True, True, q, sf)[0] is q
+    w, sfw = hq.group_wise_quant(torch.randn([128, 256], device="cuda").to(torch.bfloat16))
+    out = torch.full([64, 128], 7.0, dtype=torch.bfloat16, device="cuda")
+
+    def dense(x=q, w=w, sf=sf, sfw=sfw, out=out, bias=None, alpha=None, mode="w8a8-mxfp8", pdl=True, epilogue=0):
+        return f.dense_gemm(x, w, sf, sfw, out, bias, alpha, -1, mode, pdl, epilogue, None, 4.0, 25.0)
+
+    untouched = out.clone()
+    left = [dense(x=q.cpu()), dense(x=q.as_subclass(Sub)), dense(sf=sf.flatten()[:-1]), dense(w=w[:, :128]), dense(pdl=None),
+            dense(mode="w4a4-nvfp4"), dense(mode="bf16"), dense(epilogue=1), dense(out=out.float()), dense(alpha=sf),
+            dense(bias=torch.zeros([128], dtype=torch.bfloat16, device="cuda")), dense(out=out.t()),
+            f.group_wise_quant(x, "w8a8-mxfp8", 1, True, None, None), f.group_wise_quant(x.t(), "w8a8-mxfp8", True, True, None, None),
+            f.group_wise_quant(x.float(), "w8a8-mxfp8", True, True, None, None),
+            f.group_wise_quant(x, "w8a8-mxfp8", True, True, sf, None), f.rms_norm_quant(x, x[0, :128], 1e-6, True, True)]
+    assert left == [None] * len(left)
+    with torch.overrides.TorchFunctionMode():
+        assert dense() is None
+    torch.cuda.synchronize()
+    assert torch.equal(out, untouched)
+    assert dense() is True and not torch.equal(out, untouched)
+
+
+def test_grouped(hq, native, monkeypatch):
+    e, rows, n, k = 3, 64, 128, 256
+    x, sfa = hq.group_wise_quant(torch.randn([e * rows, k], device="cuda").to(torch.bfloat16))
+    w, sfb = (torch.stack(t) for t in zip(*(hq.group_wise_quant(torch.randn([n, k], device="cuda").to(torch.bfloat16))
+                                            for _ in range(e))))
+    counts = torch.tensor([5, 0, 64], dtype=torch.int32, device="cuda")
+    ids = torch.arange(e, dtype=torch.int32, device="cuda").repeat_interleave(rows)
+    results = []
+    for front in (native.fast_path, native._NoFastPath):
+        monkeypatch.setattr(native, "fast_path", front)
+        out = torch.zeros([2, e * rows, n], dtype=torch.bfloat16, device="cuda")
+        hq.group_masked_gemm(x, w, sfa, sfb, counts, out[0], max_m_per_expert=rows)
+        hq.group_contiguous_gemm(x, w, sfa, sfb, ids, out[1])
+        results.append(out)
+        with pytest.raises(RuntimeError, match="input M must equal num_experts"):
+            hq.group_masked_gemm(x, w, sfa, sfb, counts, out[0], max_m_per_expert=2 * rows)
+    assert torch.equal(*results)
