@@ -292,7 +292,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     volatile uint32_t* const abort = &bars->abort;
     __shared__ int s_last;  // epilogue: this CTA is the last contributor of the tile at hand
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const int cta = blockIdx.x;
     const int k_tiles = int(p.k_bytes / kBKBytes);  // 128-byte k-tiles; a k-step holds two, the last maybe one
@@ -360,7 +360,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (warp == 0) {
         // ------------------------------------------------------------ weight loader
         // One box of 128 rows x 256 bytes and one flat copy of scales per k-step.
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             bool ok = true;
             bool waited = p.early_weights == 0;
@@ -375,22 +375,28 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                             ptx::pdl_wait();
                             waited = true;
                         }
-                        ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
-                                      kStatusProducer);
+                        ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
+                                           kStatusProducer);
                         if (!ok) break;
                     }
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
                     const uint32_t sf_bytes = kPlain ? 0u : uint32_t(min(2, k_tiles - 2 * ks)) * 512;
                     // (an odd last k-tile: the box's second half lies past K and arrives as zeros,
                     // counted like the rest; no MMA reads it)
-                    ptx::mbar_arrive_expect_tx(full, C::kWBytes + sf_bytes);
+                    if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(full, C::kWBytes + sf_bytes);
                     if constexpr (kPlain) {
                         const DecSource src(plain, sg.tile, ks);
-                        ptx::tma_load_3d(w_base + s * C::kWBytes, src.other ? &plain.w2 : &tm_w, 0, src.row0, 2 * src.ks,
-                                         full);
+                        if (ptx::elect_one()) {
+                            ptx::tma_load_3d(w_base + s * C::kWBytes, src.other ? &plain.w2 : &tm_w, 0, src.row0, 2 * src.ks,
+                                             full);
+                        }
                     } else {
-                        ptx::tma_load_3d(w_base + s * C::kWBytes, &tm_w, 0, sg.tile * kDecRows, 2 * ks, full);
-                        ptx::bulk_load(sfw_base + s * C::kSfBytes, sf_row + int64_t(ks) * 1024, sf_bytes, full);
+                        if (ptx::elect_one()) {
+                            ptx::tma_load_3d(w_base + s * C::kWBytes, &tm_w, 0, sg.tile * kDecRows, 2 * ks, full);
+                        }
+                        if (ptx::elect_one()) {
+                            ptx::bulk_load(sfw_base + s * C::kSfBytes, sf_row + int64_t(ks) * 1024, sf_bytes, full);
+                        }
                     }
                 }
             }
@@ -404,7 +410,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // ------------------------------------------------------------ activation loader
         // A thread of its own: every copy holds the thread that issues it for 100 to 125 cycles,
         // and six of them per k-step were what paced the whole kernel.
-        if (lane == 0) {
+        {
             if (p.early_weights != 0) ptx::pdl_wait();
             uint32_t it = 0;
             bool ok = true;
@@ -413,11 +419,11 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             while (ok && walk.next(sg)) {
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
                     const uint32_t sf_bytes = kPlain ? 0u : uint32_t(min(2, k_tiles - 2 * ks)) * 512;
-                    ptx::mbar_arrive_expect_tx(full, uint32_t(2 * p.x_rows * kBKBytes) + sf_bytes);
+                    if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(full, uint32_t(2 * p.x_rows * kBKBytes) + sf_bytes);
                     const CUtensorMap* tm = &tm_x;
                     int kx = ks;
                     if constexpr (kPlain) {
@@ -426,9 +432,11 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                             kx = ks - plain.ksteps1;
                         }
                     }
-                    ptx::tma_load_3d(x_base + s * C::kXBytes, tm, 0, 0, 2 * kx, full);
+                    if (ptx::elect_one()) ptx::tma_load_3d(x_base + s * C::kXBytes, tm, 0, 0, 2 * kx, full);
                     if constexpr (!kPlain) {
-                        ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, sf_bytes, full);
+                        if (ptx::elect_one()) {
+                            ptx::bulk_load(sfx_base + s * C::kSfBytes, p.sfx + int64_t(ks) * 1024, sf_bytes, full);
+                        }
                     }
                 }
             }
@@ -513,7 +521,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // ------------------------------------------------------------ MMA issuers
         // Issuer `me` takes the k-steps of a piece whose index inside the piece is me modulo
         // kDecIssuers and accumulates them in its own columns; nothing orders the two threads.
-        if (lane == 0) {
+        // (the whole warp walks, one lane issues: see ptx::elect_one)
+        {
             const int me = warp == 1 ? 0 : 1;
             uint32_t it = 0;
             uint32_t t = 0;
@@ -525,7 +534,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 // both issuers wait for the drained stage, also the one that may have nothing to
                 // issue in a one-step piece: its arrival below must not run ahead of the stage's
                 // previous use
-                ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), ((t / C::kAccStages) & 1u) ^ 1u, abort, kStatusMma);
+                ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), ((t / C::kAccStages) & 1u) ^ 1u, abort, kStatusMma);
                 if (!ok) break;
                 ptx::tc_fence_after();
                 const uint32_t acc = tmem + (as * kDecIssuers + me) * NACT;
@@ -535,9 +544,9 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     const uint32_t s = it % C::kStages;
                     // scales in tensor memory (the copy thread waited for the stage before it
                     // copied); the stage's own barrier orders this thread after the TMA writes
-                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
-                                  kStatusMma) &&
-                         wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusMma);
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
+                                       kStatusMma) &&
+                         wait_bar_warp(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusMma);
                     if (!ok) break;
                     ptx::tc_fence_after();
                     const uint32_t set = tmem + C::kSfCol0 + (it % C::kSfSets) * 16;
@@ -548,20 +557,24 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             // the weights are the instruction's A (128 rows), the activations its B
-                            ptx::tc_mma_block_scaled<1, 0>(acc, wdesc + uint64_t(k * 2), xdesc + uint64_t(k * 2),
-                                                           instr_desc<NACT, 0>(uint32_t(k)), set + b * 4,
-                                                           set + 8 + b * 4, (issued || b > 0 || k > 0) ? 1u : 0u);
+                            if (ptx::elect_one()) {
+                                ptx::tc_mma_block_scaled<1, 0>(acc, wdesc + uint64_t(k * 2), xdesc + uint64_t(k * 2),
+                                                               instr_desc<NACT, 0>(uint32_t(k)), set + b * 4,
+                                                               set + 8 + b * 4, (issued || b > 0 || k > 0) ? 1u : 0u);
+                            }
                         }
                     }
                     issued = true;
-                    ptx::tc_commit(ptx::smem_u32(&bars->empty[s]));
+                    if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&bars->empty[s]));
                 }
                 if (!ok) break;
                 // a commit tracks the executing thread's operations: each issuer reports its own
-                if (issued) {
-                    ptx::tc_commit(ptx::smem_u32(&bars->acc_full[as]));
-                } else {
-                    ptx::mbar_arrive(ptx::smem_u32(&bars->acc_full[as]));
+                if (ptx::elect_one()) {
+                    if (issued) {
+                        ptx::tc_commit(ptx::smem_u32(&bars->acc_full[as]));
+                    } else {
+                        ptx::mbar_arrive(ptx::smem_u32(&bars->acc_full[as]));
+                    }
                 }
             }
         }

@@ -7,7 +7,7 @@
 // with hand-written PTX.  Per CTA (one per SM, persistent over output tiles):
 //   warp 0   TMA producer: A and B tiles (128-byte swizzle) by tensor map, the
 //            512-byte scale atoms by flat bulk copies, into a ring of stages
-//   warp 1   one thread issues the block-scaled tcgen05.mma (fp32 accumulators
+//   warp 1   one lane issues the block-scaled tcgen05.mma (fp32 accumulators
 //            in tensor memory, two accumulator stages so the epilogue overlaps
 //            the next tile)
 //   warps 2-5 epilogue: tcgen05.ld -> * alpha -> bf16 -> swizzled staging in
@@ -15,9 +15,13 @@
 //            map extent, so neither A nor the output is ever padded)
 //   warps 6-9 scales: shared memory -> registers -> tensor memory (tcgen05.st),
 //            one warp per lane quarter, a few k-tiles ahead of the MMAs
-//   warp 10  64-wide dense tiles only: a second MMA issuer that takes every other
-//            k-tile into an accumulator of its own (the epilogue adds the two); one
-//            thread needs about 600 cycles to issue and commit a k-tile of 8 KB
+//   warp 10  a second MMA issuer: every other k-tile, in k order into the same accumulator,
+//            or (one row of 64-wide dense tiles) into one of its own that the epilogue adds
+// Warps 0, 1 and 10 (and their counterparts in the 2-CTA and small-M kernels) run their loops on all
+// lanes and issue each asynchronous instruction from one elected lane (ptx::elect_one).
+// Against loops inside `if (lane == 0)`: 512 x 1536 x 4096 behind its quantizer 17.6 -> 13.9 us,
+// 128 x 8192 x 4096 17.0 -> 13.8, NVFP4 4096 x 14336 x 4096 148 -> 138, 8192 x 8192 x 8192 502 -> 483
+// (sustained, at the power cap), 5 x 3136 x 3072 on the small-M kernel 9.2 -> 8.7; same bits.
 // Every mbarrier wait is bounded: a role that waits longer than kTimeoutNs
 // records a code in the device status word, raises the CTA's abort flag and
 // all roles leave through the common teardown that frees tensor memory.
@@ -128,6 +132,14 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     }
     return true;
 }
+
+// The same for a whole warp, with a warp-uniform result (see ptx::elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort, code) ? 1 : 0) != 0;
+}
+
+// The warp's index in its CTA, known to be warp-uniform.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
 
 struct TileCoord {
     int m;
@@ -467,7 +479,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     Barriers* const bars = reinterpret_cast<Barriers*>(smem + bar_off);
     volatile uint32_t* const abort = &bars->abort;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -507,7 +519,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             bool ok = true;
             WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
@@ -520,27 +532,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 for (int kt = k_begin; kt < k_end; ++kt, ++it) {
                     const uint32_t s = it % kRing;
                     const uint32_t ph = (it / kRing) & 1u;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
                     const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
                     // The scales have a barrier of their own: they are few bytes and land early,
                     // so the scale warps are done before the operand tiles arrive.
-                    ptx::mbar_arrive_expect_tx(sf_full, C::kSfaBytes + C::kSfbBytes);
+                    if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(sf_full, C::kSfaBytes + C::kSfbBytes);
                     const int64_t koff = int64_t(kt) * C::kSfaBytes;
-                    ptx::bulk_load(sfa_base + s * C::kSfaBytes, sfa_row + koff, C::kSfaBytes, sf_full);
+                    if (ptx::elect_one()) {
+                        ptx::bulk_load(sfa_base + s * C::kSfaBytes, sfa_row + koff, C::kSfaBytes, sf_full);
+                    }
 #pragma unroll
                     for (int j = 0; j < C::kNAtoms; ++j) {
-                        ptx::bulk_load(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes,
-                                       sfb_row + int64_t(j) * kq_dim * 512 + koff, C::kSfaBytes, sf_full);
+                        if (ptx::elect_one()) {
+                            ptx::bulk_load(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes,
+                                           sfb_row + int64_t(j) * kq_dim * 512 + koff, C::kSfaBytes, sf_full);
+                        }
                     }
                     // a short activation loads only its own rows (the A box is a_rows tall)
                     // packed e2m1 weights spread to one byte per value in shared memory, but the
                     // barrier counts the bytes read from global memory: half of the stage's B bytes
-                    ptx::mbar_arrive_expect_tx(full, C::kABytes + C::kBBytes - (kBM - a_rows) * kBKBytes -
-                                                         (KIND == 3 ? C::kBBytes / 2 : 0));
-                    ptx::tma_load_2d(a_base + s * C::kABytes, &tm_a, kt * kBKBytes, m0, full);
-                    ptx::tma_load_2d(b_base + s * C::kBBytes, &tm_b, kt * kBKBytes, n0, full);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(full, C::kABytes + C::kBBytes - (kBM - a_rows) * kBKBytes -
+                                                             (KIND == 3 ? C::kBBytes / 2 : 0));
+                    }
+                    if (ptx::elect_one()) ptx::tma_load_2d(a_base + s * C::kABytes, &tm_a, kt * kBKBytes, m0, full);
+                    if (ptx::elect_one()) ptx::tma_load_2d(b_base + s * C::kBBytes, &tm_b, kt * kBKBytes, n0, full);
                 }
             }
             // let a dependent kernel start its prologue
@@ -549,7 +567,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     } else if (warp == 1 || warp == 10) {
         // ------------------------------------------------------------ MMA issuer(s)
         const int me = warp == 1 ? 0 : 1;
-        if (lane == 0 && (me == 0 || dual || ordered)) {
+        if (me == 0 || dual || ordered) {
             uint32_t it = 0;
             uint32_t t = 0;
             bool ok = true;
@@ -560,11 +578,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const uint32_t aph = (t >> 1) & 1u;
                 // (with two issuers both wait here, also the one that has no k-tile in a tile of
                 // one: its arrival below must not run ahead of the stage's previous use)
-                ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                 if (!ok) break;
                 if (C::kOverlap != 0 && t > 0) {
                     // the previous tile's epilogue has drained the columns both stages share
-                    ok = wait_bar(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
                                   abort, kStatusMma);
                     if (!ok) break;
                 }
@@ -580,12 +598,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     const uint32_t ph = (it / kRing) & 1u;
                     // the scales of this k-tile are in their set (the scale warps waited for the
                     // scale bytes); the stage's own barrier orders this thread after the TMA writes
-                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
                                   kStatusMma) &&
-                         wait_bar(ptx::smem_u32(&bars->full[s]), ph, abort, kStatusMma);
+                         wait_bar_warp(ptx::smem_u32(&bars->full[s]), ph, abort, kStatusMma);
                     // (in-order pair of issuers) the other thread has issued the MMAs of the previous k-iteration
                     if (ok && ordered && it > 0u) {
-                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
+                        ok = wait_bar_warp(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
                     }
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -606,27 +624,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                             atom = k >> 1;
                             sf_id = (k & 1) * 2;
                         }
-                        ptx::tc_mma_block_scaled<1, KIND>(
-                            acc, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2),
-                            instr_desc<BN, KIND>(sf_id), set + C::kSfaCol + atom * 4,
-                            set + C::kSfbCol + atom * C::kNAtoms * 4 + sfb_shift,
-                            (ordered ? (kt > k_begin || k > 0) : (issued || k > 0)) ? 1u : 0u);
+                        if (ptx::elect_one()) {
+                            ptx::tc_mma_block_scaled<1, KIND>(
+                                acc, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2),
+                                instr_desc<BN, KIND>(sf_id), set + C::kSfaCol + atom * 4,
+                                set + C::kSfbCol + atom * C::kNAtoms * 4 + sfb_shift,
+                                (ordered ? (kt > k_begin || k > 0) : (issued || k > 0)) ? 1u : 0u);
+                        }
                     }
                     issued = true;
                     if (ordered) {
                         // hand the turn over before the (slow) commit
                         ptx::tc_fence_before();
-                        ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1]));
+                        if (ptx::elect_one()) ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1]));
                     }
                     // stage s may be refilled once these MMAs have read it
-                    ptx::tc_commit(ptx::smem_u32(&bars->empty[s]));
+                    if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&bars->empty[s]));
                 }
                 if (!ok) break;
                 // a commit tracks the executing thread's operations: every issuer reports its own
-                if (issued) {
-                    ptx::tc_commit(ptx::smem_u32(&bars->acc_full[as]));
-                } else {
-                    ptx::mbar_arrive(ptx::smem_u32(&bars->acc_full[as]));
+                if (ptx::elect_one()) {
+                    if (issued) {
+                        ptx::tc_commit(ptx::smem_u32(&bars->acc_full[as]));
+                    } else {
+                        ptx::mbar_arrive(ptx::smem_u32(&bars->acc_full[as]));
+                    }
                 }
             }
         }
@@ -1198,7 +1220,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     Barriers* const bars = reinterpret_cast<Barriers*>(smem + bar_off);
     volatile uint32_t* const abort = &bars->abort;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();  // 0 = leader
     const bool leader = rank == 0;
@@ -1242,7 +1264,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
     if (warp == 0) {
         // ------------------------------------------------------------ box loader (both CTAs)
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             bool ok = true;
             Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
@@ -1252,7 +1274,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const int n0 = wk.b_row0 + int(rank) * (BN / 2);
                 for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                     // The MMA threads release a stage with one commit, to the leader's barrier; the
@@ -1260,22 +1282,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     // 300 cycles per k-tile, this relaxed arrival about 200 on a thread with slack
                     // (what it reports, the MMAs' reads of the stage, completed before the commit).
                     if (leader && it >= uint32_t(C::kStages)) {
-                        ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 1));
+                        if (ptx::elect_one()) {
+                            ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 1));
+                        }
                     }
                     const uint32_t full = ptx::mapa_cluster(ptx::smem_u32(&bars->full[s]), 0);
                     // Bytes of all four loader threads of the pair are counted on the leader's
                     // barrier; only this thread registers them (the count may go negative in
                     // between).
-                    if (leader) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&bars->full[s]), 2 * C::kStageTxBytes);
-                    ptx::tma_load_2d_pair(a_base + s * C::kABytes, &tm_a, kt * kBKBytes, m0, full);
-                    ptx::tma_load_2d_pair(b_base + s * C::kBBytes, &tm_b, kt * kBKBytes, n0, full);
+                    if (leader && ptx::elect_one()) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&bars->full[s]), 2 * C::kStageTxBytes);
+                    if (ptx::elect_one()) ptx::tma_load_2d_pair(a_base + s * C::kABytes, &tm_a, kt * kBKBytes, m0, full);
+                    if (ptx::elect_one()) ptx::tma_load_2d_pair(b_base + s * C::kBBytes, &tm_b, kt * kBKBytes, n0, full);
                 }
             }
             ptx::pdl_launch_dependents();
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------ scale loader (both CTAs)
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             bool ok = true;
             Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
@@ -1285,17 +1309,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const int sfb_atom_row = (wk.b_row0 / 128) * kq_dim;
                 for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::mapa_cluster(ptx::smem_u32(&bars->full[s]), 0);
                     // scale atoms are rows of 128 32-bit words
-                    ptx::tma_load_2d_pair(sfa_base + s * C::kSfaBytes, &tm_sfa, 0,
-                                          sfa_atom_row + kt * C::kSfKAtoms, full);
+                    if (ptx::elect_one()) {
+                        ptx::tma_load_2d_pair(sfa_base + s * C::kSfaBytes, &tm_sfa, 0,
+                                              sfa_atom_row + kt * C::kSfKAtoms, full);
+                    }
 #pragma unroll
                     for (int j = 0; j < C::kNAtoms; ++j) {
-                        ptx::tma_load_2d_pair(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes, &tm_sfb, 0,
-                                              sfb_atom_row + j * kq_dim + kt * C::kSfKAtoms, full);
+                        if (ptx::elect_one()) {
+                            ptx::tma_load_2d_pair(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes, &tm_sfb, 0,
+                                                  sfb_atom_row + j * kq_dim + kt * C::kSfKAtoms, full);
+                        }
                     }
                 }
             }
@@ -1303,7 +1331,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     } else if (warp >= 7 && warp < 7 + C::kCpWarps) {
         // ------------------------------------------------------------ scale copies (leader only)
         // shared memory -> tensor memory of both CTAs, into scale set it % kSfSets
-        if (leader && lane == 0) {
+        if (leader) {
             const int cw = warp - 7;
             bool ok = true;
             Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
@@ -1315,13 +1343,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     total_its += uint32_t(k_tiles);
                 }
                 const uint32_t s = it % C::kStages;
-                ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
+                ok = wait_bar_warp(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
                 if (!ok) break;
                 if (it >= uint32_t(C::kSfSets)) {
                     // the MMAs of k-tile it - kSfSets read this set: they are done once they
                     // have released their stage
                     const uint32_t prev = it - uint32_t(C::kSfSets);
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                 }
@@ -1330,25 +1358,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
                 for (int a = 0; a < C::kSfKAtoms; ++a) {
                     if ((a * (1 + C::kNAtoms)) % C::kCpWarps == cw) {
-                        ptx::tc_copy_sf<2>(set + a * 4,
-                                           ptx::smem_desc(sfa_base + s * C::kSfaBytes + a * 512, 0, 128, 0));
+                        if (ptx::elect_one()) {
+                            ptx::tc_copy_sf<2>(set + a * 4,
+                                               ptx::smem_desc(sfa_base + s * C::kSfaBytes + a * 512, 0, 128, 0));
+                        }
                     }
 #pragma unroll
                     for (int j2 = 0; j2 < C::kNAtoms; ++j2) {
                         if ((a * (1 + C::kNAtoms) + 1 + j2) % C::kCpWarps == cw) {
-                            ptx::tc_copy_sf<2>(
-                                set + C::kSfKAtoms * 4 + (a * C::kNAtoms + j2) * 4,
-                                ptx::smem_desc(sfb_base + s * C::kSfbBytes + (j2 * C::kSfKAtoms + a) * 512, 0, 128,
-                                               0));
+                            if (ptx::elect_one()) {
+                                ptx::tc_copy_sf<2>(
+                                    set + C::kSfKAtoms * 4 + (a * C::kNAtoms + j2) * 4,
+                                    ptx::smem_desc(sfb_base + s * C::kSfbBytes + (j2 * C::kSfKAtoms + a) * 512, 0, 128,
+                                                   0));
+                            }
                         }
                     }
                 }
-                ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), 0));
+                if (ptx::elect_one()) {
+                    ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), 0));
+                }
             }
         }
     } else if (warp == 1 || warp == 7 + C::kCpWarps) {
         // ------------------------------------------------------------ MMA issuers (leader only)
-        if (leader && lane == 0) {
+        if (leader) {
             const uint32_t me = warp == 1 ? 0u : 1u;  // this thread issues the k-iterations it & 1 == me
             uint32_t it = 0;
             uint32_t t = 0;
@@ -1366,20 +1400,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                             // barrier expects both threads.  The arrival may not run ahead of the
                             // previous use of this accumulator stage, hence the same wait the
                             // issuing thread makes.
-                            ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                            ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                             if (!ok) break;
                             const uint32_t accf = ptx::smem_u32(&bars->acc_full[as]);
-                            ptx::mbar_arrive(accf);
-                            ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(accf, 1));
+                            if (ptx::elect_one()) {
+                                ptx::mbar_arrive(accf);
+                                ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(accf, 1));
+                            }
                         }
                         continue;
                     }
                     const uint32_t s = it % C::kStages;
                     if (kt == 0) {
                         // first k-tile of a tile: the accumulator stage must have been drained
-                        ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                        ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                         if (ok && C::kOverlap != 0 && t > 0) {
-                            ok = wait_bar(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u, abort,
+                            ok = wait_bar_warp(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u, abort,
                                           kStatusMma);
                         }
                         if (!ok) break;
@@ -1388,11 +1424,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     // stage's barrier before it copied and committed, so the operand boxes of both
                     // CTAs have landed too: no second wait here (each one costs this thread, which
                     // sets the pace, 50-100 cycles).
-                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
+                    ok = wait_bar_warp(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
                                   kStatusMma);
                     // the other thread has issued the MMAs of the previous k-iteration
                     if (ok && it > 0u) {
-                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
+                        ok = wait_bar_warp(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
                     }
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -1412,24 +1448,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                             atom = k >> 1;
                             sf_id = (k & 1) * 2;
                         }
-                        ptx::tc_mma_block_scaled<2, KIND>(
-                            acc, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2),
-                            instr_desc_pair<BN, KIND>(sf_id), set + atom * 4,
-                            set + C::kSfKAtoms * 4 + atom * C::kNAtoms * 4, (kt > 0 || k > 0) ? 1u : 0u);
+                        if (ptx::elect_one()) {
+                            ptx::tc_mma_block_scaled<2, KIND>(
+                                acc, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2),
+                                instr_desc_pair<BN, KIND>(sf_id), set + atom * 4,
+                                set + C::kSfKAtoms * 4 + atom * C::kNAtoms * 4, (kt > 0 || k > 0) ? 1u : 0u);
+                        }
                     }
                     // hand the turn over before the (slow) commits
                     ptx::tc_fence_before();
-                    ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1u]));
+                    if (ptx::elect_one()) ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1u]));
                     // the loaders of both CTAs may refill stage s once these MMAs have read it
                     // (the leader's loader passes the release on to the other CTA)
-                    ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 0));
+                    if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 0));
                     // A commit tracks the operations of the thread that executes it, so each of
                     // the two threads commits the accumulator after its own last k-tile of the
                     // tile; the epilogue starts when both have completed.
                     if (kt >= k_tiles - 2) {
                         const uint32_t accf = ptx::smem_u32(&bars->acc_full[as]);
-                        ptx::tc_commit_pair(ptx::mapa_cluster(accf, 0));
-                        ptx::tc_commit_pair(ptx::mapa_cluster(accf, 1));
+                        if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(accf, 0));
+                        if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(accf, 1));
                     }
                 }
             }

@@ -20,6 +20,23 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// True in one lane of a converged warp, the same one every time.  The roles that issue asynchronous
+// instructions (copies, tcgen05.mma, commits) run on their whole warp, and each instruction is
+// guarded by this: the compiler then knows the loop and its addresses to be warp-uniform and keeps them
+// in uniform registers, which these instructions read.  Inside `if (lane == 0)` every operand
+// is moved there first, about 100 cycles per instruction.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---- mbarrier --------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
