@@ -437,15 +437,22 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], uint32_t
 // two CTAs works one tile, each half of the k-tiles; the second CTA sends its fp32 partial
 // sums through distributed shared memory into a 32 KB buffer of the first (carved out of the
 // last two A stages), which adds them to its accumulator before the usual epilogue.
-template <int BN, int KIND, bool kSplitK = false>
+//
+// kDense: one weight and a plain epilogue (Identity, Sigmoid), known at compile time.  The group walk in
+// every role and the quantising epilogues are then not in the code: a small problem fetches its
+// instructions anew at every launch, and they were most of them (512 x 1536 x 4096 behind its
+// quantizer 13.9 -> 12.8 us, 128 x 256 x 512 5.6 -> 5.1, NVFP4 300 x 4096 x 4096 12.0 -> 11.4; large
+// problems unchanged).  The other forms take the general code.
+template <int BN, int KIND, bool kSplitK = false, bool kDense = kSplitK>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
             const __grid_constant__ CUtensorMap tm_d, const uint8_t* __restrict__ sfa,
             const uint8_t* __restrict__ sfb, const float* __restrict__ alpha,
             const __nv_bfloat16* __restrict__ bias, int epi_op, __nv_bfloat16* __restrict__ out, int64_t ldo,
             int M, int N, int k_tiles, int kq_dim, int tiles_m, int tiles_n, int a_rows, int direct_store,
-            int dual_issue, const GroupParams grp, const SituParams situ) {
+            int dual_issue, const GroupParams grp_arg, const SituParams situ) {
     using C = Cfg<BN, KIND>;
+    const GroupParams grp = kDense ? GroupParams{kGroupDense, 1, 0, nullptr} : grp_arg;
     // Two MMA issuers with an accumulator each (64-wide dense tiles, plain epilogues): the k-tiles
     // of a tile are summed as (even ones) + (odd ones), deterministically, but not in the k order
     // of the other tiles.
@@ -705,7 +712,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
         Work wk;
         const int ar = int(lane_base) + lane;  // accumulator row of this thread
-        if (situ.sf != nullptr) zero_sf_padding(situ, (warp - 2) * 32 + lane);
+        if (!kDense && situ.sf != nullptr) zero_sf_padding(situ, (warp - 2) * 32 + lane);
         for (; ok && work.next(wk); ++t) {
             const int m0 = wk.out_row0;  // output row of accumulator row 0
             const int n0 = wk.out_col0;
@@ -725,7 +732,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t acc = tmem + as * C::kAccStride + (lane_base << 16);
-            if (KIND == 0 && epi_op == HQ_EPILOGUE_SITU_QUANT) {
+            if (!kDense && KIND == 0 && epi_op == HQ_EPILOGUE_SITU_QUANT) {
                 // quantising epilogue: 64 accumulator columns -> one group of 32 e4m3 outputs
                 constexpr int kGroups = C::kChunks / 2;
 #pragma unroll 1
@@ -876,8 +883,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const int row = m0 + ar;
                 const int col = n0 + c * kEpiChunk;
                 if (warp_idle) continue;
-                if (epi_op == HQ_EPILOGUE_QUANT || epi_op == HQ_EPILOGUE_GATE_MUL_QUANT ||
-                    epi_op == HQ_EPILOGUE_SIGMOID_GATE_MUL_QUANT) {
+                if (!kDense && (epi_op == HQ_EPILOGUE_QUANT || epi_op == HQ_EPILOGUE_GATE_MUL_QUANT ||
+                                epi_op == HQ_EPILOGUE_SIGMOID_GATE_MUL_QUANT)) {
                     // The bf16 result (times the gate, as a bf16 product) re-quantised to MXFP8 per
                     // 32 columns: the reference's batch epilogues (csrc/kernel/gemm/epilogue.cuh:990-1051).
                     if (row_ok) {
@@ -1825,6 +1832,16 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
     // Everything else: two issuers in k order (same bits as one issuer; the dense and the
     // grouped kinds alike).  HALOPS_B200_ISSUERS=1 keeps one issuer (read on every call).
     if (dual == 0 && k_tiles >= 2) dual = issuers_in_order();
+    if constexpr (KIND != 3) {  // (the e4m3 x e2m1 kind is a grouped one)
+        if (g.grp.kind == kGroupDense && (g.epi_op == HQ_EPILOGUE_IDENTITY || g.epi_op == HQ_EPILOGUE_SIGMOID)) {
+            static SmemOptIn opt_in_dense;
+            HQ_CUDA_TRY(opt_in_dense.ensure(gemm_kernel<BN, KIND, false, true>, C::kSmemBytes));
+            HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND, false, true>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
+                               g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
+                               g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.grp, g.situ));
+            return HQ_OK;
+        }
+    }
     HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
                        g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
                        g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.grp, g.situ));
