@@ -111,10 +111,12 @@ struct DecSeg {
     int tile, k0, k1;
     bool partial;  // other CTAs hold the rest of this tile's K
 };
-struct DecWalk {
+// kWhole: the deal is known to be one of whole tiles (`aligned`), 32-bit arithmetic throughout.
+template <bool kWhole>
+struct DecWalkT {
     DecPlan p;
     int64_t u, end;
-    __host__ __device__ DecWalk(const DecPlan& plan, int c) : p(plan), u(dec_begin(plan, c)), end(dec_begin(plan, c + 1)) {}
+    __host__ __device__ DecWalkT(const DecPlan& plan, int c) : p(plan), u(dec_begin(plan, c)), end(dec_begin(plan, c + 1)) {}
     __host__ __device__ bool next(DecSeg& s) {
         if (u >= end) return false;
         if (p.aligned) {
@@ -135,6 +137,23 @@ struct DecWalk {
         return true;
     }
 };
+template <>
+struct DecWalkT<true> {
+    int ksteps;
+    uint32_t tile, end;
+    __host__ __device__ DecWalkT(const DecPlan& plan, int c)
+        : ksteps(plan.ksteps), tile(uint32_t(c) * uint32_t(plan.tiles) / uint32_t(plan.ctas)),
+          end(uint32_t(c + 1) * uint32_t(plan.tiles) / uint32_t(plan.ctas)) {}
+    __host__ __device__ bool next(DecSeg& s) {
+        if (tile >= end) return false;
+        s.tile = int(tile++);
+        s.k0 = 0;
+        s.k1 = ksteps;
+        s.partial = false;
+        return true;
+    }
+};
+using DecWalk = DecWalkT<false>;
 // Scratch slot of CTA c's partial sums for `tile`: slot 0 when its run begins inside (or at
 // the start of) the tile, slot 1 when it began earlier and ends in it.  A run touches at most
 // one tile of each kind.
@@ -265,12 +284,20 @@ struct DecSource {
           row0((second ? tile - pl.tiles1 : tile) * kDecRows), ks(tail ? k - pl.ksteps1 : k) {}
 };
 
-template <int NACT, bool kPlain = false>
+// kWhole: every CTA works whole tiles.  The exchange of partial tiles and the 64-bit deal are then not in
+// the code, which a launch of a few microseconds fetches anew, and 55 registers instead of 168 leave
+// room on the SM for the CTAs of the next kernel.  Behind its quantizer, 8 x 7168 x 2048 8.0 -> 6.9 us,
+// 64 x 24576 x 1536 14.0 -> 12.1, 32 x 4096 x 4096 10.7 -> 8.7, 33 x 23552 x 7808 42.7 -> 39.9; plain scales
+// 16 x 8192 x 4096 13.4 -> 11.9.
+template <int NACT, bool kWhole, bool kPlain = false>
 __global__ void __launch_bounds__(kDecThreads + (kPlain ? 32 : 0), 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const __grid_constant__ CUtensorMap tm_o, const DecParams p,
                    const __grid_constant__ DecPlain<kPlain> plain) {
     using C = DecCfg<NACT>;
+    using Walk = DecWalkT<kWhole>;
+    static_assert(kWhole || !kPlain, "plain scales are worked in whole tiles");
+    const bool clustered = !kWhole && p.plan.cluster > 1;
     // the descriptors come from global memory: ask for them before anything else (each request
     // holds its thread for a few hundred cycles, so the loader's thread asks only for the one it
     // needs first)
@@ -309,7 +336,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         }
         for (int s = 0; s < C::kSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), kSfWarps);
         ptx::mbar_init(ptx::smem_u32(&bars->epi_sync), kEpiWarps);
-        if (p.plan.cluster > 1) {
+        if (clustered) {
             ptx::mbar_init(ptx::smem_u32(&bars->turn[0]), 1);  // "the first CTA's ring is free"
             ptx::mbar_init(ptx::smem_u32(&bars->recv_full), uint32_t(p.plan.cluster - 1) * kEpiWarps);
         }
@@ -323,7 +350,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     ptx::tc_fence_before();
     __syncthreads();
     // the other CTAs' barriers exist before anyone signals across the cluster
-    if (p.plan.cluster > 1) ptx::cluster_sync();
+    if (clustered) ptx::cluster_sync();
     ptx::tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
 
@@ -332,7 +359,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // where a write that is still to come goes, and the loads after the wait read it from there.
     // (From an epilogue warp, idle until the first tile is done.)
     if (threadIdx.x == 64 && p.prefetch_steps > 0) {
-        DecWalk ahead(p.plan, cta);
+        Walk ahead(p.plan, cta);
         DecSeg as;
         int left = p.prefetch_steps;
         while (left > 0 && ahead.next(as)) {
@@ -364,7 +391,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             uint32_t it = 0;
             bool ok = true;
             bool waited = p.early_weights == 0;
-            DecWalk walk(p.plan, cta);
+            Walk walk(p.plan, cta);
             DecSeg sg;
             while (ok && walk.next(sg)) {
                 const uint8_t* const sf_row = p.sfw + int64_t(sg.tile) * p.kq_dim * 512;
@@ -401,9 +428,9 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 }
             }
             if (!waited) ptx::pdl_wait();
-            // (triggering before this kernel's own wait was measured again with the prefetch above, which
-            // then overlaps the preceding GEMM: 64 x 24576 x 1536 15.3 against 14.2 us, 33 x 23552 x 7808
-            // 45.8 against 43.6, 8 x 7168 x 2048 8.5 against 8.4)
+            // (triggering before this kernel's own wait lets the prefetch above overlap the preceding GEMM,
+            // and disturbs it: 64 x 24576 x 1536 12.2 against 12.1 us, 33 x 23552 x 7808 41.5 against 39.9,
+            // 16 x 8192 x 4096 with plain scales 12.8 against 11.9)
             ptx::pdl_launch_dependents();
         }
     } else if (warp == 11) {
@@ -414,7 +441,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (p.early_weights != 0) ptx::pdl_wait();
             uint32_t it = 0;
             bool ok = true;
-            DecWalk walk(p.plan, cta);
+            Walk walk(p.plan, cta);
             DecSeg sg;
             while (ok && walk.next(sg)) {
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
@@ -448,7 +475,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         if constexpr (kPlain) {
             uint32_t it = 0;
             bool ok = true;
-            DecWalk walk(p.plan, cta);
+            Walk walk(p.plan, cta);
             DecSeg sg;
             while (ok && walk.next(sg)) {
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
@@ -488,7 +515,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const uint32_t quarter = (uint32_t(warp) & 3u) * 32u;
         uint32_t it = 0;
         bool ok = true;
-        DecWalk walk(p.plan, cta);
+        Walk walk(p.plan, cta);
         DecSeg sg;
         while (ok && walk.next(sg)) {
             for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
@@ -527,7 +554,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             uint32_t it = 0;
             uint32_t t = 0;
             bool ok = true;
-            DecWalk walk(p.plan, cta);
+            Walk walk(p.plan, cta);
             DecSeg sg;
             for (; ok && walk.next(sg); ++t) {
                 const uint32_t as = t % C::kAccStages;
@@ -589,7 +616,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         uint32_t stores = 0;
         uint32_t sync_phase = 0;
         bool ok = true;
-        DecWalk walk(p.plan, cta);
+        Walk walk(p.plan, cta);
         DecSeg sg;
         for (; ok && walk.next(sg); ++t) {
             const uint32_t as = t % C::kAccStages;
@@ -606,8 +633,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     tm_out = &plain.o2;
                 }
             }
-            const bool partial = !kPlain && sg.partial;  // (plain scales are always worked in whole tiles)
-            if (partial && p.plan.cluster > 1) {
+            const bool partial = !kWhole && sg.partial;
+            if (partial && clustered) {
                 // ---- the tile's CTAs are one cluster: partial tiles go into the first CTA's shared
                 // memory (its operand ring, idle once its MMAs have completed), which adds them in
                 // rank order, i.e. in K order, and stores the result
@@ -755,7 +782,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     // no CTA of a cluster leaves while another may still write into its shared memory or
     // arrive on its barriers (every wait above is bounded, so all of them get here)
-    if (p.plan.cluster > 1) ptx::cluster_sync();
+    if (clustered) ptx::cluster_sync();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc<1>(tmem, C::kTmemCols);

@@ -1965,7 +1965,7 @@ bool decode_eligible(int64_t m, int64_t n, int64_t k, int mode, int epi_op, bool
 
 int decode_width(int64_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
 
-// bytes of the operand ring of gemm_decode_kernel<NACT>: where a cluster's partial tiles land
+// bytes of the operand ring of gemm_decode_kernel<NACT, *>: where a cluster's partial tiles land
 int64_t decode_ring_bytes(int nact) {
     switch (nact) {
         case 16:
@@ -1979,7 +1979,7 @@ int64_t decode_ring_bytes(int nact) {
     }
 }
 
-// How many clusters of 2, 4 and 8 CTAs of gemm_decode_kernel<NACT> the current device can hold at
+// How many clusters of 2, 4 and 8 CTAs of gemm_decode_kernel<NACT, *> the current device can hold at
 // once; asked once per device and width.  Without a device (shape queries on a machine without
 // a GPU) the figures of a B200 stand in: 74, 36 and 14.
 template <int NACT>
@@ -1997,9 +1997,9 @@ void decode_cluster_query(DecClusterLimits* out) {
         occ.attrs = at;
         occ.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(gemm_decode_kernel<NACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(gemm_decode_kernel<NACT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  DecCfg<NACT>::kSmemBytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_decode_kernel<NACT>, &occ) != cudaSuccess) {
+            cudaOccupancyMaxActiveClusters(&n, gemm_decode_kernel<NACT, false>, &occ) != cudaSuccess) {
             cudaGetLastError();
             n = sc == 2 ? 74 : sc == 4 ? 36 : 14;
         }
@@ -2050,7 +2050,9 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     using C = DecCfg<NACT>;
     static SmemOptIn opt_in;
     int dev = 0;
-    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT>, C::kSmemBytes, &dev));
+    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, false>, C::kSmemBytes, &dev));
+    static SmemOptIn opt_in_whole;
+    HQ_CUDA_TRY(opt_in_whole.ensure(gemm_decode_kernel<NACT, true>, C::kSmemBytes));
     DecParams p;
     p.plan = decode_plan(g.m, g.n, g.k_bytes, g.sm_count);
     DecScratch scratch;
@@ -2084,7 +2086,12 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     p.kq_dim = g.kq_dim;
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
-    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes),
+    if (p.plan.aligned) {
+        HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, true>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
+                           g.pdl, 1, tm_w, tm_x, tm_o, p, DecPlain<false>{}));
+        return HQ_OK;
+    }
+    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, false>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes),
                        g.stream, g.pdl, unsigned(p.plan.cluster > 1 ? p.plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
     return HQ_OK;
 }
@@ -2137,7 +2144,7 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     using C = DecCfg<NACT>;
     static SmemOptIn opt_in;
     int dev = 0;
-    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT>, C::kSmemBytes, &dev));
+    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, false>, C::kSmemBytes, &dev));
     DecScratch scratch;
     HQ_CUDA_TRY(noalloc_scratch(dev, &scratch));
     DecParams p;
@@ -2171,7 +2178,7 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     p.kq_dim = g.kq_dim;
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
-    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT>, dim3(plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
+    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, false>, dim3(plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
                        g.pdl, unsigned(plan.cluster > 1 ? plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
     return HQ_OK;
 }
@@ -2921,8 +2928,8 @@ extern "C" int hq_low_latency_gemm(const void* a, const void* b, const void* sfa
     p.prefetch_steps = use_pdl != 0 ? hq::dec_prefetch_steps(p.plan, C::kWBytes) : 0;
 
     static hq::SmemOptIn opt_in;
-    HQ_CUDA_TRY(opt_in.ensure(hq::gemm_decode_kernel<16, true>, C::kSmemBytes));
-    HQ_CUDA_TRY(hq::launch(hq::gemm_decode_kernel<16, true>, dim3(p.plan.ctas), dim3(hq::kDecThreads + 32),
+    HQ_CUDA_TRY(opt_in.ensure(hq::gemm_decode_kernel<16, true, true>, C::kSmemBytes));
+    HQ_CUDA_TRY(hq::launch(hq::gemm_decode_kernel<16, true, true>, dim3(p.plan.ctas), dim3(hq::kDecThreads + 32),
                            size_t(C::kSmemBytes), static_cast<cudaStream_t>(stream), use_pdl != 0, 1, tm_w, tm_x, tm_o, p,
                            plain));
     return HQ_OK;
