@@ -111,8 +111,10 @@ struct DecSeg {
     int tile, k0, k1;
     bool partial;  // other CTAs hold the rest of this tile's K
 };
-// kWhole: the deal is known to be one of whole tiles (`aligned`), 32-bit arithmetic throughout.
-template <bool kWhole>
+// A CTA's walk over its units.  The two deals whose pieces are known beforehand (whole tiles; every
+// tile's K dealt to the CTAs of a cluster) walk the same units in 32-bit arithmetic.
+enum { kDealWhole = 0, kDealCluster = 1, kDealScratch = 2 };
+template <int kDeal>
 struct DecWalkT {
     DecPlan p;
     int64_t u, end;
@@ -138,7 +140,7 @@ struct DecWalkT {
     }
 };
 template <>
-struct DecWalkT<true> {
+struct DecWalkT<kDealWhole> {
     int ksteps;
     uint32_t tile, end;
     __host__ __device__ DecWalkT(const DecPlan& plan, int c)
@@ -153,7 +155,30 @@ struct DecWalkT<true> {
         return true;
     }
 };
-using DecWalk = DecWalkT<false>;
+template <>
+struct DecWalkT<kDealCluster> {  // one piece per CTA: dec_begin with ctas = tiles * cluster
+    uint32_t tile;
+    int k0, k1;
+    bool partial;
+    __host__ __device__ DecWalkT(const DecPlan& plan, int c) {
+        const uint32_t parts = uint32_t(plan.cluster);
+        tile = uint32_t(c) / parts;
+        const uint32_t r = uint32_t(c) - tile * parts;
+        k0 = int(r * uint32_t(plan.ksteps) / parts);
+        k1 = int((r + 1) * uint32_t(plan.ksteps) / parts);
+        partial = k0 != 0 || k1 != plan.ksteps;
+    }
+    __host__ __device__ bool next(DecSeg& s) {
+        if (k0 >= k1) return false;
+        s.tile = int(tile);
+        s.k0 = k0;
+        s.k1 = k1;
+        s.partial = partial;
+        k0 = k1;
+        return true;
+    }
+};
+using DecWalk = DecWalkT<kDealScratch>;
 // Scratch slot of CTA c's partial sums for `tile`: slot 0 when its run begins inside (or at
 // the start of) the tile, slot 1 when it began earlier and ends in it.  A run touches at most
 // one tile of each kind.
@@ -284,20 +309,22 @@ struct DecSource {
           row0((second ? tile - pl.tiles1 : tile) * kDecRows), ks(tail ? k - pl.ksteps1 : k) {}
 };
 
-// kWhole: every CTA works whole tiles.  The exchange of partial tiles and the 64-bit deal are then not in
-// the code, which a launch of a few microseconds fetches anew, and 55 registers instead of 168 leave
-// room on the SM for the CTAs of the next kernel.  Behind its quantizer, 8 x 7168 x 2048 8.0 -> 6.9 us,
-// 64 x 24576 x 1536 14.0 -> 12.1, 32 x 4096 x 4096 10.7 -> 8.7, 33 x 23552 x 7808 42.7 -> 39.9; plain scales
-// 16 x 8192 x 4096 13.4 -> 11.9.
-template <int NACT, bool kWhole, bool kPlain = false>
+// kDeal: how the units are dealt out, known at compile time.  With whole tiles the exchange of partial
+// tiles and the 64-bit deal are not in the code, which a launch of a few microseconds fetches anew,
+// and 55 registers instead of 168 leave room on the SM for the CTAs of the next kernel.  Behind its
+// quantizer, 8 x 7168 x 2048 8.0 -> 6.9 us, 64 x 24576 x 1536 14.0 -> 12.1, 32 x 4096 x 4096 10.7 -> 8.7,
+// 33 x 23552 x 7808 42.7 -> 39.9; plain scales
+// 16 x 8192 x 4096 13.4 -> 11.9; a deal to clusters of 8, 8 x 2048 x 7168, 9.7 -> 8.4 (39 registers).
+template <int NACT, int kDeal, bool kPlain = false>
 __global__ void __launch_bounds__(kDecThreads + (kPlain ? 32 : 0), 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const __grid_constant__ CUtensorMap tm_o, const DecParams p,
                    const __grid_constant__ DecPlain<kPlain> plain) {
     using C = DecCfg<NACT>;
-    using Walk = DecWalkT<kWhole>;
+    constexpr bool kWhole = kDeal == kDealWhole;
+    constexpr bool clustered = kDeal == kDealCluster;
+    using Walk = DecWalkT<kDeal>;
     static_assert(kWhole || !kPlain, "plain scales are worked in whole tiles");
-    const bool clustered = !kWhole && p.plan.cluster > 1;
     // the descriptors come from global memory: ask for them before anything else (each request
     // holds its thread for a few hundred cycles, so the loader's thread asks only for the one it
     // needs first)
@@ -634,7 +661,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 }
             }
             const bool partial = !kWhole && sg.partial;
-            if (partial && clustered) {
+            if (clustered && partial) {
                 // ---- the tile's CTAs are one cluster: partial tiles go into the first CTA's shared
                 // memory (its operand ring, idle once its MMAs have completed), which adds them in
                 // rank order, i.e. in K order, and stores the result
@@ -682,6 +709,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         float v[16];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = two ? __uint_as_float(r0[j]) + __uint_as_float(r1[j]) : __uint_as_float(r0[j]);
+#pragma unroll 1
                         for (int r = 1; r < p.plan.cluster; ++r) {
                             const uint32_t src = w_base + uint32_t(r - 1) * kPartBytes + uint32_t(row) * 4 + ci * 16 * (kDecRows * 4);
 #pragma unroll
@@ -700,7 +728,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 }
                 continue;
             }
-            float* const mine = !partial ? nullptr
+            constexpr bool kScratch = kDeal == kDealScratch;
+            float* const mine = !kScratch || !partial ? nullptr
                                 : p.scratch + int64_t(dec_slot(p.plan, cta, sg.tile)) * (NACT * kDecRows) + row;
 #pragma unroll 1
             for (int ci = 0; ci < m_chunks; ++ci) {
@@ -716,7 +745,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = two ? __uint_as_float(r0[j]) + __uint_as_float(r1[j]) : __uint_as_float(r0[j]);
-                if (!partial) {
+                if (!kScratch || !partial) {
                     dec_store_box<kPlain>(tm_out, my_bufs + (stores & 1u) * kDecEpiBufBytes, lane, v, p.epi_op, col0, ci * 16);
                     ++stores;
                 } else {
@@ -725,7 +754,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     for (int j = 0; j < 16; ++j) __stcg(mine + (ci * 16 + j) * kDecRows, v[j]);
                 }
             }
-            if (!partial) continue;
+            if (!kScratch || !partial) continue;
             // every thread's stores are visible device-wide before the CTA counts itself
             __threadfence();
             if (!(ok = epi_rendezvous(bars, sync_phase, lane, abort))) break;
@@ -930,6 +959,18 @@ inline bool dec_plan_selfcheck(const DecPlan& p) {
             covered += sg.k1 - sg.k0;
         }
         if (u != dec_begin(p, c + 1)) return false;
+    }
+    // the specialised walks work the same pieces
+    for (int c = 0; c < p.ctas && (p.aligned || p.cluster > 1); ++c) {
+        DecWalk general(p, c);
+        DecWalkT<kDealWhole> whole(p, c);
+        DecWalkT<kDealCluster> part(p.aligned ? DecPlan{p.tiles, p.ksteps, p.ctas, 0, 0, 1} : p, c);
+        DecSeg a, b;
+        for (bool more = true; more;) {
+            more = general.next(a);
+            if ((p.aligned ? whole.next(b) : part.next(b)) != more) return false;
+            if (more && (a.tile != b.tile || a.k0 != b.k0 || a.k1 != b.k1 || a.partial != b.partial)) return false;
+        }
     }
     return covered == units;
 }

@@ -1997,9 +1997,9 @@ void decode_cluster_query(DecClusterLimits* out) {
         occ.attrs = at;
         occ.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(gemm_decode_kernel<NACT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(gemm_decode_kernel<NACT, kDealCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  DecCfg<NACT>::kSmemBytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_decode_kernel<NACT, false>, &occ) != cudaSuccess) {
+            cudaOccupancyMaxActiveClusters(&n, gemm_decode_kernel<NACT, kDealCluster>, &occ) != cudaSuccess) {
             cudaGetLastError();
             n = sc == 2 ? 74 : sc == 4 ? 36 : 14;
         }
@@ -2045,14 +2045,35 @@ DecPlan decode_plan(int64_t m, int64_t n, int64_t k_bytes, int sm_count) {
                     sw.nocluster ? nullptr : decode_cluster_limits(nact));
 }
 
+// Launches the instantiation of the plan's deal.
+template <int NACT>
+int launch_decode_deal(const DecPlan& plan, const GemmArgs& g, const CUtensorMap& tm_w, const CUtensorMap& tm_x,
+                       const CUtensorMap& tm_o, const DecParams& p, char* err, size_t errlen) {
+    constexpr int kSmem = DecCfg<NACT>::kSmemBytes;
+    const auto run = [&](auto kernel, unsigned cluster) {
+        return launch(kernel, dim3(plan.ctas), dim3(kDecThreads), size_t(kSmem), g.stream, g.pdl, cluster, tm_w, tm_x, tm_o, p,
+                      DecPlain<false>{});
+    };
+    if (plan.aligned) {  // (the caller has opted in)
+        HQ_CUDA_TRY(run(gemm_decode_kernel<NACT, kDealWhole>, 1u));
+    } else if (plan.cluster > 1) {
+        static SmemOptIn opt_in;
+        HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, kDealCluster>, kSmem));
+        HQ_CUDA_TRY(run(gemm_decode_kernel<NACT, kDealCluster>, unsigned(plan.cluster)));
+    } else {
+        static SmemOptIn opt_in;
+        HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, kDealScratch>, kSmem));
+        HQ_CUDA_TRY(run(gemm_decode_kernel<NACT, kDealScratch>, 1u));
+    }
+    return HQ_OK;
+}
+
 template <int NACT>
 int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     using C = DecCfg<NACT>;
     static SmemOptIn opt_in;
     int dev = 0;
-    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, false>, C::kSmemBytes, &dev));
-    static SmemOptIn opt_in_whole;
-    HQ_CUDA_TRY(opt_in_whole.ensure(gemm_decode_kernel<NACT, true>, C::kSmemBytes));
+    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, kDealWhole>, C::kSmemBytes, &dev));
     DecParams p;
     p.plan = decode_plan(g.m, g.n, g.k_bytes, g.sm_count);
     DecScratch scratch;
@@ -2086,14 +2107,7 @@ int launch_decode(const GemmArgs& g, char* err, size_t errlen) {
     p.kq_dim = g.kq_dim;
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
-    if (p.plan.aligned) {
-        HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, true>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
-                           g.pdl, 1, tm_w, tm_x, tm_o, p, DecPlain<false>{}));
-        return HQ_OK;
-    }
-    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, false>, dim3(p.plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes),
-                       g.stream, g.pdl, unsigned(p.plan.cluster > 1 ? p.plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
-    return HQ_OK;
+    return launch_decode_deal<NACT>(p.plan, g, tm_w, tm_x, tm_o, p, err, errlen);
 }
 
 // ---------------------------------------------------------------------------- small M without any allocation
@@ -2144,7 +2158,7 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     using C = DecCfg<NACT>;
     static SmemOptIn opt_in;
     int dev = 0;
-    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, false>, C::kSmemBytes, &dev));
+    HQ_CUDA_TRY(opt_in.ensure(gemm_decode_kernel<NACT, kDealWhole>, C::kSmemBytes, &dev));
     DecScratch scratch;
     HQ_CUDA_TRY(noalloc_scratch(dev, &scratch));
     DecParams p;
@@ -2178,9 +2192,7 @@ int launch_decode_noalloc(const GemmArgs& g, const DecPlan& plan, char* err, siz
     p.kq_dim = g.kq_dim;
     p.x_rows = x_rows;
     p.epi_op = g.epi_op;
-    HQ_CUDA_TRY(launch(gemm_decode_kernel<NACT, false>, dim3(plan.ctas), dim3(kDecThreads), size_t(C::kSmemBytes), g.stream,
-                       g.pdl, unsigned(plan.cluster > 1 ? plan.cluster : 1), tm_w, tm_x, tm_o, p, DecPlain<false>{}));
-    return HQ_OK;
+    return launch_decode_deal<NACT>(plan, g, tm_w, tm_x, tm_o, p, err, errlen);
 }
 
 const char* mode_name(int mode) {
@@ -2928,8 +2940,8 @@ extern "C" int hq_low_latency_gemm(const void* a, const void* b, const void* sfa
     p.prefetch_steps = use_pdl != 0 ? hq::dec_prefetch_steps(p.plan, C::kWBytes) : 0;
 
     static hq::SmemOptIn opt_in;
-    HQ_CUDA_TRY(opt_in.ensure(hq::gemm_decode_kernel<16, true, true>, C::kSmemBytes));
-    HQ_CUDA_TRY(hq::launch(hq::gemm_decode_kernel<16, true, true>, dim3(p.plan.ctas), dim3(hq::kDecThreads + 32),
+    HQ_CUDA_TRY(opt_in.ensure(hq::gemm_decode_kernel<16, hq::kDealWhole, true>, C::kSmemBytes));
+    HQ_CUDA_TRY(hq::launch(hq::gemm_decode_kernel<16, hq::kDealWhole, true>, dim3(p.plan.ctas), dim3(hq::kDecThreads + 32),
                            size_t(C::kSmemBytes), static_cast<cudaStream_t>(stream), use_pdl != 0, 1, tm_w, tm_x, tm_o, p,
                            plain));
     return HQ_OK;
