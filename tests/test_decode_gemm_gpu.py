@@ -243,7 +243,8 @@ def test_chain_with_early_weight_loads(hq, monkeypatch, m, n, k, deal):
         assert torch.equal(outs[0][i], outs[1][i]) and torch.equal(outs[0][i], outs[2][i]), f"GEMM {i} of the chain differs"
 
 
-@pytest.mark.parametrize("m,n,k,deal", [(8, 7168, 2048, ""), (64, 24576, 1536, ""), (3, 320, 384, ""), (16, 1024, 8192, "split,nocluster")],
+@pytest.mark.parametrize("m,n,k,deal", [(8, 7168, 2048, ""), (64, 24576, 1536, ""), (3, 320, 384, ""), (16, 1024, 8192, "split,nocluster"),
+                                          (128, 8192, 1024, ""), (100, 192, 128, ""), (512, 1536, 1024, ""), (256, 7168, 2048, "")],
                          ids=lambda v: str(v))
 def test_weight_written_by_the_preceding_kernel(hq, monkeypatch, m, n, k, deal):
     """With a programmatic launch (use_pdl=True) the kernel asks for its weight in L2 before it waits for
