@@ -496,3 +496,26 @@ def test_pair_tile_is_bit_identical_and_deterministic(hq, monkeypatch, mode, m, 
     assert "pair=1" in hq.describe_tile(m, n, k, mode)
     for _ in range(10):
         assert torch.equal(single, _gemm(hq, aq, bq, sfa, sfb, mode))
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 256, 128), (300, 512, 384), (1000, 1024, 1152), (4096, 7168, 2048)], ids=lambda v: str(v))
+@pytest.mark.parametrize("linear_beta", [25.0, None])
+def test_situ_quant_on_the_2cta_tile(hq, monkeypatch, m, n, k, linear_beta):
+    """The quantising epilogue of the 256 x 256 pair tile gives the codes and scales of the single-CTA tile,
+    bit for bit, on one and several k-tiles, ragged rows (whose scale padding is zero) and several tiles
+    per cluster."""
+    g = torch.Generator().manual_seed(m + k)
+    xq, sfa = hq.group_wise_quant(torch.randn([m, k], generator=g).to(torch.bfloat16).cuda())
+    w = (torch.randn([n, k], generator=g) * 0.1).to(torch.bfloat16).cuda()
+    wq, sfb = hq.group_wise_quant(hq.interleave_gate_up(w))
+    bias = torch.randn([n], generator=g).to(torch.bfloat16).cuda()
+    results = []
+    for tile in ("256", "pair256"):
+        monkeypatch.setenv("HALOPS_B200_TILE", tile)
+        assert f"pair={int(tile == 'pair256')}" in hq.describe_tile(m, n, k)
+        out = torch.empty([m, n // 2], dtype=torch.float8_e4m3fn, device="cuda")
+        sf = torch.full([(m + 127) // 128 * 128, n // 64], 9, dtype=torch.uint8, device="cuda")
+        hq.dense_gemm(xq, wq, sfa, sfb, out, bias, epilogue=hq.EpilogueOp.SituQuant, output_sf=sf, situ_linear_beta=linear_beta)
+        assert hq.device_status() == 0
+        results.append((out.view(torch.uint8), sf))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
