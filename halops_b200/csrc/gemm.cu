@@ -2303,7 +2303,7 @@ struct TilePick {
 // gives every SM (or SM pair) a tile; failing that, the narrowest single-CTA
 // tile that divides N (most CTAs streaming the weight).  HALOPS_B200_TILE
 // (pair256 | pair128 | 256 | 128 | 64) overrides the choice when it is legal.
-TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count) {
+TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool grouped = false) {
     // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
     const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
     if (m < 1 || n < 1 || k < 1) return {0, false};
@@ -2334,33 +2334,40 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count) {
         }
         return {best, false};
     }
-    // Several rows of tiles: waves x time per tile.  Fitted to this build's kernels on B200
-    // (MXFP8; M = N = K = 8192, 8192 x 4096 x 4096 and 4096 x 14336 x 4096): a tile costs its
-    // k-tiles plus a fixed number of k-tile times for fill, drain and the hand-over to the
-    // next tile.  128x256: 0.46 us per k-tile + 2 (425 / 109.5 / 199 us); 256x256 pair:
-    // 0.404 + 3.2 (380 / 99.5 / 173 us); 128x128 0.35 (650 us); 256x128 pair 0.348 (633 us);
-    // 128x64 is extrapolated.  (These fits were made with one MMA issuer in the single-CTA kernel;
-    // its second, in-order issuer shortens the narrow and the FP4 tiles more than the choices made
-    // here depend on.)  The FP4 kinds stay on single-CTA tiles: the pair measured no
-    // faster there (126 against 113 us on 4096 x 14336 x 4096 with the same scale path).
+    // Several rows of tiles: a launch costs a fixed time plus, per wave of tiles, the k-tiles and a share
+    // for fill, drain and the hand-over.  Fitted (relative least squares) to 52 MXFP8 and 48 FP4 problems on B200,
+    // spread over M = 129..8192, N = 256..14336, K = 512..8192, each timed on every tile that is legal
+    // for it; residuals 3-7 %.  Choosing by it costs 0.6 % (MXFP8) and 0.1 % (FP4) over
+    // the best tile of each problem, the earlier figures (made when one thread issued all MMAs at 100 cycles
+    // each, which charged the narrow tiles most) 7 % and 2.5 %: 3139 x 1792 x 2048 behind a norm
+    // 24.4 -> 21.8 us, 937 x 4736 x 5760 36.9 -> 31.7, 256 x 7168 x 2048 behind its quantizer 11.4 -> 10.2.  The FP4 kinds stay on single-CTA tiles: the pair tile's tcgen05.cp
+    // scale copies, 12 per k-tile, are slower than its MMAs (4096 x 14336 x 4096 NVFP4 147 against 138 us).
     struct Cand {
         int bn;
         bool pair;
         double us_per_ktile;
-        double extra_ktiles;
+        double us_per_wave;
+        double us_fixed;
     };
-    const Cand cands[5] = {{256, false, 0.46, 2.0}, {256, true, 0.404, 3.2}, {128, false, 0.35, 1.0},
-                           {128, true, 0.348, 1.0},  {64, false, 0.27, 1.0}};
+    static constexpr Cand fp8_dense[5] = {{256, false, 0.340, 1.5, 3.0}, {256, true, 0.322, 1.25, 4.1}, {128, false, 0.195, 0.8, 2.7},
+                               {128, true, 0.273, 0.3, 3.7}, {64, false, 0.184, 0.5, 2.6}};
+    static constexpr Cand fp4_dense[2] = {{256, false, 0.378, 1.8, 3.0}, {128, false, 0.203, 0.9, 2.7}};
+    // the grouped kinds, whose kernels walk the groups in every role, keep the figures they were fitted with
+    static constexpr Cand any_grouped[5] = {{256, false, 0.46, 0.92, 0.0}, {256, true, 0.404, 1.293, 0.0}, {128, false, 0.35, 0.35, 0.0},
+                                 {128, true, 0.348, 0.348, 0.0}, {64, false, 0.27, 0.27, 0.0}};
+    const Cand* const cands = grouped ? any_grouped : fp8 ? fp8_dense : fp4_dense;
+    const int count = grouped || fp8 ? 5 : 2;
     const double k_tiles = double(k) / (fp8 ? 128.0 : 256.0);
     TilePick best = {0, false};
     double best_cost = 0.0;
-    for (const Cand& c : cands) {
+    for (int i = 0; i < count; ++i) {
+        const Cand& c = cands[i];
         if (n % c.bn != 0 || (c.bn == 64 && !fp8) || (c.pair && (m <= kBM || !fp8))) continue;
         const int64_t tiles = (c.pair ? tiles_m2 : tiles_m) * (n / c.bn);
         const int64_t units = c.pair ? sm_count / 2 : sm_count;
         if (units < 1) continue;
         const double waves = double((tiles + units - 1) / units);
-        const double cost = waves * (k_tiles + c.extra_ktiles) * c.us_per_ktile;
+        const double cost = c.us_fixed + waves * (k_tiles * c.us_per_ktile + c.us_per_wave);
         if (best.bn == 0 || cost < best_cost * 0.999) {
             best = {c.bn, c.pair};
             best_cost = cost;
@@ -2646,7 +2653,7 @@ TilePick pick_tile_grouped(int kind, int64_t count, int64_t rows, int64_t total_
     if (kind == kGroupMasked && rows % 64 != 0) return {0, false};
     if (kind == kGroupContiguous && total_m % 64 != 0) return {0, false};
     const int64_t pad = kind != kGroupContiguous && rows % kBM != 0 ? (count - 1) * kBM : 0;
-    TilePick pick = pick_tile(total_m + pad, n, k, mode, sm_count);
+    TilePick pick = pick_tile(total_m + pad, n, k, mode, sm_count, true);
     // The 2-CTA tile: MXFP8 (or e4m3 x MXFP4) with a plain epilogue, and no 256-row tile may hold rows of two
     // batches or expert slots (the contiguous layout is worked per run of experts, see
     // PairWorkIter).  Otherwise a forced or modelled pair choice falls back to the same width.
