@@ -5,9 +5,8 @@
 // (csrc/kernel/gemm/gemm_kernel.cuh:499-547, gemm_tile.cuh:203-216, epilogue.cuh:377-711).
 //
 // The weight streams through once, so the kernel is bound by HBM, not by the tensor cores;
-// what has to be kept small is everything else: the work of the thread that issues the MMAs
-// (about 90 cycles per tcgen05.mma and 230 per tcgen05.commit whatever their size) and the
-// epilogue.  Design:
+// what has to be kept small is everything else: the work of the warps that issue the MMAs and
+// the copies, the instructions a launch has to fetch, and the epilogue.  Design:
 //   * Operands are swapped: 128 weight rows are the M of tcgen05.mma, the activations its
 //     N (16 / 32 / 64 / 128 columns).  One instruction then consumes 4 KB of weights instead
 //     of the 2 KB of a 128 x 64 tile with the activations as M.
@@ -22,9 +21,8 @@
 //   * Before it waits for the preceding kernel of the stream a CTA asks for the start of its weight
 //     to be brought into L2 (see DecParams::prefetch_steps): 9.0 -> 8.4 us.
 //   * Two threads issue the MMAs of alternate k-steps into accumulators of their own, so
-//     they need no hand-over; the epilogue adds the two accumulators.  One thread alone
-//     needs about 1000 cycles per 32 KB step (33 bytes per cycle and CTA), less than an SM's
-//     share of HBM when fewer CTAs than SMs have work.
+//     they need no hand-over; the epilogue adds the two accumulators.  (One thread
+//     alone, issuing inside `if (lane == 0)`, needed about 1000 cycles per 32 KB step.)
 //   * Work is cut into units of (128 weight rows) x (256 bytes of K).  Normally a CTA works
 //     whole tiles.  When there are too few tiles to keep HBM busy, the units are dealt out
 //     evenly over the CTAs in one contiguous run each ("stream-K"), and a tile whose K range

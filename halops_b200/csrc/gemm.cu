@@ -1050,11 +1050,10 @@ struct Cfg2 {
     static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + kBarBytes + 1024;
     // Scale columns of one k-iteration and how many such sets rotate in tensor memory.
-    // The tcgen05.cp copies are issued by other warps than the MMAs: every asynchronous
-    // instruction stalls the thread that issues it (measured per instruction: tcgen05.cp
-    // 60-85 cycles, tcgen05.commit 88, a TMA copy 100-125) and those stalls only overlap
-    // across warps.  One thread issuing 3 copies + 4 MMAs + 2 commits per k-tile spent 850
-    // cycles on them; the MMAs alone take 512.  A set is free again once the MMAs that
+    // The tcgen05.cp copies are issued by other warps than the MMAs: a copy of one atom holds
+    // the copy unit, and the warp that waits for it, for 60-85 cycles, and 3 copies + 4 MMAs + 2 commits
+    // from one thread took 850 cycles per k-tile (measured with the issue inside `if (lane == 0)`, see
+    // ptx::elect_one); the MMAs alone take 512.  A set is free again once the MMAs that
     // read it have completed, so with 4 sets the copies run two k-tiles ahead.
     static constexpr int kSfCols = kSfKAtoms * 4 * (1 + kNAtoms);
     static constexpr int kSfSets = BN < 256 ? 4 : (kFp8Kind ? 4 : (KIND == 2 ? 3 : 2));
