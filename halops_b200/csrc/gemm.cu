@@ -114,13 +114,17 @@ struct Barriers {
     uint32_t abort;
 };
 
-// Bounded mbarrier wait.  Returns false when the CTA is aborting.
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort,
-                                         uint32_t code, uint64_t limit_ns = kTimeoutNs) {
-    if (ptx::mbar_try_wait(bar, parity)) return true;
+// Bounded mbarrier wait of one lane.  Returns false when the CTA is aborting.  kCluster: the barrier is one
+// that CTAs of the cluster arrive on with release semantics; the wait acquires what they wrote into
+// this CTA's shared memory before arriving.
+template <bool kCluster = false>
+__device__ __forceinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volatile uint32_t* abort,
+                                              uint32_t code, uint64_t limit_ns = kTimeoutNs) {
+    const auto done = [&] { return kCluster ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity); };
+    if (done()) return true;
     const uint64_t t0 = ptx::globaltimer_ns();
     uint32_t spins = 0;
-    while (!ptx::mbar_try_wait(bar, parity)) {
+    while (!done()) {
         if ((++spins & 31u) == 0u) {
             if (*abort != 0u) return false;
             if (ptx::globaltimer_ns() - t0 > limit_ns) {
@@ -133,9 +137,22 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     return true;
 }
 
-// The same for a whole warp, with a warp-uniform result (see ptx::elect_one).
-__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
-    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort, code) ? 1 : 0) != 0;
+// The wait of a role: called by all lanes of a warp, with one result for all of them.  Lanes poll for
+// themselves, so when a wait runs out while its barrier completes after all, some of them see the one and
+// some the other; leaving the role's loop on that would send a part of the warp into
+// .sync.aligned instructions, __syncwarp and elections that count on all 32 lanes.
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+    return __all_sync(0xffffffffu, wait_bar_lane(bar, parity, abort, code) ? 1 : 0) != 0;
+}
+// Two waits with one vote (the second only if `both`): a vote between a barrier and the work behind it is on the
+// critical path of a k-step.
+__device__ __forceinline__ bool wait_bars(uint32_t bar, uint32_t parity, bool both, uint32_t bar2, uint32_t parity2,
+                                          volatile uint32_t* abort, uint32_t code) {
+    const bool mine = wait_bar_lane(bar, parity, abort, code) && (!both || wait_bar_lane(bar2, parity2, abort, code));
+    return __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
+}
+__device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+    return __all_sync(0xffffffffu, wait_bar_lane<true>(bar, parity, abort, code) ? 1 : 0) != 0;
 }
 
 // The warp's index in its CTA, known to be warp-uniform.
@@ -553,7 +570,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 for (int kt = k_begin; kt < k_end; ++kt, ++it) {
                     const uint32_t s = it % kRing;
                     const uint32_t ph = (it / kRing) & 1u;
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
                     const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
@@ -599,11 +616,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const uint32_t aph = (t >> 1) & 1u;
                 // (with two issuers both wait here, also the one that has no k-tile in a tile of
                 // one: its arrival below must not run ahead of the stage's previous use)
-                ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                 if (!ok) break;
                 if (C::kOverlap != 0 && t > 0) {
                     // the previous tile's epilogue has drained the columns both stages share
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
+                    ok = wait_bar(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
                                   abort, kStatusMma);
                     if (!ok) break;
                 }
@@ -619,12 +636,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     const uint32_t ph = (it / kRing) & 1u;
                     // the scales of this k-tile are in their set (the scale warps waited for the
                     // scale bytes); the stage's own barrier orders this thread after the TMA writes
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
-                                  kStatusMma) &&
-                         wait_bar_warp(ptx::smem_u32(&bars->full[s]), ph, abort, kStatusMma);
+                    ok = wait_bars(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, true,
+                                   ptx::smem_u32(&bars->full[s]), ph, abort, kStatusMma);
                     // (in-order pair of issuers) the other thread has issued the MMAs of the previous k-iteration
                     if (ok && ordered && it > 0u) {
-                        ok = wait_bar_warp(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
+                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
                     }
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -686,14 +702,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         while (ok && work.next(wk)) {
             for (int kt = k_begin; kt < k_end; ++kt, ++it) {
                 const uint32_t s = it % kRing;
-                ok = wait_bar(ptx::smem_u32(&bars->sf_full[s]), (it / kRing) & 1u, abort, kStatusProducer);
-                if (ok && it >= uint32_t(C::kSfSets)) {
-                    // the MMAs of k-tile it - kSfSets read this set: they are done once they
-                    // have released their stage
-                    const uint32_t prev = it - uint32_t(C::kSfSets);
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[prev % kRing]), (prev / kRing) & 1u, abort,
-                                  kStatusProducer);
-                }
+                // the MMAs of k-tile it - kSfSets read this set: they are done once they
+                // have released their stage
+                const uint32_t prev = it - uint32_t(C::kSfSets);
+                ok = wait_bars(ptx::smem_u32(&bars->sf_full[s]), (it / kRing) & 1u, it >= uint32_t(C::kSfSets),
+                               ptx::smem_u32(&bars->empty[prev % kRing]), (prev / kRing) & 1u, abort, kStatusProducer);
                 if (!ok) break;
                 ptx::tc_fence_after();
                 const uint32_t set = tmem + (quarter << 16) + (it % C::kSfSets) * C::kSfCols;
@@ -833,11 +846,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     // row `ar`, columns [32 c, 32 c + 32) of the 128 x 64 fp32 buffer
                     const uint32_t slot = recv_base + uint32_t(ar) * (BN * 4) + uint32_t(c) * (kEpiChunk * 4);
                     if (k_rank != 0) {
-                        // an aborting CTA sends nothing more across the pair
-                        if (*abort != 0u) {
-                            ok = false;
-                            break;
-                        }
+                        // an aborting CTA sends nothing more across the pair (one decision per warp)
+                        ok = __any_sync(0xffffffffu, *abort != 0u ? 1 : 0) == 0;
+                        if (!ok) break;
                         const uint32_t dst = ptx::mapa_cluster(slot, 0);
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
@@ -858,15 +869,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     }
                     if (ci == 0) {
                         // this tile's partial sums (one phase of the barrier per tile)
-                        const uint64_t t0 = ptx::globaltimer_ns();
-                        while (!ptx::mbar_try_wait_cluster(ptx::smem_u32(&bars->recv_full), t & 1u)) {
-                            if (*abort != 0u || ptx::globaltimer_ns() - t0 > kTimeoutNs) {
-                                *abort = 1u;
-                                atomicOr(&g_status[0], uint32_t(kStatusEpilogue));
-                                ok = false;
-                                break;
-                            }
-                        }
+                        ok = wait_bar_cluster(ptx::smem_u32(&bars->recv_full), t & 1u, abort, kStatusEpilogue);
                         if (!ok) break;
                     }
 #pragma unroll
@@ -993,10 +996,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 // Self-test of the bounded wait and of the way a timeout spreads: thread 0 waits, with a
 // short limit, on a barrier that nothing ever arrives on; thread 32 waits on the same
 // barrier with the ordinary limit and must leave as soon as it sees the abort flag thread
-// 0 raises.  Nothing is in flight when the waits give up: no copies, no MMAs, no tensor
-// memory.  What the host then reads through hq_device_status is what it would read after a
-// GEMM role had timed out.
-__global__ void __launch_bounds__(64, 1) wait_selftest_kernel(uint64_t limit_ns) {
+// 0 raises.  The third warp makes a role's wait in which half of the lanes ask for a phase that is over and
+// half for one that never ends: all of them must be told to leave.  Nothing is in flight when the
+// waits give up: no copies, no MMAs, no tensor memory.  What the host then reads through hq_device_status
+// is what it would read after a GEMM role had timed out.
+__global__ void __launch_bounds__(96, 1) wait_selftest_kernel(uint64_t limit_ns) {
     __shared__ uint64_t bar;
     __shared__ uint32_t abort_flag;
     if (threadIdx.x == 0) {
@@ -1006,10 +1010,13 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(uint64_t limit_ns)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        wait_bar(ptx::smem_u32(&bar), 0, &abort_flag, kStatusMma, limit_ns);
+        wait_bar_lane(ptx::smem_u32(&bar), 0, &abort_flag, kStatusMma, limit_ns);
     } else if (threadIdx.x == 32) {
         // sees the flag within 32 polls of its being raised; its own limit never runs out
-        if (wait_bar(ptx::smem_u32(&bar), 0, &abort_flag, kStatusEpilogue)) atomicOr(&g_status[0], 0x80u);
+        if (wait_bar_lane(ptx::smem_u32(&bar), 0, &abort_flag, kStatusEpilogue)) atomicOr(&g_status[0], 0x80u);
+    } else if (threadIdx.x >= 64) {
+        // (the phase before the first counts as over)
+        if (wait_bar(ptx::smem_u32(&bar), threadIdx.x & 1u, &abort_flag, kStatusEpilogue)) atomicOr(&g_status[0], 0x40u);
     }
     __syncwarp();
     __syncthreads();
@@ -1315,7 +1322,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const int n0 = wk.b_row0 + int(rank) * (BN / 2);
                 for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                     // The MMA threads release a stage with one commit, to the leader's barrier; the
@@ -1350,7 +1357,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const int sfb_atom_row = (wk.b_row0 / 128) * kq_dim;
                 for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                     const uint32_t s = it % C::kStages;
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::mapa_cluster(ptx::smem_u32(&bars->full[s]), 0);
@@ -1384,13 +1391,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     total_its += uint32_t(k_tiles);
                 }
                 const uint32_t s = it % C::kStages;
-                ok = wait_bar_warp(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
+                ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
                 if (!ok) break;
                 if (it >= uint32_t(C::kSfSets)) {
                     // the MMAs of k-tile it - kSfSets read this set: they are done once they
                     // have released their stage
                     const uint32_t prev = it - uint32_t(C::kSfSets);
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
+                    ok = wait_bar(ptx::smem_u32(&bars->empty[prev % C::kStages]), (prev / C::kStages) & 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
                 }
@@ -1441,7 +1448,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                             // barrier expects both threads.  The arrival may not run ahead of the
                             // previous use of this accumulator stage, hence the same wait the
                             // issuing thread makes.
-                            ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                            ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                             if (!ok) break;
                             const uint32_t accf = ptx::smem_u32(&bars->acc_full[as]);
                             if (ptx::elect_one()) {
@@ -1454,9 +1461,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     const uint32_t s = it % C::kStages;
                     if (kt == 0) {
                         // first k-tile of a tile: the accumulator stage must have been drained
-                        ok = wait_bar_warp(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                        ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                         if (ok && C::kOverlap != 0 && t > 0) {
-                            ok = wait_bar_warp(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u, abort,
+                            ok = wait_bar(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u, abort,
                                           kStatusMma);
                         }
                         if (!ok) break;
@@ -1465,11 +1472,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     // stage's barrier before it copied and committed, so the operand boxes of both
                     // CTAs have landed too: no second wait here (each one costs this thread, which
                     // sets the pace, 50-100 cycles).
-                    ok = wait_bar_warp(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
+                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
                                   kStatusMma);
                     // the other thread has issued the MMAs of the previous k-iteration
                     if (ok && it > 0u) {
-                        ok = wait_bar_warp(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
+                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
                     }
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -3066,7 +3073,7 @@ extern "C" int hq_selftest_bounded_wait(uint32_t limit_us, int device, void* str
     }
     const hq::DeviceGuard guard(device);
     if (!guard.ok()) return hq::fail(err, errlen, HQ_ERR_CUDA, "cannot select CUDA device %d", device);
-    HQ_CUDA_TRY(hq::launch(hq::wait_selftest_kernel, dim3(1), dim3(64), size_t(0), static_cast<cudaStream_t>(stream),
+    HQ_CUDA_TRY(hq::launch(hq::wait_selftest_kernel, dim3(1), dim3(96), size_t(0), static_cast<cudaStream_t>(stream),
                            false, 1, uint64_t(limit_us) * 1000ull));
     return HQ_OK;
 }

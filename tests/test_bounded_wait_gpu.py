@@ -1,7 +1,8 @@
 """The path a GEMM role takes when one of its mbarrier waits times out, exercised with
 nothing in flight: a one-CTA kernel waits on a barrier that nothing arrives on, gives up
 after a millisecond, records its code in the device status word and raises the abort flag
-a second waiting thread leaves on.  No trap, no fault, no hang: the context stays usable
+a second waiting thread leaves on.  A third warp, half of whose lanes wait for a phase that is over, must leave
+as a whole (it would add status 0x40).  No trap, no fault, no hang: the context stays usable
 and the next GEMM is correct."""
 
 import time
