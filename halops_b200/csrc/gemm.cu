@@ -2984,6 +2984,12 @@ extern "C" int hq_low_latency_gemm(const void* a, const void* b, const void* sfa
                     "4-byte aligned");
     }
 
+    // A dual output has rows, and a first weight that may be empty is still an operand: neither has
+    // a tensor map of its own below that would refuse it.
+    if ((dual && n2 == 0) || !hq::aligned(b, 16)) {
+        return fail(err, errlen, HQ_ERR_INVALID,
+                    "TMA descriptor encoding failed: input and weight must be 16-byte aligned, contiguous rows");
+    }
     if (n == 0) {  // dual output with an empty first weight
         b = b2;
         sfb = sfb2;
@@ -3000,7 +3006,7 @@ extern "C" int hq_low_latency_gemm(const void* a, const void* b, const void* sfa
     hq::DecPlain<true> plain{};
     p.x_rows = int((m + 7) / 8 * 8);
     CUtensorMap tm_w, tm_x, tm_o;
-    const bool second_out = dual && n2 > 0;
+    const bool second_out = dual && n2 > 0;  // (n2 has become n if the first weight is empty)
     const bool maps_ok =
         hq::make_tmap_ktiles(&tm_w, b, uint64_t(n), uint64_t(k1), hq::kDecRows, 2) &&
         hq::make_tmap_ktiles(&tm_x, a, uint64_t(m), uint64_t(k1), uint32_t(p.x_rows), 2) &&

@@ -209,3 +209,33 @@ def test_tile_edges(hq, m, n, n2, k1, k2):
     assert hq.device_status() == 0
     for got, want in [(out, ref)] + refs:
         assert ((got.double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5).all()
+
+
+def test_dual_output_with_an_empty_weight(hq):
+    """C ABI only (an empty torch tensor has no address): with no rows in the first weight the call is the
+    plain product with the second one, bit for bit; with none in the second it is refused, and so is a first
+    weight that is empty but not aligned."""
+    from halops_b200 import _native
+
+    m, n2, k = 5, 264, 512
+    g = torch.Generator().manual_seed(8)
+    x, sx = hq.group_wise_quant(torch.randn([m, k], generator=g).to(torch.bfloat16).cuda(), use_swizzle=False)
+    w, sw = hq.group_wise_quant((torch.randn([n2, k], generator=g) * 0.02).to(torch.bfloat16).cuda(), use_swizzle=False)
+    expected = _run(hq, x, w, sx, sw)
+    first, sfirst = torch.zeros([8, k], dtype=torch.uint8, device="cuda"), torch.zeros([8, k // 32], dtype=torch.uint8, device="cuda")
+    out = torch.full([m, 8], 7.0, dtype=torch.bfloat16, device="cuda")
+    out2 = torch.empty_like(expected)
+
+    def call(n, n2, offset=0):
+        _native.call("hq_low_latency_gemm", x.data_ptr(), first.data_ptr() + offset, sx.data_ptr(), sfirst.data_ptr(), out.data_ptr(),
+                     None, w.data_ptr(), None, sw.data_ptr(), out2.data_ptr(), m, n, n2, k, 0, sx.stride(0), sfirst.stride(0), 0,
+                     sw.stride(0), 8, out2.stride(0), 0, -1, 1, 0, torch.cuda.current_stream().cuda_stream)
+
+    call(0, n2)
+    torch.cuda.synchronize()
+    assert torch.equal(out2, expected) and bool((out == 7.0).all())
+    for args in ((8, 0), (0, n2, 8)):
+        with pytest.raises(RuntimeError, match="TMA descriptor encoding failed"):
+            call(*args)
+    torch.cuda.synchronize()
+    assert torch.equal(out2, expected) and bool((out == 7.0).all())
