@@ -26,6 +26,10 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
 
 
+def cuda_root() -> str:
+    return os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+
+
 def _stale(target: str, deps) -> bool:
     return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
 
@@ -49,7 +53,7 @@ def _build_fast_path(force: bool, verbose: bool) -> None:
     import torch
 
     root = os.path.dirname(torch.__file__)
-    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cuda = cuda_root()
     _run([
         os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
         "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),

@@ -106,15 +106,23 @@ bool u8(const at::Tensor& t) { return t.scalar_type() == at::kByte; }
 
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
-// The C ABI call itself runs without the interpreter lock, as a ctypes call does.
+// Gives the interpreter lock away for its lifetime.
+class Unlocked {
+    PyThreadState* const state_ = PyEval_SaveThread();
+
+public:
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state_); }
+};
+
+// Runs without the interpreter lock, as torch.empty and a ctypes call do: the C ABI call, and the allocation of the
+// outputs, which may wait for the device when the allocator has to free memory for it.
 template <typename F>
 int unlocked(F&& f) {
     char err[kErrLen];
-    int rc = 0;
-    Py_BEGIN_ALLOW_THREADS
-    rc = f(err);
-    Py_END_ALLOW_THREADS
-    return rc;
+    const Unlocked scope;
+    return f(err);
 }
 
 PyObject* pair_of(const at::Tensor& a, const at::Tensor& b) {
@@ -148,18 +156,14 @@ PyObject* group_wise_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int64_t qk = mode == 0 ? k : k / 2;
     const auto qt = mode == 0 ? at::kFloat8_e4m3fn : at::kByte;
     at::Tensor q, sf;
-    if (a[4] == Py_None) {
-        q = at::empty({m, qk}, at::TensorOptions().dtype(qt).device(x->device()));
-    } else {
+    if (a[4] != Py_None) {
         const at::Tensor* const t = plain_tensor(a[4]);
         if (t == nullptr || !t->is_contiguous() || t->scalar_type() != qt || t->numel() != m * qk || t->device() != x->device()) {
             Py_RETURN_NONE;
         }
         q = *t;
     }
-    if (a[5] == Py_None) {
-        sf = at::empty({m_sf, kb}, at::TensorOptions().dtype(at::kByte).device(x->device()));
-    } else {
+    if (a[5] != Py_None) {
         const at::Tensor* const t = plain_tensor(a[5]);
         if (t == nullptr || !t->is_contiguous() || !u8(*t) || t->numel() != m_sf * kb || t->device() != x->device()) {
             Py_RETURN_NONE;
@@ -168,12 +172,13 @@ PyObject* group_wise_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     }
     const void* const px = x->data_ptr();
     const int64_t ld = x->stride(0);
-    void* const pq = q.data_ptr();
-    void* const psf = sf.data_ptr();
     const int dev = x->get_device();
     void* const st = stream_of(*x);
+    const auto on_device = at::TensorOptions().device(x->device());
     if (unlocked([&](char* err) {
-            return g_fn.quant(px, ld, bf16 ? 0 : 1, m, k, mode, swizzle, pdl, pq, psf, dev, st, err, kErrLen);
+            if (!q.defined()) q = at::empty({m, qk}, on_device.dtype(qt));
+            if (!sf.defined()) sf = at::empty({m_sf, kb}, on_device.dtype(at::kByte));
+            return g_fn.quant(px, ld, bf16 ? 0 : 1, m, k, mode, swizzle, pdl, q.data_ptr(), sf.data_ptr(), dev, st, err, kErrLen);
         }) != 0) {
         Py_RETURN_NONE;
     }
@@ -198,17 +203,18 @@ PyObject* rms_norm_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         Py_RETURN_NONE;
     }
     const int64_t m_sf = swizzle != 0 ? (m + 127) / 128 * 128 : m;
-    const at::Tensor q = at::empty({m, k}, at::TensorOptions().dtype(at::kFloat8_e4m3fn).device(x->device()));
-    const at::Tensor sf = at::empty({m_sf, k / 32}, at::TensorOptions().dtype(at::kByte).device(x->device()));
     const void* const px = x->data_ptr();
     const int64_t ld = x->stride(0);
     const void* const pw = w->data_ptr();
-    void* const pq = q.data_ptr();
-    void* const psf = sf.data_ptr();
     const int dev = x->get_device();
     void* const st = stream_of(*x);
-    if (unlocked([&](char* err) { return g_fn.rms(px, ld, pw, eps, m, k, swizzle, pdl, pq, psf, dev, st, err, kErrLen); }) !=
-        0) {
+    const auto on_device = at::TensorOptions().device(x->device());
+    at::Tensor q, sf;
+    if (unlocked([&](char* err) {
+            q = at::empty({m, k}, on_device.dtype(at::kFloat8_e4m3fn));
+            sf = at::empty({m_sf, k / 32}, on_device.dtype(at::kByte));
+            return g_fn.rms(px, ld, pw, eps, m, k, swizzle, pdl, q.data_ptr(), sf.data_ptr(), dev, st, err, kErrLen);
+        }) != 0) {
         Py_RETURN_NONE;
     }
     return pair_of(q, sf);

@@ -1,6 +1,10 @@
 """The native front of the entry points (csrc/fast_path.cpp) takes the ordinary call of every mode and
 gives what the wrapper's own way gives; whatever is not ordinary it leaves to the wrapper, unlaunched."""
 
+import ctypes
+import subprocess
+import threading
+
 import pytest
 import torch
 
@@ -95,3 +99,84 @@ def test_grouped(hq, native, monkeypatch):
         with pytest.raises(RuntimeError, match="input M must equal num_experts"):
             hq.group_masked_gemm(x, w, sfa, sfb, counts, out[0], max_m_per_expert=2 * rows)
     assert torch.equal(*results)
+
+
+ALLOCATOR = """
+#include <cuda_runtime.h>
+#include <sys/types.h>
+extern "C" int PyGILState_Check(void);
+static int calls, locked;
+extern "C" void* count_alloc(ssize_t size, int, cudaStream_t) {
+    ++calls;
+    locked += PyGILState_Check();
+    void* p = nullptr;
+    return cudaMalloc(&p, size) == cudaSuccess ? p : nullptr;
+}
+extern "C" void count_free(void* p, ssize_t, int, cudaStream_t) { cudaFree(p); }
+extern "C" int count_calls(void) { return calls; }
+extern "C" int count_locked(void) { return locked; }
+"""
+
+
+@pytest.mark.parametrize("entry", ["group_wise_quant", "rms_norm_quant"])
+def test_outputs_are_allocated_without_the_interpreter_lock(hq, native, tmp_path, entry):
+    """An allocation may wait for the device (a full card, a stream that a host function in Python holds up):
+    other Python threads must be able to run meanwhile."""
+    from halops_b200 import build
+
+    source, lib = tmp_path / "alloc.cpp", tmp_path / "alloc.so"
+    source.write_text(ALLOCATOR)
+    cuda = build.cuda_root()
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", lib, source, f"-I{cuda}/include", f"-L{cuda}/lib64", "-lcudart"], check=True)
+    x = torch.randn([64, 256], device="cuda").to(torch.bfloat16)
+    weight = x[0].contiguous()
+    pool = torch.cuda.MemPool(torch.cuda.memory.CUDAPluggableAllocator(str(lib), "count_alloc", "count_free").allocator())
+    counts = ctypes.CDLL(str(lib))
+    with torch.cuda.use_mem_pool(pool):
+        if entry == "group_wise_quant":
+            outputs = native.fast_path.group_wise_quant(x, "w8a8-mxfp8", True, True, None, None)
+        else:
+            outputs = native.fast_path.rms_norm_quant(x, weight, 1e-6, True, True)
+    assert outputs is not None
+    torch.cuda.synchronize()
+    assert counts.count_calls() > 0 and counts.count_locked() == 0
+    del outputs
+
+
+def test_two_threads(hq, native):
+    """Each thread on a stream of its own, with its own inputs, outputs and weights: what one thread alone gets."""
+    g = torch.Generator().manual_seed(4)
+    sizes = [(8, 1024, 512), (200, 256, 384)]
+    jobs = []
+    for m, n, k in sizes:
+        x = torch.randn([m, k], generator=g).to(torch.bfloat16).cuda()
+        w, sfw = hq.group_wise_quant(torch.randn([n, k], generator=g).to(torch.bfloat16).cuda())
+        jobs.append((x, w, sfw, n))
+
+    def chain(job):
+        x, w, sfw, n = job
+        outs = []
+        for _ in range(50):
+            q, sf = hq.group_wise_quant(x)
+            out = torch.empty([x.size(0), n], dtype=torch.bfloat16, device="cuda")
+            hq.dense_gemm(q, w, sf, sfw, out)
+            outs.append(out)
+        return outs
+
+    expected = [chain(job)[0] for job in jobs]
+    torch.cuda.synchronize()
+    results = [None] * len(jobs)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            results[i] = chain(jobs[i])
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert hq.device_status() == 0
+    for want, outs in zip(expected, results):
+        assert outs is not None and all(torch.equal(want, out) for out in outs)
