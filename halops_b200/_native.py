@@ -6,6 +6,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import warnings
 
 _LIB_PATH = os.environ.get("HALOPS_B200_LIB") or os.path.join(
     os.path.dirname(os.path.abspath(__file__)), "lib", "libhalops_b200.so")
@@ -89,8 +90,8 @@ def lib() -> ctypes.CDLL:
 
 
 class _NoFastPath:
-    """Stands in while the shared library has not been built: every call takes the wrappers' own
-    way, whose argument checks need no library and whose first use of it says that it is missing."""
+    """Stands in where there is no native front: every call takes the wrappers' own way, whose argument
+    checks need no library and whose first use of it says if it is missing."""
 
     @staticmethod
     def _none(*args):
@@ -105,28 +106,39 @@ fast_path = None
 _FAST_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "halops_b200_fast_path.so")
 
 
+def _import_fast_path(handle):
+    import importlib.util
+
+    import torch  # noqa: F401  (the module's symbols are torch's)
+
+    spec = importlib.util.spec_from_file_location("halops_b200_fast_path", _FAST_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
+        "hq_group_wise_quant", "hq_rms_norm_quant", "hq_dense_gemm", "hq_dense_gemm_situ_quant",
+        "hq_describe_group_tile", "hq_group_masked_gemm", "hq_group_contiguous_gemm")))
+    return module
+
+
 def load_fast_path():
-    """Loads the module once and hands it the entry points of the loaded library."""
+    """Loads the module once and hands it the entry points of the loaded library.  It only saves host time:
+    where it has not been built (a library that HALOPS_B200_LIB names may come without one) or does not load, the
+    wrappers make every call, and one warning says so."""
     global fast_path
     if not os.path.exists(_LIB_PATH):
         return _NoFastPath
     handle = lib()
+    problem = None
     with _lock:
         if fast_path is None:
-            if not os.path.exists(_FAST_PATH):
-                raise RuntimeError(f"halops_b200: native module not found at {_FAST_PATH}; build it with "
-                                   "`python -m halops_b200.build` (needs a C++ compiler, no GPU).")
-            import importlib.util
-
-            import torch  # noqa: F401  (the module's symbols are torch's)
-
-            spec = importlib.util.spec_from_file_location("halops_b200_fast_path", _FAST_PATH)
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
-            module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
-                "hq_group_wise_quant", "hq_rms_norm_quant", "hq_dense_gemm", "hq_dense_gemm_situ_quant",
-                "hq_describe_group_tile", "hq_group_masked_gemm", "hq_group_contiguous_gemm")))
-            fast_path = module
+            try:
+                fast_path = _import_fast_path(handle)
+            except (ImportError, OSError, AttributeError) as e:
+                problem, fast_path = e, _NoFastPath
+    if problem is not None:
+        warnings.warn(f"halops_b200: the native front of the Python calls is not used, each call costs the host more time ({problem}); "
+                      "`python -m halops_b200.build` builds it (needs a C++ compiler and torch with CUDA, no GPU).",
+                      RuntimeWarning, stacklevel=3)
     return fast_path
 
 
