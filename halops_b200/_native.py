@@ -8,6 +8,10 @@ import os
 import threading
 import warnings
 
+import torch
+
+from ._paths import fast_path_file
+
 _LIB_PATH = os.environ.get("HALOPS_B200_LIB") or os.path.join(
     os.path.dirname(os.path.abspath(__file__)), "lib", "libhalops_b200.so")
 _lock = threading.Lock()
@@ -103,13 +107,11 @@ class _NoFastPath:
 # The module of csrc/fast_path.cpp, which makes the ordinary call of an entry point natively; None until
 # load_fast_path has run.  Its functions return None for a call they leave to the wrapper.
 fast_path = None
-_FAST_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "halops_b200_fast_path.so")
+_FAST_PATH = fast_path_file(torch.__version__)
 
 
 def _import_fast_path(handle):
     import importlib.util
-
-    import torch  # noqa: F401  (the module's symbols are torch's)
 
     spec = importlib.util.spec_from_file_location("halops_b200_fast_path", _FAST_PATH)
     module = importlib.util.module_from_spec(spec)
@@ -157,8 +159,6 @@ def current_stream(device) -> int:
     """Handle of torch's current CUDA stream on ``device`` (a ``torch.device`` with an index).
     ``torch.cuda.current_stream`` builds a Stream object for this, which costs the host several
     microseconds per call; torch's raw getter does not."""
-    import torch
-
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
     if raw is not None and device.index is not None:
         return raw(device.index)

@@ -1,6 +1,7 @@
 """Builds the C-ABI shared library ``halops_b200/lib/libhalops_b200.so`` in-tree
-with nvcc for sm_100a, and beside it the CPython module that the Python entry
-points call it through.  No GPU is needed to build."""
+with nvcc for sm_100a, and beside it, where torch with CUDA and a C++ compiler are
+there, the CPython module that the Python entry points call it through.  No GPU is
+needed to build."""
 
 from __future__ import annotations
 
@@ -14,9 +15,16 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libhalops_b200.so")
-FAST_PATH = os.path.join(LIB_DIR, "halops_b200_fast_path.so")
 SOURCES = ("quant.cu", "gemm.cu")
-HEADERS = ("common.cuh", "ptx.cuh", "decode.cuh", os.path.join("..", "..", "include", "halops_b200.h"))
+ABI_HEADER = os.path.join(PKG, "..", "include", "halops_b200.h")
+FAST_PATH_DEPS = (os.path.join(CSRC, "fast_path.cpp"), ABI_HEADER)
+HEADERS = ("common.cuh", "ptx.cuh", "decode.cuh")
+
+
+try:
+    from ._paths import fast_path_file
+except ImportError:  # run as a file, for the C ABI alone
+    from _paths import fast_path_file
 
 
 def _nvcc() -> str:
@@ -35,7 +43,11 @@ def _stale(target: str, deps) -> bool:
 
 
 def is_stale() -> bool:
-    return _stale(LIB_PATH, [os.path.join(CSRC, f) for f in SOURCES + HEADERS])
+    return _stale(LIB_PATH, [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [ABI_HEADER])
+
+
+def fast_path_is_stale(torch_version: str) -> bool:
+    return _stale(fast_path_file(torch_version), FAST_PATH_DEPS)
 
 
 def _run(cmd, verbose: bool) -> None:
@@ -47,19 +59,26 @@ def _run(cmd, verbose: bool) -> None:
 
 
 def _build_fast_path(force: bool, verbose: bool) -> None:
-    source = os.path.join(CSRC, "fast_path.cpp")
-    if not force and not _stale(FAST_PATH, [source]):
+    compiler = os.environ.get("CXX") or "g++"
+    try:
+        import torch
+    except ImportError:
+        torch = None
+    if torch is None or torch.version.cuda is None or shutil.which(compiler) is None:
+        # the C ABI does not need it, and the Python wrappers do without
+        sys.stderr.write("halops_b200: the native front of the Python calls is not built: it needs torch with CUDA and "
+                         f"a C++ compiler ({compiler})\n")
         return
-    import torch
-
+    if not force and not fast_path_is_stale(torch.__version__):
+        return
     root = os.path.dirname(torch.__file__)
     cuda = cuda_root()
     _run([
-        os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+        compiler, "-O2", "-std=c++17", "-fPIC", "-shared",
         "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
         "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"],
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-        "-o", FAST_PATH, source,
+        "-o", fast_path_file(torch.__version__), FAST_PATH_DEPS[0],
         "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
     ], verbose)
 

@@ -22,21 +22,20 @@
 
 #include <cstring>
 
+#include "../../include/halops_b200.h"
+
 namespace {
 
 constexpr int kErrLen = 512;
 
-using QuantFn = int (*)(const void*, int64_t, int, int64_t, int64_t, int, int, int, void*, void*, int, void*, char*, size_t);
-using RmsFn = int (*)(const void*, int64_t, const void*, float, int64_t, int64_t, int, int, void*, void*, int, void*, char*,
-                      size_t);
-using DenseFn = int (*)(const void*, const void*, const void*, const void*, void*, const void*, const float*, int64_t, int64_t,
-                        int64_t, int64_t, int64_t, int64_t, int, int, int, int, int, void*, char*, size_t);
-using SituFn = int (*)(const void*, const void*, const void*, const void*, void*, void*, const void*, int64_t, int64_t, int64_t,
-                       int64_t, int64_t, int64_t, float, float, int, int, int, void*, char*, size_t);
-using DescribeGroupFn = int (*)(int, int64_t, int64_t, int64_t, int64_t, int64_t, int, int, int, char*, size_t);
-using MaskedFn = int (*)(const void*, const void*, const void*, const void*, const void*, void*, const void*, const float*,
-                         int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, int, int, int, void*, char*,
-                         size_t);
+// The signatures are the header's, so a changed one does not compile here until its call is changed too.
+using QuantFn = decltype(&hq_group_wise_quant);
+using RmsFn = decltype(&hq_rms_norm_quant);
+using DenseFn = decltype(&hq_dense_gemm);
+using SituFn = decltype(&hq_dense_gemm_situ_quant);
+using DescribeGroupFn = decltype(&hq_describe_group_tile);
+using MaskedFn = decltype(&hq_group_masked_gemm);
+using ContiguousFn = decltype(&hq_group_contiguous_gemm);
 
 // the entry points of the shared library that the Python package has loaded
 struct {
@@ -46,10 +45,10 @@ struct {
     SituFn situ;
     DescribeGroupFn describe_group;
     MaskedFn masked;
-    MaskedFn contiguous;  // the same signature: table of expert ids, M instead of rows per expert
+    ContiguousFn contiguous;
 } g_fn;
 
-// MODE_IDS of the package: w8a8-mxfp8, w4a4-mxfp4, w4a4-nvfp4, w4a8-mxfp4
+// the package's mode names
 int mode_id(PyObject* o) {
     if (!PyUnicode_CheckExact(o)) return -1;
     const char* s = PyUnicode_AsUTF8(o);
@@ -57,10 +56,10 @@ int mode_id(PyObject* o) {
         PyErr_Clear();
         return -1;
     }
-    if (std::strcmp(s, "w8a8-mxfp8") == 0) return 0;
-    if (std::strcmp(s, "w4a4-mxfp4") == 0) return 1;
-    if (std::strcmp(s, "w4a4-nvfp4") == 0) return 2;
-    if (std::strcmp(s, "w4a8-mxfp4") == 0) return 3;
+    if (std::strcmp(s, "w8a8-mxfp8") == 0) return HQ_MODE_W8A8_MXFP8;
+    if (std::strcmp(s, "w4a4-mxfp4") == 0) return HQ_MODE_W4A4_MXFP4;
+    if (std::strcmp(s, "w4a4-nvfp4") == 0) return HQ_MODE_W4A4_NVFP4;
+    if (std::strcmp(s, "w4a8-mxfp4") == 0) return HQ_MODE_W4A8_MXFP4;
     return -1;
 }
 
@@ -147,14 +146,14 @@ PyObject* group_wise_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (nargs != 6 || g_fn.quant == nullptr || at::impl::torch_function_mode_enabled()) Py_RETURN_NONE;
     const at::Tensor* const x = plain_tensor(a[0]);
     const int mode = mode_id(a[1]);
-    if (x == nullptr || mode < 0 || mode > 2 || !flag(a[2], &swizzle) || !flag(a[3], &pdl)) Py_RETURN_NONE;
+    if (x == nullptr || mode < 0 || mode == HQ_MODE_W4A8_MXFP4 || !flag(a[2], &swizzle) || !flag(a[3], &pdl)) Py_RETURN_NONE;
     const bool bf16 = x->scalar_type() == at::kBFloat16;
     if ((!bf16 && x->scalar_type() != at::kHalf) || !quant_input(*x)) Py_RETURN_NONE;
-    const int64_t m = x->size(0), k = x->size(1), group = mode == 2 ? 16 : 32, kb = k / group;
+    const int64_t m = x->size(0), k = x->size(1), group = mode == HQ_MODE_W4A4_NVFP4 ? 16 : 32, kb = k / group;
     if (m == 0 || k == 0 || k % group != 0 || (swizzle != 0 && kb % 4 != 0)) Py_RETURN_NONE;
     const int64_t m_sf = swizzle != 0 ? (m + 127) / 128 * 128 : m;
-    const int64_t qk = mode == 0 ? k : k / 2;
-    const auto qt = mode == 0 ? at::kFloat8_e4m3fn : at::kByte;
+    const int64_t qk = mode == HQ_MODE_W8A8_MXFP8 ? k : k / 2;
+    const auto qt = mode == HQ_MODE_W8A8_MXFP8 ? at::kFloat8_e4m3fn : at::kByte;
     at::Tensor q, sf;
     if (a[4] != Py_None) {
         const at::Tensor* const t = plain_tensor(a[4]);
@@ -178,7 +177,7 @@ PyObject* group_wise_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (unlocked([&](char* err) {
             if (!q.defined()) q = at::empty({m, qk}, on_device.dtype(qt));
             if (!sf.defined()) sf = at::empty({m_sf, kb}, on_device.dtype(at::kByte));
-            return g_fn.quant(px, ld, bf16 ? 0 : 1, m, k, mode, swizzle, pdl, q.data_ptr(), sf.data_ptr(), dev, st, err, kErrLen);
+            return g_fn.quant(px, ld, bf16 ? HQ_DTYPE_BF16 : HQ_DTYPE_FP16, m, k, mode, swizzle, pdl, q.data_ptr(), sf.data_ptr(), dev, st, err, kErrLen);
         }) != 0) {
         Py_RETURN_NONE;
     }
@@ -225,7 +224,7 @@ PyObject* rms_norm_quant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 //            situ_beta, situ_linear_beta) -> True, or None when the call is not an ordinary one
 PyObject* dense_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
-    constexpr int kIdentity = 0, kSigmoid = 3, kSitu = 4;
+    constexpr int kIdentity = HQ_EPILOGUE_IDENTITY, kSigmoid = HQ_EPILOGUE_SIGMOID, kSitu = HQ_EPILOGUE_SITU_QUANT;
     int sm_count, pdl, epilogue;
     if (nargs != 14 || g_fn.dense == nullptr || at::impl::torch_function_mode_enabled()) Py_RETURN_NONE;
     const at::Tensor* const x = plain_tensor(a[0]);
@@ -234,11 +233,11 @@ PyObject* dense_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const at::Tensor* const sfb = plain_tensor(a[3]);
     const at::Tensor* const out = plain_tensor(a[4]);
     const int mode = mode_id(a[8]);
-    if (x == nullptr || w == nullptr || sfa == nullptr || sfb == nullptr || out == nullptr || mode < 0 || mode > 2 ||
-        !small_int(a[7], &sm_count) || !small_int(a[9], &pdl) || pdl < 0 || pdl > 2 || !small_int(a[10], &epilogue)) {
+    if (x == nullptr || w == nullptr || sfa == nullptr || sfb == nullptr || out == nullptr || mode < 0 ||
+        mode == HQ_MODE_W4A8_MXFP4 || !small_int(a[7], &sm_count) || !small_int(a[9], &pdl) || pdl < 0 || pdl > 2 || !small_int(a[10], &epilogue)) {
         Py_RETURN_NONE;
     }
-    const bool fp8 = mode == 0, situ = epilogue == kSitu;
+    const bool fp8 = mode == HQ_MODE_W8A8_MXFP8, nvfp4 = mode == HQ_MODE_W4A4_NVFP4, situ = epilogue == kSitu;
     if (epilogue != kIdentity && epilogue != kSigmoid && !(situ && fp8)) Py_RETURN_NONE;
     if (x->dim() != 2 || w->dim() != 2 || out->dim() != 2 || sfa->dim() < 1 || sfb->dim() < 1) Py_RETURN_NONE;
     if (!bytes(*x) || !bytes(*w) || !u8(*sfa) || !u8(*sfb)) Py_RETURN_NONE;
@@ -248,7 +247,7 @@ PyObject* dense_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int64_t m = x->size(0), n = w->size(0), k = fp8 ? w->size(1) : w->size(1) * 2;
     if (m == 0 || n == 0 || x->size(1) != w->size(1)) Py_RETURN_NONE;
     if (out->size(0) != m || out->size(1) != (situ ? n / 2 : n)) Py_RETURN_NONE;
-    const int64_t sf_k = k / (mode == 2 ? 16 : 32), m_sf = (m + 127) / 128 * 128;
+    const int64_t sf_k = k / (nvfp4 ? 16 : 32), m_sf = (m + 127) / 128 * 128;
     if (sfa->numel() < m_sf * sf_k) Py_RETURN_NONE;
     if (!fp8 && (sfa->size(-1) != sf_k || sfb->size(-1) != sf_k)) Py_RETURN_NONE;
     const void* bias = nullptr;
@@ -263,9 +262,9 @@ PyObject* dense_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const float* alpha = nullptr;
     if (a[6] != Py_None) {
         const at::Tensor* const t = plain_tensor(a[6]);
-        if (mode != 2 || t == nullptr || t->scalar_type() != at::kFloat || t->numel() < 1 || t->device() != dev) Py_RETURN_NONE;
+        if (!nvfp4 || t == nullptr || t->scalar_type() != at::kFloat || t->numel() < 1 || t->device() != dev) Py_RETURN_NONE;
         alpha = static_cast<const float*>(t->data_ptr());
-    } else if (mode == 2) {
+    } else if (nvfp4) {
         Py_RETURN_NONE;
     }
     const void* const px = x->data_ptr();
@@ -319,7 +318,8 @@ PyObject* grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         !small_int(a[0], &kind) || !small_int(a[9], &max_m) || !small_int(a[10], &sm_count)) {
         Py_RETURN_NONE;
     }
-    const bool masked = kind == 2, fp8 = mode == 0, w4a8 = mode == 3;
+    const bool masked = kind == 2, fp8 = mode == HQ_MODE_W8A8_MXFP8, nvfp4 = mode == HQ_MODE_W4A4_NVFP4,
+               w4a8 = mode == HQ_MODE_W4A8_MXFP4;
     if (x->dim() != 2 || w->dim() != 3 || table->dim() != 1 || out->dim() != 2 || sfa->dim() < 1 || sfb->dim() < 1) {
         Py_RETURN_NONE;
     }
@@ -336,7 +336,7 @@ PyObject* grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         !table->is_contiguous()) {
         Py_RETURN_NONE;
     }
-    const int64_t sf_k = k / (mode == 2 ? 16 : 32);
+    const int64_t sf_k = k / (nvfp4 ? 16 : 32);
     if (!fp8 && (sfa->size(-1) != sf_k || sfb->size(-1) != sf_k)) Py_RETURN_NONE;
     const void* bias = nullptr;
     if (a[7] != Py_None) {
@@ -350,19 +350,19 @@ PyObject* grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const float* alpha = nullptr;
     if (a[8] != Py_None) {
         const at::Tensor* const t = plain_tensor(a[8]);
-        if (mode != 2 || t == nullptr || t->scalar_type() != at::kFloat || t->numel() != e || !t->is_contiguous() ||
+        if (!nvfp4 || t == nullptr || t->scalar_type() != at::kFloat || t->numel() != e || !t->is_contiguous() ||
             t->device() != dev) {
             Py_RETURN_NONE;
         }
         alpha = static_cast<const float*>(t->data_ptr());
-    } else if (mode == 2) {
+    } else if (nvfp4) {
         Py_RETURN_NONE;
     }
     const void* const px = x->data_ptr();
     const void* const pw = w->data_ptr();
     const void* const psa = sfa->data_ptr();
     const void* const psb = sfb->data_ptr();
-    const void* const pt = table->data_ptr();
+    const int32_t* const pt = static_cast<const int32_t*>(table->data_ptr());
     void* const po = out->data_ptr();
     const int64_t na = sfa->numel(), nb = sfb->numel(), ldo = out->stride(0);
     const int d = x->get_device();
@@ -388,7 +388,7 @@ PyObject* bind(PyObject*, PyObject* args) {
     g_fn.situ = reinterpret_cast<SituFn>(p[3]);
     g_fn.describe_group = reinterpret_cast<DescribeGroupFn>(p[4]);
     g_fn.masked = reinterpret_cast<MaskedFn>(p[5]);
-    g_fn.contiguous = reinterpret_cast<MaskedFn>(p[6]);
+    g_fn.contiguous = reinterpret_cast<ContiguousFn>(p[6]);
     Py_RETURN_NONE;
 }
 
