@@ -904,9 +904,16 @@ inline DecPlan dec_plan(int n, int64_t k_bytes, int sm_count, bool allow_split, 
 // step), about what HBM brings while an activation's quantizer runs and the wait is released.
 // More evicts and queues in front of the loads (whole runs: 33 x 23552 x 7808 45.0 us, 5 steps
 // 43.6, none 44.7), less leaves HBM idle (8 x 7168 x 2048: 2 or 5 steps 8.45 us, all 8 8.2).
+// And no more than one tile's steps per CTA (but up to 8): few CTAs (a caller's sm_count) would each ask for
+// hundreds, at some 100 cycles each, from the warp that has to drain their first tile meanwhile.  Behind their
+// quantizers, on 4 / 16 / 148 SMs: 8 x 7168 x 2048 without the limit 41.0 / 13.5 / 6.2 us, with it 27.6 / 11.3 / 6.2,
+// without a prefetch 27.5 / 11.2 / 6.2; 8 x 24576 x 1536 98.7 / 26.7 / 10.9, 82.1 / 24.5 / 10.9 and 83.7 / 25.2 / 11.8.
+// (8 steps for all took 7.4 instead of 7.1 us on 5 x 3136 x 3072, one tile of 12 steps per CTA.)
+constexpr int kDecPrefetchSteps = 8;
 inline int dec_prefetch_steps(const DecPlan& p, int64_t step_bytes) {
     const int64_t steps = (int64_t(24) << 20) / (int64_t(p.ctas) * step_bytes);
-    return steps < 1 ? 1 : steps > p.ksteps * int64_t(p.tiles) ? int(p.ksteps * int64_t(p.tiles)) : int(steps);
+    const int limit = p.ksteps > kDecPrefetchSteps ? p.ksteps : kDecPrefetchSteps;
+    return steps < 1 ? 1 : steps > limit ? limit : int(steps);
 }
 
 // Host check of the unit deal, for tests: every unit is worked exactly once, the owner

@@ -467,7 +467,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const uint8_t* __restrict__ sfb, const float* __restrict__ alpha,
             const __nv_bfloat16* __restrict__ bias, int epi_op, __nv_bfloat16* __restrict__ out, int64_t ldo,
             int M, int N, int k_tiles, int kq_dim, int tiles_m, int tiles_n, int a_rows, int direct_store,
-            int dual_issue, const GroupParams grp_arg, const SituParams situ) {
+            int dual_issue, int prefetch_weight, const GroupParams grp_arg, const SituParams situ) {
     using C = Cfg<BN, KIND>;
     const GroupParams grp = kDense ? GroupParams{kGroupDense, 1, 0, nullptr} : grp_arg;
     // Two MMA issuers with an accumulator each (64-wide dense tiles, plain epilogues): the k-tiles
@@ -540,9 +540,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     // The first k-tiles of this CTA's weight into L2 while the preceding kernel finishes: a hint, as in the
     // small-M kernel, up to 160 KB per CTA (24 MB in all).  The CTAs that share a column of tiles share
     // the k-tiles too.  128 x 8192 x 4096 behind its quantizer 13.2 -> 12.5 us, 512 x 1536 x 4096 12.8 -> 12.7.
+    // Only under a programmatic launch: a CTA that starts after the preceding kernel has ended would ask for
+    // everything twice (128 x 8192 x 4096 launched without, 11.7 us, was 12.8 with it).
     // (Dense only: which weight a grouped tile takes is only known after the wait.)
     if constexpr (kDense) {
-        if (threadIdx.x == 64 && first_item < tiles_m * tiles_n) {
+        if (threadIdx.x == 64 && prefetch_weight != 0 && first_item < tiles_m * tiles_n) {
             const TileCoord tc = tile_coord(first_item, tiles_m, tiles_n);
             const int end = min(k_end, k_begin + 1280 / BN);
             for (int kt = k_begin + (tc.m & 7); kt < end; kt += min(8, tiles_m)) {
@@ -1240,7 +1242,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ CUtensorMap tm_sfa,
                  const __grid_constant__ CUtensorMap tm_sfb, const float* __restrict__ alpha,
                  const __nv_bfloat16* __restrict__ bias, int epi_op, int k_tiles, int kq_dim, int tiles_m,
-                 int tiles_n, const __grid_constant__ GatherMaps<kGather> peers, const PairGroupArgs ga,
+                 int tiles_n, int prefetch_weight, const __grid_constant__ GatherMaps<kGather> peers, const PairGroupArgs ga,
                  const PairSitu<kSitu> situ) {
     using C = Cfg2<BN, KIND>;
     using Iter = PairWorkIter<BN, kGrouped>;
@@ -1299,7 +1301,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // as in the single-CTA kernel (256 x 7168 x 2048 behind its quantizer 11.8 -> 11.3 us, more rows
     // of tiles: no change); this CTA's half of the columns
     if constexpr (!kGrouped) {
-        if (threadIdx.x == 64 && cluster_id < tiles_m * tiles_n) {
+        if (threadIdx.x == 64 && prefetch_weight != 0 && cluster_id < tiles_m * tiles_n) {
             const TileCoord tc = tile_coord(cluster_id, tiles_m, tiles_n);
             const int end = min(k_tiles, 2560 / BN);
             for (int kt = (tc.m & 7); kt < end; kt += min(8, tiles_m)) {
@@ -1903,7 +1905,7 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
             HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND, true>, dim3(2 * tiles_n), dim3(kThreads), size_t(C::kSmemBytes),
                                g.stream, g.pdl, 2, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out,
                                g.ldo, g.m, g.n, k_tiles, g.kq_dim, tiles_m, tiles_n, a_rows,
-                               g.direct_store ? 1 : 0, issuers_in_order(), g.grp, g.situ));
+                               g.direct_store ? 1 : 0, issuers_in_order(), g.pdl ? 1 : 0, g.grp, g.situ));
             return HQ_OK;
         }
     }
@@ -1924,13 +1926,13 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
             HQ_CUDA_TRY(opt_in_dense.ensure(gemm_kernel<BN, KIND, false, true>, C::kSmemBytes));
             HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND, false, true>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
                                g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
-                               g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.grp, g.situ));
+                               g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.pdl ? 1 : 0, g.grp, g.situ));
             return HQ_OK;
         }
     }
     HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
                        g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
-                       g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.grp, g.situ));
+                       g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.pdl ? 1 : 0, g.grp, g.situ));
     return HQ_OK;
 }
 
@@ -2013,7 +2015,7 @@ int launch_pair(const GemmArgs& g, char* err, size_t errlen, __nv_bfloat16* cons
     if constexpr (kSitu) situ.p = g.situ;
     HQ_CUDA_TRY(launch(gemm_pair_kernel<BN, KIND, kGather, kGrouped, kSitu>, dim3(2 * clusters), dim3(C::kThreads),
                        size_t(C::kSmemBytes), g.stream, g.pdl, 2, tm_a, tm_b, tm_d, tm_sfa, tm_sfb, g.alpha, g.bias,
-                       g.epi_op, k_tiles, g.kq_dim, tiles_m, tiles_n, peers, ga, situ));
+                       g.epi_op, k_tiles, g.kq_dim, tiles_m, tiles_n, g.pdl ? 1 : 0, peers, ga, situ));
     return HQ_OK;
 }
 
@@ -2418,9 +2420,11 @@ extern "C" int hq_describe_tile(int64_t m, int64_t n, int64_t k, int mode, int s
         const hq::DecPlan plan = hq::decode_plan(m, n, k, sm > 0 ? sm : 148);
         if (buf != nullptr && buflen > 0) {
             snprintf(buf, buflen,
-                     "[gemm] mode=dense kind=%s m=%lld n=%lld k=%lld sm=%d -> swap 128x%d/256 pair=0 splitk=%d ctas=%d cluster=%d",
+                     "[gemm] mode=dense kind=%s m=%lld n=%lld k=%lld sm=%d -> swap 128x%d/256 pair=0 splitk=%d ctas=%d cluster=%d "
+                     "prefetch=%d",
                      hq::mode_name(mode), (long long)m, (long long)n, (long long)k, sm, hq::decode_width(m),
-                     plan.aligned ? 0 : 1, plan.ctas, plan.cluster > 1 ? plan.cluster : 1);
+                     plan.aligned ? 0 : 1, plan.ctas, plan.cluster > 1 ? plan.cluster : 1,
+                     hq::dec_prefetch_steps(plan, hq::kDecRows * hq::kDecStepBytes));
         }
         return HQ_OK;
     }

@@ -331,6 +331,17 @@ def test_decode_unit_deal_is_consistent(native):
         _native.call("hq_selftest_decode_plan", 128, 100, 148, 0)
 
 
+def test_weight_prefetch_of_the_small_m_kernel_is_bounded(native):
+    """24 MB over the grid, and at most one tile's steps of 32 KB (or 8) from the one thread of a CTA that asks for them."""
+    import halops_b200 as hq
+
+    for m, n, k in ((8, 24576, 1536), (16, 7168, 2048), (33, 23552, 7808), (1, 64, 128), (64, 64, 8192)):
+        for sm in (1, 4, 16, 64, 148):
+            line = hq.describe_tile(m, n, k, sm_count=sm)
+            steps, ctas = (int(re.search(rf"{name}=(\d+)", line).group(1)) for name in ("prefetch", "ctas"))
+            assert 1 <= steps <= max(8, -(-k // 256)) and (steps == 1 or steps * ctas <= 24 * 32), line
+
+
 def test_describe_tile(native):
     import halops_b200 as hq
 
