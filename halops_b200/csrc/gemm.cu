@@ -2311,7 +2311,7 @@ struct TilePick {
 // gives every SM (or SM pair) a tile; failing that, the narrowest single-CTA
 // tile that divides N (most CTAs streaming the weight).  HALOPS_B200_TILE
 // (pair256 | pair128 | 256 | 128 | 64) overrides the choice when it is legal.
-TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int64_t runs = 1) {
+TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int64_t boundaries = 0) {
     // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
     const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
     if (m < 1 || n < 1 || k < 1) return {0, false};
@@ -2368,15 +2368,18 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
     for (int i = 0; i < count; ++i) {
         const Cand& c = cands[i];
         if (n % c.bn != 0 || (c.bn == 64 && !fp8) || (c.pair && (m <= kBM || !fp8))) continue;
-        // contiguous experts (`runs` of rows that start on multiples of 64): a tile with a boundary inside is
-        // worked once more, as half of the boundaries are in a 128-row tile and three of four in a 256-row one
-        // (16 experts on 4096 rows, N = 4096, K = 2048: 76 us on the pair tile, 60 on the 128-wide one;
-        // 14 on 2816 rows, w4a8, N = 4352, K = 1280: 40 -> 34)
-        const int64_t extra = c.pair ? (runs - 1) * 3 / 4 : (runs - 1) / 2;
-        const int64_t tiles = ((c.pair ? tiles_m2 : tiles_m) + extra) * (n / c.bn);
+        const int64_t rows = c.pair ? tiles_m2 : tiles_m;
+        const int64_t tiles = rows * (n / c.bn);
         const int64_t units = c.pair ? sm_count / 2 : sm_count;
         if (units < 1) continue;
-        const double waves = double((tiles + units - 1) / units);
+        // Contiguous experts (runs of rows that start on multiples of 64): a CTA works a tile with a boundary inside
+        // once per run, one after the other.  Half of the boundaries are inside a 128-row tile, which has room
+        // for one, three of four inside a 256-row one, which has room for three.  On 80 problems (512 to 16384 rows, 8 to
+        // 256 experts, MXFP8 and NVFP4) choosing by this costs 0.65 % (MXFP8) and 0.3 % (NVFP4) over the best tile of each,
+        // without a term for the boundaries 3.6 % and 0.9 %, counting them as tiles of their own, which other CTAs
+        // could take, 9.1 % and 6.0 % (16 experts on 512 rows, N = K = 2048: 16.3 us; now 10.8).
+        const double passes = 1.0 + std::min(c.pair ? 3.0 : 1.0, double(boundaries) * (c.pair ? 0.75 : 0.5) / double(rows));
+        const double waves = double((tiles + units - 1) / units) * passes;
         const double cost = c.us_fixed + waves * (k_tiles * c.us_per_ktile + c.us_per_wave);
         if (best.bn == 0 || cost < best_cost * 0.999) {
             best = {c.bn, c.pair};
@@ -2665,7 +2668,9 @@ TilePick pick_tile_grouped(int kind, int64_t count, int64_t rows, int64_t total_
     if (kind == kGroupMasked && rows % 64 != 0) return {0, false};
     if (kind == kGroupContiguous && total_m % 64 != 0) return {0, false};
     const int64_t pad = kind != kGroupContiguous && rows % kBM != 0 ? (count - 1) * kBM : 0;
-    TilePick pick = pick_tile(total_m + pad, n, k, mode, sm_count, kind == kGroupContiguous ? count : 1);
+    // boundaries between the experts' runs: as many as there are experts, or as the rows have room for
+    const int64_t boundaries = kind == kGroupContiguous ? std::min(count, total_m / 64) - 1 : 0;
+    TilePick pick = pick_tile(total_m + pad, n, k, mode, sm_count, boundaries);
     // The 2-CTA tile: MXFP8 (or e4m3 x MXFP4) with a plain epilogue, and no 256-row tile may hold rows of two
     // batches or expert slots (the contiguous layout is worked per run of experts, see
     // PairWorkIter).  Otherwise a forced or modelled pair choice falls back to the same width.
