@@ -519,3 +519,50 @@ def test_situ_quant_on_the_2cta_tile(hq, monkeypatch, m, n, k, linear_beta):
         assert hq.device_status() == 0
         results.append((out.view(torch.uint8), sf))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("mode,m,n,k,tile", [("w8a8-mxfp8", 512, 1536, 1024, "pair256"), ("w8a8-mxfp8", 300, 1536, 1024, "pair128"),
+                                             ("w8a8-mxfp8", 300, 1536, 1024, "256"), ("w8a8-mxfp8", 300, 1536, 1024, "128"),
+                                             ("w4a4-nvfp4", 300, 1536, 1024, "256"), ("w4a4-mxfp4", 130, 256, 512, "128"),
+                                             ("situ", 512, 1536, 1024, "pair256"), ("w8a8-mxfp8", 40, 512, 2048, "64")],
+                         ids=lambda v: str(v))
+def test_weight_rewritten_by_the_preceding_kernel_on_every_tile(hq, monkeypatch, mode, m, n, k, tile):
+    """With a programmatic launch every dense kernel asks for its weight in L2 before it waits for the preceding
+    kernel.  Only a hint: a weight that the preceding quantizer rewrites is used in its new form, bit for
+    bit what a launch after a synchronise gives.  (The last case is the split of K over two CTAs.)"""
+    monkeypatch.setenv("HALOPS_B200_TILE", tile)
+    situ = mode == "situ"
+    mode = "w8a8-mxfp8" if situ else mode
+    described = hq.describe_tile(m, n, k, mode)
+    assert f"x{tile.replace('pair', '')}/" in described and f"pair={int('pair' in tile)}" in described
+    assert "splitk=1" in described if tile == "64" else "splitk=0" in described
+    g = torch.Generator().manual_seed(n + k)
+    a, sfa = hq.group_wise_quant(torch.randn([m, k], generator=g).to(torch.bfloat16).cuda(), mode)
+    weights = [(torch.randn([n, k], generator=g) * 0.05).to(torch.bfloat16).cuda() for _ in range(2)]
+    alpha = torch.full([1], 0.5, device="cuda") if mode == "w4a4-nvfp4" else None
+
+    def gemm(w, sfb):
+        if not situ:
+            out = torch.empty([m, n], dtype=torch.bfloat16, device="cuda")
+            hq.dense_gemm(a, w, sfa, sfb, out, alpha=alpha, mode=mode, use_pdl=True)
+            return (out,)
+        out = torch.empty([m, n // 2], dtype=torch.float8_e4m3fn, device="cuda")
+        sf = torch.empty([(m + 127) // 128 * 128, n // 64], dtype=torch.uint8, device="cuda")
+        hq.dense_gemm(a, w, sfa, sfb, out, epilogue=hq.EpilogueOp.SituQuant, output_sf=sf, use_pdl=True)
+        return out.view(torch.uint8), sf
+
+    expected = []
+    for weight in weights:
+        w, sfb = hq.group_wise_quant(weight, mode)
+        torch.cuda.synchronize()
+        expected.append(gemm(w, sfb))
+        torch.cuda.synchronize()
+    assert not torch.equal(expected[0][0], expected[1][0])
+    got = []
+    for i in range(8):
+        hq.group_wise_quant(weights[i & 1], mode, True, True, w, sfb)
+        got.append(gemm(w, sfb))
+    torch.cuda.synchronize()
+    assert hq.device_status() == 0
+    for i, outs in enumerate(got):
+        assert all(torch.equal(x, y) for x, y in zip(outs, expected[i & 1])), f"call {i} used stale weight bytes"

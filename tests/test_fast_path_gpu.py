@@ -180,3 +180,82 @@ def test_two_threads(hq, native):
     assert hq.device_status() == 0
     for want, outs in zip(expected, results):
         assert outs is not None and all(torch.equal(want, out) for out in outs)
+
+
+class Recorder:
+    """The native front, noting whether it took each call."""
+
+    def __init__(self, front):
+        self.front, self.took = front, []
+
+    def __getattr__(self, name):
+        def call(*args):
+            result = getattr(self.front, name)(*args)
+            self.took.append(result is not None)
+            return result
+        return call
+
+
+def _both_ways(native, monkeypatch, calls):
+    """The results of ``calls`` through the native front, which must take every call, and through the wrappers."""
+    recorder = Recorder(native.load_fast_path())
+    results = []
+    for front in (recorder, native._NoFastPath):
+        monkeypatch.setattr(native, "fast_path", front)
+        results.append([t.view(torch.uint8) for call in calls for t in call()])
+        torch.cuda.synchronize()
+    assert recorder.took and all(recorder.took), recorder.took
+    for x, y in zip(*results):
+        assert x.shape == y.shape and torch.equal(x, y)
+
+
+def test_dense_options_both_ways(hq, native, monkeypatch):
+    m, n, k = 256, 512, 384
+    g = torch.Generator().manual_seed(21)
+    wide = torch.randn([m, k + 128], generator=g).to(torch.bfloat16).cuda()
+    a, sfa = hq.group_wise_quant(wide[:, :k].contiguous())
+    b, sfb = hq.group_wise_quant((torch.randn([n, k], generator=g) * 0.1).to(torch.bfloat16).cuda())
+    bias = torch.randn([n], generator=g).to(torch.bfloat16).cuda()
+
+    def dense(**kw):
+        out = torch.zeros([m, n + 64], dtype=torch.bfloat16, device="cuda")
+        hq.dense_gemm(a, b, sfa, sfb, out[:, :n], **kw)  # (rows of the output are strided)
+        return [out]
+
+    def situ(**kw):
+        out = torch.zeros([m, n // 2], dtype=torch.float8_e4m3fn, device="cuda")
+        sf = torch.zeros([m, n // 64], dtype=torch.uint8, device="cuda")
+        hq.dense_gemm(a, b, sfa, sfb, out, epilogue=hq.EpilogueOp.SituQuant, output_sf=sf, **kw)
+        return [out, sf]
+
+    _both_ways(native, monkeypatch, [
+        lambda: hq.group_wise_quant(wide[:, :k]), lambda: hq.group_wise_quant(wide[:, :k], use_swizzle=False, use_pdl=False),
+        lambda: hq.rms_norm_quant(wide[:, :k], bias[:k]),
+        lambda: dense(), lambda: dense(bias=bias), lambda: dense(epilogue=hq.EpilogueOp.Sigmoid, sm_count=64), lambda: dense(use_pdl=2),
+        lambda: situ(), lambda: situ(bias=bias, situ_linear_beta=None), lambda: situ(situ_beta=2, use_pdl=False)])
+
+
+@pytest.mark.parametrize("mode", MODES + ("w4a8-mxfp4",))
+def test_grouped_options_both_ways(hq, native, monkeypatch, mode):
+    e, rows, n, k = 3, 128, 256, 512
+    g = torch.Generator().manual_seed(22)
+    act, wgt = ("w8a8-mxfp8", "w4a4-mxfp4") if mode == "w4a8-mxfp4" else (mode, mode)
+    x, sfa = hq.group_wise_quant(torch.randn([e * rows, k], generator=g).to(torch.bfloat16).cuda(), act)
+    w, sfb = hq.group_wise_quant((torch.randn([e * n, k], generator=g) * 0.1).to(torch.bfloat16).cuda(), wgt)
+    w, sfb = w.view(e, n, -1), sfb.view(e, n, -1)
+    alpha = torch.tensor([0.5, 1.0, 2.0], device="cuda") if mode == "w4a4-nvfp4" else None
+    biases = [None] + ([torch.randn([e, n], generator=g).to(torch.bfloat16).cuda()] if mode == "w8a8-mxfp8" else [])
+    counts = torch.tensor([5, 0, 128], dtype=torch.int32, device="cuda")
+    ids = torch.tensor([0] * 64 + [1] * 192 + [2] * 128, dtype=torch.int32, device="cuda")
+
+    def masked(bias):
+        out = torch.zeros([e * rows, n + 8], dtype=torch.bfloat16, device="cuda")
+        hq.group_masked_gemm(x, w, sfa, sfb, counts, out[:, :n], bias, alpha, rows, mode=mode)
+        return [out]
+
+    def contiguous(bias):
+        out = torch.zeros([e * rows, n], dtype=torch.bfloat16, device="cuda")
+        hq.group_contiguous_gemm(x, w, sfa, sfb, ids, out, bias, alpha, mode=mode)
+        return [out]
+
+    _both_ways(native, monkeypatch, [lambda f=f, b=b: f(b) for f in (masked, contiguous) for b in biases])

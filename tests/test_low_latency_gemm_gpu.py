@@ -239,3 +239,44 @@ def test_dual_output_with_an_empty_weight(hq):
             call(*args)
     torch.cuda.synchronize()
     assert torch.equal(out2, expected) and bool((out == 7.0).all())
+
+
+@pytest.mark.parametrize("form", ["plain", "concat", "dual"])
+def test_weight_rewritten_by_the_preceding_kernel(hq, form):
+    """The kernel asks for its weights in L2 before it waits for the preceding kernel, here the quantizer that
+    rewrites them (the second one of the fused forms last): the new values are used, bit for bit."""
+    m, n, k = 7, 1032, 1024
+    g = torch.Generator().manual_seed(12)
+
+    def quant(rows, scale):
+        return hq.group_wise_quant((torch.randn([rows, k], generator=g) * scale).to(torch.bfloat16).cuda(), use_swizzle=False)
+
+    x, x2 = quant(m, 1.0), quant(m, 1.0)
+    values = [[(torch.randn([n, k], generator=g) * 0.02).to(torch.bfloat16).cuda() for _ in range(2)] for _ in range(2)]
+
+    def gemm(w, w2):
+        out = torch.empty([m, n], dtype=torch.bfloat16, device="cuda")
+        out2 = torch.empty_like(out) if form == "dual" else None
+        kw = {}
+        if form != "plain":
+            kw = dict(weight2=w2[0], sfb2=w2[1])
+            kw.update(dict(input2=x2[0], sfa2=x2[1]) if form == "concat" else dict(output2=out2))
+        hq.low_latency_mma_gemm(x[0], w[0], x[1], w[1], out, **kw)
+        return [out] if out2 is None else [out, out2]
+
+    expected = []
+    for pair in values:
+        w, w2 = (hq.group_wise_quant(v, use_swizzle=False) for v in pair)
+        torch.cuda.synchronize()
+        expected.append(gemm(w, w2))
+        torch.cuda.synchronize()
+    assert not any(torch.equal(a, b) for a, b in zip(*expected))
+    got = []
+    for i in range(8):
+        for buffers, v in zip((w, w2) if form != "plain" else (w2, w), values[i & 1] if form != "plain" else values[i & 1][::-1]):
+            hq.group_wise_quant(v, "w8a8-mxfp8", False, True, *buffers)
+        got.append(gemm(w, w2))
+    torch.cuda.synchronize()
+    assert hq.device_status() == 0
+    for i, outs in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(outs, expected[i & 1])), f"call {i} used stale weight bytes"
