@@ -473,7 +473,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     // Two MMA issuers with an accumulator each (64-wide dense tiles, plain epilogues): the k-tiles
     // of a tile are summed as (even ones) + (odd ones), deterministically, but not in the k order
     // of the other tiles.
-    const bool dual = BN == 64 && !kSplitK && dual_issue == 1;
+    const bool dual = BN == 64 && kDense && !kSplitK && dual_issue == 1;
     // dual_issue == 2: two issuers as well, but into ONE accumulator and in k order, as in the
     // 2-CTA kernel: the threads take alternate k-iterations and hand each other the turn (tcgen05
     // fences around an mbarrier arrival), so the MMAs reach the tensor core in the order one thread
@@ -834,7 +834,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     ptx::tc_load_32x32(acc + c * kEpiChunk, r);
                     ptx::tc_wait_ld();
                 }
-                if constexpr (BN == 64 && !kSplitK) {
+                if constexpr (BN == 64 && kDense && !kSplitK) {
                     // the second issuer's accumulator (it has k-tiles whenever the tile has two or more)
                     if (dual && k_end - k_begin > 1) {
                         uint32_t r2[32];
@@ -2389,6 +2389,21 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
     return best;
 }
 
+template <int KIND>
+int launch_single(const TilePick& pick, const GemmArgs& g, char* err, size_t errlen) {
+    if (pick.bn == 256) return launch_tile<256, KIND>(g, err, errlen);
+    if (pick.bn == 128) return launch_tile<128, KIND>(g, err, errlen);
+    if constexpr (KIND == 0 || KIND == 3) return launch_tile<64, KIND>(g, err, errlen);
+    // (the packed modes have no 64-wide tile: their problems need N % 128 == 0)
+    return fail(err, errlen, HQ_ERR_INVALID, "no %d-wide tile for this mode", pick.bn);
+}
+
+template <int KIND>
+int launch_dense(const TilePick& pick, const GemmArgs& g, char* err, size_t errlen) {
+    if (!pick.pair) return launch_single<KIND>(pick, g, err, errlen);
+    return pick.bn == 256 ? launch_pair<256, KIND>(g, err, errlen) : launch_pair<128, KIND>(g, err, errlen);
+}
+
 std::mutex g_sm_mutex;
 int g_sm_cache[64];
 
@@ -2579,27 +2594,9 @@ int dense_gemm_impl(const void* a, const void* b, const void* sfa, const void* s
     }
 
     if (is_situ && pick.pair) return hq::launch_pair<256, 0, false, false, true>(g, err, errlen);
-#define HQ_DISPATCH(KIND)                                                            \
-    if (pick.pair) {                                                                 \
-        return pick.bn == 256 ? hq::launch_pair<256, KIND>(g, err, errlen)           \
-                              : hq::launch_pair<128, KIND>(g, err, errlen);          \
-    }                                                                                \
-    switch (pick.bn) {                                                               \
-        case 256:                                                                    \
-            return hq::launch_tile<256, KIND>(g, err, errlen);                       \
-        case 128:                                                                    \
-            return hq::launch_tile<128, KIND>(g, err, errlen);                       \
-        default:                                                                     \
-            return hq::launch_tile<64, KIND>(g, err, errlen);                        \
-    }
-    if (mode == HQ_MODE_W8A8_MXFP8) {
-        HQ_DISPATCH(0)
-    } else if (mode == HQ_MODE_W4A4_NVFP4) {
-        HQ_DISPATCH(1)
-    } else {
-        HQ_DISPATCH(2)
-    }
-#undef HQ_DISPATCH
+    if (mode == HQ_MODE_W8A8_MXFP8) return hq::launch_dense<0>(pick, g, err, errlen);
+    if (mode == HQ_MODE_W4A4_NVFP4) return hq::launch_dense<1>(pick, g, err, errlen);
+    return hq::launch_dense<2>(pick, g, err, errlen);
 }
 
 }  // namespace
@@ -2795,15 +2792,6 @@ int grouped_gemm_impl(int kind, const void* a, const void* b, const void* sfa, c
     g.pdl = use_pdl != 0;
     g.direct_store = false;
     g.stream = static_cast<cudaStream_t>(stream);
-#define HQ_DISPATCH(KIND)                                      \
-    switch (pick.bn) {                                         \
-        case 256:                                              \
-            return launch_tile<256, KIND>(g, err, errlen);     \
-        case 128:                                              \
-            return launch_tile<128, KIND>(g, err, errlen);     \
-        default:                                               \
-            return launch_tile<64, KIND>(g, err, errlen);      \
-    }
     if (pick.pair && w4a8) {
         return pick.bn == 256 ? launch_pair<256, 3, false, true>(g, err, errlen)
                               : launch_pair<128, 3, false, true>(g, err, errlen);
@@ -2812,16 +2800,10 @@ int grouped_gemm_impl(int kind, const void* a, const void* b, const void* sfa, c
         return pick.bn == 256 ? launch_pair<256, 0, false, true>(g, err, errlen)
                               : launch_pair<128, 0, false, true>(g, err, errlen);
     }
-    if (mode == HQ_MODE_W8A8_MXFP8) {
-        HQ_DISPATCH(0)
-    } else if (w4a8) {
-        HQ_DISPATCH(3)
-    } else if (mode == HQ_MODE_W4A4_NVFP4) {
-        HQ_DISPATCH(1)
-    } else {
-        HQ_DISPATCH(2)
-    }
-#undef HQ_DISPATCH
+    if (mode == HQ_MODE_W8A8_MXFP8) return launch_single<0>(pick, g, err, errlen);
+    if (w4a8) return launch_single<3>(pick, g, err, errlen);
+    if (mode == HQ_MODE_W4A4_NVFP4) return launch_single<1>(pick, g, err, errlen);
+    return launch_single<2>(pick, g, err, errlen);
 }
 
 }  // namespace
