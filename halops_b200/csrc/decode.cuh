@@ -20,8 +20,8 @@
 //     near what L2 delivers to one SM.  8 x 7168 x 2048 behind its quantizer: 10.0 -> 9.0 us.
 //   * Before it waits for the preceding kernel of the stream a CTA asks for the start of its weight
 //     to be brought into L2 (see DecParams::prefetch_steps): 9.0 -> 8.4 us.
-//   * Two threads issue the MMAs of alternate k-steps into accumulators of their own, so
-//     they need no hand-over; the epilogue adds the two accumulators.  (One thread
+//   * Two warps issue the MMAs of alternate k-steps (one elected lane of each) into accumulators of their
+//     own, so they need no hand-over; the epilogue adds the two accumulators.  (One thread
 //     alone, issuing inside `if (lane == 0)`, needed about 1000 cycles per 32 KB step.)
 //   * Work is cut into units of (128 weight rows) x (256 bytes of K).  Normally a CTA works
 //     whole tiles.  When there are too few tiles to keep HBM busy, the units are dealt out
@@ -67,7 +67,7 @@ struct DecCfg {
     // Tensor memory: kAccStages accumulator stages of kDecIssuers x NACT fp32 columns (one
     // stage for the widest activations: two would not fit beside the scales), then kSfSets
     // sets of 16 scale columns (weights: 2 atoms x 4 columns, activations: 2 x 4).  A set is
-    // reused once the MMAs that read it have released their stage, which the copy thread can
+    // reused once the MMAs that read it have released their stage, which the scale warps can
     // only tell apart from a later release of the same stage when there are no more sets than
     // stages.
     static constexpr int kAccStages = NACT == 128 ? 1 : 2;
@@ -553,7 +553,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     } else if (warp == 1 || warp == 10) {
         // ------------------------------------------------------------ MMA issuers
         // Issuer `me` takes the k-steps of a piece whose index inside the piece is me modulo
-        // kDecIssuers and accumulates them in its own columns; nothing orders the two threads.
+        // kDecIssuers and accumulates them in its own columns; nothing orders the two.
         // (the whole warp walks, one lane issues: see ptx::elect_one)
         {
             const int me = warp == 1 ? 0 : 1;
@@ -575,7 +575,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 for (int ks = sg.k0; ks < sg.k1; ++ks, ++it) {
                     if (((ks - sg.k0) & (kDecIssuers - 1)) != me) continue;
                     const uint32_t s = it % C::kStages;
-                    // scales in tensor memory (the copy thread waited for the stage before it
+                    // scales in tensor memory (the scale warps waited for the stage before they
                     // copied); the stage's own barrier orders this thread after the TMA writes
                     ok = wait_bars(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, true,
                                    ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusMma);
@@ -874,10 +874,13 @@ inline DecPlan dec_plan(int n, int64_t k_bytes, int sm_count, bool allow_split, 
         sc = s > 8 ? 8 : s;
         while (sc > 1 && (int64_t(sc - 1) * nact * kDecRows * 4 > ring_bytes || p.tiles > clusters->max_active[sc])) sc /= 2;
     }
-    // Measured on B200: a CTA streams one 32 KB step per 0.42 us at most (what its shared memory
-    // holds in flight per memory round trip); the exchange through a cluster costs 2 us plus
-    // 0.3 us per CTA of the cluster, through the scratch buffer 5.5 us (fences, an atomic and
-    // the loads of the last CTA to arrive), both plus the partial tiles' own bytes.
+    // The figures are those of an earlier form of the kernel, both sides of the comparison: a 32 KB step took a CTA
+    // 0.42 us (now 0.26 with the weight in L2); the exchange through a cluster 2 us plus 0.3 us per CTA of the
+    // cluster, through the scratch buffer 5.5 us (fences, an atomic and the loads of the last CTA to
+    // arrive), both plus the partial tiles' own bytes.  On the kernel as it is the choice costs 0.5 % on average,
+    // 6.6 % at most, over the best of the three deals on 84 problems (8 to 64 rows, N = 1024..12288, K = 1024..7168):
+    // 8 x 1024 x 7168 behind its quantizer whole 11.9, cluster (taken) 8.3 us, scratch 13.9; 64 x 6144 x 7168 whole
+    // (taken) 16.4, cluster 15.4.
     const double step_us = 0.42, hbm_bytes_per_us = 6.0e6;
     const double bytes = double(p.tiles) * kDecRows * double(k_bytes);
     const double hbm_us = bytes / hbm_bytes_per_us;

@@ -1298,8 +1298,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
 
-    // as in the single-CTA kernel (256 x 7168 x 2048 behind its quantizer 11.8 -> 11.3 us, more rows
-    // of tiles: no change); this CTA's half of the columns
+    // as in the single-CTA kernel (300 x 8192 x 8192 behind its quantizer 33.1 -> 32.7 us, 512 x 14336 x 4096
+    // 32.3 -> 32.2, four rows of tiles and more: no change); this CTA's half of the columns
     if constexpr (!kGrouped) {
         if (threadIdx.x == 64 && prefetch_weight != 0 && cluster_id < tiles_m * tiles_n) {
             const TileCoord tc = tile_coord(cluster_id, tiles_m, tiles_n);
@@ -2046,8 +2046,9 @@ bool decode_eligible(int64_t m, int64_t n, int64_t k, int mode, int epi_op, bool
     if (forced != nullptr && forced[0] != '\0') return false;
     if ((n / 128 + 1) * (k / 256 + 1) >= (int64_t(1) << 31)) return false;
     // Up to 64 activation rows by default.  With 65 to 128 a stage is half activations, the
-    // weight in flight per CTA halves, and the 128 x 64 tile is faster (18.8 against 16.9 us on
-    // 128 x 8192 x 4096); HALOPS_B200_DECODE=wide sends them here all the same.
+    // weight in flight per CTA halves, and the best 128-row tile was faster on each of 33 problems (128 x 8192 x 4096
+    // behind its quantizer 15.5 against 12.8 us on the 128 x 64 tile, 96 x 24576 x 1536 14.9 against 12.5 on the
+    // 128 x 128 one); HALOPS_B200_DECODE=wide sends them here all the same.
     const DecodeSwitches sw = decode_switches();
     const int64_t m_max = sw.wide ? 128 : 64;
     return mode == HQ_MODE_W8A8_MXFP8 && m >= 1 && m <= m_max && n % 64 == 0 && k % 128 == 0 && !has_bias &&
@@ -2307,10 +2308,9 @@ struct TilePick {
 // Shape legality follows the reference's "some compiled tile fits" rule
 // (csrc/kernel/gemm/gemm_dispatch.cuh:65-100 over the tiles of gemm_tile.cuh:371-395):
 // MXFP8 needs K % 128 == 0 and N % 64 == 0, the FP4 modes K % 256 == 0 and
-// N % 128 == 0; any M >= 1.  Among the legal tiles: the largest that still
-// gives every SM (or SM pair) a tile; failing that, the narrowest single-CTA
-// tile that divides N (most CTAs streaming the weight).  HALOPS_B200_TILE
-// (pair256 | pair128 | 256 | 128 | 64) overrides the choice when it is legal.
+// N % 128 == 0; any M >= 1.  Among the legal tiles: the one that the figures
+// below make cheapest.  HALOPS_B200_TILE (pair256 | pair128 | 256 | 128 | 64)
+// overrides the choice when it is legal.
 TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int64_t boundaries = 0) {
     // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
     const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
@@ -2343,13 +2343,14 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
         return {best, false};
     }
     // Several rows of tiles: a launch costs a fixed time plus, per wave of tiles, the k-tiles and a share
-    // for fill, drain and the hand-over.  Fitted (relative least squares) to 52 MXFP8 and 48 FP4 problems on B200,
-    // spread over M = 129..8192, N = 256..14336, K = 512..8192, each timed on every tile that is legal
-    // for it; residuals 3-7 %.  Choosing by it costs 0.6 % (MXFP8) and 0.1 % (FP4) over
-    // the best tile of each problem, the earlier figures (made when one thread issued all MMAs at 100 cycles
-    // each, which charged the narrow tiles most) 7 % and 2.5 %: 3139 x 1792 x 2048 behind a norm
-    // 24.4 -> 21.8 us, 937 x 4736 x 5760 36.9 -> 31.7, 256 x 7168 x 2048 behind its quantizer 11.4 -> 10.2.  The FP4 kinds stay on single-CTA tiles: the pair tile's tcgen05.cp
-    // scale copies, 12 per k-tile, are slower than its MMAs (4096 x 14336 x 4096 NVFP4 147 against 138 us).
+    // for fill, drain and the hand-over.  Fitted (relative least squares) to 51 MXFP8 and 48 FP4 problems on B200,
+    // spread over M = 129..8192, N = 256..14336, K = 512..8192, each
+    // timed on every tile that is legal for it; residuals 3-7 %.  Choosing by it costs 0.6 % (MXFP8) and
+    // 0.1 % (FP4) over the best tile of each problem, the earlier figures (made when one thread issued all MMAs
+    // at 100 cycles each, which charged the narrow tiles most) 7 % and 2.5 %: 3139 x 1792 x 2048 behind a
+    // norm 24.4 -> 21.8 us, 937 x 4736 x 5760 36.9 -> 31.7, 256 x 7168 x 2048 behind its quantizer 11.4 -> 10.2.
+    // The FP4 kinds stay on single-CTA tiles: the pair tile's tcgen05.cp scale copies, 12 per k-tile, are slower
+    // than its MMAs (4096 x 14336 x 4096 NVFP4 147 against 138 us).
     struct Cand {
         int bn;
         bool pair;
@@ -2374,9 +2375,9 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
         if (units < 1) continue;
         // Contiguous experts (runs of rows that start on multiples of 64): a CTA works a tile with a boundary inside
         // once per run, one after the other.  Half of the boundaries are inside a 128-row tile, which has room
-        // for one, three of four inside a 256-row one, which has room for three.  On 80 problems (512 to 16384 rows, 8 to
-        // 256 experts, MXFP8 and NVFP4) choosing by this costs 0.65 % (MXFP8) and 0.3 % (NVFP4) over the best tile of each,
-        // without a term for the boundaries 3.6 % and 0.9 %, counting them as tiles of their own, which other CTAs
+        // for one, three of four inside a 256-row one, which has room for three.  On 80 problems (512 to 16384
+        // rows, 8 to 256 experts, MXFP8 and NVFP4) choosing by this costs 0.65 % (MXFP8) and 0.3 % (NVFP4) over
+        // the best tile of each, without a term for the boundaries 3.6 % and 0.9 %, counting them as tiles of their own, which other CTAs
         // could take, 9.1 % and 6.0 % (16 experts on 512 rows, N = K = 2048: 16.3 us; now 10.8).
         const double passes = 1.0 + std::min(c.pair ? 3.0 : 1.0, double(boundaries) * (c.pair ? 0.75 : 0.5) / double(rows));
         const double waves = double((tiles + units - 1) / units) * passes;
