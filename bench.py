@@ -47,8 +47,8 @@ WORKLOAD = (f"C5 N-sharded MXFP8 dense GEMM M={M5} N={N5} K={K5}, weight rows sp
 # on 16384 x 7168 x 8192 (ncu, one launch); a rank's launch covers N5 / world / 7168 such
 # column blocks, whose tiles are walked one block of 8 row tiles x all columns at a time,
 # so the traffic grows in proportion
-TRAFFIC_PER_7168_COLUMNS = 897.6e6
-TRAFFIC_SOURCE = ("ncu capture of one launch of this kernel on 16384 x 7168 x 8192 (677.5 MB read + 220.1 MB "
+TRAFFIC_PER_7168_COLUMNS = 864.5e6
+TRAFFIC_SOURCE = ("ncu capture of one launch of this kernel on 16384 x 7168 x 8192 (645.7 MB read + 218.8 MB "
                   "written), times the number of 7168-column blocks of the rank's shard")
 
 

@@ -2329,6 +2329,9 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
         // One row of tiles: the weight streams through once, so what counts is the
         // largest share of weight rows any CTA has to stream (tiles per CTA x width,
         // plus a fixed cost per tile of about 16 rows' worth); ties go to the wider tile.
+        // (From before the uniform issue, which sped the wider tiles up most: of 33 problems of 65 to 128 rows the choice is
+        // within 5 % of the best on 25, and takes 9.3 instead of 6.4 us on 96 x 4096 x 1024, 10.8 instead of 9.9 on
+        // 96 x 1024 x 4096, where the 64-wide tile with K split over two CTAs loses to the 128-wide one.)
         int best = 0;
         int64_t best_cost = 0;
         for (int w : {256, 128, 64}) {
