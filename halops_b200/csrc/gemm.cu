@@ -707,24 +707,44 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 // the MMAs of k-tile it - kSfSets read this set: they are done once they
                 // have released their stage
                 const uint32_t prev = it - uint32_t(C::kSfSets);
-                ok = wait_bars(ptx::smem_u32(&bars->sf_full[s]), (it / kRing) & 1u, it >= uint32_t(C::kSfSets),
-                               ptx::smem_u32(&bars->empty[prev % kRing]), (prev / kRing) & 1u, abort, kStatusProducer);
-                if (!ok) break;
-                ptx::tc_fence_after();
-                const uint32_t set = tmem + (quarter << 16) + (it % C::kSfSets) * C::kSfCols;
-                const uint32_t src_a = sfa_base + s * C::kSfaBytes + uint32_t(lane) * 16u;
-                const uint32_t src_b = sfb_base + s * C::kSfbBytes + uint32_t(lane) * 16u;
+                const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
+                const uint32_t set_free = ptx::smem_u32(&bars->empty[prev % kRing]);
+                // A k-tile's scales go to registers first, in the order of the set's columns (SFA by atom along
+                // K, then SFB by atom along K and 128 columns), and on with as few stores as there are.  Where only
+                // two sets rotate and a set is large, the loads do not wait for it: what lies between its release and
+                // the MMAs that wait for its next scales is on the critical path there, and it was 12 loads and 12
+                // stores one after the other, some 700 cycles against 512 of one k-tile's MMAs (NVFP4 512 x 4096 x 4096 on the
+                // 128 x 256 tile 10.9 -> 9.9 us, 4096 x 14336 x 4096 128 -> 121, 8192 x 8192 x 8192 270 -> 254, sustained).
+                // Elsewhere the second vote costs more than it saves (NVFP4 4096 x 4096 x 4096 on 128 x 128 36.2 -> 36.8).
+                uint32_t r[C::kSfCols];
+                const auto load = [&] {
+                    const uint32_t src_a = sfa_base + s * C::kSfaBytes + uint32_t(lane) * 16u;
+                    const uint32_t src_b = sfb_base + s * C::kSfbBytes + uint32_t(lane) * 16u;
 #pragma unroll
-                for (int a = 0; a < C::kSfKAtoms; ++a) {
-                    uint32_t r0, r1, r2, r3;
-                    ptx::ld_shared_v4(src_a + a * 512, r0, r1, r2, r3);
-                    ptx::tc_store_32x32_x4(set + C::kSfaCol + a * 4, r0, r1, r2, r3);
+                    for (int a = 0; a < C::kSfKAtoms; ++a) {
+                        ptx::ld_shared_v4(src_a + a * 512, r[4 * a], r[4 * a + 1], r[4 * a + 2], r[4 * a + 3]);
 #pragma unroll
-                    for (int j = 0; j < C::kNAtoms; ++j) {
-                        ptx::ld_shared_v4(src_b + (j * C::kSfKAtoms + a) * 512, r0, r1, r2, r3);
-                        ptx::tc_store_32x32_x4(set + C::kSfbCol + (a * C::kNAtoms + j) * 4, r0, r1, r2, r3);
+                        for (int j = 0; j < C::kNAtoms; ++j) {
+                            const int c = 4 * (C::kSfKAtoms + a * C::kNAtoms + j);
+                            ptx::ld_shared_v4(src_b + (j * C::kSfKAtoms + a) * 512, r[c], r[c + 1], r[c + 2], r[c + 3]);
+                        }
                     }
+                };
+                if constexpr (C::kSfSets == 2 && C::kSfKAtoms > 1) {
+                    ok = wait_bar(sf_full, (it / kRing) & 1u, abort, kStatusProducer);
+                    if (!ok) break;
+                    load();
+                    if (it >= uint32_t(C::kSfSets)) ok = wait_bar(set_free, (prev / kRing) & 1u, abort, kStatusProducer);
+                    if (!ok) break;
+                } else {
+                    ok = wait_bars(sf_full, (it / kRing) & 1u, it >= uint32_t(C::kSfSets), set_free, (prev / kRing) & 1u,
+                                   abort, kStatusProducer);
+                    if (!ok) break;
+                    load();
                 }
+                ptx::tc_fence_after();
+                const uint32_t set = tmem + (quarter << 16) + C::kSfaCol + (it % C::kSfSets) * C::kSfCols;
+                ptx::tc_store_32x32<C::kSfCols>(set, r);
                 ptx::tc_wait_st();
                 ptx::tc_fence_before();
                 __syncwarp();

@@ -388,6 +388,20 @@ __device__ __forceinline__ void tc_store_32x32_x16(uint32_t taddr, const uint32_
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
+// N columns (a multiple of 4), in as few instructions.
+template <int N>
+__device__ __forceinline__ void tc_store_32x32(uint32_t taddr, const uint32_t (&r)[N]) {
+    static_assert(N % 4 == 0, "columns");
+#pragma unroll
+    for (int c = 0; c + 16 <= N; c += 16) {
+        uint32_t q[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) q[i] = r[c + i];
+        tc_store_32x32_x16(taddr + c, q);
+    }
+#pragma unroll
+    for (int c = N / 16 * 16; c < N; c += 4) tc_store_32x32_x4(taddr + c, r[c], r[c + 1], r[c + 2], r[c + 3]);
+}
 __device__ __forceinline__ void tc_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
