@@ -200,6 +200,7 @@ struct Work {
     int b_row0;     // first row of the B box in the stacked weights
     int sfb_tile;   // 128-row scale atom row of the B box
     int sfb_shift;  // 32-row group of the B box inside that atom (BN = 64 only)
+    int cols;       // weight rows of the tile that exist; its other columns are neither loaded for nor stored
     int group;      // weight index: selects alpha and the bias row
     int row_lo;     // accumulator rows [row_lo, row_hi) belong to this item; the others
     int row_hi;     //   are padding or belong to the neighbouring group
@@ -229,6 +230,7 @@ struct WorkIter {
 
     __device__ __forceinline__ void set_b(Work& w, int group, int nt) const {
         w.group = group;
+        w.cols = min(BN, N - nt * BN);
         w.b_row0 = group * N + nt * BN;
         w.sfb_tile = group * ((N + 127) / 128) + (nt * BN) / 128;
         w.sfb_shift = ((nt * BN) % 128) / 32;
@@ -585,9 +587,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     }
 #pragma unroll
                     for (int j = 0; j < C::kNAtoms; ++j) {
+                        // (a ragged last tile takes the atoms that exist once more)
+                        const int ja = (j * 128 < wk.cols) ? j : 0;
                         if (ptx::elect_one()) {
                             ptx::bulk_load(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes,
-                                           sfb_row + int64_t(j) * kq_dim * 512 + koff, C::kSfaBytes, sf_full);
+                                           sfb_row + int64_t(ja) * kq_dim * 512 + koff, C::kSfaBytes, sf_full);
                         }
                     }
                     // a short activation loads only its own rows (the A box is a_rows tall)
@@ -801,7 +805,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars->acc_empty[as]));
                     }
-                    if (warp_idle) continue;
+                    if (warp_idle || 2 * g * kEpiChunk >= wk.cols) continue;
                     uint32_t y[16];
                     const __nv_bfloat16* const bc = bias != nullptr ? bias + n0 + 2 * g * kEpiChunk : nullptr;
                     situ_chunk(r0, bc, situ, &y[0]);
@@ -916,12 +920,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars->acc_empty[as]));
                 }
+                if (warp_idle || c * kEpiChunk >= wk.cols) continue;
                 uint32_t p[16];
                 epilogue_chunk(r, p, scale, bias != nullptr ? bias + wk.bias_col0 + c * kEpiChunk : nullptr,
                                epi_op);
                 const int row = m0 + ar;
                 const int col = n0 + c * kEpiChunk;
-                if (warp_idle) continue;
                 if (!kDense && (epi_op == HQ_EPILOGUE_QUANT || epi_op == HQ_EPILOGUE_GATE_MUL_QUANT ||
                                 epi_op == HQ_EPILOGUE_SIGMOID_GATE_MUL_QUANT)) {
                     // The bf16 result (times the gate, as a bf16 product) re-quantised to MXFP8 per
@@ -1121,6 +1125,8 @@ __device__ __forceinline__ uint32_t instr_desc_pair(uint32_t sf_id) {
 struct PairWork {
     int a_row0;     // first of the tile's 256 stacked A rows (a multiple of 256)
     int b_row0;     // first of the BN weight rows in the stacked weights
+    int sfb_tile;   // 128-row scale atom row of that row
+    int cols;       // weight rows of the tile that exist (see Work)
     int row_lo;     // tile rows [row_lo, row_hi) belong to this item; the others are padding,
     int row_hi;     //   belong to another expert, or lie beyond M
     int out_row0;   // output row of tile row 0
@@ -1146,6 +1152,13 @@ struct PairWorkIter {
 
     __device__ PairWorkIter(const GroupParams& grp, int m, int n, int tm, int tn, int first, int step)
         : g(grp), M(m), N(n), tiles_m(tm), tiles_n(tn), tile(first), stride(step) {}
+
+    __device__ __forceinline__ void set_b(PairWork& w, int group, int nt) const {
+        w.cols = min(BN, N - nt * BN);
+        w.b_row0 = group * N + nt * BN;
+        w.sfb_tile = group * ((N + 127) / 128) + (nt * BN) / 128;
+        w.bias_col0 = w.b_row0;
+    }
 
     __device__ bool next(PairWork& w) {
         if (!kGrouped || g.kind == kGroupContiguous) {
@@ -1187,8 +1200,7 @@ struct PairWorkIter {
                 }
                 pass = last ? 0 : pass + 1;
             }
-            w.b_row0 = group * N + tc.n * BN;
-            w.bias_col0 = w.b_row0;
+            set_b(w, group, tc.n);
             if (last) tile += stride;
             return true;
         }
@@ -1209,8 +1221,7 @@ struct PairWorkIter {
         w.a_row0 = first + rt * 256;
         w.row_lo = 0;
         w.row_hi = min(256, valid - rt * 256);
-        w.b_row0 = walk_group * N + nt * BN;
-        w.bias_col0 = w.b_row0;
+        set_b(w, walk_group, nt);
         if (g.kind == kGroupBatch) {
             w.out_row0 = w.a_row0 - first;
             w.out_col0 = w.b_row0;
@@ -1376,7 +1387,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             PairWork wk;
             while (ok && walk.next(wk)) {
                 const int sfa_atom_row = (wk.a_row0 / 128 + int(rank)) * kq_dim;
-                const int sfb_atom_row = (wk.b_row0 / 128) * kq_dim;
+                const int sfb_atom_row = wk.sfb_tile * kq_dim;
                 for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                     const uint32_t s = it % C::kStages;
                     ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
@@ -1594,6 +1605,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                             ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->acc_empty[as]), 0));
                         }
                     }
+                    if (2 * g * kEpiChunk >= wk.cols) continue;
                     uint32_t y[16];
                     const __nv_bfloat16* const bc = bias != nullptr ? bias + n0 + 2 * g * kEpiChunk : nullptr;
                     situ_chunk(r0, bc, situ.p, &y[0]);
@@ -1661,6 +1673,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                         ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->acc_empty[as]), 0));
                     }
                 }
+                if (c * kEpiChunk >= wk.cols) continue;
                 uint32_t p[16];
                 epilogue_chunk(r, p, scale, bias != nullptr ? bias + wk.bias_col0 + c * kEpiChunk : nullptr, epi_op);
                 if constexpr (kGrouped) {
@@ -1914,7 +1927,7 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
             tiles_m += int(((int64_t(b) + 1) * g.grp.rows - 1) / kBM - (int64_t(b) * g.grp.rows) / kBM + 1);
         }
     }
-    const int tiles_n = g.n / BN;
+    const int tiles_n = (g.n + BN - 1) / BN;
     const int grid = min(g.sm_count, tiles_m * tiles_n);
     const int k_tiles = int(g.k_bytes / kBKBytes);
     if constexpr (BN == 64) {
@@ -1996,7 +2009,7 @@ int launch_pair(const GemmArgs& g, char* err, size_t errlen, __nv_bfloat16* cons
         return fail(err, errlen, HQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the GEMM operands");
     }
     const int tiles_m = (g.m + 255) / 256;
-    const int tiles_n = g.n / BN;
+    const int tiles_n = (g.n + BN - 1) / BN;
     // persistent grid: no more clusters than can be resident at once
     static int max_clusters[64];
     static std::mutex max_clusters_mutex;
@@ -2328,9 +2341,11 @@ struct TilePick {
 // Shape legality follows the reference's "some compiled tile fits" rule
 // (csrc/kernel/gemm/gemm_dispatch.cuh:65-100 over the tiles of gemm_tile.cuh:371-395):
 // MXFP8 needs K % 128 == 0 and N % 64 == 0, the FP4 modes K % 256 == 0 and
-// N % 128 == 0; any M >= 1.  Among the legal tiles: the one that the figures
-// below make cheapest.  HALOPS_B200_TILE (pair256 | pair128 | 256 | 128 | 64)
-// overrides the choice when it is legal.
+// N % 128 == 0; any M >= 1.  A tile may stick out beyond N (the copies fill its rows beyond the weight with
+// zeros, the epilogue skips its columns), so every width is open to every N: when a width had to divide N, an odd
+// multiple of 64 left the 64-wide tile alone (3000 x 7232 x 4096 115 us there, 71 on the pair tile;
+// 1000 x 1984 x 4096 15.0 and 10.1).  Among the tiles: the one that the figures below make cheapest.
+// HALOPS_B200_TILE (pair256 | pair128 | 256 | 128 | 64) overrides the choice (64: the 8-bit modes only).
 TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int64_t boundaries = 0) {
     // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
     const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
@@ -2342,7 +2357,7 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
     if (forced != nullptr && forced[0] != '\0') {
         const bool pair = strncmp(forced, "pair", 4) == 0;
         const int w = atoi(pair ? forced + 4 : forced);
-        const bool legal = (w == 256 || w == 128 || (w == 64 && fp8 && !pair)) && n % w == 0;
+        const bool legal = w == 256 || w == 128 || (w == 64 && fp8 && !pair);
         if (legal) return {w, pair};
     }
     if (tiles_m == 1) {
@@ -2355,8 +2370,8 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
         int best = 0;
         int64_t best_cost = 0;
         for (int w : {256, 128, 64}) {
-            if (n % w != 0 || (w == 64 && !fp8)) continue;
-            const int64_t tiles = n / w;
+            if (w == 64 && !fp8) continue;
+            const int64_t tiles = (n + w - 1) / w;
             const int64_t cost = ((tiles + sm_count - 1) / sm_count) * (w + 16);
             if (best == 0 || cost < best_cost) {
                 best = w;
@@ -2391,9 +2406,9 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int6
     double best_cost = 0.0;
     for (int i = 0; i < count; ++i) {
         const Cand& c = cands[i];
-        if (n % c.bn != 0 || (c.bn == 64 && !fp8) || (c.pair && (m <= kBM || !fp8))) continue;
+        if ((c.bn == 64 && !fp8) || (c.pair && (m <= kBM || !fp8))) continue;
         const int64_t rows = c.pair ? tiles_m2 : tiles_m;
-        const int64_t tiles = rows * (n / c.bn);
+        const int64_t tiles = rows * ((n + c.bn - 1) / c.bn);
         const int64_t units = c.pair ? sm_count / 2 : sm_count;
         if (units < 1) continue;
         // Contiguous experts (runs of rows that start on multiples of 64): a CTA works a tile with a boundary inside

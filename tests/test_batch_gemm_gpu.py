@@ -325,3 +325,19 @@ def test_quant_epilogue_rules(hq):
     alpha = torch.ones([2], dtype=torch.float32, device="cuda")
     with pytest.raises(RuntimeError, match="Unsupported epilogue 1 for w4a4-nvfp4"):
         hq.batch_gemm(xq, wq, sfa4, sfb4, q, None, alpha, -1, "w4a4-nvfp4", hq.EpilogueOp.Quant, sf)
+
+
+@pytest.mark.parametrize("tile", ["128", "256", "pair128", "pair256"])
+@pytest.mark.parametrize("n", [64, 192, 320])
+def test_columns_that_do_not_fill_the_last_tile(hq, monkeypatch, tile, n):
+    """The columns behind a batch's last ones are the next batch's: the same bits as on the tile that divides N."""
+    b, m, k = 3, 256, 384
+    xq, wq, sfa, sfb = _inputs(hq, b, m, n, k, "w8a8-mxfp8", seed=14)
+    bias = torch.rand([b, n], generator=torch.Generator().manual_seed(9)).to(torch.bfloat16).cuda()
+    outs = []
+    for t in ("64", tile):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert f"pair={int('pair' in t)}" in hq.describe_group_tile("batch", b, m, n, k)
+        outs.append(_run(hq, xq, wq, sfa, sfb, "w8a8-mxfp8", bias=bias))
+    assert torch.equal(outs[0], outs[1])
+    _compare(outs[1], xq, wq, sfa, sfb, "w8a8-mxfp8", bias=bias)

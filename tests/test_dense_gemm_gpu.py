@@ -566,3 +566,34 @@ def test_weight_rewritten_by_the_preceding_kernel_on_every_tile(hq, monkeypatch,
     assert hq.device_status() == 0
     for i, outs in enumerate(got):
         assert all(torch.equal(x, y) for x, y in zip(outs, expected[i & 1])), f"call {i} used stale weight bytes"
+
+
+@pytest.mark.parametrize("mode,tile", [("w8a8-mxfp8", t) for t in ("128", "256", "pair128", "pair256")] +
+                         [("w4a4-nvfp4", "256"), ("w4a4-mxfp4", "256")], ids=lambda v: str(v))
+@pytest.mark.parametrize("m", [100, 300, 512])
+@pytest.mark.parametrize("n_extra", [64, 128, 192])
+def test_columns_that_do_not_fill_the_last_tile(hq, monkeypatch, mode, tile, m, n_extra):
+    """A tile may stick out beyond N: the result is that of a tile that divides N, bit for bit, the columns behind
+    the output stay as they were, and the last scale atoms of the weight are read, not what lies behind them."""
+    if mode != "w8a8-mxfp8" and n_extra != 128:
+        pytest.skip("the FP4 modes need N % 128 == 0")
+    n, k = 512 + n_extra, 1024
+    a, b = _rand(m, k, 61), _rand(n, k, 62)
+    aq, bq, sfa, sfb = _quantize(hq, a, b, mode)
+    alpha = torch.full([1], 0.7, device="cuda") if mode == "w4a4-nvfp4" else None
+    bias = torch.rand([n], generator=torch.Generator().manual_seed(63)).to(torch.bfloat16).cuda() if m % 256 == 0 and mode == "w8a8-mxfp8" else None
+    results = []
+    monkeypatch.setenv("HALOPS_B200_SPLITK", "0")
+    # (one row of 64-wide tiles sums in another order, so a width that divides N and walks K in order)
+    whole = "128" if n % 128 == 0 or m <= 128 else "64"
+    for t in (whole, tile):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert ("256x" if "pair" in t else "128x") + t.replace("pair", "") in hq.describe_tile(m, n, k, mode)
+        wide = torch.full([m, n + 64], 7.0, dtype=torch.bfloat16, device="cuda")
+        hq.dense_gemm(aq, bq, sfa, sfb, wide[:, :n], bias, alpha, mode=mode)
+        assert hq.device_status() == 0
+        assert torch.all(wide[:, n:] == 7.0)
+        results.append(wide[:, :n].contiguous())
+    assert torch.equal(results[0], results[1])
+    if bias is None:
+        _check(results[1], aq, bq, sfa, sfb, mode, alpha=None if alpha is None else 0.7)

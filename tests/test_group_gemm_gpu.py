@@ -435,3 +435,32 @@ def test_w4a8_rules(hq):
         hq.group_masked_gemm(xq[:, :128].contiguous(), wq, sfa, sfb, masked, out, None, None, max_m, -1, "w4a8-mxfp4")
     with pytest.raises(RuntimeError, match="requires SF K = 8"):
         hq.group_masked_gemm(xq, wq, sfa, sfb[:, :, :4].contiguous(), masked, out, None, None, max_m, -1, "w4a8-mxfp4")
+
+
+@pytest.mark.parametrize("mode,tile", [("w8a8-mxfp8", "256"), ("w8a8-mxfp8", "pair256"), ("w4a8-mxfp4", "pair256"), ("w4a8-mxfp4", "256"),
+                                       ("w4a4-nvfp4", "256")], ids=lambda v: str(v))
+def test_columns_that_do_not_fill_the_last_tile(hq, monkeypatch, mode, tile):
+    """384 columns on a 256-wide tile: behind an expert's last weight rows lie the next expert's."""
+    n, k = 384, 512
+    results = []
+    for t in ("128", tile):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert f"x{t.replace('pair', '')}/" in hq.describe_group_tile("masked", 4, 256, n, k, mode)
+        if mode == "w4a8-mxfp4":
+            results.append(_w4a8_pair_of_outputs(hq, n, k))
+            continue
+        results.append((_masked_case(hq, 256, 4, n, k, mode, [256, 0, 129, 200]), _contiguous_case(hq, [64, 192, 256, 256], n, k, mode)))
+    assert all(torch.equal(x, y) for x, y in zip(*results))
+
+
+def _w4a8_pair_of_outputs(hq, n, k):
+    xq, _, sfa, _ = _inputs(hq, 768, 1, n, k, "w8a8-mxfp8", seed=4)
+    _, wq, _, sfb = _inputs(hq, 128, 4, n, k, "w4a4-mxfp4", seed=5)
+    masked = torch.full([4 * 256, n], 3.0, dtype=torch.bfloat16, device="cuda")
+    x4, sf4 = torch.cat([xq, xq[:256]]), torch.cat([sfa, sfa[:256]])
+    hq.group_masked_gemm(x4, wq, sf4, sfb, torch.tensor([256, 0, 129, 200], dtype=torch.int32).cuda(), masked, None, None, 256, -1, "w4a8-mxfp4")
+    out = torch.full([768, n], 3.0, dtype=torch.bfloat16, device="cuda")
+    ids = torch.from_numpy(np.repeat(np.arange(4, dtype=np.int32), [64, 192, 256, 256])).cuda()
+    hq.group_contiguous_gemm(xq, wq, sfa, sfb, ids, out, mode="w4a8-mxfp4")
+    assert hq.device_status() == 0
+    return masked, out
