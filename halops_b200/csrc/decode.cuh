@@ -488,7 +488,9 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     const uint32_t s = it % C::kStages;
                     // (no vote: every lane copies and arrives for itself, and this warp paces the first ring of
                     // stages; with a vote per step 16 x 8192 x 4096 took 12.3 instead of 12.1 us)
-                    ok = wait_bar_lane(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort, kStatusProducer);
+                    const uint32_t empty = ptx::smem_u32(&bars->empty[s]);
+                    const uint32_t free_phase = ((it / C::kStages) & 1u) ^ 1u;
+                    ok = ptx::mbar_try_wait(empty, free_phase) || wait_bar_lane(empty, free_phase, abort, kStatusProducer);
                     if (!ok) break;
                     const DecSource src(plain, sg.tile, ks);
                     const int64_t koff = int64_t(src.ks) * 8;

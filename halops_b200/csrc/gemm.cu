@@ -116,10 +116,12 @@ struct Barriers {
 
 // Bounded mbarrier wait of one lane.  Returns false when the CTA is aborting.  kCluster: the barrier is one
 // that CTAs of the cluster arrive on with release semantics; the wait acquires what they wrote into
-// this CTA's shared memory before arriving.
+// this CTA's shared memory before arriving.  A function of its own: the roles come here only when a first
+// try_wait, which holds a converged warp until the phase ends (woken 84 cycles after the arrival, also after
+// 6000 cycles), has returned without it, and the polling code is not in their loops.
 template <bool kCluster = false>
-__device__ __forceinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volatile uint32_t* abort,
-                                              uint32_t code, uint64_t limit_ns = kTimeoutNs) {
+__device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code,
+                                           uint64_t limit_ns = kTimeoutNs) {
     const auto done = [&] { return kCluster ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity); };
     if (done()) return true;
     const uint64_t t0 = ptx::globaltimer_ns();
@@ -141,17 +143,25 @@ __device__ __forceinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, vol
 // themselves, so when a wait runs out while its barrier completes after all, some of them see the one and
 // some the other; leaving the role's loop on that would send a part of the warp into
 // .sync.aligned instructions, __syncwarp and elections that count on all 32 lanes.
+// The first try and its vote are straight-line code (a completed barrier: 58 cycles); with the polling loop inline, lane by
+// lane, a wait on a completed barrier took a role 125: 512 x 1536 x 4096 8.8 -> 8.5 us, 1024 x 1536 x 8192 26.0 -> 24.9 (both on
+// the 128 x 64 tile), NVFP4 512 x 4096 x 8192 12.9 -> 12.7, 64 x 24576 x 1536 10.2 -> 10.0, GEMM alone.
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+    if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
     return __all_sync(0xffffffffu, wait_bar_lane(bar, parity, abort, code) ? 1 : 0) != 0;
 }
 // Two waits with one vote (the second only if `both`): a vote between a barrier and the work behind it is on the
 // critical path of a k-step.
 __device__ __forceinline__ bool wait_bars(uint32_t bar, uint32_t parity, bool both, uint32_t bar2, uint32_t parity2,
                                           volatile uint32_t* abort, uint32_t code) {
-    const bool mine = wait_bar_lane(bar, parity, abort, code) && (!both || wait_bar_lane(bar2, parity2, abort, code));
+    bool mine = ptx::mbar_try_wait(bar, parity);
+    if (both) mine = ptx::mbar_try_wait(bar2, parity2) && mine;
+    if (__all_sync(0xffffffffu, mine ? 1 : 0) != 0) return true;
+    mine = wait_bar_lane(bar, parity, abort, code) && (!both || wait_bar_lane(bar2, parity2, abort, code));
     return __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
 }
 __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
+    if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar, parity) ? 1 : 0) != 0) return true;
     return __all_sync(0xffffffffu, wait_bar_lane<true>(bar, parity, abort, code) ? 1 : 0) != 0;
 }
 
