@@ -462,6 +462,23 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], uint32_t
     }
 }
 
+// The scale atoms of one stage (512 bytes each, 16 for a lane) into registers, in the order of a scale set's columns:
+// SFA by atom along K, then SFB by atom along K and 128 columns.
+template <typename C>
+__device__ __forceinline__ void load_scales(uint32_t sfa_stage, uint32_t sfb_stage, int lane, uint32_t (&r)[C::kSfCols]) {
+    const uint32_t a0 = sfa_stage + uint32_t(lane) * 16u;
+    const uint32_t b0 = sfb_stage + uint32_t(lane) * 16u;
+#pragma unroll
+    for (int a = 0; a < C::kSfKAtoms; ++a) {
+        ptx::ld_shared_v4(a0 + a * 512, r[4 * a], r[4 * a + 1], r[4 * a + 2], r[4 * a + 3]);
+#pragma unroll
+        for (int j = 0; j < C::kNAtoms; ++j) {
+            const int c = 4 * (C::kSfKAtoms + a * C::kNAtoms + j);
+            ptx::ld_shared_v4(b0 + (j * C::kSfKAtoms + a) * 512, r[c], r[c + 1], r[c + 2], r[c + 3]);
+        }
+    }
+}
+
 // kSplitK (64-wide tiles, one row of tiles, at most half as many tiles as SMs): a cluster of
 // two CTAs works one tile, each half of the k-tiles; the second CTA sends its fp32 partial
 // sums through distributed shared memory into a 32 KB buffer of the first (carved out of the
@@ -723,27 +740,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const uint32_t prev = it - uint32_t(C::kSfSets);
                 const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
                 const uint32_t set_free = ptx::smem_u32(&bars->empty[prev % kRing]);
-                // A k-tile's scales go to registers first, in the order of the set's columns (SFA by atom along
-                // K, then SFB by atom along K and 128 columns), and on with as few stores as there are.  Where only
+                // A k-tile's scales go to registers first, and on with as few stores as there are.  Where only
                 // two sets rotate and a set is large, the loads do not wait for it: what lies between its release and
                 // the MMAs that wait for its next scales is on the critical path there, and it was 12 loads and 12
                 // stores one after the other, some 700 cycles against 512 of one k-tile's MMAs (NVFP4 512 x 4096 x 4096 on the
                 // 128 x 256 tile 10.9 -> 9.9 us, 4096 x 14336 x 4096 128 -> 121, 8192 x 8192 x 8192 270 -> 254, sustained).
                 // Elsewhere the second vote costs more than it saves (NVFP4 4096 x 4096 x 4096 on 128 x 128 36.2 -> 36.8).
                 uint32_t r[C::kSfCols];
-                const auto load = [&] {
-                    const uint32_t src_a = sfa_base + s * C::kSfaBytes + uint32_t(lane) * 16u;
-                    const uint32_t src_b = sfb_base + s * C::kSfbBytes + uint32_t(lane) * 16u;
-#pragma unroll
-                    for (int a = 0; a < C::kSfKAtoms; ++a) {
-                        ptx::ld_shared_v4(src_a + a * 512, r[4 * a], r[4 * a + 1], r[4 * a + 2], r[4 * a + 3]);
-#pragma unroll
-                        for (int j = 0; j < C::kNAtoms; ++j) {
-                            const int c = 4 * (C::kSfKAtoms + a * C::kNAtoms + j);
-                            ptx::ld_shared_v4(src_b + (j * C::kSfKAtoms + a) * 512, r[c], r[c + 1], r[c + 2], r[c + 3]);
-                        }
-                    }
-                };
+                const auto load = [&] { load_scales<C>(sfa_base + s * C::kSfaBytes, sfb_base + s * C::kSfbBytes, lane, r); };
                 if constexpr (C::kSfSets == 2 && C::kSfKAtoms > 1) {
                     ok = wait_bar(sf_full, (it / kRing) & 1u, abort, kStatusProducer);
                     if (!ok) break;
@@ -1066,11 +1070,18 @@ __global__ void __launch_bounds__(96, 1) wait_selftest_kernel(uint64_t limit_ns)
 // matching half of the accumulator; both CTAs hold the scales of all BN columns.
 // Every CTA loads its own halves with plain (non-broadcast) TMA copies in the
 // cta_group::2 form, which lets the bytes be counted on the leader's (rank 0)
-// barrier; only the leader issues tcgen05.cp / tcgen05.mma.  It releases a stage with
-// one tcgen05.commit to its own barrier, which its loader passes on to the other CTA,
-// and publishes an accumulator with one commit per CTA.  The epilogue warps of
-// both CTAs report to the leader's barriers.  Per CTA this halves the B traffic from
-// L2 and leaves room for 6 stages instead of 4.
+// barrier; only the leader issues tcgen05.mma.  It releases a stage, and publishes an accumulator, with
+// one tcgen05.commit that arrives in both CTAs.  The scales of a k-tile go from shared to tensor memory
+// by four warps of each CTA, as in the single-CTA kernel, which report to the leader, as the epilogue warps of
+// both CTAs do.  Per CTA this halves the B traffic from L2 and leaves room for 6 stages instead of 4.
+//
+// What bounds it: large problems the power cap (clocks of 1.1 to 1.4 GHz), so the bytes that each product moves count
+// more than the cycles between them; small ones the hand-over between the k-tiles.  Against scales copied by
+// tcgen05.cp from one warp (75 to 90 cycles a copy, a commit behind them) and a release that the leader's loader
+// passed on: MXFP8 8192 x 8192 x 8192 462 -> 448 us, 4096 x 7168 x 2048 58.4 -> 56.5, 512 x 4096 x 4096 16.4 -> 15.0,
+// 4096 x 4096 x 4096 on the 256 x 128 tile 80 -> 64 (sustained, GEMM alone; the waits' part of the last is 10).  NVFP4, with
+// 12 copies a k-tile: 8192 x 8192 x 8192 295 -> 230, which made it the better tile for the FP4 kinds too
+// (single-CTA 128 x 256: 251); 4096 x 4096 x 4096 44 -> 35.5 (41).
 
 template <int BN, int KIND>
 struct Cfg2 {
@@ -1083,31 +1094,26 @@ struct Cfg2 {
     static constexpr int kSfaBytes = kSfKAtoms * 512;
     static constexpr int kSfbBytes = kNAtoms * kSfaBytes;
     static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
-    // bytes a stage reads from global memory: packed e2m1 weights (KIND 3) are spread to one byte
+    // operand bytes a stage reads from global memory: packed e2m1 weights (KIND 3) are spread to one byte
     // per value by the copy, and the barrier counts what was read
-    static constexpr int kStageTxBytes = kStageBytes - (KIND == 3 ? kBBytes / 2 : 0);
+    static constexpr int kStageTxBytes = kABytes + kBBytes - (KIND == 3 ? kBBytes / 2 : 0);
     static constexpr int kEpiBufs = 2;
     static constexpr int kEpiBytes = kEpiWarps * kEpiBufs * kEpiBufBytes;
     static constexpr int kBarBytes = 1024;
     static constexpr int kStagesFit = (kSmemBudget - kEpiBytes - kBarBytes - 1024) / kStageBytes;
     static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + kBarBytes + 1024;
-    // Scale columns of one k-iteration and how many such sets rotate in tensor memory.
-    // The tcgen05.cp copies are issued by other warps than the MMAs: a copy of one atom holds
-    // the copy unit, and the warp that waits for it, for 60-85 cycles, and 3 copies + 4 MMAs + 2 commits
-    // from one thread took 850 cycles per k-tile (measured with the issue inside `if (lane == 0)`, see
-    // ptx::elect_one); the MMAs alone take 512.  A set is free again once the MMAs that
-    // read it have completed, so with 4 sets the copies run two k-tiles ahead.
+    // Scale columns of one k-iteration and how many such sets rotate in tensor memory.  A set is free again once the
+    // MMAs that read it have completed, so with 4 sets the scales run two k-tiles ahead; NVFP4's 48 columns
+    // leave room for 2.
     static constexpr int kSfCols = kSfKAtoms * 4 * (1 + kNAtoms);
-    static constexpr int kSfSets = BN < 256 ? 4 : (kFp8Kind ? 4 : (KIND == 2 ? 3 : 2));
-    // warps: 0 box loader, 1 MMA issuer, 2-5 epilogue, 6 scale loader, 7.. scale copies
-    static constexpr int kCpWarps = kFp8Kind ? 1 : (KIND == 1 ? 3 : 2);
-    // Two threads (warp 1 and the last warp) issue the MMAs of alternate k-tiles: issuing
-    // 4 MMAs and the commit that releases the stage keeps one thread busy for longer
-    // than the 512 cycles the MMAs run.  After its MMAs a thread
+    static constexpr int kSfSets = BN < 256 || KIND != 1 ? 4 : 2;
+    // warps: 0 box loader, 1 MMA issuer, 2-5 epilogue, 6 scale loader, 7-10 scales to tensor memory, 11 MMA issuer
+    // Two threads (of warp 1 and of the last warp) issue the MMAs of alternate k-tiles.  After its MMAs a thread
     // hands the turn to the other one (tcgen05 fences around an mbarrier arrive), so the
     // MMAs still reach the tensor core in k order.
-    static constexpr int kThreads = 32 * (8 + kCpWarps);
+    static constexpr int kMma2Warp = 7 + kSfWarps;
+    static constexpr int kThreads = 32 * (kMma2Warp + 1);
     static constexpr int kSfRegion = kSfCols * kSfSets;
     static constexpr int kOverlap = BN == 256 ? (kSfRegion + 15) / 16 * 16 : 0;
     static constexpr int kAccStride = BN - kOverlap;
@@ -1308,9 +1314,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
-            // the leader's copy collects the bytes of both CTAs after one
-            // expect_tx arrival of the leader's producer
+            // the leader's copy collects the operand bytes of both CTAs after one
+            // expect_tx arrival of the leader's producer; the scales' bytes are each CTA's own matter
             ptx::mbar_init(ptx::smem_u32(&bars->full[s]), 1);
+            ptx::mbar_init(ptx::smem_u32(&bars->sf_full[s]), 1);
             ptx::mbar_init(ptx::smem_u32(&bars->empty[s]), 1);  // one tcgen05.commit
         }
         for (int s = 0; s < 2; ++s) {
@@ -1318,7 +1325,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             ptx::mbar_init(ptx::smem_u32(&bars->acc_empty[s]), 2 * kEpiWarps);  // leader's copy is used
             ptx::mbar_init(ptx::smem_u32(&bars->overlap_free[s]), 2 * kEpiWarps);
         }
-        for (int s = 0; s < C::kSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), C::kCpWarps);
+        // (the leader's copy is used)
+        for (int s = 0; s < C::kSfSets; ++s) ptx::mbar_init(ptx::smem_u32(&bars->sf_ready[s]), 2 * kSfWarps);
         for (int s = 0; s < 2; ++s) ptx::mbar_init(ptx::smem_u32(&bars->turn[s]), 1);
         bars->abort = 0;
         ptx::fence_mbar_init();
@@ -1368,18 +1376,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
-                    // The MMA threads release a stage with one commit, to the leader's barrier; the
-                    // leader's loader passes it on.  A second commit costs the issuing thread about
-                    // 300 cycles per k-tile, this relaxed arrival about 200 on a thread with slack
-                    // (what it reports, the MMAs' reads of the stage, completed before the commit).
-                    if (leader && it >= uint32_t(C::kStages)) {
-                        if (ptx::elect_one()) {
-                            ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 1));
-                        }
-                    }
                     const uint32_t full = ptx::mapa_cluster(ptx::smem_u32(&bars->full[s]), 0);
-                    // Bytes of all four loader threads of the pair are counted on the leader's
-                    // barrier; only this thread registers them (the count may go negative in
+                    // The bytes of both loaders of the pair are counted on the leader's
+                    // barrier; only its own registers them (the count may go negative in
                     // between).
                     if (leader && ptx::elect_one()) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&bars->full[s]), 2 * C::kStageTxBytes);
                     if (ptx::elect_one()) ptx::tma_load_2d_pair(a_base + s * C::kABytes, &tm_a, kt * kBKBytes, m0, full);
@@ -1403,39 +1402,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ((it / C::kStages) & 1u) ^ 1u, abort,
                                   kStatusProducer);
                     if (!ok) break;
-                    const uint32_t full = ptx::mapa_cluster(ptx::smem_u32(&bars->full[s]), 0);
-                    // scale atoms are rows of 128 32-bit words
+                    const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
+                    if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(sf_full, C::kSfaBytes + C::kSfbBytes);
+                    // scale atoms are rows of 128 32-bit words (those beyond the weight arrive as zeros)
                     if (ptx::elect_one()) {
-                        ptx::tma_load_2d_pair(sfa_base + s * C::kSfaBytes, &tm_sfa, 0,
-                                              sfa_atom_row + kt * C::kSfKAtoms, full);
+                        ptx::tma_load_2d(sfa_base + s * C::kSfaBytes, &tm_sfa, 0, sfa_atom_row + kt * C::kSfKAtoms, sf_full);
                     }
 #pragma unroll
                     for (int j = 0; j < C::kNAtoms; ++j) {
                         if (ptx::elect_one()) {
-                            ptx::tma_load_2d_pair(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes, &tm_sfb, 0,
-                                                  sfb_atom_row + j * kq_dim + kt * C::kSfKAtoms, full);
+                            ptx::tma_load_2d(sfb_base + s * C::kSfbBytes + j * C::kSfaBytes, &tm_sfb, 0,
+                                             sfb_atom_row + j * kq_dim + kt * C::kSfKAtoms, sf_full);
                         }
                     }
                 }
             }
         }
-    } else if (warp >= 7 && warp < 7 + C::kCpWarps) {
-        // ------------------------------------------------------------ scale copies (leader only)
-        // shared memory -> tensor memory of both CTAs, into scale set it % kSfSets
-        if (leader) {
-            const int cw = warp - 7;
-            bool ok = true;
-            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
-            PairWork wk;
-            uint32_t total_its = 0;
-            for (uint32_t it = 0; ok; ++it) {
-                if (it == total_its) {  // the k-tiles of the next item
-                    if (!walk.next(wk)) break;
-                    total_its += uint32_t(k_tiles);
-                }
+    } else if (warp >= 7 && warp < 7 + kSfWarps) {
+        // ------------------------------------------------------------ scales -> tensor memory (both CTAs)
+        // as in the single-CTA kernel: every warp fills its quarter of the lanes with the same image
+        const uint32_t quarter = (uint32_t(warp) & 3u) * 32u;
+        uint32_t it = 0;
+        bool ok = true;
+        Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+        PairWork wk;
+        while (ok && walk.next(wk)) {
+            for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                 const uint32_t s = it % C::kStages;
-                ok = wait_bar(ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
+                ok = wait_bar(ptx::smem_u32(&bars->sf_full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
                 if (!ok) break;
+                // into registers before the set is free, in the order of its columns
+                uint32_t r[C::kSfCols];
+                load_scales<C>(sfa_base + s * C::kSfaBytes, sfb_base + s * C::kSfbBytes, lane, r);
                 if (it >= uint32_t(C::kSfSets)) {
                     // the MMAs of k-tile it - kSfSets read this set: they are done once they
                     // have released their stage
@@ -1445,33 +1443,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     if (!ok) break;
                 }
                 ptx::tc_fence_after();
-                const uint32_t set = tmem + C::kSfCol0 + (it % C::kSfSets) * C::kSfCols;
-#pragma unroll
-                for (int a = 0; a < C::kSfKAtoms; ++a) {
-                    if ((a * (1 + C::kNAtoms)) % C::kCpWarps == cw) {
-                        if (ptx::elect_one()) {
-                            ptx::tc_copy_sf<2>(set + a * 4,
-                                               ptx::smem_desc(sfa_base + s * C::kSfaBytes + a * 512, 0, 128, 0));
-                        }
-                    }
-#pragma unroll
-                    for (int j2 = 0; j2 < C::kNAtoms; ++j2) {
-                        if ((a * (1 + C::kNAtoms) + 1 + j2) % C::kCpWarps == cw) {
-                            if (ptx::elect_one()) {
-                                ptx::tc_copy_sf<2>(
-                                    set + C::kSfKAtoms * 4 + (a * C::kNAtoms + j2) * 4,
-                                    ptx::smem_desc(sfb_base + s * C::kSfbBytes + (j2 * C::kSfKAtoms + a) * 512, 0, 128,
-                                                   0));
-                            }
-                        }
-                    }
-                }
+                ptx::tc_store_32x32<C::kSfCols>(tmem + (quarter << 16) + C::kSfCol0 + (it % C::kSfSets) * C::kSfCols, r);
+                ptx::tc_wait_st();
+                ptx::tc_fence_before();
+                __syncwarp();
+                // (what it reports is in tensor memory, and complete)
                 if (ptx::elect_one()) {
-                    ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), 0));
+                    ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), 0));
                 }
             }
         }
-    } else if (warp == 1 || warp == 7 + C::kCpWarps) {
+    } else if (warp == 1 || warp == C::kMma2Warp) {
         // ------------------------------------------------------------ MMA issuers (leader only)
         if (leader) {
             const uint32_t me = warp == 1 ? 0u : 1u;  // this thread issues the k-iterations it & 1 == me
@@ -1511,12 +1493,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                         }
                         if (!ok) break;
                     }
-                    // The scale copies of this k-tile have landed.  Every copy warp waited for the
-                    // stage's barrier before it copied and committed, so the operand boxes of both
-                    // CTAs have landed too: no second wait here (each one costs this thread, which
-                    // sets the pace, 50-100 cycles).
-                    ok = wait_bar(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, abort,
-                                  kStatusMma);
+                    // the scales of both CTAs are in tensor memory and the operand boxes of both have landed
+                    ok = wait_bars(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, true,
+                                   ptx::smem_u32(&bars->full[s]), (it / C::kStages) & 1u, abort, kStatusMma);
                     // the other thread has issued the MMAs of the previous k-iteration
                     if (ok && it > 0u) {
                         ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
@@ -1546,19 +1525,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                                 set + C::kSfKAtoms * 4 + atom * C::kNAtoms * 4, (kt > 0 || k > 0) ? 1u : 0u);
                         }
                     }
-                    // hand the turn over before the (slow) commits
+                    // hand the turn over before the commits
                     ptx::tc_fence_before();
                     if (ptx::elect_one()) ptx::mbar_arrive(ptx::smem_u32(&bars->turn[me ^ 1u]));
                     // the loaders of both CTAs may refill stage s once these MMAs have read it
-                    // (the leader's loader passes the release on to the other CTA)
-                    if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(ptx::smem_u32(&bars->empty[s]), 0));
+                    if (ptx::elect_one()) ptx::tc_commit_both(ptx::smem_u32(&bars->empty[s]));
                     // A commit tracks the operations of the thread that executes it, so each of
                     // the two threads commits the accumulator after its own last k-tile of the
                     // tile; the epilogue starts when both have completed.
                     if (kt >= k_tiles - 2) {
-                        const uint32_t accf = ptx::smem_u32(&bars->acc_full[as]);
-                        if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(accf, 0));
-                        if (ptx::elect_one()) ptx::tc_commit_pair(ptx::mapa_cluster(accf, 1));
+                        if (ptx::elect_one()) ptx::tc_commit_both(ptx::smem_u32(&bars->acc_full[as]));
                     }
                 }
             }

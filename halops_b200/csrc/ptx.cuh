@@ -282,19 +282,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     }
 }
 
-// 32 rows x 16 bytes of shared memory (one quarter of a 512-byte SfAtom row
-// set) -> 4 tensor-memory columns, replicated into all four 32-lane quadrants.
-template <int kCtaGroup>
-__device__ __forceinline__ void tc_copy_sf(uint32_t taddr, uint64_t sdesc) {
-    if constexpr (kCtaGroup == 1) {
-        asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc)
-                     : "memory");
-    } else {
-        asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc)
-                     : "memory");
-    }
-}
-
 // Block-scaled MMA, both operands from shared memory, accumulator and scale
 // factors in tensor memory.  kKind: 0 = mxf8f6f4 (1 scale / 32), 1 = mxf4nvf4
 // with 4 scales per K=64 (NVFP4), 2 = mxf4nvf4 with 2 scales per K=64 (MXFP4),
@@ -338,11 +325,12 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
-// Pair form: `bar` is a shared::cluster address, so it may name a barrier of
-// either CTA of the pair (see mapa_cluster).
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
+// Pair form: one arrival on the barrier at `bar`'s offset in the shared memory of each of the two CTAs.
+__device__ __forceinline__ void tc_commit_both(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"(uint16_t(3))
+        : "memory");
 }
 // shared::cluster address of this CTA's shared-memory address `addr` in CTA
 // `cta` of the cluster.
