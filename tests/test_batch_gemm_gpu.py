@@ -341,3 +341,18 @@ def test_columns_that_do_not_fill_the_last_tile(hq, monkeypatch, tile, n):
         outs.append(_run(hq, xq, wq, sfa, sfb, "w8a8-mxfp8", bias=bias))
     assert torch.equal(outs[0], outs[1])
     _compare(outs[1], xq, wq, sfa, sfb, "w8a8-mxfp8", bias=bias)
+
+
+@pytest.mark.parametrize("mode", ["w4a4-nvfp4", "w4a4-mxfp4"])
+@pytest.mark.parametrize("tile", ["pair256", "pair128"])
+def test_fp4_batches_on_the_2cta_tile(hq, monkeypatch, mode, tile):
+    b, m, n, k = 3, 256, 384, 1536
+    xq, wq, sfa, sfb = _inputs(hq, b, m, n, k, mode, seed=15)
+    alpha = (0.5 + torch.arange(b, dtype=torch.float32) * 0.25).cuda() if mode == "w4a4-nvfp4" else None
+    outs = []
+    for t in ("128", tile):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert f"pair={int('pair' in t)}" in hq.describe_group_tile("batch", b, m, n, k, mode)
+        outs.append(_run(hq, xq, wq, sfa, sfb, mode, alpha=alpha))
+    assert torch.equal(outs[0], outs[1])
+    _compare(outs[1], xq, wq, sfa, sfb, mode, alpha=alpha)

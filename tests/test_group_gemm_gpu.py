@@ -464,3 +464,19 @@ def _w4a8_pair_of_outputs(hq, n, k):
     hq.group_contiguous_gemm(xq, wq, sfa, sfb, ids, out, mode="w4a8-mxfp4")
     assert hq.device_status() == 0
     return masked, out
+
+
+@pytest.mark.parametrize("mode", ["w4a4-nvfp4", "w4a4-mxfp4"])
+@pytest.mark.parametrize("tile", ["pair256", "pair128"])
+def test_fp4_experts_on_the_2cta_tile(hq, monkeypatch, mode, tile):
+    """The FP4 kinds on the pair tile, each expert with its own alpha: full and partly filled tiles, empty slots, several runs of
+    experts in a tile, more k-tiles than stages; the bits of the single-CTA tile."""
+    results = []
+    for t in ("128", tile):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert f"pair={int('pair' in t)}" in hq.describe_group_tile("masked", 4, 512, 512, 2048, mode)
+        assert f"pair={int('pair' in t)}" in hq.describe_group_tile("contiguous", 5, 256, 512, 2048, mode, total_m=1280)
+        results.append((_masked_case(hq, 512, 4, 512, 2048, mode, [512, 300, 0, 257]),
+                        _contiguous_case(hq, [64, 192, 128, 640, 256], 512, 2048, mode),
+                        _contiguous_case(hq, [64] * 4, 256, 256, mode)))
+    assert all(torch.equal(x, y) for x, y in zip(*results))
