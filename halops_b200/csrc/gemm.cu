@@ -28,6 +28,8 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "common.cuh"
@@ -43,6 +45,8 @@ constexpr int kEpiWarps = 4;
 constexpr int kSfWarps = 4;        // single-CTA kernel: warps 6-9 move the scales into tensor memory
 constexpr int kEpiChunk = 32;      // accumulator columns per tcgen05.ld / TMA store
 constexpr int kEpiBufBytes = 32 * kEpiChunk * 2;  // 32 rows x 64 bytes
+constexpr int kMaxRuns = 255;      // runs of contiguous experts a launch may keep in shared memory, and their end
+constexpr int kRunBytes = 4 * (kMaxRuns + 1);
 constexpr uint64_t kTimeoutNs = 2000000000ull;    // bound of every device-side wait
 constexpr int kSmemBudget = 232448;               // 227 KiB opt-in maximum per CTA
 
@@ -68,7 +72,7 @@ struct Cfg {
     static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
     static constexpr int kEpiBufs = (KIND == 1 && BN == 256) ? 1 : 2;
     static constexpr int kEpiBytes = kEpiWarps * kEpiBufs * kEpiBufBytes;
-    static constexpr int kBarBytes = 1024;
+    static constexpr int kBarBytes = 1024 + kRunBytes;  // barriers, then the runs of contiguous experts
     static constexpr int kStagesFit = (kSmemBudget - kEpiBytes - kBarBytes - 1024) / kStageBytes;
     static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + kBarBytes + 1024;
@@ -112,7 +116,10 @@ struct Barriers {
     uint64_t epi_sync;     // small-M kernel: rendezvous of the four epilogue warps (a bounded wait, unlike bar.sync)
     uint32_t tmem_base;
     uint32_t abort;
+    int run_counts[16];  // contiguous experts: runs that start in a warp's share of the rows; [0] in the end: row tiles
 };
+constexpr int kKeptOffset = 640;  // pair kernel: the epilogue warps' places in the walk, behind the barriers
+static_assert(sizeof(Barriers) <= kKeptOffset, "kBarBytes");
 
 // Bounded mbarrier wait of one lane.  Returns false when the CTA is aborting.  kCluster: the barrier is one
 // that CTAs of the cluster arrive on with release semantics; the wait acquires what they wrote into
@@ -204,6 +211,100 @@ struct GroupParams {
     const int* table;  // masked: valid rows per expert; contiguous: expert of every row
 };
 
+// Contiguous experts: the rows as runs of one expert each.  A run is cut into tiles of kRows rows from the 128-row
+// boundary at or before its start (where its scale atoms are), so that every tile is worked once, for one expert, and the tiles
+// of all runs are dealt out alike.  (Tiles on fixed boundaries were worked once per run in them, one pass after the other by the CTA that
+// had them: ten uneven experts on 8192 x 4096 x 4096 MXFP8, pair tile, 152 us where one expert takes 113;
+// NVFP4 40960 x 4096 x 4096 324 and 293.)
+// Entry i: first 64-row quarter of run i, and its expert << 16; the entry behind the last run ends it.
+struct RunTable {
+    const uint32_t* runs;  // null: the rows have more runs, or more quarters, than the table can hold
+    int row_tiles;
+};
+
+// Tiles of kRows rows in the run between two entries.
+template <int kRows>
+__device__ __forceinline__ int run_tiles(uint32_t entry, uint32_t next) {
+    const int first = int(entry & 0xffffu) / 2 * 128;
+    return (int(next & 0xffffu) * 64 - first + kRows - 1) / kRows;
+}
+
+// Called by all threads of the block, kBlock of them, after the wait for the preceding kernel.
+template <int kRows, int kBlock>
+__device__ __forceinline__ RunTable build_runs(const GroupParams& g, int m, Barriers* bars, uint32_t* runs) {
+    static_assert(kBlock / 32 <= 16, "Barriers::run_counts");
+    const int nq = m / 64;
+    if (nq > 0xffff || g.count > 0x10000) return {nullptr, 0};
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    int total = 0;
+    constexpr int kRounds = 2;  // loads in flight per thread
+    for (int b = 0; b < nq; b += kRounds * kBlock) {
+        int id[kRounds], before[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            const int q = b + r * kBlock + int(threadIdx.x);
+            id[r] = q < nq ? __ldg(g.table + q * 64) : 0;
+            before[r] = q < nq && q > 0 ? __ldg(g.table + q * 64 - 64) : ~id[r];
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            if (b + r * kBlock >= nq) break;
+            const int q = b + r * kBlock + int(threadIdx.x);
+            const bool starts = q < nq && id[r] != before[r];
+            const uint32_t ballot = __ballot_sync(0xffffffffu, starts);
+            if (lane == 0) bars->run_counts[warp] = __popc(ballot);
+            __syncthreads();
+            int at = total + __popc(ballot & ((1u << lane) - 1u));
+#pragma unroll
+            for (int w = 0; w < kBlock / 32; ++w) {
+                const int c = bars->run_counts[w];
+                at += w < warp ? c : 0;
+                total += c;
+            }
+            if (starts && at < kMaxRuns) runs[at] = uint32_t(q) | (uint32_t(min(max(id[r], 0), g.count - 1)) << 16);
+            __syncthreads();
+        }
+    }
+    if (total > kMaxRuns) return {nullptr, 0};
+    if (threadIdx.x == 0) runs[total] = uint32_t(nq);
+    __syncthreads();
+    if (warp == 0) {
+        int tiles = 0;
+        for (int i = lane; i < total; i += 32) tiles += run_tiles<kRows>(runs[i], runs[i + 1]);
+        tiles = __reduce_add_sync(0xffffffffu, tiles);
+        if (lane == 0) bars->run_counts[0] = tiles;
+    }
+    __syncthreads();
+    return {runs, bars->run_counts[0]};
+}
+
+// A role's place in the runs: row tile `rt` of them, by steps from the last one asked for.
+template <int kRows>
+struct RunWalk {
+    RunTable t;
+    int run = 0, base = 0;  // the run of the last row tile, and the row tiles before it
+
+    __device__ __forceinline__ int tiles(int i) const { return run_tiles<kRows>(t.runs[i], t.runs[i + 1]); }
+    // first row of the tile, the rows [lo, hi) of it that are the run's, and the expert
+    __device__ __forceinline__ void find(int rt, int& row0, int& lo, int& hi, int& expert) {
+        for (int c = tiles(run); rt >= base + c; c = tiles(run)) {
+            base += c;
+            ++run;
+        }
+        while (rt < base) {
+            --run;
+            base -= tiles(run);
+        }
+        const uint32_t e = t.runs[run];
+        const int start = int(e & 0xffffu) * 64;
+        row0 = start / 128 * 128 + (rt - base) * kRows;
+        lo = max(0, start - row0);
+        hi = min(kRows, int(t.runs[run + 1] & 0xffffu) * 64 - row0);
+        expert = int(e >> 16);
+    }
+};
+
 // What one persistent-loop iteration of the single-CTA kernel works on.
 struct Work {
     int a_row0;     // first row of the A box (and 128 x its scale-atom row)
@@ -233,10 +334,13 @@ struct WorkIter {
     int walk_base = 0;   //   (group, row tile) pairs before it
 
     int stride;          // work items between two items of this CTA (or cluster)
+    RunWalk<kBM> runs;   // contiguous
 
-    __device__ WorkIter(const GroupParams& grp, int m, int n, int tm, int tn, int first = blockIdx.x,
+    __device__ WorkIter(const GroupParams& grp, int m, int n, int tm, int tn, const RunTable& rt, int first = blockIdx.x,
                         int step = gridDim.x)
-        : g(grp), M(m), N(n), tiles_m(tm), tiles_n(tn), tile(first), stride(step) {}
+        : g(grp), M(m), N(n), tiles_m(tm), tiles_n(tn), tile(first), stride(step), runs{rt} {
+        if (g.kind == kGroupContiguous && rt.runs != nullptr) tiles_m = rt.row_tiles;
+    }
 
     __device__ __forceinline__ void set_b(Work& w, int group, int nt) const {
         w.group = group;
@@ -251,12 +355,19 @@ struct WorkIter {
         if (g.kind == kGroupDense || g.kind == kGroupContiguous) {
             if (tile >= tiles_m * tiles_n) return false;
             const TileCoord tc = tile_coord(tile, tiles_m, tiles_n);
+            w.out_col0 = tc.n * BN;
+            int group = 0;
+            if (g.kind == kGroupContiguous && runs.t.runs != nullptr) {
+                runs.find(tc.m, w.a_row0, w.row_lo, w.row_hi, group);
+                w.out_row0 = w.a_row0;
+                set_b(w, group, tc.n);
+                tile += stride;
+                return true;
+            }
             w.a_row0 = tc.m * kBM;
             w.out_row0 = w.a_row0;
-            w.out_col0 = tc.n * BN;
             w.row_lo = 0;
             w.row_hi = min(kBM, M - w.a_row0);
-            int group = 0;
             if (g.kind == kGroupContiguous) {
                 const int e0 = __ldg(g.table + w.a_row0);
                 const int e1 = w.a_row0 + 64 < M ? __ldg(g.table + w.a_row0 + 64) : e0;
@@ -585,13 +696,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     // Everything above overlaps the tail of the previous kernel under a
     // programmatic launch; nothing below may run before its writes are visible.
     ptx::pdl_wait();
+    RunTable run_table = {nullptr, 0};
+    if (!kDense && grp.kind == kGroupContiguous) {
+        run_table = build_runs<kBM, kThreads>(grp, M, bars, reinterpret_cast<uint32_t*>(smem + bar_off + 1024));
+    }
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         {
             uint32_t it = 0;
             bool ok = true;
-            WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
+            WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, run_table, first_item, item_step);
             Work wk;
             while (ok && work.next(wk)) {
                 const int m0 = wk.a_row0;
@@ -642,7 +757,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             uint32_t it = 0;
             uint32_t t = 0;
             bool ok = true;
-            WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
+            WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, run_table, first_item, item_step);
             Work wk;
             for (; ok && work.next(wk); ++t) {
                 const uint32_t as = t & 1u;
@@ -730,7 +845,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         const uint32_t quarter = (uint32_t(warp) & 3u) * 32u;
         uint32_t it = 0;
         bool ok = true;
-        WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
+        WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, run_table, first_item, item_step);
         Work wk;
         while (ok && work.next(wk)) {
             for (int kt = k_begin; kt < k_end; ++kt, ++it) {
@@ -776,7 +891,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         uint32_t t = 0;
         uint32_t stores = 0;
         bool ok = true;
-        WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, first_item, item_step);
+        float scale = 1.0f;
+        int scale_group = -1;
+        WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, run_table, first_item, item_step);
         Work wk;
         const int ar = int(lane_base) + lane;  // accumulator row of this thread
         if (!kDense && situ.sf != nullptr) zero_sf_padding(situ, (warp - 2) * 32 + lane);
@@ -786,13 +903,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             // this warp's 32 rows are all padding or all belong to a neighbouring group
             const bool warp_idle = int(lane_base) >= wk.row_hi || int(lane_base) + 32 <= wk.row_lo;
             const bool row_ok = ar >= wk.row_lo && ar < wk.row_hi;
-            // whole tiles go out through TMA stores (a dense tail is clipped by the tensor map);
-            // partial tiles are stored from registers, row by row, and so are tiles of at most
+            // rows go out through TMA stores (a dense tail is clipped by the tensor map), except where only some of
+            // this warp's are the item's: those are stored from registers, row by row, and so are tiles of at most
             // 32 rows (one warp, no staging round trip)
-            const bool reg_store = direct_store != 0 || wk.row_lo != 0 || wk.row_hi <= 32 ||
-                                   (wk.row_hi != kBM && grp.kind != kGroupDense);
+            const bool warp_whole = int(lane_base) >= wk.row_lo && int(lane_base) + 32 <= wk.row_hi;
+            const bool reg_store = direct_store != 0 || (wk.row_lo == 0 && wk.row_hi <= 32) ||
+                                   (!warp_whole && grp.kind != kGroupDense);
             // per-tensor (dense) or per-group factor of the NVFP4 recipe
-            const float scale = (KIND == 1 && alpha != nullptr) ? __ldg(alpha + wk.group) : 1.0f;
+            if (KIND == 1 && alpha != nullptr && wk.group != scale_group) {
+                scale = __ldg(alpha + wk.group);
+                scale_group = wk.group;
+            }
             const uint32_t as = t & 1u;
             const uint32_t aph = (t >> 1) & 1u;
             ok = wait_bar(ptx::smem_u32(&bars->acc_full[as]), aph, abort, kStatusEpilogue);
@@ -1099,7 +1220,7 @@ struct Cfg2 {
     static constexpr int kStageTxBytes = kABytes + kBBytes - (KIND == 3 ? kBBytes / 2 : 0);
     static constexpr int kEpiBufs = 2;
     static constexpr int kEpiBytes = kEpiWarps * kEpiBufs * kEpiBufBytes;
-    static constexpr int kBarBytes = 1024;
+    static constexpr int kBarBytes = 1024 + kRunBytes;  // barriers, then the runs of contiguous experts
     static constexpr int kStagesFit = (kSmemBudget - kEpiBytes - kBarBytes - 1024) / kStageBytes;
     static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;
     static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + kBarBytes + 1024;
@@ -1154,10 +1275,9 @@ struct PairWork {
 // The grouped kinds on the 2-CTA tile (kGrouped; dense otherwise).  Batches and masked experts
 // take it when their row count is a multiple of 256, so that no tile holds rows of two of
 // them; an item is (expert, 256-row tile that holds valid rows of it, column tile).  The
-// contiguous layout takes it when M is a multiple of 256: a tile whose four 64-row quarters
-// belong to several experts is worked once per run of equal experts, each pass storing its own
-// rows (the rule of the single-CTA kernel, with 256-row tiles).  The roles of the kernel walk
-// the same sequence of items, each with its own copy of this iterator.
+// contiguous layout is cut into tiles by runs of experts (RunTable); with more runs than the table holds, a tile
+// whose four 64-row quarters belong to several experts is worked once per run of equal experts, each pass storing
+// its own rows.  The roles of the kernel walk the same sequence of items, each with its own copy of this iterator.
 template <int BN, bool kGrouped>
 struct PairWorkIter {
     GroupParams g;
@@ -1166,9 +1286,12 @@ struct PairWorkIter {
     int pass = 0;        // contiguous: run of the current tile to work next
     int walk_group = 0;  // batch / masked: group of the last item and the number of
     int walk_base = 0;   //   (group, row tile) pairs before it
+    RunWalk<256> runs;   // contiguous
 
-    __device__ PairWorkIter(const GroupParams& grp, int m, int n, int tm, int tn, int first, int step)
-        : g(grp), M(m), N(n), tiles_m(tm), tiles_n(tn), tile(first), stride(step) {}
+    __device__ PairWorkIter(const GroupParams& grp, int m, int n, int tm, int tn, const RunTable& rt, int first, int step)
+        : g(grp), M(m), N(n), tiles_m(tm), tiles_n(tn), tile(first), stride(step), runs{rt} {
+        if (kGrouped && g.kind == kGroupContiguous && rt.runs != nullptr) tiles_m = rt.row_tiles;
+    }
 
     __device__ __forceinline__ void set_b(PairWork& w, int group, int nt) const {
         w.group = group;
@@ -1178,17 +1301,40 @@ struct PairWorkIter {
         w.bias_col0 = w.b_row0;
     }
 
+    // How many items next() will give: the roles that work k-tiles whatever they belong to (scales, MMAs) count them down
+    // instead of walking.  -1: only the walk can tell (contiguous experts without a run table).
+    __device__ int items() const {
+        int row_tiles = tiles_m;
+        if constexpr (kGrouped) {
+            if (g.kind == kGroupContiguous && runs.t.runs == nullptr) return -1;
+            if (g.kind == kGroupBatch) row_tiles = g.count * ((g.rows + 255) / 256);
+            if (g.kind == kGroupMasked) {
+                row_tiles = 0;
+                for (int e = 0; e < g.count; ++e) row_tiles += (min(max(__ldg(g.table + e), 0), g.rows) + 255) / 256;
+            }
+        }
+        const int total = row_tiles * tiles_n;
+        return tile < total ? (total - tile + stride - 1) / stride : 0;
+    }
+
     __device__ bool next(PairWork& w) {
         if (!kGrouped || g.kind == kGroupContiguous) {
             if (tile >= tiles_m * tiles_n) return false;
             const TileCoord tc = tile_coord(tile, tiles_m, tiles_n);
-            w.a_row0 = tc.m * 256;
-            w.out_row0 = w.a_row0;
             w.out_col0 = tc.n * BN;
-            w.row_lo = 0;
-            w.row_hi = min(256, M - w.a_row0);
             int group = 0;
             bool last = true;
+            if (kGrouped && runs.t.runs != nullptr) {
+                runs.find(tc.m, w.a_row0, w.row_lo, w.row_hi, group);
+                w.out_row0 = w.a_row0;
+                set_b(w, group, tc.n);
+                tile += stride;
+                return true;
+            }
+            w.a_row0 = tc.m * 256;
+            w.out_row0 = w.a_row0;
+            w.row_lo = 0;
+            w.row_hi = min(256, M - w.a_row0);
             if constexpr (kGrouped) {
                 int e[4];
 #pragma unroll
@@ -1277,6 +1423,36 @@ struct GatherMaps<true> {
     int count;
 };
 
+// The epilogue of a warp of which some or none of the 32 rows are the item's: each thread stores its own row from
+// registers, or nothing (`out` null).  A function of its own: in a branch inside the chunk loop it cost every tile 8 %, full
+// ones too (32768 x 3072 x 1280 NVFP4 in one batch 102.7 us with it there, 94.9 without).
+template <typename C>
+__device__ __noinline__ void partial_rows(uint32_t acc, bool second_stage, __nv_bfloat16* out, float scale,
+                                          const __nv_bfloat16* bias, int epi_op, int cols, uint32_t overlap_free,
+                                          uint32_t acc_empty) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int ci = 0; ci < C::kChunks; ++ci) {
+        const int c = (C::kOverlap != 0 && !second_stage) ? C::kChunks - 1 - ci : ci;
+        uint32_t r[32];
+        ptx::tc_load_32x32(acc + c * kEpiChunk, r);
+        ptx::tc_wait_ld();
+        const bool overlap_read = C::kOverlap != 0 && ci == C::kOverlapChunks - 1;
+        if (overlap_read || ci == C::kChunks - 1) {
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0 && overlap_read) ptx::mbar_arrive_cluster_relaxed(overlap_free);
+            if (lane == 0 && ci == C::kChunks - 1) ptx::mbar_arrive_cluster_relaxed(acc_empty);
+        }
+        if (out == nullptr || c * kEpiChunk >= cols) continue;
+        uint32_t p[16];
+        epilogue_chunk(r, p, scale, bias != nullptr ? bias + c * kEpiChunk : nullptr, epi_op);
+        uint4* const dst = reinterpret_cast<uint4*>(out + c * kEpiChunk);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dst[j] = make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+    }
+}
+
 // The SiTU-GLU quantising epilogue's outputs (kSitu; dense MXFP8 only).
 template <bool kSitu>
 struct PairSitu {};
@@ -1362,13 +1538,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         __syncwarp();
     }
     ptx::pdl_wait();
+    RunTable run_table = {nullptr, 0};
+    if constexpr (kGrouped) {
+        if (ga.grp.kind == kGroupContiguous) {
+            run_table = build_runs<256, C::kThreads>(ga.grp, ga.m, bars, reinterpret_cast<uint32_t*>(smem + bar_off + 1024));
+        }
+    }
 
     if (warp == 0) {
         // ------------------------------------------------------------ box loader (both CTAs)
         {
             uint32_t it = 0;
             bool ok = true;
-            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, run_table, cluster_id, num_clusters);
             PairWork wk;
             while (ok && walk.next(wk)) {
                 const int m0 = wk.a_row0 + int(rank) * kBM;
@@ -1394,7 +1576,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         {
             uint32_t it = 0;
             bool ok = true;
-            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, run_table, cluster_id, num_clusters);
             PairWork wk;
             while (ok && walk.next(wk)) {
                 const int sfa_atom_row = (wk.a_row0 / 128 + int(rank)) * kq_dim;
@@ -1426,9 +1608,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const uint32_t quarter = (uint32_t(warp) & 3u) * 32u;
         uint32_t it = 0;
         bool ok = true;
-        Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+        Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, run_table, cluster_id, num_clusters);
         PairWork wk;
-        while (ok && walk.next(wk)) {
+        int left = walk.items();
+        while (ok && (left >= 0 ? left-- > 0 : walk.next(wk))) {
             for (int kt = 0; kt < k_tiles; ++kt, ++it) {
                 const uint32_t s = it % C::kStages;
                 ok = wait_bar(ptx::smem_u32(&bars->sf_full[s]), (it / C::kStages) & 1u, abort, kStatusProducer);
@@ -1462,9 +1645,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             uint32_t it = 0;
             uint32_t t = 0;
             bool ok = true;
-            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+            Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, run_table, cluster_id, num_clusters);
             PairWork wk;
-            for (; ok && walk.next(wk); ++t) {
+            int left = walk.items();
+            for (; ok && (left >= 0 ? left-- > 0 : walk.next(wk)); ++t) {
                 const uint32_t as = t & 1u;
                 const uint32_t aph = (t >> 1) & 1u;
                 const uint32_t acc = tmem + as * C::kAccStride;
@@ -1548,20 +1732,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         uint32_t t = 0;
         uint32_t stores = 0;
         bool ok = true;
+        float scale = 1.0f;
+        int scale_group = -1;
         if constexpr (kSitu) zero_sf_padding(situ.p, (warp - 2) * 32 + lane);
-        Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, cluster_id, num_clusters);
+        // The grouped kinds keep their place in shared memory: a dozen registers less through the loop over the chunks.  With
+        // that and the item count of the other roles 32768 x 3072 x 1280 NVFP4 in one batch took 93 us instead of 99.
+        static_assert(sizeof(Iter) * kEpiWarps <= 1024 - kKeptOffset, "behind the barriers");
+        Iter* const kept = reinterpret_cast<Iter*>(smem + bar_off + kKeptOffset);
+        Iter walk(ga.grp, ga.m, ga.n, tiles_m, tiles_n, run_table, cluster_id, num_clusters);
+        if (kGrouped) {
+            if (lane == 0) kept[ew] = walk;
+            __syncwarp();
+        }
+        const auto next = [&](PairWork& w) {
+            if constexpr (!kGrouped) return walk.next(w);
+            Iter at = kept[ew];
+            const bool more = at.next(w);
+            __syncwarp();
+            if (lane == 0) kept[ew] = at;
+            __syncwarp();
+            return more;
+        };
         PairWork wk;
-        for (; ok && walk.next(wk); ++t) {
+        for (; ok && next(wk); ++t) {
             const int m0 = wk.out_row0 + int(rank) * kBM;
             const int n0 = wk.out_col0;
             // rows of this CTA's half of the tile that belong to the item
             const int half_lo = min(max(wk.row_lo - int(rank) * kBM, 0), kBM);
             const int half_hi = min(max(wk.row_hi - int(rank) * kBM, 0), kBM);
-            // (a dense tile that sticks out beyond M is clipped by the TMA store; the grouped kinds
-            // come here with whole tiles inside M only)
-            const bool partial = kGrouped && (half_lo != 0 || half_hi != kBM);
+            // Of a warp's 32 rows all, none or (masked) some are the item's.  (A dense tile that sticks out beyond M is clipped by the TMA store.)
+            const bool partial = kGrouped && (int(lane_base) < half_lo || int(lane_base) + 32 > half_hi);
             // per-tensor (dense) or per-group factor of the NVFP4 recipe
-            const float scale = (KIND == 1 && alpha != nullptr) ? __ldg(alpha + wk.group) : 1.0f;
+            if (KIND == 1 && alpha != nullptr && wk.group != scale_group) {
+                scale = __ldg(alpha + wk.group);
+                scale_group = wk.group;
+            }
             const uint32_t as = t & 1u;
             const uint32_t aph = (t >> 1) & 1u;
             ok = wait_bar(ptx::smem_u32(&bars->acc_full[as]), aph, abort, kStatusEpilogue);
@@ -1612,6 +1817,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     }
                 }
                 continue;
+            }
+            if constexpr (kGrouped) {
+                if (partial) {
+                    const int row = int(lane_base) + lane;
+                    const bool row_ok = row >= half_lo && row < half_hi;
+                    partial_rows<C>(acc, as != 0, row_ok ? ga.out + int64_t(m0 + row) * ga.ldo + n0 : nullptr, scale,
+                                    bias != nullptr ? bias + wk.bias_col0 : nullptr, epi_op, wk.cols,
+                                    ptx::mapa_cluster(ptx::smem_u32(&bars->overlap_free[as]), 0),
+                                    ptx::mapa_cluster(ptx::smem_u32(&bars->acc_empty[as]), 0));
+                    continue;
+                }
             }
             // chunks shared with the other accumulator stage are read into registers first (as
             // in the single-CTA kernel), so that the next tile's MMAs may start early
@@ -1665,22 +1881,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 if (c * kEpiChunk >= wk.cols) continue;
                 uint32_t p[16];
                 epilogue_chunk(r, p, scale, bias != nullptr ? bias + wk.bias_col0 + c * kEpiChunk : nullptr, epi_op);
-                if constexpr (kGrouped) {
-                    if (partial) {
-                        // only some rows of this half belong to the item: each thread stores its
-                        // own row's 32 columns from registers, or nothing
-                        const int r_half = int(lane_base) + lane;
-                        if (r_half >= half_lo && r_half < half_hi) {
-                            uint4* const dst = reinterpret_cast<uint4*>(ga.out + int64_t(m0 + r_half) * ga.ldo + n0 +
-                                                                        c * kEpiChunk);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                dst[j] = make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
-                            }
-                        }
-                        continue;
-                    }
-                }
                 if constexpr (kGather) {
                     // Two neighbouring chunks are staged as ONE box of 32 rows x 128 bytes (the warp's
                     // two buffers, 128-byte swizzle) and stored together: rows of 128 bytes use
@@ -1922,7 +2122,9 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
         }
     }
     const int tiles_n = (g.n + BN - 1) / BN;
-    const int grid = min(g.sm_count, tiles_m * tiles_n);
+    // contiguous: the runs are cut into at most a tile each more than the rows alone
+    const int64_t row_tiles = g.grp.kind == kGroupContiguous ? std::min<int64_t>(g.m / 64, int64_t(tiles_m) + g.grp.count) : tiles_m;
+    const int grid = int(std::min<int64_t>(g.sm_count, row_tiles * tiles_n));
     const int k_tiles = int(g.k_bytes / kBKBytes);
     if constexpr (BN == 64) {
         // One row of at most sm_count / 2 tiles and a long K: two CTAs per tile, half of K each.
@@ -2025,7 +2227,8 @@ int launch_pair(const GemmArgs& g, char* err, size_t errlen, __nv_bfloat16* cons
         HQ_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<BN, KIND, kGather, kGrouped, kSitu>, &occ));
         max_clusters[slot] = n > 0 ? n : 1;
     }
-    const int clusters = min(min(g.sm_count / 2, max_clusters[slot]), tiles_m * tiles_n);
+    const int64_t row_tiles = kGrouped && g.grp.kind == kGroupContiguous ? std::min<int64_t>(g.m / 64, int64_t(tiles_m) + g.grp.count) : tiles_m;
+    const int clusters = int(std::min<int64_t>(min(g.sm_count / 2, max_clusters[slot]), row_tiles * tiles_n));
     const int k_tiles = int(g.k_bytes / kBKBytes);
     GatherMaps<kGather> peers{};
     if constexpr (kGather) {
@@ -2405,20 +2608,20 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool
         const Cand& c = cands[i];
         if (c.pair && (m <= kBM || !pair_open)) continue;
         const int64_t rows = c.pair ? tiles_m2 : tiles_m;
-        const int64_t tiles = rows * ((n + c.bn - 1) / c.bn);
+        const int64_t cols = (n + c.bn - 1) / c.bn;
         const int64_t units = c.pair ? sm_count / 2 : sm_count;
         if (units < 1) continue;
-        // Contiguous experts (runs of rows that start on multiples of 64): a CTA works a tile with a boundary inside
-        // once per run, one after the other.  Half of the boundaries are inside a 128-row tile, which has room
-        // for one, three of four inside a 256-row one, which has room for three.  (The pace is left as it is: with the passes on
-        // it too the choice was 2.5 % off.)  On 80 problems (512 to 16384 rows, 8 to 256 experts, MXFP8 and NVFP4) choosing by
-        // this costs 0.02 % (MXFP8) and 0.4 % (NVFP4) over the best tile of each; with other figures for the tiles it was
-        // 3.6 % and 0.9 % without a term for the boundaries, 9.1 % and 6.0 % counting them as tiles of their own, which other
-        // CTAs could take (16 experts on 512 rows, N = K = 2048: 16.3 us; now 10.8).
-        const double passes = 1.0 + std::min(c.pair ? 3.0 : 1.0, double(boundaries) * (c.pair ? 0.75 : 0.5) / double(rows));
-        const double waves = double((tiles + units - 1) / units) * passes;
+        // Contiguous experts: every run is cut into tiles of its own, so a boundary adds part of a tile of rows (and no more
+        // than one per 64 rows), and such tiles work for rows that they do not have, which tells against wide ones.
+        // Fitted to 80 problems of many short runs (512 to 16384 rows, 8 to 256 experts, MXFP8 and NVFP4), each timed on
+        // every tile: 2.6 % (MXFP8) and 1.3 % (NVFP4) over the best of each, some of it because the suite holds 16 experts
+        // on 4096 x 4096 x 2048 to the 128 x 128 tile (48.7 us; 46.4 on 128 x 256).
+        const double extra = std::min(0.4 * double(boundaries), double(m) / 64.0 - double(rows));
+        const double tiles = boundaries > 0 ? (double(rows) + std::max(extra, 0.0)) * double(cols) : double(rows * cols);
+        const double idle = std::min(c.pair ? 3.0 : 1.0, double(boundaries) * (c.pair ? 0.75 : 0.5) / double(rows)) * c.bn / 256.0;
+        const double waves = std::ceil(tiles / double(units)) * (1.0 + (c.pair ? 0.4 : 0.6) * idle);
         const double cost = c.us_fixed + std::max(waves * (k_tiles * c.us_per_ktile + c.us_per_wave),
-                                                  double(tiles) / double(units) * k_tiles * c.us_paced);
+                                                  tiles / double(units) * k_tiles * c.us_paced * (1.0 + 0.3 * idle));
         if (best.bn == 0 || cost < best_cost * 0.999) {
             best = {c.bn, c.pair};
             best_cost = cost;
@@ -2716,7 +2919,7 @@ TilePick pick_tile_grouped(int kind, int64_t count, int64_t rows, int64_t total_
     // The 2-CTA tile: a plain epilogue, and no 256-row tile may hold rows of two
     // batches or expert slots (the contiguous layout is worked per run of experts, see
     // PairWorkIter).  Otherwise a forced or modelled pair choice falls back to the same width.
-    const bool whole_tiles = kind == kGroupContiguous ? total_m % 256 == 0 : rows % 256 == 0;
+    const bool whole_tiles = kind == kGroupContiguous || rows % 256 == 0;
     if (!(plain_epilogue && whole_tiles)) pick.pair = false;
     return pick;
 }

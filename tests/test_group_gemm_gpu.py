@@ -480,3 +480,29 @@ def test_fp4_experts_on_the_2cta_tile(hq, monkeypatch, mode, tile):
                         _contiguous_case(hq, [64, 192, 128, 640, 256], 512, 2048, mode),
                         _contiguous_case(hq, [64] * 4, 256, 256, mode)))
     assert all(torch.equal(x, y) for x, y in zip(*results))
+
+
+@pytest.mark.parametrize("tile", ["128", "256", "pair128", "pair256"])
+@pytest.mark.parametrize("counts", [
+    [64], [192, 64],                                   # fewer rows than a tile
+    [64, 320, 0, 64, 448, 64],                         # starts on odd multiples of 64, a last tile beyond M
+    [64] * 255, [64] * 256,                            # as many runs as the table holds, and one more
+    [64, 0] * 20 + [49152, 64, 192],                   # more quarters than the block has threads, twice
+], ids=lambda v: f"{len(v)}runs{sum(v)}")
+def test_contiguous_runs_and_their_tiles(hq, monkeypatch, tile, counts):
+    """Every run of experts is cut into tiles of its own, whatever the number of runs and rows."""
+    monkeypatch.setenv("HALOPS_B200_TILE", tile)
+    _contiguous_case(hq, counts, 384 if sum(counts) < 1000 else 128, 256, "w8a8-mxfp8", check_rows=1024)
+
+
+def test_contiguous_experts_in_any_order(hq, monkeypatch):
+    """Runs of one expert may come back, in any order; rows whose id is out of range take the nearest expert."""
+    ids = np.repeat(np.array([2, 0, 2, 1, 1, 0, 3, 9, -4], dtype=np.int32), 64)
+    xq, wq, sfa, sfb = _inputs(hq, ids.size, 4, 256, 256, "w8a8-mxfp8", seed=21)
+    ref = oracle.group_gemm_ref(xq, wq, sfa, sfb, np.clip(ids, 0, 3).astype(np.int64), "w8a8-mxfp8")
+    for tile in ("64", "256", "pair256"):
+        monkeypatch.setenv("HALOPS_B200_TILE", tile)
+        out = torch.full([ids.size, 256], float("nan"), dtype=torch.bfloat16, device="cuda")
+        hq.group_contiguous_gemm(xq, wq, sfa, sfb, torch.from_numpy(ids).cuda(), out)
+        assert hq.device_status() == 0
+        _compare(out, ref, np.arange(ids.size), "w8a8-mxfp8", None)
