@@ -116,9 +116,9 @@ struct Barriers {
     uint64_t epi_sync;     // small-M kernel: rendezvous of the four epilogue warps (a bounded wait, unlike bar.sync)
     uint32_t tmem_base;
     uint32_t abort;
-    int run_counts[16];  // contiguous experts: runs that start in a warp's share of the rows; [0] in the end: row tiles
+    int run_counts[16];  // contiguous experts: runs that start in a warp's share of the rows
 };
-constexpr int kKeptOffset = 640;  // pair kernel: the epilogue warps' places in the walk, behind the barriers
+constexpr int kKeptOffset = 576;  // pair kernel: the epilogue warps' places in the walk, behind the barriers
 static_assert(sizeof(Barriers) <= kKeptOffset, "kBarBytes");
 
 // Bounded mbarrier wait of one lane.  Returns false when the CTA is aborting.  kCluster: the barrier is one
@@ -263,45 +263,46 @@ __device__ __forceinline__ RunTable build_runs(const GroupParams& g, int m, Barr
                 total += c;
             }
             if (starts && at < kMaxRuns) runs[at] = uint32_t(q) | (uint32_t(min(max(id[r], 0), g.count - 1)) << 16);
-            __syncthreads();
+            if (b + (r + 1) * kBlock < nq) __syncthreads();  // run_counts are written again
         }
     }
     if (total > kMaxRuns) return {nullptr, 0};
     if (threadIdx.x == 0) runs[total] = uint32_t(nq);
     __syncthreads();
-    if (warp == 0) {
-        int tiles = 0;
-        for (int i = lane; i < total; i += 32) tiles += run_tiles<kRows>(runs[i], runs[i + 1]);
-        tiles = __reduce_add_sync(0xffffffffu, tiles);
-        if (lane == 0) bars->run_counts[0] = tiles;
-    }
-    __syncthreads();
-    return {runs, bars->run_counts[0]};
+    int tiles = 0;  // every warp for itself
+    for (int i = lane; i < total; i += 32) tiles += run_tiles<kRows>(runs[i], runs[i + 1]);
+    return {runs, int(__reduce_add_sync(0xffffffffu, tiles))};
 }
 
 // A role's place in the runs: row tile `rt` of them, by steps from the last one asked for.
 template <int kRows>
 struct RunWalk {
     RunTable t;
-    int run = 0, base = 0;  // the run of the last row tile, and the row tiles before it
+    int run = -1, base = 0, count = 0;  // the run of the last row tile, the row tiles before it and in it
+    uint32_t entry = 0, next = 0;       // its entry and the one behind it
 
-    __device__ __forceinline__ int tiles(int i) const { return run_tiles<kRows>(t.runs[i], t.runs[i + 1]); }
+    __device__ __forceinline__ void take(int i) {
+        run = i;
+        entry = t.runs[i];
+        next = t.runs[i + 1];
+        count = run_tiles<kRows>(entry, next);
+    }
     // first row of the tile, the rows [lo, hi) of it that are the run's, and the expert
     __device__ __forceinline__ void find(int rt, int& row0, int& lo, int& hi, int& expert) {
-        for (int c = tiles(run); rt >= base + c; c = tiles(run)) {
-            base += c;
-            ++run;
+        if (run < 0) take(0);
+        while (rt >= base + count) {
+            base += count;
+            take(run + 1);
         }
         while (rt < base) {
-            --run;
-            base -= tiles(run);
+            take(run - 1);
+            base -= count;
         }
-        const uint32_t e = t.runs[run];
-        const int start = int(e & 0xffffu) * 64;
+        const int start = int(entry & 0xffffu) * 64;
         row0 = start / 128 * 128 + (rt - base) * kRows;
         lo = max(0, start - row0);
-        hi = min(kRows, int(t.runs[run + 1] & 0xffffu) * 64 - row0);
-        expert = int(e >> 16);
+        hi = min(kRows, int(next & 0xffffu) * 64 - row0);
+        expert = int(entry >> 16);
     }
 };
 
