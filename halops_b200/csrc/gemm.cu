@@ -28,6 +28,8 @@
 
 #include <cuda_bf16.h>
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -2054,15 +2056,46 @@ struct GemmArgs {
     cudaStream_t stream;
 };
 
+// The environment switches (HALOPS_B200_*, for experiments and tests), read on every call: entry points that lead to one
+// of them begin with a SwitchScope, which goes through the environment once.  (A dense call made six to nine getenv, 106 ns
+// each among 135 variables: 3.9 -> 3.6 us of the host's time per call with the shape rule taken out of the cost model.)
+struct Switches {
+    const char* tile = nullptr;
+    const char* splitk = nullptr;
+    const char* issuers = nullptr;
+    const char* decode = nullptr;
+    const char* epilogue = nullptr;
+};
+thread_local Switches t_switches;
+
+struct SwitchScope {
+    SwitchScope() {
+        Switches s;
+        for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
+            if ((*e)[0] != 'H' || strncmp(*e, "HALOPS_B200_", 12) != 0) continue;
+            const auto take = [v = *e + 12](const char* name, const char*& value) {
+                const size_t len = strlen(name);
+                if (value == nullptr && strncmp(v, name, len) == 0 && v[len] == '=') value = v + len + 1;
+            };
+            take("TILE", s.tile);
+            take("SPLITK", s.splitk);
+            take("ISSUERS", s.issuers);
+            take("DECODE", s.decode);
+            take("EPILOGUE", s.epilogue);
+        }
+        t_switches = s;
+    }
+};
+
 // Split-K is taken for a dense problem with one row of at most sm_count / 2 64-wide tiles and at least 192 k-tiles
 // (HALOPS_B200_SPLITK=0 turns it off; read on every call).  The cluster and its exchange cost 3.6 us: behind
 // a quantizer the split took 9.1 us at 8 k-tiles and 0.133 for each further one, the whole tile 5.5 and 0.154 (16 problems of 65 to
 // 128 rows; 69 x 1088 x 1024 9.1 against 5.5, 65 x 1088 x 4992 13.1 against 10.4, 80 x 1792 x 7680 15.8 against 13.5).
 // With the 64-wide tile forced, from 8 k-tiles on.
 bool split_k_chosen(int group_kind, int tiles_m, int tiles_n, int k_tiles, int sm_count, int epi_op) {
-    const char* e = getenv("HALOPS_B200_SPLITK");
+    const char* e = t_switches.splitk;
     if (e != nullptr && e[0] == '0') return false;
-    const char* forced = getenv("HALOPS_B200_TILE");
+    const char* forced = t_switches.tile;
     const int least = forced != nullptr && strcmp(forced, "64") == 0 ? 8 : 192;
     return group_kind == kGroupDense && tiles_m == 1 && 2 * tiles_n <= sm_count && k_tiles >= least &&
            (epi_op == HQ_EPILOGUE_IDENTITY || epi_op == HQ_EPILOGUE_SIGMOID);
@@ -2071,7 +2104,7 @@ bool split_k_chosen(int group_kind, int tiles_m, int tiles_n, int k_tiles, int s
 // 2: the single-CTA kernel issues its MMAs from two threads in k order (see the kernel);
 // 0 with HALOPS_B200_ISSUERS=1 (read on every call)
 int issuers_in_order() {
-    const char* e = getenv("HALOPS_B200_ISSUERS");
+    const char* e = t_switches.issuers;
     return e != nullptr && e[0] == '1' ? 0 : 2;
 }
 
@@ -2260,7 +2293,7 @@ struct DecodeSwitches {
 };
 DecodeSwitches decode_switches() {
     DecodeSwitches d;
-    const char* e = getenv("HALOPS_B200_DECODE");
+    const char* e = t_switches.decode;
     if (e == nullptr) return d;
     d.off = strstr(e, "off") != nullptr;
     d.nosplit = strstr(e, "nosplit") != nullptr;
@@ -2273,7 +2306,7 @@ DecodeSwitches decode_switches() {
 // Small M goes to the operand-swapped kernel: dense MXFP8 without bias, plain or sigmoid
 // epilogue, no forced tile.
 bool decode_eligible(int64_t m, int64_t n, int64_t k, int mode, int epi_op, bool has_bias) {
-    const char* forced = getenv("HALOPS_B200_TILE");
+    const char* forced = t_switches.tile;
     if (forced != nullptr && forced[0] != '\0') return false;
     if ((n / 128 + 1) * (k / 256 + 1) >= (int64_t(1) << 31)) return false;
     // Up to 64 activation rows by default.  With 65 to 128 a stage is half activations, the
@@ -2544,14 +2577,19 @@ struct TilePick {
 // multiple of 64 left the 64-wide tile alone (3000 x 7232 x 4096 115 us there, 71 on the pair tile;
 // 1000 x 1984 x 4096 15.0 and 10.1).  Among the tiles: the one that the figures below make cheapest.
 // HALOPS_B200_TILE (pair256 | pair128 | 256 | 128 | 64) overrides the choice (64: the 8-bit modes only).
+bool tile_fits(int64_t m, int64_t n, int64_t k, int mode) {
+    const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
+    if (m < 1 || n < 1 || k < 1) return false;
+    return fp8 ? k % 128 == 0 && n % 64 == 0 : k % 256 == 0 && n % 128 == 0;
+}
+
 TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool grouped = false, int64_t boundaries = 0) {
     // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
     const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
-    if (m < 1 || n < 1 || k < 1) return {0, false};
-    if (fp8 ? (k % 128 != 0 || n % 64 != 0) : (k % 256 != 0 || n % 128 != 0)) return {0, false};
+    if (!tile_fits(m, n, k, mode)) return {0, false};
     const int64_t tiles_m = (m + kBM - 1) / kBM;
     const int64_t tiles_m2 = (m + 255) / 256;
-    const char* forced = getenv("HALOPS_B200_TILE");
+    const char* forced = t_switches.tile;
     if (forced != nullptr && forced[0] != '\0') {
         const bool pair = strncmp(forced, "pair", 4) == 0;
         const int w = atoi(pair ? forced + 4 : forced);
@@ -2675,6 +2713,7 @@ extern "C" int hq_sm_count(int device) {
 extern "C" int hq_describe_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, int device,
                                 char* buf, size_t buflen) {
     if (hq_group_size(mode) == 0) return hq::fail(buf, buflen, HQ_ERR_INVALID, "Unsupported mode: %d", mode);
+    const hq::SwitchScope switches;
     const int sm = sm_count > 0 ? sm_count : hq_sm_count(device);
     const hq::TilePick pick = hq::pick_tile(m, n, k, mode, sm > 0 ? sm : 148);
     if (pick.bn == 0) {
@@ -2755,9 +2794,10 @@ int dense_gemm_impl(const void* a, const void* b, const void* sfa, const void* s
                     "W4A4-nvfp4 mode requires alpha input (per-batch scaling).");
     }
     if (m == 0 || n == 0) return HQ_OK;
+    const SwitchScope switches;
 
     // shape legality first: it needs no device
-    if (hq::pick_tile(m, n, k, mode, 148).bn == 0) {
+    if (!tile_fits(m, n, k, mode)) {
         return fail(err, errlen, HQ_ERR_INVALID, "No dense %s tile for M=%lld (grid M=%lld), N=%lld, K=%lld",
                     hq::mode_name(mode), (long long)(m < 128 ? m : hq_sf_rows(m)),
                     (long long)(m < 128 ? m : hq_sf_rows(m)), (long long)n, (long long)k);
@@ -2824,7 +2864,7 @@ int dense_gemm_impl(const void* a, const void* b, const void* sfa, const void* s
     g.early_weights = use_pdl == 2;
     {
         // test switch, read on every call: store every tile from registers
-        const char* e = getenv("HALOPS_B200_EPILOGUE");
+        const char* e = t_switches.epilogue;
         g.direct_store = e != nullptr && strcmp(e, "direct") == 0;
     }
     g.stream = static_cast<cudaStream_t>(stream);
@@ -2981,6 +3021,7 @@ int grouped_gemm_impl(int kind, const void* a, const void* b, const void* sfa, c
                           : "W4A4-nvfp4 mode requires alpha input (per-expert scaling factor).");
     }
     if (count == 0 || total_m == 0 || n == 0) return HQ_OK;
+    const SwitchScope switches;
     if (pick_tile_grouped(kind, count, rows, total_m, n, k, mode, 148).bn == 0) {
         return no_group_tile(err, errlen, kind, mode, rows, total_m, n, k);
     }
@@ -3057,6 +3098,7 @@ extern "C" int hq_describe_group_tile(int kind, int64_t count, int64_t rows, int
     if (kind < hq::kGroupBatch || kind > hq::kGroupContiguous) {
         return hq::fail(buf, buflen, HQ_ERR_INVALID, "Unsupported group kind: %d", kind);
     }
+    const hq::SwitchScope switches;
     const int sm = sm_count > 0 ? sm_count : hq_sm_count(device);
     const hq::TilePick pick = hq::pick_tile_grouped(kind, count, rows, total_m, n, k, mode, sm > 0 ? sm : 148);
     if (pick.bn == 0) return hq::no_group_tile(buf, buflen, kind, mode, rows, total_m, n, k);
@@ -3431,6 +3473,7 @@ extern "C" int hq_dense_gemm_small_m_noalloc(const void* a, const void* b, const
                     "multiple of 8 elements");
     }
     // the same deal of the work as hq_dense_gemm makes for this shape, capped by the array's size
+    const hq::SwitchScope switches;
     hq::DecPlan plan = hq::decode_plan(m, n, k, sm);
     if (plan.ctas > hq::kNoAllocMaxCtas) {
         return fail(err, errlen, HQ_ERR_INVALID,
