@@ -1573,6 +1573,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 }
             }
             ptx::pdl_launch_dependents();
+            // The releases of the last stages, which no load waits for any more: commits that arrive in both CTAs, so
+            // neither may leave before it has seen its own (the closing cluster_sync orders what threads did, not these).
+            for (uint32_t d = it > uint32_t(C::kStages) ? it - C::kStages : 0u; ok && d < it; ++d) {
+                ok = wait_bar(ptx::smem_u32(&bars->empty[d % C::kStages]), (d / C::kStages) & 1u, abort, kStatusProducer);
+            }
         }
     } else if (warp == 6) {
         // ------------------------------------------------------------ scale loader (both CTAs)
@@ -1952,8 +1957,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
     ptx::tc_fence_before();
     __syncthreads();
-    // neither CTA may leave while the other can still signal its barriers or
-    // while MMAs of the pair read its shared memory
+    // neither CTA may leave while the other can still signal its barriers or while MMAs of the pair read its shared
+    // memory: threads' arrivals are ordered by this barrier, the commits of both kinds have been waited for
+    // (acc_full by the epilogue, empty by the loader)
     ptx::cluster_sync();
     if (warp == 1) {
         ptx::tc_fence_after();

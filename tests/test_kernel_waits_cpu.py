@@ -44,3 +44,23 @@ def test_roles_read_the_abort_flag_as_whole_warps(name):
             line = m.group(0).strip()
             # declarations, votes, and the grace period of the teardown, which every warp reaches
             assert "uint32_t" in line or "_sync(" in line or "__nanosleep" in body[m.end():m.end() + 400], line
+
+
+def test_commits_that_arrive_in_both_ctas_are_waited_for():
+    """A commit with a destination in each CTA of the pair is asynchronous: a CTA that left before it arrived would have
+    its barriers written afterwards.  So whatever such a commit signals is waited for to the last phase: the accumulators
+    by the epilogue of every tile, the stages by the loads that refill them and, the last ring of them, behind the loop."""
+    pair = [body for head, body in _functions("gemm.cu") if "gemm_pair_kernel(" in head]
+    assert len(pair) == 1
+    barriers = set(re.findall(r"tc_commit_both\(ptx::smem_u32\(&bars->(\w+)\[", pair[0]))
+    assert barriers == {"empty", "acc_full"} and pair[0].count("tc_commit_both(") == 2
+    loader = re.search(r"if \(warp == 0\) \{.*?\} else if", pair[0], re.S).group(0)
+    refill, drain = re.search(r"(.*)pdl_launch_dependents\(\);(.*)", loader, re.S).groups()
+    assert re.search(r"wait_bar\(ptx::smem_u32\(&bars->empty\[s\]\), \(\(it / C::kStages\) & 1u\) \^ 1u", refill)
+    assert re.search(r"for \(uint32_t d = it > uint32_t\(C::kStages\) \? it - C::kStages : 0u; ok && d < it; \+\+d\)", drain)
+    assert re.search(r"wait_bar\(ptx::smem_u32\(&bars->empty\[d % C::kStages\]\), \(d / C::kStages\) & 1u", drain)
+    # the k-tile whose release a refill waits for and the phase that the drain waits for are the same
+    for stages in (3, 4, 6, 8):
+        for it in range(stages, 5 * stages):
+            d = it - stages
+            assert (d % stages, (d // stages) & 1) == (it % stages, ((it // stages) & 1) ^ 1)
