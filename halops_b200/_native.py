@@ -56,6 +56,7 @@ SIGNATURES = {
     "hq_describe_group_tile": (c_int, [c_int, c_i64, c_i64, c_i64, c_i64, c_i64, c_int, c_int, c_int, c_char_p,
                                        c_size_t]),
     "hq_sm_count": (c_int, [c_int]),
+    "hq_hold_switches": (None, [c_int]),
     "hq_device_status": (c_int, [c_int, c_void_p, ctypes.POINTER(ctypes.c_uint32), c_char_p, c_size_t]),
     "hq_selftest_bounded_wait": (c_int, [ctypes.c_uint32, c_int, c_void_p, c_char_p, c_size_t]),
     "hq_dense_gemm_allgather": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_void_p), c_int, c_int,
@@ -118,7 +119,7 @@ def _import_fast_path(handle):
     spec.loader.exec_module(module)
     module.bind(*(ctypes.cast(getattr(handle, name), c_void_p).value for name in (
         "hq_group_wise_quant", "hq_rms_norm_quant", "hq_dense_gemm", "hq_dense_gemm_situ_quant",
-        "hq_describe_group_tile", "hq_group_masked_gemm", "hq_group_contiguous_gemm")))
+        "hq_describe_group_tile", "hq_group_masked_gemm", "hq_group_contiguous_gemm", "hq_hold_switches")))
     return module
 
 

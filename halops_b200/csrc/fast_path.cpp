@@ -46,6 +46,7 @@ struct {
     DescribeGroupFn describe_group;
     MaskedFn masked;
     ContiguousFn contiguous;
+    decltype(&hq_hold_switches) hold_switches;
 } g_fn;
 
 // the package's mode names
@@ -122,6 +123,18 @@ int unlocked(F&& f) {
     char err[kErrLen];
     const Unlocked scope;
     return f(err);
+}
+
+// The same for the GEMMs, whose C ABI reads environment switches: they are read before the lock is given away, since an
+// assignment to os.environ in another thread moves the array that they are in.
+template <typename F>
+int unlocked_gemm(F&& f) {
+    const struct Held {
+        Held() { g_fn.hold_switches(1); }
+        Held(const Held&) = delete;
+        ~Held() { g_fn.hold_switches(0); }
+    } held;
+    return unlocked(f);
 }
 
 PyObject* pair_of(const at::Tensor& a, const at::Tensor& b) {
@@ -285,13 +298,13 @@ PyObject* dense_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         }
         void* const pos = osf->data_ptr();
         const int64_t no = osf->numel();
-        rc = unlocked([&](char* err) {
+        rc = unlocked_gemm([&](char* err) {
             return g_fn.situ(px, pw, psa, psb, po, pos, bias, m, n, k, na, nb, no, beta, lin, sm_count, pdl != 0 ? 1 : 0, d, st,
                              err, kErrLen);
         });
     } else {
         if (out->scalar_type() != at::kBFloat16 || out->stride(1) != 1) Py_RETURN_NONE;
-        rc = unlocked([&](char* err) {
+        rc = unlocked_gemm([&](char* err) {
             return g_fn.dense(px, pw, psa, psb, po, bias, alpha, m, n, k, na, nb, ldo, mode, epilogue, sm_count, pdl, d, st, err,
                               kErrLen);
         });
@@ -367,7 +380,7 @@ PyObject* grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int64_t na = sfa->numel(), nb = sfb->numel(), ldo = out->stride(0);
     const int d = x->get_device();
     void* const st = stream_of(*x);
-    const int rc = unlocked([&](char* err) {
+    const int rc = unlocked_gemm([&](char* err) {
         // the shape rules that the wrapper asks for first
         if (g_fn.describe_group(kind, e, masked ? max_m : m / e, m, n, k, mode, 148, -1, err, kErrLen) != 0) return 1;
         return (masked ? g_fn.masked : g_fn.contiguous)(px, pw, psa, psb, pt, po, bias, alpha, e, masked ? max_m : m, n, k, na,
@@ -378,10 +391,10 @@ PyObject* grouped_gemm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
-// bind(quant, rms, dense, situ, describe_group, masked, contiguous): addresses of the C ABI's entry points
+// bind(quant, rms, dense, situ, describe_group, masked, contiguous, hold_switches): addresses of the C ABI's entry points
 PyObject* bind(PyObject*, PyObject* args) {
-    unsigned long long p[7];
-    if (!PyArg_ParseTuple(args, "KKKKKKK", &p[0], &p[1], &p[2], &p[3], &p[4], &p[5], &p[6])) return nullptr;
+    unsigned long long p[8];
+    if (!PyArg_ParseTuple(args, "KKKKKKKK", &p[0], &p[1], &p[2], &p[3], &p[4], &p[5], &p[6], &p[7])) return nullptr;
     g_fn.quant = reinterpret_cast<QuantFn>(p[0]);
     g_fn.rms = reinterpret_cast<RmsFn>(p[1]);
     g_fn.dense = reinterpret_cast<DenseFn>(p[2]);
@@ -389,6 +402,7 @@ PyObject* bind(PyObject*, PyObject* args) {
     g_fn.describe_group = reinterpret_cast<DescribeGroupFn>(p[4]);
     g_fn.masked = reinterpret_cast<MaskedFn>(p[5]);
     g_fn.contiguous = reinterpret_cast<ContiguousFn>(p[6]);
+    g_fn.hold_switches = reinterpret_cast<decltype(&hq_hold_switches)>(p[7]);
     Py_RETURN_NONE;
 }
 

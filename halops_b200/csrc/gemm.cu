@@ -2063,33 +2063,47 @@ struct GemmArgs {
 };
 
 // The environment switches (HALOPS_B200_*, for experiments and tests), read on every call: entry points that lead to one
-// of them begin with a SwitchScope, which goes through the environment once.  (A dense call made six to nine getenv, 106 ns
-// each among 135 variables: 3.9 -> 3.6 us of the host's time per call with the shape rule taken out of the cost model.)
+// of them begin with a SwitchScope.  It asks getenv, which a thread that changes the environment meanwhile is kept from
+// by nothing but the C library; a caller that has a lock for that reads them under it (hq_hold_switches), in one walk over
+// the environment, and the calls that follow on its thread take that reading.  (Five getenv are 0.5 us among 135 variables.)
 struct Switches {
-    const char* tile = nullptr;
-    const char* splitk = nullptr;
-    const char* issuers = nullptr;
-    const char* decode = nullptr;
-    const char* epilogue = nullptr;
+    char tile[16] = "", splitk[8] = "", issuers[8] = "", decode[64] = "", epilogue[16] = "";
+
+    template <typename F>
+    void each(F&& f) {
+        f("HALOPS_B200_TILE", tile, sizeof(tile));
+        f("HALOPS_B200_SPLITK", splitk, sizeof(splitk));
+        f("HALOPS_B200_ISSUERS", issuers, sizeof(issuers));
+        f("HALOPS_B200_DECODE", decode, sizeof(decode));
+        f("HALOPS_B200_EPILOGUE", epilogue, sizeof(epilogue));
+    }
+    void clear() {
+        each([](const char*, char* to, size_t) { to[0] = '\0'; });
+    }
+    void ask() {
+        each([](const char* name, char* to, size_t size) {
+            const char* const v = getenv(name);
+            to[0] = '\0';
+            if (v != nullptr) snprintf(to, size, "%s", v);
+        });
+    }
+    void walk() {
+        clear();
+        for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
+            if ((*e)[0] != 'H' || strncmp(*e, "HALOPS_B200_", 12) != 0) continue;
+            each([v = *e](const char* name, char* to, size_t size) {
+                const size_t len = strlen(name);
+                if (to[0] == '\0' && strncmp(v, name, len) == 0 && v[len] == '=') snprintf(to, size, "%s", v + len + 1);
+            });
+        }
+    }
 };
 thread_local Switches t_switches;
+thread_local bool t_switches_held = false;
 
 struct SwitchScope {
     SwitchScope() {
-        Switches s;
-        for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
-            if ((*e)[0] != 'H' || strncmp(*e, "HALOPS_B200_", 12) != 0) continue;
-            const auto take = [v = *e + 12](const char* name, const char*& value) {
-                const size_t len = strlen(name);
-                if (value == nullptr && strncmp(v, name, len) == 0 && v[len] == '=') value = v + len + 1;
-            };
-            take("TILE", s.tile);
-            take("SPLITK", s.splitk);
-            take("ISSUERS", s.issuers);
-            take("DECODE", s.decode);
-            take("EPILOGUE", s.epilogue);
-        }
-        t_switches = s;
+        if (!t_switches_held) t_switches.ask();
     }
 };
 
@@ -2099,10 +2113,8 @@ struct SwitchScope {
 // 128 rows; 69 x 1088 x 1024 9.1 against 5.5, 65 x 1088 x 4992 13.1 against 10.4, 80 x 1792 x 7680 15.8 against 13.5).
 // With the 64-wide tile forced, from 8 k-tiles on.
 bool split_k_chosen(int group_kind, int tiles_m, int tiles_n, int k_tiles, int sm_count, int epi_op) {
-    const char* e = t_switches.splitk;
-    if (e != nullptr && e[0] == '0') return false;
-    const char* forced = t_switches.tile;
-    const int least = forced != nullptr && strcmp(forced, "64") == 0 ? 8 : 192;
+    if (t_switches.splitk[0] == '0') return false;
+    const int least = strcmp(t_switches.tile, "64") == 0 ? 8 : 192;
     return group_kind == kGroupDense && tiles_m == 1 && 2 * tiles_n <= sm_count && k_tiles >= least &&
            (epi_op == HQ_EPILOGUE_IDENTITY || epi_op == HQ_EPILOGUE_SIGMOID);
 }
@@ -2110,8 +2122,7 @@ bool split_k_chosen(int group_kind, int tiles_m, int tiles_n, int k_tiles, int s
 // 2: the single-CTA kernel issues its MMAs from two threads in k order (see the kernel);
 // 0 with HALOPS_B200_ISSUERS=1 (read on every call)
 int issuers_in_order() {
-    const char* e = t_switches.issuers;
-    return e != nullptr && e[0] == '1' ? 0 : 2;
+    return t_switches.issuers[0] == '1' ? 0 : 2;
 }
 
 template <int BN, int KIND>
@@ -2299,8 +2310,8 @@ struct DecodeSwitches {
 };
 DecodeSwitches decode_switches() {
     DecodeSwitches d;
-    const char* e = t_switches.decode;
-    if (e == nullptr) return d;
+    const char* const e = t_switches.decode;
+    if (e[0] == '\0') return d;
     d.off = strstr(e, "off") != nullptr;
     d.nosplit = strstr(e, "nosplit") != nullptr;
     d.split = !d.nosplit && strstr(e, "split") != nullptr;
@@ -2312,8 +2323,7 @@ DecodeSwitches decode_switches() {
 // Small M goes to the operand-swapped kernel: dense MXFP8 without bias, plain or sigmoid
 // epilogue, no forced tile.
 bool decode_eligible(int64_t m, int64_t n, int64_t k, int mode, int epi_op, bool has_bias) {
-    const char* forced = t_switches.tile;
-    if (forced != nullptr && forced[0] != '\0') return false;
+    if (t_switches.tile[0] != '\0') return false;
     if ((n / 128 + 1) * (k / 256 + 1) >= (int64_t(1) << 31)) return false;
     // Up to 64 activation rows by default.  With 65 to 128 a stage is half activations, the
     // weight in flight per CTA halves, and the best 128-row tile was faster on each of 33 problems (128 x 8192 x 4096
@@ -2595,8 +2605,8 @@ TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool
     if (!tile_fits(m, n, k, mode)) return {0, false};
     const int64_t tiles_m = (m + kBM - 1) / kBM;
     const int64_t tiles_m2 = (m + 255) / 256;
-    const char* forced = t_switches.tile;
-    if (forced != nullptr && forced[0] != '\0') {
+    const char* const forced = t_switches.tile;
+    if (forced[0] != '\0') {
         const bool pair = strncmp(forced, "pair", 4) == 0;
         const int w = atoi(pair ? forced + 4 : forced);
         const bool legal = w == 256 || w == 128 || (w == 64 && fp8 && !pair);
@@ -2702,6 +2712,11 @@ int g_sm_cache[64];
 
 }  // namespace
 }  // namespace hq
+
+extern "C" void hq_hold_switches(int hold) {
+    hq::t_switches_held = hold != 0;
+    if (hold != 0) hq::t_switches.walk();
+}
 
 extern "C" int hq_sm_count(int device) {
     if (device < 0 || device >= 64) {
@@ -2868,11 +2883,8 @@ int dense_gemm_impl(const void* a, const void* b, const void* sfa, const void* s
     g.sm_count = sm;
     g.pdl = use_pdl != 0;
     g.early_weights = use_pdl == 2;
-    {
-        // test switch, read on every call: store every tile from registers
-        const char* e = t_switches.epilogue;
-        g.direct_store = e != nullptr && strcmp(e, "direct") == 0;
-    }
+    // test switch, read on every call: store every tile from registers
+    g.direct_store = strcmp(t_switches.epilogue, "direct") == 0;
     g.stream = static_cast<cudaStream_t>(stream);
 
     if (!is_situ && hq::decode_eligible(m, n, k, mode, epilogue, bias != nullptr)) {

@@ -291,6 +291,11 @@ int hq_describe_group_tile(int kind, int64_t count, int64_t rows, int64_t total_
  * keyed by nothing and so returns the first device's count on every device. */
 int hq_sm_count(int device);
 
+/* The environment switches (HALOPS_B200_*) are read on every call, with getenv.  A caller that holds a lock under which
+ * the environment is changed (CPython's interpreter lock), and gives it up for the call, reads them itself before it
+ * does: hold != 0 reads them now, and the calls of this thread take that reading until hold == 0. */
+void hq_hold_switches(int hold);
+
 /*
  * Reads (and clears) the device-side status word of `device` after
  * synchronising `stream`: 0 when no kernel of this library gave up on a

@@ -361,6 +361,49 @@ def test_describe_tile(native):
         hq.describe_tile(128, 96, 128, sm_count=148)
 
 
+def test_switches_can_be_read_under_the_callers_lock(native, monkeypatch):
+    """A held reading serves the calls of its thread until it is let go, whatever happens to the environment."""
+    import threading
+
+    import halops_b200 as hq
+
+    def width():
+        return int(re.search(r"128x(\d+)/", hq.describe_tile(1000, 4096, 4096, sm_count=148)).group(1))
+
+    lib = native.lib()
+    monkeypatch.setenv("HALOPS_B200_TILE", "64")
+    lib.hq_hold_switches(1)
+    try:
+        monkeypatch.setenv("HALOPS_B200_TILE", "256")
+        assert width() == 64
+        seen = []
+        other = threading.Thread(target=lambda: seen.append(width()))
+        other.start()
+        other.join()
+        assert seen == [256]
+        lib.hq_hold_switches(1)
+        assert width() == 256
+    finally:
+        lib.hq_hold_switches(0)
+    monkeypatch.setenv("HALOPS_B200_TILE", "128")
+    assert width() == 128
+
+
+def test_switches_of_the_native_front_are_read_under_the_interpreter_lock():
+    """Assignments to os.environ may move the array that the C library's functions walk; only the lock keeps them apart."""
+    with open(os.path.join(ROOT, "halops_b200", "csrc", "gemm.cu")) as f:
+        gemm = f.read()
+    assert len(re.findall(r"\benviron\b(?=[;,) ])", re.sub(r"//[^\n]*", "", gemm))) == 1  # one walk, of the held reading
+    assert re.findall(r"\.walk\(\)", gemm) == [".walk()"]
+    assert re.search(r"void hq_hold_switches\(int hold\) \{[^}]*\.walk\(\);\s*\}", gemm)
+    with open(os.path.join(ROOT, "halops_b200", "csrc", "fast_path.cpp")) as f:
+        front = re.sub(r"//[^\n]*", "", f.read())
+    held = front.index("hold_switches(1)")
+    assert held < front.index("return unlocked(f);", held)
+    gemms = front[front.index("PyObject* dense_gemm("):]
+    assert gemms.count("unlocked_gemm(") == 3 and not re.search(r"\bunlocked\(", gemms)
+
+
 def test_wide_tiles_for_columns_that_do_not_fill_them(native):
     """A width need not divide N (timed: 71 us on the pair tile against 115 on the 64-wide one, 110 against 175, 67 against 75)."""
     import halops_b200 as hq
