@@ -127,10 +127,14 @@ static_assert(sizeof(Barriers) <= kKeptOffset, "kBarBytes");
 // that CTAs of the cluster arrive on with release semantics; the wait acquires what they wrote into
 // this CTA's shared memory before arriving.  A function of its own: the roles come here only when a first
 // try_wait, which holds a converged warp until the phase ends (woken 84 cycles after the arrival, also after
-// 6000 cycles), has returned without it, and the polling code is not in their loops.
+// 6000 cycles), has returned without it, and the polling code is not in their loops.  (InPlace: inline after all, for the split-K
+// kernel, which took 170 cycles a k-tile longer with the calls in its loops: 125 x 704 x 8064 10.8 us, 13.7 with them.  Inline in every
+// kernel: SituQuant 300 x 5120 x 2048 7.5 -> 8.6 us, NVFP4 2048 x 8192 x 2048 20.7 -> 26.0, W4A8 12 slots of 256 x 3072 x 2048
+// 18.7 -> 25.5.)
+enum class InPlace {};
 template <bool kCluster = false>
-__device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code,
-                                           uint64_t limit_ns = kTimeoutNs) {
+__device__ __forceinline__ bool wait_bar_lane(InPlace, uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code,
+                                              uint64_t limit_ns = kTimeoutNs) {
     const auto done = [&] { return kCluster ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity); };
     if (done()) return true;
     const uint64_t t0 = ptx::globaltimer_ns();
@@ -147,6 +151,11 @@ __device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volati
     }
     return true;
 }
+template <bool kCluster = false>
+__device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code,
+                                           uint64_t limit_ns = kTimeoutNs) {
+    return wait_bar_lane<kCluster>(InPlace{}, bar, parity, abort, code, limit_ns);
+}
 
 // The wait of a role: called by all lanes of a warp, with one result for all of them.  Lanes poll for
 // themselves, so when a wait runs out while its barrier completes after all, some of them see the one and
@@ -155,23 +164,32 @@ __device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volati
 // The first try and its vote are straight-line code (a completed barrier: 58 cycles); with the polling loop inline, lane by
 // lane, a wait on a completed barrier took a role 125: 512 x 1536 x 4096 8.8 -> 8.5 us, 1024 x 1536 x 8192 26.0 -> 24.9 (both on
 // the 128 x 64 tile), NVFP4 512 x 4096 x 8192 12.9 -> 12.7, 64 x 24576 x 1536 10.2 -> 10.0, GEMM alone.
+template <bool kInPlace = false>
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
     if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
-    return __all_sync(0xffffffffu, wait_bar_lane(bar, parity, abort, code) ? 1 : 0) != 0;
+    const bool mine = kInPlace ? wait_bar_lane(InPlace{}, bar, parity, abort, code) : wait_bar_lane(bar, parity, abort, code);
+    return __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
 }
 // Two waits with one vote (the second only if `both`): a vote between a barrier and the work behind it is on the
 // critical path of a k-step.
+template <bool kInPlace = false>
 __device__ __forceinline__ bool wait_bars(uint32_t bar, uint32_t parity, bool both, uint32_t bar2, uint32_t parity2,
                                           volatile uint32_t* abort, uint32_t code) {
     bool mine = ptx::mbar_try_wait(bar, parity);
     if (both) mine = ptx::mbar_try_wait(bar2, parity2) && mine;
     if (__all_sync(0xffffffffu, mine ? 1 : 0) != 0) return true;
-    mine = wait_bar_lane(bar, parity, abort, code) && (!both || wait_bar_lane(bar2, parity2, abort, code));
+    if constexpr (kInPlace) {
+        mine = wait_bar_lane(InPlace{}, bar, parity, abort, code) && (!both || wait_bar_lane(InPlace{}, bar2, parity2, abort, code));
+    } else {
+        mine = wait_bar_lane(bar, parity, abort, code) && (!both || wait_bar_lane(bar2, parity2, abort, code));
+    }
     return __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
 }
+template <bool kInPlace = false>
 __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
     if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar, parity) ? 1 : 0) != 0) return true;
-    return __all_sync(0xffffffffu, wait_bar_lane<true>(bar, parity, abort, code) ? 1 : 0) != 0;
+    const bool mine = kInPlace ? wait_bar_lane<true>(InPlace{}, bar, parity, abort, code) : wait_bar_lane<true>(bar, parity, abort, code);
+    return __all_sync(0xffffffffu, mine ? 1 : 0) != 0;
 }
 
 // The warp's index in its CTA, known to be warp-uniform.
@@ -719,7 +737,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 for (int kt = k_begin; kt < k_end; ++kt, ++it) {
                     const uint32_t s = it % kRing;
                     const uint32_t ph = (it / kRing) & 1u;
-                    ok = wait_bar(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
+                    ok = wait_bar<kSplitK>(ptx::smem_u32(&bars->empty[s]), ph ^ 1u, abort, kStatusProducer);
                     if (!ok) break;
                     const uint32_t full = ptx::smem_u32(&bars->full[s]);
                     const uint32_t sf_full = ptx::smem_u32(&bars->sf_full[s]);
@@ -767,11 +785,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 const uint32_t aph = (t >> 1) & 1u;
                 // (with two issuers both wait here, also the one that has no k-tile in a tile of
                 // one: its arrival below must not run ahead of the stage's previous use)
-                ok = wait_bar(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
+                ok = wait_bar<kSplitK>(ptx::smem_u32(&bars->acc_empty[as]), aph ^ 1u, abort, kStatusMma);
                 if (!ok) break;
                 if (C::kOverlap != 0 && t > 0) {
                     // the previous tile's epilogue has drained the columns both stages share
-                    ok = wait_bar(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
+                    ok = wait_bar<kSplitK>(ptx::smem_u32(&bars->overlap_free[as ^ 1u]), ((t - 1) >> 1) & 1u,
                                   abort, kStatusMma);
                     if (!ok) break;
                 }
@@ -787,11 +805,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     const uint32_t ph = (it / kRing) & 1u;
                     // the scales of this k-tile are in their set (the scale warps waited for the
                     // scale bytes); the stage's own barrier orders this thread after the TMA writes
-                    ok = wait_bars(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, true,
+                    ok = wait_bars<kSplitK>(ptx::smem_u32(&bars->sf_ready[it % C::kSfSets]), (it / C::kSfSets) & 1u, true,
                                    ptx::smem_u32(&bars->full[s]), ph, abort, kStatusMma);
                     // (in-order pair of issuers) the other thread has issued the MMAs of the previous k-iteration
                     if (ok && ordered && it > 0u) {
-                        ok = wait_bar(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
+                        ok = wait_bar<kSplitK>(ptx::smem_u32(&bars->turn[me]), ((it - 1u) >> 1) & 1u, abort, kStatusMma);
                     }
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -867,13 +885,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 uint32_t r[C::kSfCols];
                 const auto load = [&] { load_scales<C>(sfa_base + s * C::kSfaBytes, sfb_base + s * C::kSfbBytes, lane, r); };
                 if constexpr (C::kSfSets == 2 && C::kSfKAtoms > 1) {
-                    ok = wait_bar(sf_full, (it / kRing) & 1u, abort, kStatusProducer);
+                    ok = wait_bar<kSplitK>(sf_full, (it / kRing) & 1u, abort, kStatusProducer);
                     if (!ok) break;
                     load();
-                    if (it >= uint32_t(C::kSfSets)) ok = wait_bar(set_free, (prev / kRing) & 1u, abort, kStatusProducer);
+                    if (it >= uint32_t(C::kSfSets)) ok = wait_bar<kSplitK>(set_free, (prev / kRing) & 1u, abort, kStatusProducer);
                     if (!ok) break;
                 } else {
-                    ok = wait_bars(sf_full, (it / kRing) & 1u, it >= uint32_t(C::kSfSets), set_free, (prev / kRing) & 1u,
+                    ok = wait_bars<kSplitK>(sf_full, (it / kRing) & 1u, it >= uint32_t(C::kSfSets), set_free, (prev / kRing) & 1u,
                                    abort, kStatusProducer);
                     if (!ok) break;
                     load();
@@ -919,7 +937,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             }
             const uint32_t as = t & 1u;
             const uint32_t aph = (t >> 1) & 1u;
-            ok = wait_bar(ptx::smem_u32(&bars->acc_full[as]), aph, abort, kStatusEpilogue);
+            ok = wait_bar<kSplitK>(ptx::smem_u32(&bars->acc_full[as]), aph, abort, kStatusEpilogue);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t acc = tmem + as * C::kAccStride + (lane_base << 16);
@@ -1033,7 +1051,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     }
                     if (ci == 0) {
                         // this tile's partial sums (one phase of the barrier per tile)
-                        ok = wait_bar_cluster(ptx::smem_u32(&bars->recv_full), t & 1u, abort, kStatusEpilogue);
+                        ok = wait_bar_cluster<kSplitK>(ptx::smem_u32(&bars->recv_full), t & 1u, abort, kStatusEpilogue);
                         if (!ok) break;
                     }
 #pragma unroll
@@ -2107,14 +2125,14 @@ struct SwitchScope {
     }
 };
 
-// Split-K is taken for a dense problem with one row of at most sm_count / 2 64-wide tiles and at least 192 k-tiles
-// (HALOPS_B200_SPLITK=0 turns it off; read on every call).  The cluster and its exchange cost 3.6 us: behind
-// a quantizer the split took 9.1 us at 8 k-tiles and 0.133 for each further one, the whole tile 5.5 and 0.154 (16 problems of 65 to
-// 128 rows; 69 x 1088 x 1024 9.1 against 5.5, 65 x 1088 x 4992 13.1 against 10.4, 80 x 1792 x 7680 15.8 against 13.5).
-// With the 64-wide tile forced, from 8 k-tiles on.
+// Split-K is taken for a dense problem with one row of 64-wide tiles and a long K: at least 56 k-tiles where its two CTAs per tile
+// fill at most half of the SMs, 96 where they fill more (a tile's weights then come no faster to two CTAs than to one).
+// HALOPS_B200_SPLITK=0 turns it off; read on every call.  The cluster and its exchange cost 3.5 us; N = 704 (11 tiles) takes
+// 9.6 us split and 9.2 whole at 48 k-tiles, 10.2 and 10.4 at 56, 13.2 and 16.1 at 96; N = 3712 13.9 and 13.1 at 64, 17.1 and 17.9
+// at 96 (112 problems of 66 and 128 rows).  With the 64-wide tile forced, from 8 k-tiles on.
 bool split_k_chosen(int group_kind, int tiles_m, int tiles_n, int k_tiles, int sm_count, int epi_op) {
     if (t_switches.splitk[0] == '0') return false;
-    const int least = strcmp(t_switches.tile, "64") == 0 ? 8 : 192;
+    const int least = strcmp(t_switches.tile, "64") == 0 ? 8 : 4 * tiles_n <= sm_count ? 56 : 96;
     return group_kind == kGroupDense && tiles_m == 1 && 2 * tiles_n <= sm_count && k_tiles >= least &&
            (epi_op == HQ_EPILOGUE_IDENTITY || epi_op == HQ_EPILOGUE_SIGMOID);
 }

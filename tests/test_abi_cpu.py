@@ -433,6 +433,18 @@ def test_contiguous_tile_with_experts_that_meet_inside_tiles(native):
     assert tile(1, 4096, 4096, 2048) == hq.describe_tile(4096, 4096, 2048, sm_count=148).split("-> ")[1].split(" splitk")[0]
 
 
+def test_split_k_from_the_k_that_repays_its_exchange(native):
+    """Timed split and whole: 9.6 / 9.2 us at 48 k-tiles, 10.2 / 10.4 at 56 on 11 tiles; 13.9 / 13.1 at 64, 17.1 / 17.9 at 96 on 58."""
+    import halops_b200 as hq
+
+    def split(n, k_tiles):
+        return re.search(r"splitk=(\d)", hq.describe_tile(100, n, 128 * k_tiles, sm_count=148)).group(1)
+
+    assert [split(704, kt) for kt in (8, 48, 55, 56, 64, 192)] == ["0", "0", "0", "1", "1", "1"]
+    assert [split(3712, kt) for kt in (56, 95, 96)] == ["0", "0", "1"]
+    assert split(2368, 56) == "1" and split(2432, 56) == "0" and split(4800, 192) == "0"
+
+
 def test_product_never_imports_the_oracle():
     """The library must not route through the CPU oracle."""
     pkg = os.path.join(ROOT, "halops_b200")

@@ -435,8 +435,8 @@ def test_situ_quant_epilogue(hq, m, n, k, with_bias, beta, linear_beta):
     ("w8a8-mxfp8", 5, 64, 2048), ("w8a8-mxfp8", 33, 4736, 1152), ("w8a8-mxfp8", 100, 1024, 1024)],
     ids=lambda v: str(v))
 def test_split_k_shapes(hq, monkeypatch, mode, m, n, k):
-    """One row of at most 74 64-wide tiles and at least 8 k-tiles: two CTAs share a tile, half
-    of K each, partial sums through distributed shared memory.  Without the split the same tile
+    """One row of at most 74 64-wide tiles (forced here, where 8 k-tiles are enough; see test_split_k_by_default): two CTAs share
+    a tile, half of K each, partial sums through distributed shared memory.  Without the split the same tile
     runs with two MMA issuers that take alternate k-tiles into accumulators of their own.  Both
     are deterministic and within a bfloat16 rounding of each other and of the 128-wide tile
     (which sums the k-tiles in order)."""
@@ -463,6 +463,17 @@ def test_split_k_shapes(hq, monkeypatch, mode, m, n, k):
         monkeypatch.setenv("HALOPS_B200_TILE", "128")
         in_order = _gemm(hq, aq, bq, sfa, sfb, mode)
         assert close(out, in_order) and close(unsplit, in_order)
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 256, 7168), (128, 704, 7296), (100, 3712, 12288)])
+def test_split_k_by_default(hq, m, n, k):
+    """Without any switch, from 56 k-tiles on (96 where the tiles fill more than a quarter of the SMs)."""
+    assert "128x64" in hq.describe_tile(m, n, k) and "splitk=1" in hq.describe_tile(m, n, k)
+    assert "splitk=0" in hq.describe_tile(m, n, k - 256 if k < 10000 else k - 128)
+    aq, bq, sfa, sfb = _quantize(hq, _rand(m, k, 24), _rand(n, k, 25, "weight"), "w8a8-mxfp8")
+    out = _gemm(hq, aq, bq, sfa, sfb, "w8a8-mxfp8")
+    _check(out, aq, bq, sfa, sfb, "w8a8-mxfp8")
+    assert torch.equal(out, _gemm(hq, aq, bq, sfa, sfb, "w8a8-mxfp8", use_pdl=True))
 
 
 @pytest.mark.parametrize("mode, m, n, k", [("w8a8-mxfp8", 256, 512, 1024), ("w8a8-mxfp8", 100, 256, 512),
