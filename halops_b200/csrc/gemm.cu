@@ -621,7 +621,13 @@ __device__ __forceinline__ void load_scales(uint32_t sfa_stage, uint32_t sfb_sta
 // instructions anew at every launch, and they were most of them (512 x 1536 x 4096 behind its
 // quantizer 13.9 -> 12.8 us, 128 x 256 x 512 5.6 -> 5.1, NVFP4 300 x 4096 x 4096 12.0 -> 11.4; large
 // problems unchanged).  The other forms take the general code.
-template <int BN, int KIND, bool kSplitK = false, bool kDense = kSplitK>
+//
+// kRuns: contiguous experts, cut into tiles by their runs (RunTable), known at compile time.  Batches, masked experts and the contiguous
+// problems worked on fixed tiles (HALOPS_B200_RUNS=0) carry none of its code, and the runs none of theirs: MXFP8 5504 x 3456 x 768
+// with 12 experts on the 128 x 128 tile 35 -> 24 us, NVFP4 21504 x 2432 x 1024 with 18 75 (pair tile) -> 47; masked and batch 2 % faster.
+// (The pair kernel has one grouped form for all: with the runs in one of their own they took 1.17 and 1.25 of the time on
+// the 256 x 128 tile in MXFP8 and W4A8.)
+template <int BN, int KIND, bool kSplitK = false, bool kDense = kSplitK, bool kRuns = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
             const __grid_constant__ CUtensorMap tm_d, const uint8_t* __restrict__ sfa,
@@ -630,7 +636,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             int M, int N, int k_tiles, int kq_dim, int tiles_m, int tiles_n, int a_rows, int direct_store,
             int dual_issue, int prefetch_weight, const GroupParams grp_arg, const SituParams situ) {
     using C = Cfg<BN, KIND>;
-    const GroupParams grp = kDense ? GroupParams{kGroupDense, 1, 0, nullptr} : grp_arg;
+    const GroupParams grp = kDense ? GroupParams{kGroupDense, 1, 0, nullptr}
+                            : kRuns ? GroupParams{kGroupContiguous, grp_arg.count, grp_arg.rows, grp_arg.table} : grp_arg;
+    constexpr bool kPlain = kDense || kRuns;  // Identity or Sigmoid
     // Two MMA issuers with an accumulator each (64-wide dense tiles, plain epilogues): the k-tiles
     // of a tile are summed as (even ones) + (odd ones), deterministically, but not in the k order
     // of the other tiles.
@@ -718,7 +726,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     // programmatic launch; nothing below may run before its writes are visible.
     ptx::pdl_wait();
     RunTable run_table = {nullptr, 0};
-    if (!kDense && grp.kind == kGroupContiguous) {
+    if constexpr (kRuns) {
         run_table = build_runs<kBM, kThreads>(grp, M, bars, reinterpret_cast<uint32_t*>(smem + bar_off + 1024));
     }
 
@@ -917,7 +925,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         WorkIter<BN> work(grp, M, N, tiles_m, tiles_n, run_table, first_item, item_step);
         Work wk;
         const int ar = int(lane_base) + lane;  // accumulator row of this thread
-        if (!kDense && situ.sf != nullptr) zero_sf_padding(situ, (warp - 2) * 32 + lane);
+        if (!kPlain && situ.sf != nullptr) zero_sf_padding(situ, (warp - 2) * 32 + lane);
         for (; ok && work.next(wk); ++t) {
             const int m0 = wk.out_row0;  // output row of accumulator row 0
             const int n0 = wk.out_col0;
@@ -941,7 +949,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             if (!ok) break;
             ptx::tc_fence_after();
             const uint32_t acc = tmem + as * C::kAccStride + (lane_base << 16);
-            if (!kDense && KIND == 0 && epi_op == HQ_EPILOGUE_SITU_QUANT) {
+            if (!kPlain && KIND == 0 && epi_op == HQ_EPILOGUE_SITU_QUANT) {
                 // quantising epilogue: 64 accumulator columns -> one group of 32 e4m3 outputs
                 constexpr int kGroups = C::kChunks / 2;
 #pragma unroll 1
@@ -1082,7 +1090,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                                epi_op);
                 const int row = m0 + ar;
                 const int col = n0 + c * kEpiChunk;
-                if (!kDense && (epi_op == HQ_EPILOGUE_QUANT || epi_op == HQ_EPILOGUE_GATE_MUL_QUANT ||
+                if (!kPlain && (epi_op == HQ_EPILOGUE_QUANT || epi_op == HQ_EPILOGUE_GATE_MUL_QUANT ||
                                 epi_op == HQ_EPILOGUE_SIGMOID_GATE_MUL_QUANT)) {
                     // The bf16 result (times the gate, as a bf16 product) re-quantised to MXFP8 per
                     // 32 columns: the reference's batch epilogues (csrc/kernel/gemm/epilogue.cuh:990-1051).
@@ -1487,10 +1495,13 @@ __global__ void __launch_bounds__((Cfg2<BN, KIND>::kThreads), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ CUtensorMap tm_sfa,
                  const __grid_constant__ CUtensorMap tm_sfb, const float* __restrict__ alpha,
-                 const __nv_bfloat16* __restrict__ bias, int epi_op, int k_tiles, int kq_dim, int tiles_m,
+                 const __nv_bfloat16* __restrict__ bias_arg, int epi_arg, int k_tiles, int kq_dim, int tiles_m,
                  int tiles_n, int prefetch_weight, const __grid_constant__ GatherMaps<kGather> peers, const PairGroupArgs ga,
                  const PairSitu<kSitu> situ) {
     using C = Cfg2<BN, KIND>;
+    // (only MXFP8 takes a bias, only the dense form another epilogue than Identity: less to hold through the loop over the chunks)
+    const __nv_bfloat16* const bias = KIND == 0 ? bias_arg : nullptr;
+    const int epi_op = kGrouped ? HQ_EPILOGUE_IDENTITY : epi_arg;
     using Iter = PairWorkIter<BN, kGrouped>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -2075,6 +2086,7 @@ struct GemmArgs {
     int kq_dim;
     int sm_count;
     bool pdl;
+    bool runs = false;           // contiguous experts: tiles by runs (RunTable)
     bool early_weights = false;  // with pdl: b and sfb may be read before the preceding kernel completes
     bool direct_store;
     cudaStream_t stream;
@@ -2085,7 +2097,7 @@ struct GemmArgs {
 // by nothing but the C library; a caller that has a lock for that reads them under it (hq_hold_switches), in one walk over
 // the environment, and the calls that follow on its thread take that reading.  (Five getenv are 0.5 us among 135 variables.)
 struct Switches {
-    char tile[16] = "", splitk[8] = "", issuers[8] = "", decode[64] = "", epilogue[16] = "";
+    char tile[16] = "", splitk[8] = "", issuers[8] = "", decode[64] = "", epilogue[16] = "", runs[8] = "";
 
     template <typename F>
     void each(F&& f) {
@@ -2094,6 +2106,7 @@ struct Switches {
         f("HALOPS_B200_ISSUERS", issuers, sizeof(issuers));
         f("HALOPS_B200_DECODE", decode, sizeof(decode));
         f("HALOPS_B200_EPILOGUE", epilogue, sizeof(epilogue));
+        f("HALOPS_B200_RUNS", runs, sizeof(runs));
     }
     void clear() {
         each([](const char*, char* to, size_t) { to[0] = '\0'; });
@@ -2191,8 +2204,8 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
         }
     }
     const int tiles_n = (g.n + BN - 1) / BN;
-    // contiguous: the runs are cut into at most a tile each more than the rows alone
-    const int64_t row_tiles = g.grp.kind == kGroupContiguous ? std::min<int64_t>(g.m / 64, int64_t(tiles_m) + g.grp.count) : tiles_m;
+    // runs are cut into at most a tile each more than the rows alone
+    const int64_t row_tiles = g.runs ? std::min<int64_t>(g.m / 64, int64_t(tiles_m) + g.grp.count) : tiles_m;
     const int grid = int(std::min<int64_t>(g.sm_count, row_tiles * tiles_n));
     const int k_tiles = int(g.k_bytes / kBKBytes);
     if constexpr (BN == 64) {
@@ -2227,6 +2240,14 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
                                g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.pdl ? 1 : 0, g.grp, g.situ));
             return HQ_OK;
         }
+    }
+    if (g.runs) {
+        static SmemOptIn opt_in_runs;
+        HQ_CUDA_TRY(opt_in_runs.ensure(gemm_kernel<BN, KIND, false, false, true>, C::kSmemBytes));
+        HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND, false, false, true>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
+                           g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
+                           g.kq_dim, tiles_m, tiles_n, a_rows, g.direct_store ? 1 : 0, dual, g.pdl ? 1 : 0, g.grp, g.situ));
+        return HQ_OK;
     }
     HQ_CUDA_TRY(launch(gemm_kernel<BN, KIND>, dim3(grid), dim3(kThreads), size_t(C::kSmemBytes), g.stream,
                        g.pdl, 1, tm_a, tm_b, tm_d, g.sfa, g.sfb, g.alpha, g.bias, g.epi_op, g.out, g.ldo, g.m, g.n, k_tiles,
@@ -2601,6 +2622,7 @@ const char* mode_name(int mode) {
 struct TilePick {
     int bn;     // tile width, 0 = no tile fits
     bool pair;  // 256-row tile on a pair of CTAs
+    bool runs = false;  // contiguous experts: tiles by their runs
 };
 
 // Shape legality follows the reference's "some compiled tile fits" rule
@@ -2998,6 +3020,7 @@ TilePick pick_tile_grouped(int kind, int64_t count, int64_t rows, int64_t total_
     // PairWorkIter).  Otherwise a forced or modelled pair choice falls back to the same width.
     const bool whole_tiles = kind == kGroupContiguous || rows % 256 == 0;
     if (!(plain_epilogue && whole_tiles)) pick.pair = false;
+    pick.runs = kind == kGroupContiguous && (pick.pair || t_switches.runs[0] != '0');
     return pick;
 }
 
@@ -3111,6 +3134,7 @@ int grouped_gemm_impl(int kind, const void* a, const void* b, const void* sfa, c
     g.m = int(total_m);
     g.n = int(n);
     g.grp = GroupParams{kind, int(count), int(rows), table};
+    g.runs = pick.runs;
     g.k_bytes = (mode == HQ_MODE_W8A8_MXFP8 || w4a8) ? k : k / 2;  // bytes of one A row
     g.kq_dim = int(sf_k / 4);
     g.sm_count = sm;

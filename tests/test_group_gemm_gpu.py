@@ -495,6 +495,20 @@ def test_contiguous_runs_and_their_tiles(hq, monkeypatch, tile, counts):
     _contiguous_case(hq, counts, 384 if sum(counts) < 1000 else 128, 256, "w8a8-mxfp8", check_rows=1024)
 
 
+@pytest.mark.parametrize("mode,tile", [("w8a8-mxfp8", "64"), ("w8a8-mxfp8", "128"), ("w8a8-mxfp8", "256"), ("w8a8-mxfp8", "pair256"),
+                                       ("w4a4-nvfp4", "128"), ("w4a4-nvfp4", "256"), ("w4a4-mxfp4", "128")], ids=lambda v: str(v))
+@pytest.mark.parametrize("counts", [[64], [64, 64], [64, 192, 0, 128], [128, 64, 320, 64], [64] * 40], ids=lambda v: f"{len(v)}runs{sum(v)}")
+def test_contiguous_by_rows_and_by_runs(hq, monkeypatch, mode, tile, counts):
+    """Tiles on fixed boundaries, worked once per expert in them, and tiles cut by the runs give the same bits (the pair tile is
+    always cut by runs)."""
+    monkeypatch.setenv("HALOPS_B200_TILE", tile)
+    results = []
+    for runs in ("0", "1"):
+        monkeypatch.setenv("HALOPS_B200_RUNS", runs)
+        results.append(_contiguous_case(hq, counts, 384, 512, mode))
+    assert torch.equal(*results)
+
+
 def test_contiguous_experts_in_any_order(hq, monkeypatch):
     """Runs of one expert may come back, in any order; rows whose id is out of range take the nearest expert."""
     ids = np.repeat(np.array([2, 0, 2, 1, 1, 0, 3, 9, -4], dtype=np.int32), 64)
