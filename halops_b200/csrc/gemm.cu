@@ -933,10 +933,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const bool warp_idle = int(lane_base) >= wk.row_hi || int(lane_base) + 32 <= wk.row_lo;
             const bool row_ok = ar >= wk.row_lo && ar < wk.row_hi;
             // rows go out through TMA stores (a dense tail is clipped by the tensor map), except where only some of
-            // this warp's are the item's: those are stored from registers, row by row, and so are tiles of at most
-            // 32 rows (one warp, no staging round trip)
+            // this warp's are the item's: those are stored from registers, row by row, and so are items of at most
+            // 32 rows (no staging round trip: NVFP4, two batches of 32 x 1792 x 768, 4.0 us with it)
             const bool warp_whole = int(lane_base) >= wk.row_lo && int(lane_base) + 32 <= wk.row_hi;
-            const bool reg_store = direct_store != 0 || (wk.row_lo == 0 && wk.row_hi <= 32) ||
+            const bool reg_store = direct_store != 0 || wk.row_hi - wk.row_lo <= 32 ||
                                    (!warp_whole && grp.kind != kGroupDense);
             // per-tensor (dense) or per-group factor of the NVFP4 recipe
             if (KIND == 1 && alpha != nullptr && wk.group != scale_group) {

@@ -356,3 +356,18 @@ def test_fp4_batches_on_the_2cta_tile(hq, monkeypatch, mode, tile):
         outs.append(_run(hq, xq, wq, sfa, sfb, mode, alpha=alpha))
     assert torch.equal(outs[0], outs[1])
     _compare(outs[1], xq, wq, sfa, sfb, mode, alpha=alpha)
+
+
+@pytest.mark.parametrize("mode", ["w8a8-mxfp8", "w4a4-nvfp4"])
+@pytest.mark.parametrize("m", [16, 32, 40, 96])
+def test_batches_of_few_rows(hq, monkeypatch, mode, m):
+    """Batches that share a 128-row tile, with and without whole 32-row warps of their own."""
+    b, n, k = 5, 384, 512
+    xq, wq, sfa, sfb = _inputs(hq, b, m, n, k, mode, seed=19)
+    alpha = (0.5 + torch.arange(b, dtype=torch.float32) * 0.25).cuda() if mode == "w4a4-nvfp4" else None
+    outs = []
+    for tile in ("128", "256"):
+        monkeypatch.setenv("HALOPS_B200_TILE", tile)
+        outs.append(_run(hq, xq, wq, sfa, sfb, mode, alpha=alpha))
+    assert torch.equal(outs[0], outs[1])
+    _compare(outs[1], xq, wq, sfa, sfb, mode, alpha=alpha)
