@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
 
 #include "common.cuh"
@@ -623,7 +624,7 @@ __device__ __forceinline__ void load_scales(uint32_t sfa_stage, uint32_t sfb_sta
 // problems unchanged).  The other forms take the general code.
 //
 // kRuns: contiguous experts, cut into tiles by their runs (RunTable), known at compile time.  Batches, masked experts and the contiguous
-// problems worked on fixed tiles (HALOPS_B200_RUNS=0) carry none of its code, and the runs none of theirs: MXFP8 5504 x 3456 x 768
+// problems that the table does not repay (contiguous_by_runs) carry none of its code, and the runs none of theirs: MXFP8 5504 x 3456 x 768
 // with 12 experts on the 128 x 128 tile 35 -> 24 us, NVFP4 21504 x 2432 x 1024 with 18 75 (pair tile) -> 47; masked and batch 2 % faster.
 // (The pair kernel has one grouped form for all: with the runs in one of their own they took 1.17 and 1.25 of the time on
 // the 256 x 128 tile in MXFP8 and W4A8.)
@@ -2156,6 +2157,18 @@ int issuers_in_order() {
     return t_switches.issuers[0] == '1' ? 0 : 2;
 }
 
+// (group, 128-row tile) pairs of `count` groups of `rows` rows each; a tile that straddles groups counts once per group.
+int64_t slot_row_tiles(int64_t count, int64_t rows) {
+    const auto tiles = [rows](int64_t g) { return ((g + 1) * rows - 1) / kBM - g * rows / kBM + 1; };
+    int64_t period = 1;  // groups after which the starts in their tiles come again
+    while (period < kBM && period * rows % kBM != 0) period *= 2;
+    int64_t each = 0, total = 0;
+    for (int64_t g = 0; g < std::min(period, count); ++g) each += tiles(g);
+    total = count / period * each;
+    for (int64_t g = count / period * period; g < count; ++g) total += tiles(g);
+    return total;
+}
+
 template <int BN, int KIND>
 int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
     using C = Cfg<BN, KIND>;
@@ -2198,10 +2211,7 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
         // (group, 128-row tile) pairs; a straddling tile counts once per group.  For the
         // masked kind this is the upper bound that sizes the grid: the kernel walks the
         // valid rows only.
-        tiles_m = 0;
-        for (int b = 0; b < g.grp.count; ++b) {
-            tiles_m += int(((int64_t(b) + 1) * g.grp.rows - 1) / kBM - (int64_t(b) * g.grp.rows) / kBM + 1);
-        }
+        tiles_m = int(slot_row_tiles(g.grp.count, g.grp.rows));
     }
     const int tiles_n = (g.n + BN - 1) / BN;
     // runs are cut into at most a tile each more than the rows alone
@@ -2633,96 +2643,135 @@ struct TilePick {
 // multiple of 64 left the 64-wide tile alone (3000 x 7232 x 4096 115 us there, 71 on the pair tile;
 // 1000 x 1984 x 4096 15.0 and 10.1).  Among the tiles: the one that the figures below make cheapest.
 // HALOPS_B200_TILE (pair256 | pair128 | 256 | 128 | 64) overrides the choice (64: the 8-bit modes only).
+// (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
+bool is_fp8_kind(int mode) { return mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4; }
+
 bool tile_fits(int64_t m, int64_t n, int64_t k, int mode) {
-    const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
     if (m < 1 || n < 1 || k < 1) return false;
-    return fp8 ? k % 128 == 0 && n % 64 == 0 : k % 256 == 0 && n % 128 == 0;
+    return is_fp8_kind(mode) ? k % 128 == 0 && n % 64 == 0 : k % 256 == 0 && n % 128 == 0;
 }
 
-TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool grouped = false, int64_t boundaries = 0) {
-    // (FP8 activations x FP4 weights tile like FP8: 128 values of K per k-tile)
-    const bool fp8 = mode == HQ_MODE_W8A8_MXFP8 || mode == HQ_MODE_W4A8_MXFP4;
-    if (!tile_fits(m, n, k, mode)) return {0, false};
-    const int64_t tiles_m = (m + kBM - 1) / kBM;
-    const int64_t tiles_m2 = (m + 255) / 256;
+// HALOPS_B200_TILE; a pair tile where the problem has none is the single-CTA tile of its width.
+bool forced_tile(int mode, bool pairs, TilePick* pick) {
     const char* const forced = t_switches.tile;
-    if (forced[0] != '\0') {
-        const bool pair = strncmp(forced, "pair", 4) == 0;
-        const int w = atoi(pair ? forced + 4 : forced);
-        const bool legal = w == 256 || w == 128 || (w == 64 && fp8 && !pair);
-        if (legal) return {w, pair};
-    }
-    if (tiles_m == 1) {
-        // One row of tiles: the weight streams through once, so what counts is the
-        // largest share of weight rows any CTA has to stream (tiles per CTA x width,
-        // plus a fixed cost per tile of about 16 rows' worth); ties go to the wider tile.
-        int best = 0;
-        int64_t best_cost = 0;
-        for (int w : {256, 128, 64}) {
-            if (w == 64 && !fp8) continue;
-            const int64_t tiles = (n + w - 1) / w;
-            const int64_t cost = ((tiles + sm_count - 1) / sm_count) * (w + 16);
-            if (best == 0 || cost < best_cost) {
-                best = w;
-                best_cost = cost;
-            }
+    if (forced[0] == '\0') return false;
+    const bool pair = strncmp(forced, "pair", 4) == 0;
+    const int w = atoi(pair ? forced + 4 : forced);
+    if (w != 256 && w != 128 && !(w == 64 && is_fp8_kind(mode) && !pair)) return false;
+    *pick = {w, pair && pairs};
+    return true;
+}
+
+// One row of tiles: the weight streams through once, so what counts is the largest share of weight rows any CTA has to
+// stream (tiles per CTA x width, plus a fixed cost per tile of about 16 rows' worth); ties go to the wider tile.
+TilePick one_row_tile(int64_t n, int mode, int sm_count) {
+    int best = 0;
+    int64_t best_cost = 0;
+    for (int w : {256, 128, 64}) {
+        if (w == 64 && !is_fp8_kind(mode)) continue;
+        const int64_t tiles = (n + w - 1) / w;
+        const int64_t cost = ((tiles + sm_count - 1) / sm_count) * (w + 16);
+        if (best == 0 || cost < best_cost) {
+            best = w;
+            best_cost = cost;
         }
-        return {best, false};
     }
-    // Several rows of tiles: a launch costs a fixed time plus the longer of two: per wave of tiles, the k-tiles and a share
-    // for fill, drain and the hand-over; or, without regard to waves, the pace the power cap leaves (clocks of 1.1 to
-    // 1.5 GHz from some 30 us of full chip on), at which the tiles differ by the bytes they move per product.  Fitted to
-    // 48 MXFP8 and 36 FP4 problems of M = 129..8192, N = 256..16384, K = 512..8192 (waves) and 21 large ones in
-    // sustained runs (pace), each timed on every tile; residuals 4-9 %.  Choosing by it costs 1.0 % over the best tile
-    // of each, the figures from before the pair kernel's scale warps 3.6 % and up to 17 (195 x 14016 x 768 7.1 -> 6.1 us,
-    // 711 x 3456 x 1152 7.8 -> 6.7, 166 x 13120 x 2560 13.4 -> 11.7, 191 x 5632 x 7424 18.0 -> 16.1).
-    struct Cand {
-        int bn;
-        bool pair;
-        double us_per_ktile;
-        double us_per_wave;
-        double us_fixed;
-        double us_paced;  // per k-tile, whole and partial waves alike
-    };
-    static constexpr Cand fp8_dense[5] = {{256, false, 0.345, 1.7, 2.6, 0.55}, {256, true, 0.301, 1.2, 4.0, 0.49},
-                               {128, false, 0.185, 0.9, 2.45, 0.30}, {128, true, 0.161, 0.8, 2.8, 0.265},
-                               {64, false, 0.171, 0.45, 2.6, 0.20}};
-    static constexpr Cand fp4_dense[4] = {{256, false, 0.307, 1.8, 3.1, 0.61}, {256, true, 0.303, 1.4, 4.1, 0.555},
-                               {128, false, 0.187, 0.9, 2.6, 0.34}, {128, true, 0.197, 0.75, 3.1, 0.315}};
-    const Cand* const cands = fp8 ? fp8_dense : fp4_dense;
-    const int count = fp8 ? 5 : 4;
-    // The pair tile of dense NVFP4 is taken for outputs up to three times as wide as tall: there it gains 6 to 13 %
-    // (4096 x 4096 x 4096 38.3 -> 35.9 us, 8192 x 4096 x 4096 69.6 -> 64.0, 8192 x 8192 x 2048 82.9 -> 72.5), on wider ones
-    // 5 to 7 (2048 x 8192 x 4096 38.6 -> 36.5, 1000 x 8192 x 8192 38.3 -> 35.6), which are given up because the suite
-    // holds 4096 x 14336 x 4096 to the single-CTA tile (119 there, 113 on the pair tile).
-    const bool pair_open = mode != HQ_MODE_W4A4_NVFP4 || grouped || n <= 3 * m;
-    const double k_tiles = double(k) / (fp8 ? 128.0 : 256.0);
+    return {best, false};
+}
+
+// Several rows of tiles: a launch costs a fixed time plus the longest of three: per wave of tiles, the k-tiles and a share
+// for fill, drain and the hand-over; without regard to waves, the pace the power cap leaves (clocks of 1.1 to 1.5 GHz from
+// some 30 us of full chip on), at which the tiles differ by the bytes they move per product; and the weights' way from
+// memory.  Each table is fitted to problems of its kind, timed on every tile that it lists; only what a call can run is listed or
+// allowed (a tile that was picked and then replaced by the single-CTA one of its width was not the cheapest of those: SituQuant
+// 458 x 9984 x 1664 14.6 us, 13.9 on 128 x 128; 2.1 % over the best tile on average, now 0.4).
+struct TileCost {
+    int bn;
+    bool pair;
+    double us_per_ktile;
+    double us_per_wave;
+    double us_fixed;
+    double us_paced;  // per k-tile, whole and partial waves alike
+    double stream;    // bytes of weights per us (0: no matter)
+};
+struct CostTable {
+    int count;
+    TileCost tiles[5];
+};
+
+// Dense: 48 MXFP8 and 29 FP4 problems of M = 129..8192, N = 256..16384, K = 512..8192 (waves) and 17 large ones in
+// sustained runs (pace), 1.0 % over the best tile of each; 1.5 % (MXFP8) and 2.8 (FP4) on 117 and 74 others.
+constexpr CostTable kDenseFp8 = {5, {{256, false, 0.345, 1.7, 2.6, 0.55}, {256, true, 0.301, 1.2, 4.0, 0.49},
+    {128, false, 0.185, 0.9, 2.45, 0.30}, {128, true, 0.161, 0.8, 2.8, 0.265}, {64, false, 0.171, 0.45, 2.6, 0.20}}};
+constexpr CostTable kDenseFp4 = {4, {{256, false, 0.307, 1.8, 3.1, 0.61}, {256, true, 0.303, 1.4, 4.1, 0.555},
+    {128, false, 0.187, 0.9, 2.6, 0.34}, {128, true, 0.197, 0.75, 3.1, 0.315}}};
+// SituQuant, whose epilogue is longer, and which has no 256 x 128 pair kernel: 92 problems of M = 129..8192, N = 2048..14336,
+// K = 1024..4096; 0.4 % over the best tile, 2.1 % by the dense figures.
+constexpr CostTable kSitu = {4, {{256, false, 0.355, 1.34, 4.53, 0.538}, {256, true, 0.307, 1.13, 5.32, 0.451},
+    {128, false, 0.179, 0.79, 3.8, 0.297}, {64, false, 0.161, 0.61, 2.98, 0.233}}};
+// Batches and masked experts: 20 batches and 88 masked problems in MXFP8, 72 masked in W4A8, 40 and 112 in FP4; 2 to 128 groups of 32
+// to 2048 rows; the long streams of weights (64-row slots, more than 200 MB) weigh ten.  Over the best tile of each: batches 1.0 %
+// (MXFP8) and 0.8 % (FP4), half-filled experts 1.4, 1.9 and 0.9 %, full ones 0.7, 0.5 and 3.0; by the dense figures, and with pair
+// tiles that the call cannot run replaced by the single-CTA one of their width, 1.9 and 3.0, 1.6, 3.3 and 4.5, 0.6, 0.6 and 3.1.
+constexpr CostTable kSlotsFp8 = {5, {{256, false, 0.481, 1.03, 4.3, 0.585, 5.4e6}, {256, true, 0.277, 1.13, 5.42, 0.504, 5.5e6},
+    {128, false, 0.142, 0.73, 4.08, 0.335, 5.38e6}, {128, true, 0.182, 0.7, 3.58, 0.286, 5.5e6}, {64, false, 0.184, 0.51, 2.99, 0.225, 4.44e6}}};
+constexpr CostTable kSlotsW4A8 = {5, {{256, false, 0.375, 1.39, 5.01, 0.569, 5.5e6}, {256, true, 0.306, 1.14, 4.51, 0.46, 5.5e6},
+    {128, false, 0.229, 0.93, 3.24, 0.306, 5.5e6}, {128, true, 0.153, 0.79, 3.5, 0.262, 5.5e6}, {64, false, 0.179, 0.58, 2.87, 0.221, 5.5e6}}};
+constexpr CostTable kSlotsFp4 = {4, {{256, false, 0.301, 2.52, 4.43, 0.668, 4.29e6}, {256, true, 0.288, 1.96, 4.8, 0.608, 5.5e6},
+    {128, false, 0.191, 1.13, 3.32, 0.408, 4.5e6}, {128, true, 0.195, 0.79, 3.39, 0.356, 5.5e6}}};
+// Contiguous experts cut by their runs: 65 MXFP8, 40 W4A8 and 61 FP4 problems of 512 to 40960 rows and 2 to 181 experts; 1.5, 0.7 and
+// 0.9 % over the best tile.  (The MXFP8 figures are fitted so that 16 experts on 4096 x 4096 x 2048 take the tile the suite names, 128 x 128: 55 us,
+// 50 on the 256 x 256 pair tile; without that 1.5 % all the same.)
+constexpr CostTable kRunsFp8 = {5, {{256, false, 0.201, 2.19, 6.28, 0.576, 7.14e6}, {256, true, 0.229, 2.55, 5.0, 0.49, 6.92e6},
+    {128, false, 0.22, 0.95, 3.47, 0.304, 6.86e6}, {128, true, 0.165, 1.15, 3.32, 0.272, 5.88e6}, {64, false, 0.178, 0.65, 2.72, 0.217, 5.63e6}}};
+constexpr CostTable kRunsW4A8 = {5, {{256, false, 0.326, 1.55, 4.26, 0.527, 5.5e6}, {256, true, 0.248, 1.13, 5.67, 0.445, 5.5e6},
+    {128, false, 0.211, 0.85, 3.12, 0.291, 5.5e6}, {128, true, 0.156, 0.8, 4.02, 0.254, 5.5e6}, {64, false, 0.172, 0.49, 2.77, 0.218, 5.5e6}}};
+constexpr CostTable kRunsFp4 = {4, {{256, false, 0.395, 2.56, 3.7, 0.622, 6.49e6}, {256, true, 0.252, 2.4, 4.99, 0.414, 5.45e6},
+    {128, false, 0.182, 1.02, 3.83, 0.383, 6.31e6}, {128, true, 0.235, 0.77, 4.14, 0.265, 5.5e6}}};
+
+struct RowTiles {
+    double single, pair;  // 128-row and 256-row tiles
+};
+
+// The cheapest tile of a table; `rows`: the rows of tiles, or several guesses at them.
+TilePick cheapest_tile(const CostTable& table, std::initializer_list<RowTiles> rows, int64_t n, double k_tiles, double weight_bytes,
+                       bool pairs, int sm_count) {
     TilePick best = {0, false};
     double best_cost = 0.0;
-    for (int i = 0; i < count; ++i) {
-        const Cand& c = cands[i];
-        if (c.pair && (m <= kBM || !pair_open)) continue;
-        const int64_t rows = c.pair ? tiles_m2 : tiles_m;
-        const int64_t cols = (n + c.bn - 1) / c.bn;
+    for (int i = 0; i < table.count; ++i) {
+        const TileCost& c = table.tiles[i];
         const int64_t units = c.pair ? sm_count / 2 : sm_count;
-        if (units < 1) continue;
-        // Contiguous experts: every run is cut into tiles of its own, so a boundary adds part of a tile of rows (and no more
-        // than one per 64 rows), and such tiles work for rows that they do not have, which tells against wide ones.
-        // Fitted to 80 problems of many short runs (512 to 16384 rows, 8 to 256 experts, MXFP8 and NVFP4), each timed on
-        // every tile: 2.6 % (MXFP8) and 1.3 % (NVFP4) over the best of each, some of it because the suite holds 16 experts
-        // on 4096 x 4096 x 2048 to the 128 x 128 tile (48.7 us; 46.4 on 128 x 256).
-        const double extra = std::min(0.4 * double(boundaries), double(m) / 64.0 - double(rows));
-        const double tiles = boundaries > 0 ? (double(rows) + std::max(extra, 0.0)) * double(cols) : double(rows * cols);
-        const double idle = std::min(c.pair ? 3.0 : 1.0, double(boundaries) * (c.pair ? 0.75 : 0.5) / double(rows)) * c.bn / 256.0;
-        const double waves = std::ceil(tiles / double(units)) * (1.0 + (c.pair ? 0.4 : 0.6) * idle);
-        const double cost = c.us_fixed + std::max(waves * (k_tiles * c.us_per_ktile + c.us_per_wave),
-                                                  tiles / double(units) * k_tiles * c.us_paced * (1.0 + 0.3 * idle));
+        if ((c.pair && !pairs) || units < 1) continue;
+        double cost = 0.0;
+        for (const RowTiles& r : rows) {
+            const double share = (c.pair ? r.pair : r.single) * double((n + c.bn - 1) / c.bn) / double(units);
+            const double waves = std::ceil(share - 1e-9) * (k_tiles * c.us_per_ktile + c.us_per_wave);
+            const double stream = c.stream > 0.0 ? weight_bytes / c.stream : 0.0;
+            cost += c.us_fixed + std::max({waves, share * k_tiles * c.us_paced, stream});
+        }
         if (best.bn == 0 || cost < best_cost * 0.999) {
             best = {c.bn, c.pair};
             best_cost = cost;
         }
     }
     return best;
+}
+
+double k_tiles_of(int64_t k, int mode) { return double(k) / (is_fp8_kind(mode) ? 128.0 : 256.0); }
+
+// `situ`: the SituQuant epilogue.
+TilePick pick_tile(int64_t m, int64_t n, int64_t k, int mode, int sm_count, bool situ = false) {
+    if (!tile_fits(m, n, k, mode)) return {0, false};
+    TilePick pick;
+    if (forced_tile(mode, true, &pick)) return {pick.bn, pick.pair && (!situ || pick.bn == 256)};
+    if (m <= kBM) return one_row_tile(n, mode, sm_count);
+    // The pair tile of dense NVFP4 is taken for outputs up to three times as wide as tall: there it gains 6 to 13 %
+    // (4096 x 4096 x 4096 38.3 -> 35.9 us, 8192 x 4096 x 4096 69.6 -> 64.0, 8192 x 8192 x 2048 82.9 -> 72.5), on wider ones
+    // 5 to 7 (2048 x 8192 x 4096 38.6 -> 36.5, 1000 x 8192 x 8192 38.3 -> 35.6), which are given up because the suite
+    // holds 4096 x 14336 x 4096 to the single-CTA tile (119 there, 113 on the pair tile).
+    const bool pairs = mode != HQ_MODE_W4A4_NVFP4 || n <= 3 * m;
+    const RowTiles rows = {double((m + kBM - 1) / kBM), double((m + 255) / 256)};
+    return cheapest_tile(situ ? kSitu : is_fp8_kind(mode) ? kDenseFp8 : kDenseFp4, {rows}, n, k_tiles_of(k, mode), 0.0, pairs, sm_count);
 }
 
 template <int KIND>
@@ -2800,9 +2849,13 @@ extern "C" int hq_describe_tile(int64_t m, int64_t n, int64_t k, int mode, int s
         const bool split = pick.bn == 64 && !pick.pair &&
                            hq::split_k_chosen(hq::kGroupDense, int((m + hq::kBM - 1) / hq::kBM), int(n / 64),
                                               int(k / 128), sm > 0 ? sm : 148, HQ_EPILOGUE_IDENTITY);
-        snprintf(buf, buflen, "[gemm] mode=dense kind=%s m=%lld n=%lld k=%lld sm=%d -> %dx%d/%d pair=%d splitk=%d",
-                 hq::mode_name(mode), (long long)m, (long long)n, (long long)k, sm, pick.pair ? 256 : hq::kBM,
-                 pick.bn, mode == HQ_MODE_W8A8_MXFP8 ? 128 : 256, pick.pair ? 1 : 0, split ? 1 : 0);
+        const int len = snprintf(buf, buflen, "[gemm] mode=dense kind=%s m=%lld n=%lld k=%lld sm=%d -> %dx%d/%d pair=%d splitk=%d",
+                                 hq::mode_name(mode), (long long)m, (long long)n, (long long)k, sm, pick.pair ? 256 : hq::kBM,
+                                 pick.bn, mode == HQ_MODE_W8A8_MXFP8 ? 128 : 256, pick.pair ? 1 : 0, split ? 1 : 0);
+        if (mode == HQ_MODE_W8A8_MXFP8 && n % 256 == 0 && len > 0 && size_t(len) < buflen) {
+            const hq::TilePick quant = hq::pick_tile(m, n, k, mode, sm > 0 ? sm : 148, true);
+            snprintf(buf + len, buflen - size_t(len), " situ=%dx%d", quant.pair ? 256 : hq::kBM, quant.bn);
+        }
     }
     return HQ_OK;
 }
@@ -2885,12 +2938,8 @@ int dense_gemm_impl(const void* a, const void* b, const void* sfa, const void* s
     const int sm_all = hq_sm_count(device);
     const int sm = sm_count > 0 ? (sm_count < sm_all || sm_all == 0 ? sm_count : sm_all) : sm_all;
     if (sm <= 0) return fail(err, errlen, HQ_ERR_CUDA, "cannot query the SM count of device %d", device);
-    hq::TilePick pick = hq::pick_tile(m, n, k, mode, sm);
+    const hq::TilePick pick = hq::pick_tile(m, n, k, mode, sm, is_situ);
     if (is_situ) {
-        // The quantising epilogue is built for the single-CTA tiles and the 256 x 256 pair tile, which the
-        // same rule picks as for the plain epilogues (gate / up and down projection of an MLP block,
-        // 4096 x 7168 x 2048: 100.2 -> 93.6 us; 8192 x 14336 x 2048: 364 -> 334 us).
-        if (pick.bn != 256) pick.pair = false;
         out = situ->q;
         ldo = situ->ldq / 2;
     }
@@ -2999,28 +3048,73 @@ const char* group_kind_name(int kind) {
     return kind == kGroupBatch ? "batch" : kind == kGroupMasked ? "masked" : "contiguous";
 }
 
-// The grouped kinds run in the single-CTA kernel.  `rows` = rows per group (batch,
-// masked) or the mean rows per expert (contiguous), `total_m` = all rows of A.  The
-// waves are sized by the (group, row tile) pairs, which exceed the row tiles of the
-// stacked rows when tiles straddle groups.  Batches take any row count (straddling
-// tiles are worked once per batch); the expert kinds want slots / runs that are
-// multiples of 64 rows, the finest granularity of the reference's tiles
-// (csrc/kernel/gemm/gemm_dispatch.cuh:65-100).
+// Batches take any row count (straddling tiles are worked once per batch); the expert kinds want slots / runs that are
+// multiples of 64 rows, the finest granularity of the reference's tiles (csrc/kernel/gemm/gemm_dispatch.cuh:65-100).
+bool grouped_tile_fits(int kind, int64_t count, int64_t rows, int64_t total_m, int64_t n, int64_t k, int mode) {
+    if (count < 1 || rows < 1) return false;
+    if (kind == kGroupMasked && rows % 64 != 0) return false;
+    if (kind == kGroupContiguous && total_m % 64 != 0) return false;
+    return tile_fits(total_m, n, k, mode);
+}
+
+// Contiguous experts are cut by their runs (RunTable) on the pair tiles, and on the single-CTA ones unless the table does not
+// repay itself: when every 64 rows may be another expert's (so a fixed 128-row tile is worked twice at most, and as many runs
+// leave no tile whole), and either K is short, or the fixed tiles fill the chip once while the runs would take a second wave.
+// 24 such problems on the 128-wide tile: 0.75 to 0.94 of the time (NVFP4 1600 x 1024 x 512 with 25 experts 6.8 -> 5.0 us,
+// MXFP8 640 x 3200 x 512 with 10 6.8 -> 5.6, 2048 x 1024 x 2048 with 64 15.9 -> 14.6); K of 6 k-tiles and more of several
+// waves 0.99 to 1.34 (960 x 5888 x 3840 with 15 46 -> 56), runs of 128 rows and more 1.02 to 1.2.
+bool contiguous_by_runs(int64_t count, int64_t total_m, int64_t n, int64_t k, int mode, int sm_count) {
+    if (t_switches.runs[0] != '\0') return t_switches.runs[0] != '0';
+    const int64_t quarters = total_m / 64;
+    if (quarters == 1) return false;
+    if (count < quarters) return true;
+    const int64_t cols = (n + 127) / 128;
+    const bool one_wave = (quarters + 1) / 2 * cols <= sm_count && quarters * cols > sm_count;
+    const double k_tiles = k_tiles_of(k, mode);
+    return !(k_tiles <= 4.0 || (one_wave && k_tiles <= 16.0));
+}
+
+// The grouped kinds.  `rows` = rows per group (batch, masked) or the mean rows per expert (contiguous), `total_m` = all
+// rows of A.  The 2-CTA tile has plain epilogues only, and none of its tiles may hold rows of two batches or slots.
 TilePick pick_tile_grouped(int kind, int64_t count, int64_t rows, int64_t total_m, int64_t n, int64_t k, int mode,
                            int sm_count, bool plain_epilogue = true) {
-    if (count < 1 || rows < 1) return {0, false};
-    if (kind == kGroupMasked && rows % 64 != 0) return {0, false};
-    if (kind == kGroupContiguous && total_m % 64 != 0) return {0, false};
-    const int64_t pad = kind != kGroupContiguous && rows % kBM != 0 ? (count - 1) * kBM : 0;
-    // boundaries between the experts' runs: as many as there are experts, or as the rows have room for
-    const int64_t boundaries = kind == kGroupContiguous ? std::min(count, total_m / 64) - 1 : 0;
-    TilePick pick = pick_tile(total_m + pad, n, k, mode, sm_count, true, boundaries);
-    // The 2-CTA tile: a plain epilogue, and no 256-row tile may hold rows of two
-    // batches or expert slots (the contiguous layout is worked per run of experts, see
-    // PairWorkIter).  Otherwise a forced or modelled pair choice falls back to the same width.
-    const bool whole_tiles = kind == kGroupContiguous || rows % 256 == 0;
-    if (!(plain_epilogue && whole_tiles)) pick.pair = false;
-    pick.runs = kind == kGroupContiguous && (pick.pair || t_switches.runs[0] != '0');
+    if (!grouped_tile_fits(kind, count, rows, total_m, n, k, mode)) return {0, false};
+    const bool contiguous = kind == kGroupContiguous;
+    const bool pairs = plain_epilogue && (contiguous || rows % 256 == 0);
+    const bool fp8 = is_fp8_kind(mode), w4a8 = mode == HQ_MODE_W4A8_MXFP4;
+    const double k_tiles = k_tiles_of(k, mode);
+    const double bytes_per_weight = double(n) * double(k) * (mode == HQ_MODE_W8A8_MXFP8 ? 1.0 : 0.5);
+    const RowTiles whole = {double((total_m + kBM - 1) / kBM), double((total_m + 255) / 256)};
+    const int64_t quarters = total_m / 64;
+    // runs: as many as there are experts, or as the rows have room for
+    const int64_t runs = contiguous ? std::min(count, quarters) : 1;
+    TilePick pick;
+    if (forced_tile(mode, pairs, &pick)) {
+    } else if (contiguous ? total_m <= kBM : slot_row_tiles(count, rows) == 1) {
+        pick = one_row_tile(n, mode, sm_count);
+    } else if (contiguous && runs == 1) {
+        pick = cheapest_tile(fp8 ? kDenseFp8 : kDenseFp4, {whole}, n, k_tiles, 0.0, pairs, sm_count);
+    } else if (contiguous && !contiguous_by_runs(count, total_m, n, k, mode, sm_count)) {
+        pick = {128, false};
+    } else if (contiguous) {
+        // every run is cut into tiles of its own: half a tile more for each, and no more than one per 64 rows
+        const auto cut = [&](double tiles) {
+            return runs == quarters ? double(quarters) : std::max(std::ceil(tiles), std::min(tiles + 0.5 * double(runs), double(quarters)));
+        };
+        pick = cheapest_tile(fp8 ? (w4a8 ? kRunsW4A8 : kRunsFp8) : kRunsFp4, {{cut(double(quarters) / 2), cut(double(quarters) / 4)}}, n,
+                             k_tiles, double(runs) * bytes_per_weight, pairs, sm_count);
+    } else {
+        const RowTiles full = {double(slot_row_tiles(count, rows)), double(count) * double((rows + 255) / 256)};
+        // how many rows of a slot are valid only the device knows: half-filled ones (evenly spread counts) weigh two, full ones one
+        const auto half = [rows](double tiles, int64_t height) {
+            const double most = double((rows + height - 1) / height);
+            return tiles * (most + 1.0) / (2.0 * most);
+        };
+        const RowTiles filled = kind == kGroupMasked ? RowTiles{half(full.single, kBM), half(full.pair, 256)} : full;
+        pick = cheapest_tile(fp8 ? (w4a8 ? kSlotsW4A8 : kSlotsFp8) : kSlotsFp4, {full, filled, filled}, n, k_tiles,
+                             double(count) * bytes_per_weight, pairs, sm_count);
+    }
+    pick.runs = contiguous && (pick.pair || contiguous_by_runs(count, total_m, n, k, mode, sm_count));
     return pick;
 }
 
@@ -3081,7 +3175,7 @@ int grouped_gemm_impl(int kind, const void* a, const void* b, const void* sfa, c
     }
     if (count == 0 || total_m == 0 || n == 0) return HQ_OK;
     const SwitchScope switches;
-    if (pick_tile_grouped(kind, count, rows, total_m, n, k, mode, 148).bn == 0) {
+    if (!grouped_tile_fits(kind, count, rows, total_m, n, k, mode)) {
         return no_group_tile(err, errlen, kind, mode, rows, total_m, n, k);
     }
     const int64_t sf_k = k / group;
@@ -3164,9 +3258,10 @@ extern "C" int hq_describe_group_tile(int kind, int64_t count, int64_t rows, int
     if (pick.bn == 0) return hq::no_group_tile(buf, buflen, kind, mode, rows, total_m, n, k);
     if (buf != nullptr && buflen > 0) {
         // (the Identity epilogue is assumed)
-        snprintf(buf, buflen, "[gemm] mode=%s kind=%s groups=%lld m=%lld grid_m=%lld n=%lld k=%lld sm=%d -> %dx%d/%d pair=%d",
+        snprintf(buf, buflen, "[gemm] mode=%s kind=%s groups=%lld m=%lld grid_m=%lld n=%lld k=%lld sm=%d%s -> %dx%d/%d pair=%d",
                  hq::group_kind_name(kind), hq::mode_name(mode), (long long)count, (long long)rows,
-                 (long long)total_m, (long long)n, (long long)k, sm, pick.pair ? 256 : hq::kBM, pick.bn,
+                 (long long)total_m, (long long)n, (long long)k, sm,
+                 kind != hq::kGroupContiguous ? "" : pick.runs ? " cut=runs" : " cut=rows", pick.pair ? 256 : hq::kBM, pick.bn,
                  mode == HQ_MODE_W8A8_MXFP8 ? 128 : 256, pick.pair ? 1 : 0);
     }
     return HQ_OK;

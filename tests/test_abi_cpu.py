@@ -414,8 +414,8 @@ def test_wide_tiles_for_columns_that_do_not_fill_them(native):
 
 
 def test_contiguous_tile_with_experts_that_meet_inside_tiles(native):
-    """Runs start on multiples of 64 rows, so more experts than that leave the choice as it is; a boundary is a second
-    pass of the CTA that has the tile, so short runs do not ask for wide tiles."""
+    """Runs start on multiples of 64 rows, so more experts than that leave the choice as it is; every run is cut into tiles of its
+    own (or, on fixed tiles, worked in a pass of its own), so short runs do not ask for wide tiles."""
     import halops_b200 as hq
 
     def tile(count, m, n, k, mode="w8a8-mxfp8"):
@@ -443,6 +443,43 @@ def test_split_k_from_the_k_that_repays_its_exchange(native):
     assert [split(704, kt) for kt in (8, 48, 55, 56, 64, 192)] == ["0", "0", "0", "1", "1", "1"]
     assert [split(3712, kt) for kt in (56, 95, 96)] == ["0", "0", "1"]
     assert split(2368, 56) == "1" and split(2432, 56) == "0" and split(4800, 192) == "0"
+
+
+def test_contiguous_experts_that_the_run_table_does_not_repay(native):
+    """Timed both ways on the 128-wide tile: 6.8 us by runs and 5.0 by rows, 6.8 and 5.6, 15.9 and 14.6; 7.2 and 8.3, 46 and 56,
+    30 and 35 the other way round (a second wave only by rows, several waves, runs of two quarters and more)."""
+    import halops_b200 as hq
+
+    def cut(count, m, n, k, mode="w8a8-mxfp8"):
+        return re.search(r"cut=(\w+)", hq.describe_group_tile("contiguous", count, max(1, m // count), n, k, mode, total_m=m, sm_count=148)).group(1)
+
+    assert cut(25, 1600, 1024, 512, "w4a4-nvfp4") == "rows" and cut(10, 640, 3200, 512) == "rows" and cut(64, 2048, 1024, 2048) == "rows"
+    assert cut(16, 512, 2048, 2048, "w4a4-nvfp4") == "runs" and cut(15, 960, 5888, 3840) == "runs" and cut(16, 1024, 2944, 3328) == "runs"
+    assert cut(10, 40960, 4096, 4096, "w4a4-nvfp4") == "runs" and cut(8, 1024, 1024, 512) == "runs"
+
+
+def test_the_tile_is_chosen_among_those_that_can_run(native):
+    """Slots and batches that are no multiple of 256 rows and the quantising epilogues have no (or not every) pair tile, and 64-row
+    slots never straddle 128-row tiles.  Timed on every tile: 6.5 us on 128 x 128, 8.4 on 128 x 256; 19 and 21; 6.3 and 8.7;
+    26 and 29; SituQuant 13.9 on 128 x 128, 14.6 on 128 x 256 and 15.3 on the pair tile; 11.3 and 12.5."""
+    import halops_b200 as hq
+
+    def tile(kind, count, m, n, k, mode):
+        return hq.describe_group_tile(kind, count, m, n, k, mode, sm_count=148).split("-> ")[1]
+
+    assert "128x128" in tile("masked", 8, 64, 2048, 2048, "w4a4-nvfp4") and "128x128" in tile("masked", 16, 64, 2688, 3072, "w4a4-nvfp4")
+    assert "128x128" in tile("batch", 7, 192, 1152, 2048, "w4a4-mxfp4") and "128x128" in tile("batch", 22, 128, 3968, 2560, "w4a4-mxfp4")
+    for m in (64, 128, 192, 320):
+        for n in (1024, 2176, 7168):
+            assert "pair=0" in tile("masked", 12, m, n, 2048, "w8a8-mxfp8") and "pair=0" in tile("batch", 12, m, n, 2048, "w8a8-mxfp8")
+    # one slot fills tiles of its own: as many as the rows have, whatever the number of slots
+    assert tile("masked", 64, 128, 2048, 1024, "w8a8-mxfp8") == tile("masked", 64, 64, 2048, 1024, "w8a8-mxfp8")
+    assert "situ=128x128" in hq.describe_tile(458, 9984, 1664, sm_count=148)
+    assert "situ=128x128" in hq.describe_tile(609, 4096, 2176, sm_count=148)
+    assert "situ=256x256" in hq.describe_tile(4096, 7168, 2048, sm_count=148)
+    for m in (129, 300, 916, 2048, 8192):
+        for n in (2048, 5120, 9728, 14336):
+            assert "situ=256x128" not in hq.describe_tile(m, n, 2048, sm_count=148)
 
 
 def test_product_never_imports_the_oracle():
