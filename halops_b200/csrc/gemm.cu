@@ -970,7 +970,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars->acc_empty[as]));
                     }
-                    if (warp_idle || 2 * g * kEpiChunk >= wk.cols) continue;
+                    if (warp_idle) continue;  // (N is a multiple of 256 here: no ragged tile)
                     uint32_t y[16];
                     const __nv_bfloat16* const bc = bias != nullptr ? bias + n0 + 2 * g * kEpiChunk : nullptr;
                     situ_chunk(r0, bc, situ, &y[0]);
@@ -1290,7 +1290,7 @@ __device__ __forceinline__ uint32_t instr_desc_pair(uint32_t sf_id) {
 // What one persistent-loop iteration of the 2-CTA kernel works on: a 256-row tile of the
 // stacked A rows against BN rows of one weight.
 struct PairWork {
-    int a_row0;     // first of the tile's 256 stacked A rows (a multiple of 256)
+    int a_row0;     // first of the tile's 256 stacked A rows (a multiple of 128: runs of experts start there; of 256 otherwise)
     int b_row0;     // first of the BN weight rows in the stacked weights
     int sfb_tile;   // 128-row scale atom row of that row
     int cols;       // weight rows of the tile that exist (see Work)
@@ -1837,7 +1837,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                             ptx::mbar_arrive_cluster_relaxed(ptx::mapa_cluster(ptx::smem_u32(&bars->acc_empty[as]), 0));
                         }
                     }
-                    if (2 * g * kEpiChunk >= wk.cols) continue;
                     uint32_t y[16];
                     const __nv_bfloat16* const bc = bias != nullptr ? bias + n0 + 2 * g * kEpiChunk : nullptr;
                     situ_chunk(r0, bc, situ.p, &y[0]);
@@ -2218,7 +2217,7 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
     const int64_t row_tiles = g.runs ? std::min<int64_t>(g.m / 64, int64_t(tiles_m) + g.grp.count) : tiles_m;
     const int grid = int(std::min<int64_t>(g.sm_count, row_tiles * tiles_n));
     const int k_tiles = int(g.k_bytes / kBKBytes);
-    if constexpr (BN == 64) {
+    if constexpr (BN == 64 && KIND != 3) {  // (the e4m3 x e2m1 kind is a grouped one)
         // One row of at most sm_count / 2 tiles and a long K: two CTAs per tile, half of K each.
         if (split_k_chosen(g.grp.kind, tiles_m, tiles_n, k_tiles, g.sm_count, g.epi_op)) {
             static SmemOptIn opt_in_split;
@@ -2241,7 +2240,7 @@ int launch_tile(const GemmArgs& g, char* err, size_t errlen) {
     // Everything else: two issuers in k order (same bits as one issuer; the dense and the
     // grouped kinds alike).  HALOPS_B200_ISSUERS=1 keeps one issuer (read on every call).
     if (dual == 0 && k_tiles >= 2) dual = issuers_in_order();
-    if constexpr (KIND != 3) {  // (the e4m3 x e2m1 kind is a grouped one)
+    if constexpr (KIND != 3) {
         if (g.grp.kind == kGroupDense && (g.epi_op == HQ_EPILOGUE_IDENTITY || g.epi_op == HQ_EPILOGUE_SIGMOID)) {
             static SmemOptIn opt_in_dense;
             HQ_CUDA_TRY(opt_in_dense.ensure(gemm_kernel<BN, KIND, false, true>, C::kSmemBytes));

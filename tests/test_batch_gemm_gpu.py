@@ -358,6 +358,26 @@ def test_fp4_batches_on_the_2cta_tile(hq, monkeypatch, mode, tile):
     _compare(outs[1], xq, wq, sfa, sfb, mode, alpha=alpha)
 
 
+@pytest.mark.parametrize("op", ["Quant", "GateMulQuant", "SigmoidGateMulQuant"])
+@pytest.mark.parametrize("b,m,n", [(3, 200, 384), (2, 32, 128), (5, 96, 640)], ids=lambda v: str(v))
+def test_quantising_epilogues_on_a_tile_that_sticks_out(hq, monkeypatch, op, b, m, n):
+    """256-wide tiles on columns that do not fill them: the bytes and scales of the 128-wide tile, and none behind a batch's last column."""
+    args = _inputs(hq, b, m, n, 256, "w8a8-mxfp8", seed=17)
+    gate = None
+    if op != "Quant":
+        gate = (torch.rand([m, b * n], generator=torch.Generator().manual_seed(18)) * 2 - 0.5).to(torch.bfloat16).cuda()
+    results = []
+    for tile in ("128", "256"):
+        monkeypatch.setenv("HALOPS_B200_TILE", tile)
+        results.append(_quant_run(hq, args, m, b * n, hq.EpilogueOp[op], gate))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    if op != "SigmoidGateMulQuant":
+        y = _run(hq, *args, "w8a8-mxfp8")
+        ref_q, ref_sf = _ref_quant_e4m3((y if gate is None else y * gate).cpu())
+        assert torch.equal(results[1][0].cpu(), ref_q)
+        assert torch.equal(results[1][1].cpu()[torch.from_numpy(oracle.sf_atom_offsets(m, b * n // 32))], ref_sf)
+
+
 @pytest.mark.parametrize("mode", ["w8a8-mxfp8", "w4a4-nvfp4"])
 @pytest.mark.parametrize("m", [16, 32, 40, 96])
 def test_batches_of_few_rows(hq, monkeypatch, mode, m):

@@ -608,3 +608,20 @@ def test_columns_that_do_not_fill_the_last_tile(hq, monkeypatch, mode, tile, m, 
     assert torch.equal(results[0], results[1])
     if bias is None:
         _check(results[1], aq, bq, sfa, sfb, mode, alpha=None if alpha is None else 0.7)
+
+
+@pytest.mark.parametrize("mode", ["w4a4-nvfp4", "w4a4-mxfp4"])
+@pytest.mark.parametrize("m,n,k", [(300, 640, 1024), (512, 128, 256), (257, 896, 2304)], ids=lambda v: str(v))
+def test_fp4_columns_that_do_not_fill_the_pair_tile(hq, monkeypatch, mode, m, n, k):
+    aq, bq, sfa, sfb = _quantize(hq, _rand(m, k, 71), _rand(n, k, 72), mode)
+    alpha = torch.full([1], 0.7, device="cuda") if mode == "w4a4-nvfp4" else None
+    results = []
+    for t in ("128", "pair256"):
+        monkeypatch.setenv("HALOPS_B200_TILE", t)
+        assert ("256x256" if "pair" in t else "128x128") in hq.describe_tile(m, n, k, mode)
+        wide = torch.full([m, n + 64], 7.0, dtype=torch.bfloat16, device="cuda")
+        hq.dense_gemm(aq, bq, sfa, sfb, wide[:, :n], None, alpha, mode=mode)
+        assert hq.device_status() == 0 and torch.all(wide[:, n:] == 7.0)
+        results.append(wide[:, :n].contiguous())
+    assert torch.equal(*results)
+    _check(results[1], aq, bq, sfa, sfb, mode, alpha=None if alpha is None else 0.7)
