@@ -329,7 +329,7 @@ def bench_c2(hq, dev, steps, peaks):
                   "frac_of_hbm": qbytes / (quant_alone * 1e-3) / 1e9 / peaks["hbm_gbs"], "bytes_per_element": 3.03125},
         "roofline": {"kernel": "gemm_pair_kernel<256, mxfp8>" if pair else "gemm_kernel<256, mxfp8>",
                      "bound": "tensor", "achieved": gemm_tflops, "peak": fp8_peak, "unit": "TFLOP/s",
-                     "frac": gemm_tflops / fp8_peak, "traffic": 487.5e6 if pair else 605.2e6,
+                     "frac": gemm_tflops / fp8_peak, "traffic": 478.3e6 if pair else 605.2e6,
                      "traffic_source": "ncu capture of one launch of this kernel on this shape",
                      "algorithmic_bytes": 64 * 2**20 * 2 + 4 * 2**20 + 128 * 2**20,
                      "peak_source": f"2 x {peaks['source']} cuBLAS bf16 (burst) as the dense fp8 peak"},

@@ -164,7 +164,7 @@ __device__ __noinline__ bool wait_bar_lane(uint32_t bar, uint32_t parity, volati
 // .sync.aligned instructions, __syncwarp and elections that count on all 32 lanes.
 // The first try and its vote are straight-line code (a completed barrier: 58 cycles); with the polling loop inline, lane by
 // lane, a wait on a completed barrier took a role 125: 512 x 1536 x 4096 8.8 -> 8.5 us, 1024 x 1536 x 8192 26.0 -> 24.9 (both on
-// the 128 x 64 tile), NVFP4 512 x 4096 x 8192 12.9 -> 12.7, 64 x 24576 x 1536 10.2 -> 10.0, GEMM alone.
+// the 128 x 64 tile), NVFP4 512 x 4096 x 8192 12.9 -> 12.7, GEMM alone.
 template <bool kInPlace = false>
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t code) {
     if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar, parity) ? 1 : 0) != 0) return true;
@@ -1231,8 +1231,8 @@ __global__ void __launch_bounds__(96, 1) wait_selftest_kernel(uint64_t limit_ns)
 // tcgen05.cp from one warp (75 to 90 cycles a copy, a commit behind them) and a release that the leader's loader
 // passed on: MXFP8 8192 x 8192 x 8192 462 -> 448 us, 4096 x 7168 x 2048 58.4 -> 56.5, 512 x 4096 x 4096 16.4 -> 15.0,
 // 4096 x 4096 x 4096 on the 256 x 128 tile 80 -> 64 (sustained, GEMM alone; the waits' part of the last is 10).  NVFP4, with
-// 12 copies a k-tile: 8192 x 8192 x 8192 295 -> 230, which made it the better tile for the FP4 kinds too
-// (single-CTA 128 x 256: 251); 4096 x 4096 x 4096 44 -> 35.5 (41).
+// 12 copies a k-tile: 8192 x 8192 x 8192 295 -> 233, which made it the better tile for the FP4 kinds too
+// (single-CTA 128 x 256: 248); 4096 x 4096 x 4096 44 -> 35.5 (41).
 
 template <int BN, int KIND>
 struct Cfg2 {
